@@ -37,26 +37,24 @@ __device__ __forceinline__ int cell_of(float y, float x, float G, int ncy, int n
     return cy * ncx + cx;
 }
 
-// Counting sort of n points into cells: start[ncell+1], idx[n].
-__device__ void build_grid(const float* ys, const float* xs, const int* sel, int n, float G,
-                           int ncy, int ncx, int* cnt_s, int* start, int* idx, int* warp_tot,
-                           int* s_total) {
+// Counting sort of n points into cells: start[ncell+1], idx[n] and, when
+// asked for, their positions in that order.
+__device__ void build_grid(const float* ys, const float* xs, int n, float G, int ncy, int ncx, int* cnt_s, int* start,
+                           int* idx, float2* pos, int* warp_tot, int* s_total) {
     const int ncell = ncy * ncx;
     for (int c = threadIdx.x; c < ncell; c += NTF) cnt_s[c] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += NTF) {
-        const int j = sel ? sel[i] : i;
-        atomicAdd(&cnt_s[cell_of(ys[j], xs[j], G, ncy, ncx)], 1);
-    }
+    for (int i = threadIdx.x; i < n; i += NTF) atomicAdd(&cnt_s[cell_of(ys[i], xs[i], G, ncy, ncx)], 1);
     __syncthreads();
     block_scan_inplace(cnt_s, ncell, warp_tot, s_total);
     for (int c = threadIdx.x; c < ncell; c += NTF) start[c] = cnt_s[c];
     if (threadIdx.x == 0) start[ncell] = n;
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += NTF) {
-        const int j = sel ? sel[i] : i;
-        const int k = atomicAdd(&cnt_s[cell_of(ys[j], xs[j], G, ncy, ncx)], 1);
+        const float y = ys[i], x = xs[i];
+        const int k = atomicAdd(&cnt_s[cell_of(y, x, G, ncy, ncx)], 1);
         idx[k] = i;
+        if (pos) pos[k] = make_float2(y, x);
     }
     __syncthreads();
 }
@@ -135,7 +133,7 @@ __global__ void __launch_bounds__(NTF) finalize_kernel(const LocParams p, MovieB
     const int ncell = b.ncx * b.ncy;
     int* cstart = b.cstart + (size_t)t * (ncell + 1);
     int* cidx = b.cidx + (size_t)t * cap_c;
-    build_grid(cy, cx, nullptr, ne, G, b.ncy, b.ncx, cnt_s, cstart, cidx, warp_tot, &s_total);
+    build_grid(cy, cx, ne, G, b.ncy, b.ncx, cnt_s, cstart, cidx, nullptr, warp_tot, &s_total);
     for (int i = threadIdx.x; i < ne; i += NTF) {
         const float qy = cy[i], qx = cx[i], qm = cm[i];
         const int c = cell_of(qy, qx, G, b.ncy, b.ncx);
@@ -185,22 +183,22 @@ __global__ void __launch_bounds__(NTF) finalize_kernel(const LocParams p, MovieB
     // 5. grid over the particles for the linker
     if (link_grid) {
         const int n = over ? b.cap_p : np;
-        build_grid(py, px, nullptr, n, G, b.ncy, b.ncx, cnt_s, b.gstart + (size_t)t * (ncell + 1),
-                   b.gidx + (size_t)t * b.cap_p, warp_tot, &s_total);
+        build_grid(py, px, n, G, b.ncy, b.ncx, cnt_s, b.gstart + (size_t)t * (ncell + 1),
+                   b.gidx + (size_t)t * b.cap_p, b.gpos + (size_t)t * b.cap_p, warp_tot, &s_total);
     }
 }
 
 // Grid over externally supplied particle tables (standalone linking).
 __global__ void __launch_bounds__(NTF) grid_kernel(const float* py, const float* px, const int* npart,
                                                    int cap_p, int G, int ncy, int ncx, int* gstart,
-                                                   int* gidx) {
+                                                   int* gidx, float2* gpos) {
     __shared__ int warp_tot[NTF / 32];
     __shared__ int s_total;
     extern __shared__ int cnt_s[];
     const int t = blockIdx.x;
     const int ncell = ncx * ncy;
-    build_grid(py + (size_t)t * cap_p, px + (size_t)t * cap_p, nullptr, npart[t], (float)G, ncy, ncx, cnt_s,
-               gstart + (size_t)t * (ncell + 1), gidx + (size_t)t * cap_p, warp_tot, &s_total);
+    build_grid(py + (size_t)t * cap_p, px + (size_t)t * cap_p, npart[t], (float)G, ncy, ncx, cnt_s,
+               gstart + (size_t)t * (ncell + 1), gidx + (size_t)t * cap_p, gpos + (size_t)t * cap_p, warp_tot, &s_total);
 }
 
 }  // namespace gt

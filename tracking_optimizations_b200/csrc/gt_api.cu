@@ -30,15 +30,18 @@ namespace gt {
 __global__ void locate_tiles_kernel(const LocParams p, const MovieBufs b, int frame0);
 __global__ void fallback_walk_kernel(const LocParams p, const MovieBufs b, int win, const int* pbeg);
 __global__ void finalize_kernel(const LocParams p, MovieBufs b, float sep, int link_grid, int frame0);
-cudaError_t link_fixpoint_occupancy(int nt, int smem, int* per_sm);
-cudaError_t launch_link_fixpoint(int nt, int grid, void** args, int smem, cudaStream_t st);
+cudaError_t link_blocks_per_sm(bool multi, int* per_sm);
+cudaError_t launch_link(const LinkBufs& L, int max_passes, int* passes, unsigned long long* stat, int grid,
+                        cudaStream_t st);
+cudaError_t launch_link_multi(const LinkBufs* d_L, int nm, int max_passes, int* passes, unsigned long long* stat,
+                              int grid, cudaStream_t st);
 __global__ void scan_frames_kernel(const int* in, int* out, int n);
 __global__ void scan_frames_from_kernel(const int* in, int* out, int f0, int n);
 __global__ void newid_kernel(const int* newrank, const int* newbase, const int* off, const int* npart,
                              int* newid, int T);
 __global__ void assemble_kernel(AsmArgs a);
 __global__ void grid_kernel(const float* py, const float* px, const int* npart, int cap_p, int G,
-                            int ncy, int ncx, int* gstart, int* gidx);
+                            int ncy, int ncx, int* gstart, int* gidx, float2* gpos);
 bool fast_supported(int kr, int dd, int rc, int diameter);
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, int T, int frame0, int* used_tma);
@@ -48,8 +51,6 @@ cudaError_t launch_adjoint_particles(int mode, const AdjParams& p, const float* 
                                      double* gpart, int* err, int num_sms, cudaStream_t st);
 int adjoint_particle_blocks_max(int num_sms);
 cudaError_t launch_adjoint_transpose(const AdjParams& p, const float* gR, float* gI, cudaStream_t st);
-__global__ void link_fixpoint_multi_kernel(const LinkBufs* Ls, const int* memory, const int* fstart, int nm,
-                                           int max_passes, int* ndirty, int* passes);
 int traj_filter_stubs(const int64_t* h_ids, int64_t n, int64_t threshold, uint8_t* h_keep, int64_t* h_count,
                       int64_t* nkept, cudaStream_t st, int num_sms, std::string* msg);
 int traj_steps(const int64_t* h_ids, const float* h_x, const float* h_y, int64_t n, float mppf, float* h_xs,
@@ -109,8 +110,7 @@ struct gt_ctx {
     cudaEvent_t bev[20] = {};         // fork/join events
     int* h_status = nullptr;          // pinned: 8 ints per movie
     int* h_stage = nullptr;           // pinned: one call's statistics, read back in one go
-    int link_per_sm = 0;              // resident link_fixpoint_kernel<256> blocks per SM (queried once)
-    int link_per_sm_big = 0;          // the same for link_fixpoint_kernel<1024>
+    int link_grid[2] = {0, 0};        // resident blocks of the one-movie and the batched linker (queried once)
     size_t h_stage_n = 0;
     uint16_t* h_frames = nullptr;     // pinned: decoded file frames
     size_t h_frames_n = 0;
@@ -128,15 +128,6 @@ constexpr int LOC_TW = 64;
 constexpr int LOC_CMAX = 512;
 constexpr int FB_WIN_MAX = 100;
 constexpr long long SUBNET_BUDGET = 1LL << 26;  // option trials per subnet
-// shared-memory pool of a linker block: 4 blocks of 256 threads per SM, so
-// that one round of blocks covers ~600 frames; frames whose data does not
-// fit use the block's global scratch slot
-constexpr int LINK_POOL_BYTES = 48 * 1024;
-// frames of at least this many pixels are linked by 1024-thread blocks (one
-// per SM, a larger shared-memory pool): their linking is latency-bound on
-// global scratch, and 32 warps per frame hide four times more of it
-constexpr long long LINK_BIG_PIXELS = 1LL << 20;
-constexpr int LINK_POOL_BYTES_BIG = 160 * 1024;
 constexpr int LINK_WINDOWS = 16;  // upload chunks of the host-frames path, at most
 
 struct Resolved {
@@ -225,21 +216,16 @@ void dilation(uint32_t sep, int* D, int* o) {
     *o = (int)half;
 }
 
-int next_pow2(long long x) {
-    int p = 1;
-    while (p < x) p <<= 1;
-    return p;
-}
-
 struct Plan {
     int T = 0, H = 0, W = 0, dtype = 0;
     Resolved r{};
     LocParams lp{};
     float sep = 0.f;
     int link = 0;
-    int cap_c = 0, cap_p = 0, cap_m = 0, cap_s = 0, cap_e = 0;
+    int cap_c = 0, cap_p = 0;
     int G = 8, ncx = 1, ncy = 1;
-    int nslot = 1, hsize = 64;
+    // linker scratch for components beyond a thread's own arrays
+    int nslot = 0, big_d = 1, big_s = 1, big_e = 1;
     size_t smem_loc = 0, smem_fb = 0, smem_fin = 0;
     int fb_win = 0;
     int fast = 0;
@@ -280,6 +266,20 @@ void annulus_inds_f(float outer, float inner, std::vector<int>& off) {
             float r2 = (float)(i * i + j * j);
             if (r2 <= or2 && r2 >= ir2) { off.push_back(i); off.push_back(j); }
         }
+}
+
+size_t big_ints(const Plan& P) { return 8 * (size_t)P.big_d + 1 + 3 * (size_t)P.big_s + 5 * (size_t)P.big_e; }
+
+// Scratch slots of the linker's large components: room for 4096
+// destinations, 8192 sources and 32768 edges each (a component that the
+// search budget lets finish is far smaller), four times more per capacity
+// retry.
+void link_scratch(Plan* pl, int scale) {
+    Plan& P = *pl;
+    P.nslot = P.link ? 64 : 0;
+    P.big_d = (int)std::min<long long>(4096LL * scale, P.cap_p);
+    P.big_s = (int)std::min<long long>(8192LL * scale, (long long)P.cap_p * (P.r.memory + 1));
+    P.big_e = (int)std::min<long long>(32768LL * scale, (long long)P.big_d * P.big_s);
 }
 
 int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int num_sms, Plan* pl,
@@ -352,25 +352,13 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     const double ext_h = H + 2.0 * lp.rint_c + s, ext_w = W + 2.0 * lp.rint_c + s;
     long long pack = (long long)(ext_h * ext_w / (0.785 * s * s)) + 16;
     P.cap_p = (int)std::min<long long>(P.cap_c, pack * scale);
-    P.cap_m = (int)std::max<long long>(1, (long long)r.memory * P.cap_p);
-    P.cap_s = P.cap_p + P.cap_m;
-    const double sr = P.link ? r.search_range : 1.0;
-    long long deg = (long long)((2 * sr + s) * (2 * sr + s) / (0.785 * s * s)) + 2;
-    P.cap_e = (int)std::min<long long>((long long)P.cap_s * std::min<long long>(deg * scale, P.cap_p),
-                                       (long long)1 << 30);
     P.G = std::max({(int)std::ceil(P.sep) + 1, P.link ? (int)std::ceil(r.search_range) + 1 : 0, 8,
                     (int)std::ceil(std::sqrt((double)HW / 16384.0))});
     P.ncy = (H + P.G - 1) / P.G;
     P.ncx = (W + P.G - 1) / P.G;
     P.smem_fin = sizeof(int) * (size_t)P.ncx * P.ncy;
     if (P.smem_fin > 200 * 1024) { *msg = "grid too fine"; return GT_ERR_ARG; }
-    P.hsize = 2 * next_pow2(2LL * std::max({P.cap_p, P.cap_m, 32}));
-    // link slots: bounded scratch
-    const size_t nn = (size_t)P.cap_s + P.cap_p;
-    const size_t per_slot = 4 * (3 * (size_t)P.cap_s + 1) + 8 * (size_t)P.cap_e * 2 + 4 * ((size_t)P.cap_p + 1) +
-                            4 * 4 * nn + nn + 16 * nn + 4 + 8 * (size_t)P.hsize;
-    const size_t budget = (size_t)6 << 30;
-    P.nslot = (int)std::max<size_t>(1, std::min<size_t>({(size_t)T, (size_t)num_sms * 4, budget / per_slot}));
+    link_scratch(&P, scale);
     column_list(r, P.names, P.types);
     return GT_OK;
 }
@@ -387,13 +375,13 @@ struct Work {
     float *char_tab, *gchar_tab;
     int *char_off, *sig_off, *bg_off;
     int* err;
-    int *off, *pred, *mlist, *mcount, *dirty, *ndirty, *newrank, *newcount, *newbase, *root, *lroot, *newid;
+    int *off, *pred, *newrank, *newcount, *newbase, *root, *lroot, *newid;
     int* pbeg;  // fallback list position at the start of each chunk's locate
-    unsigned long long* phase_ns;
-    unsigned char* lnext;
-    float *s_y, *s_x, *e_w, *d_w;
-    int *s_h, *s_deg, *e_dst, *d_cnt, *d_src, *uf, *c_nd, *c_ns, *c_min, *work, *bump, *hkey, *hval;
-    unsigned char* vis;
+    // linker (LinkBufs)
+    float2* gpos;
+    unsigned *lnk, *mm, *pres;
+    int *stamp, *rstamp, *seedq, *recq, *deferq, *gframe, *head, *nextc, *fstamp, *big;
+    unsigned long long* lstat;  // 4 phase times, 8 frame counts, then the linker's counters (16 ints)
     float* out;
 };
 
@@ -443,40 +431,32 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->err = c.take<int>(4);
     w->off = c.take<int>(T + 1);
     const size_t np = P.link ? T * P.cap_p : 1;
+    const size_t nm = P.link && P.r.memory > 0 ? np : 1;   // memory entries
+    const size_t nl = P.link && P.r.memory > 2 ? np : 1;   // and by trajectory root
+    const size_t nw = (P.r.memory + 31) / 32;
+    w->gpos = c.take<float2>(np);
     w->pred = c.take<int>(np);
-    w->lnext = c.take<unsigned char>(np);
-    w->mlist = c.take<int>(P.link ? T * P.cap_m : 1);
-    w->mcount = c.take<int>(T);
-    w->dirty = c.take<int>(T);
-    w->ndirty = c.take<int>((T + 2) * LINK_WINDOWS);  // per linker launch (frame window)
-    w->pbeg = c.take<int>(LINK_WINDOWS);
-    w->phase_ns = c.take<unsigned long long>(4);
     w->newrank = c.take<int>(np);
     w->newcount = c.take<int>(T);
     w->newbase = c.take<int>(T + 1);
     w->root = c.take<int>(np);
-    w->lroot = c.take<int>(P.link ? np : 1);
+    w->lroot = c.take<int>(np);
     w->newid = c.take<int>(np);
-    const size_t S = P.link ? P.nslot : 0;
-    const size_t nn = (size_t)P.cap_s + P.cap_p;
-    w->s_y = c.take<float>(S * P.cap_s);
-    w->s_x = c.take<float>(S * P.cap_s);
-    w->s_h = c.take<int>(S * P.cap_s);
-    w->s_deg = c.take<int>(S * (P.cap_s + 1));
-    w->e_dst = c.take<int>(S * P.cap_e);
-    w->e_w = c.take<float>(S * P.cap_e);
-    w->d_cnt = c.take<int>(S * (P.cap_p + 1));
-    w->d_src = c.take<int>(S * P.cap_e);
-    w->d_w = c.take<float>(S * P.cap_e);
-    w->uf = c.take<int>(S * nn);
-    w->c_nd = c.take<int>(S * nn);
-    w->c_ns = c.take<int>(S * nn);
-    w->c_min = c.take<int>(S * nn);
-    w->vis = c.take<unsigned char>(S * nn);
-    w->work = c.take<int>(S * 4 * nn);
-    w->bump = c.take<int>(S);
-    w->hkey = c.take<int>(S * P.hsize);
-    w->hval = c.take<int>(S * P.hsize);
+    w->pbeg = c.take<int>(LINK_WINDOWS);
+    w->lnk = c.take<unsigned>(nm);
+    w->mm = c.take<unsigned>(nm * nw);
+    w->stamp = c.take<int>(nm);
+    w->rstamp = c.take<int>(nm);
+    w->seedq = c.take<int>(nm);
+    w->recq = c.take<int>(nm);
+    w->deferq = c.take<int>(np);
+    w->gframe = c.take<int>(nl);
+    w->head = c.take<int>(nl);
+    w->nextc = c.take<int>(nl);
+    w->pres = c.take<unsigned>(nl * nw);
+    w->fstamp = c.take<int>(T);
+    w->lstat = c.take<unsigned long long>(12 + 8);
+    w->big = c.take<int>((size_t)P.nslot * big_ints(P));
     w->out = c.take<float>(need_locate && own_out ? T * P.cap_p * P.names.size() : 1);
     return c.off + 256;
 }
@@ -503,20 +483,20 @@ LinkBufs link_bufs(const Plan& P, const Work& w, long long budget) {
     LinkBufs L{};
     L.tb = 0;
     L.te = P.T;
-    L.T = P.T; L.cap_p = P.cap_p; L.cap_m = P.cap_m; L.cap_e = P.cap_e; L.cap_s = P.cap_s;
+    L.T = P.T; L.cap_p = P.cap_p; L.memory = (int)P.r.memory;
     L.r = P.r.search_range;
-    L.G = P.G; L.ncx = P.ncx; L.ncy = P.ncy;
-    L.py = w.py; L.px = w.px; L.npart = w.npart; L.off = w.off; L.gstart = w.gstart; L.gidx = w.gidx;
-    L.pred = w.pred; L.lnext = w.lnext; L.mlist = w.mlist; L.mcount = w.mcount; L.dirty = w.dirty;
-    L.ndirty = w.ndirty; L.newrank = w.newrank; L.newcount = w.newcount; L.root = w.root; L.lroot = w.lroot; L.err = w.err;
+    L.inv_g = 1.0f / (float)P.G;
+    L.ncx = P.ncx; L.ncy = P.ncy;
+    L.py = w.py; L.px = w.px; L.npart = w.npart; L.off = w.off; L.gstart = w.gstart; L.gidx = w.gidx; L.gpos = w.gpos;
+    L.np = (size_t)P.T * P.cap_p;
+    L.pred = w.pred; L.lnk = w.lnk; L.mm = w.mm; L.stamp = w.stamp; L.rstamp = w.rstamp;
+    L.seedq = w.seedq; L.recq = w.recq; L.deferq = w.deferq;
+    L.newrank = w.newrank; L.newcount = w.newcount; L.root = w.root; L.lroot = w.lroot;
+    L.gframe = w.gframe; L.head = w.head; L.nextc = w.nextc; L.pres = w.pres;
+    L.fstamp = w.fstamp; L.ctr = (int*)(w.lstat + 12); L.err = w.err;
     L.budget = budget;
-    L.nslot = P.nslot;
-    L.s_y = w.s_y; L.s_x = w.s_x; L.s_h = w.s_h; L.s_deg = w.s_deg; L.e_dst = w.e_dst; L.e_w = w.e_w;
-    L.d_cnt = w.d_cnt; L.d_src = w.d_src; L.d_w = w.d_w; L.uf = w.uf; L.c_nd = w.c_nd; L.c_ns = w.c_ns;
-    L.c_min = w.c_min; L.vis = w.vis; L.work = w.work; L.bump = w.bump; L.hkey = w.hkey; L.hval = w.hval;
-    L.hsize = P.hsize;
-    L.st_s = P.cap_s; L.st_s1 = (long long)P.cap_s + 1; L.st_p1 = (long long)P.cap_p + 1;
-    L.st_n = (long long)P.cap_s + P.cap_p; L.st_e = P.cap_e; L.st_h = P.hsize;
+    L.nslot = P.nslot; L.big_d = P.big_d; L.big_s = P.big_s; L.big_e = P.big_e;
+    L.big_ints = big_ints(P); L.big = w.big;
     return L;
 }
 
@@ -531,49 +511,32 @@ LinkBufs link_bufs(const Plan& P, const Work& w, long long budget) {
 // order give the sequential result (the host-frames path links each
 // uploaded chunk while the next one is copied).  link_prepare runs once
 // before the first window, link_finish once after the last.
-int link_prepare(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st) {
-    const int T = P.T;
-    CK(cudaMemsetAsync(w.mcount, 0, sizeof(int) * T, st));
-    CK(cudaMemsetAsync(w.dirty, 0, sizeof(int) * T, st));
-    CK(cudaMemsetAsync(w.ndirty, 0, sizeof(int) * (T + 2) * LINK_WINDOWS, st));
-    CK(cudaMemsetAsync(w.phase_ns, 0, sizeof(unsigned long long) * 4, st));
+int link_prepare(gt_ctx* ctx, const Work& w, cudaStream_t st) {
+    CK(cudaMemsetAsync(w.lstat, 0, sizeof(unsigned long long) * (12 + 8), st));
     return GT_OK;
 }
 
-// Threads per linker block for frames of H x W pixels, its resident blocks
-// per SM (queried once per context) and its shared-memory pool.
-int link_shape(gt_ctx* ctx, long long px, int* nt, int* per_sm, int* pool) {
-    const bool big = px >= LINK_BIG_PIXELS;
-    *nt = big ? 1024 : 256;
-    *pool = big ? LINK_POOL_BYTES_BIG : LINK_POOL_BYTES;
-    int& cached = big ? ctx->link_per_sm_big : ctx->link_per_sm;
-    if (!cached) {
+// Resident blocks of the one-movie (0) or the batched (1) linker.
+int link_grid(gt_ctx* ctx, int multi, int* grid) {
+    if (!ctx->link_grid[multi]) {
         int q = 0;
-        CK(link_fixpoint_occupancy(*nt, *pool, &q));
-        cached = std::max(1, q);
+        CK(link_blocks_per_sm(multi != 0, &q));
+        ctx->link_grid[multi] = std::max(1, q) * ctx->num_sms;
     }
-    *per_sm = cached;
+    *grid = ctx->link_grid[multi];
     return GT_OK;
 }
 
-int link_window(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st, int tb, int te, int wi) {
+int link_window(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st, int tb, int te) {
     LinkBufs L = link_bufs(P, w, ctx->subnet_budget);
     L.tb = tb;
     L.te = te;
-    const int T = P.T;
-    int rounds = 0;
-    int nt = 256, per_sm = 1, pool = LINK_POOL_BYTES;
-    int rc = link_shape(ctx, (long long)P.H * P.W, &nt, &per_sm, &pool);
+    int grid = 1;
+    const int rc = link_grid(ctx, 0, &grid);
     if (rc) return rc;
-    L.lsm_bytes = pool;
-    const int grid = std::max(1, std::min(P.nslot, per_sm * ctx->num_sms));
-    int memory = (int)P.r.memory;
-    int max_passes = te - tb + 1;
-    int* ndirty = w.ndirty + (size_t)wi * (T + 2);
-    int* passes = w.err + 1;
-    unsigned long long* phase_ns = w.phase_ns;
-    void* args[] = {&L, &memory, &max_passes, &rounds, &ndirty, &passes, &phase_ns};
-    CK(launch_link_fixpoint(nt, grid, args, pool, st));
+    // the pass counters start at zero (the statistics add up over windows)
+    if (tb > 0) CK(cudaMemsetAsync(w.lstat + 12, 0, sizeof(unsigned long long) * 8, st));
+    CK(launch_link(L, te - tb + 1, w.err + 1, w.lstat, grid, st));
     ctx->stats.launches += 1;
     return GT_OK;
 }
@@ -588,8 +551,8 @@ int link_finish(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st) {
 }
 
 int run_link(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st) {
-    int rc = link_prepare(ctx, P, w, st);
-    if (!rc) rc = link_window(ctx, P, w, st, 0, P.T, 0);
+    int rc = link_prepare(ctx, w, st);
+    if (!rc) rc = link_window(ctx, P, w, st, 0, P.T);
     if (!rc) rc = link_finish(ctx, P, w, st);
     return rc;
 }
@@ -612,10 +575,10 @@ MovieBufs movie_bufs(const Plan& P, const Work& w, const void* frames) {
     MovieBufs b{};
     b.frames = frames;
     b.T = P.T;
-    b.cap_c = P.cap_c; b.cap_p = P.cap_p; b.cap_m = P.cap_m; b.cap_e = P.cap_e;
+    b.cap_c = P.cap_c; b.cap_p = P.cap_p;
     b.cand = w.cand; b.fcount = w.fcount; b.rowcnt = w.rowcnt; b.pend = w.pend; b.npend = w.npend;
     b.py = w.py; b.px = w.px; b.pm = w.pm; b.prec = w.prec; b.npart = w.npart;
-    b.G = P.G; b.ncx = P.ncx; b.ncy = P.ncy; b.gstart = w.gstart; b.gidx = w.gidx;
+    b.G = P.G; b.ncx = P.ncx; b.ncy = P.ncy; b.gstart = w.gstart; b.gidx = w.gidx; b.gpos = w.gpos;
     b.cperm = w.cperm; b.cy = w.cy; b.cx = w.cx; b.cm = w.cm; b.crec = w.crec; b.ccell = w.ccell;
     b.cstart = w.cstart; b.cidx = w.cidx;
     b.char_tab = w.char_tab; b.char_off = w.char_off; b.gchar_tab = w.gchar_tab;
@@ -679,7 +642,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     const int nchunks = (T + chunk - 1) / chunk;
     const bool chunked = h_frames && P.link && nchunks > 1 && nchunks <= LINK_WINDOWS;
     if (P.link) {
-        rc = link_prepare(ctx, P, w, st);
+        rc = link_prepare(ctx, w, st);
         if (rc) return rc;
     }
     CK(cudaMemsetAsync(w.pbeg, 0, sizeof(int) * LINK_WINDOWS, st));
@@ -693,7 +656,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
         CK(cudaGetLastError());
         ctx->stats.launches += 3;
         if (P.link) {
-            const int r2 = link_window(ctx, P, w, st, f0, f0 + nf, wi);
+            const int r2 = link_window(ctx, P, w, st, f0, f0 + nf);
             if (r2) return r2;
         }
         ++wi;
@@ -748,7 +711,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     }
     CK(cudaEventRecord(ctx->ev[2], st));
     if (P.link) {
-        if (!chunked) rc = link_window(ctx, P, w, st, 0, T, 0);
+        if (!chunked) rc = link_window(ctx, P, w, st, 0, T);
         if (!rc) rc = link_finish(ctx, P, w, st);
         if (rc) return rc;
     }
@@ -773,11 +736,9 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     ctx->stats.launches += 1;
     CK(cudaEventRecord(ctx->ev[4], st));
     // every statistic of the call in one readback: error words, row count,
-    // pending walks, per-frame record counts, linker phases and dirty counts
-    const int nwin = std::max(wi, 1);
-    const size_t n_nd = P.link ? (size_t)(T + 2) * nwin : 0;
-    const size_t ph_off = (6 + (size_t)T + 1) & ~(size_t)1;  // 8-byte aligned for the phase times
-    const size_t need_ints = ph_off + 8 + n_nd;
+    // pending walks, per-frame record counts, linker phases and frame counts
+    const size_t ph_off = (6 + (size_t)T + 1) & ~(size_t)1;  // 8-byte aligned for the linker's statistics
+    const size_t need_ints = ph_off + 2 * 12;
     if (ctx->h_stage_n < need_ints) {
         if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
         ctx->h_stage = nullptr;
@@ -790,11 +751,8 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     CK(cudaMemcpyAsync(hs + 4, w.off + T, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(hs + 5, w.npend, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(hs + 6, w.fcount, sizeof(int) * T, cudaMemcpyDeviceToHost, st));
-    unsigned long long* hph = (unsigned long long*)(hs + ph_off);  // 4 u64
-    if (P.link) {
-        CK(cudaMemcpyAsync(hph, w.phase_ns, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(hs + ph_off + 8, w.ndirty, sizeof(int) * n_nd, cudaMemcpyDeviceToHost, st));
-    }
+    unsigned long long* hph = (unsigned long long*)(hs + ph_off);
+    if (P.link) CK(cudaMemcpyAsync(hph, w.lstat, sizeof(unsigned long long) * 12, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     int hb[5] = {hs[0], hs[1], hs[2], hs[3], hs[4]};
     const int np = hs[5];
@@ -805,12 +763,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     ctx->stats.link_iterations = P.link ? hb[1] : 0;
     if (P.link) {
         for (int i = 0; i < 4; ++i) ctx->stats.link_phase_ms[i] = (float)(hph[i] * 1e-6);
-        const int* nd = hs + ph_off + 8;
-        for (int i = 0; i < 8; ++i) {
-            int v = 0;
-            for (int c = 0; c < nwin; ++c) v += i + 1 < T + 2 ? nd[(size_t)c * (T + 2) + i + 1] : 0;
-            ctx->stats.link_dirty[i] = v;
-        }
+        for (int i = 0; i < 8; ++i) ctx->stats.link_dirty[i] = (int)hph[4 + i];
     }
     ctx->stats.fallback_walks = np;
     ctx->stats.particles = hb[4];
@@ -997,22 +950,14 @@ struct BatchMovie {
     size_t off = 0;
     bool fast = false;
     int link_slot = -1;  // index among the movies of the shared linker launch
-    bool solo = false;   // linked by its own cooperative launch (large movie)
-    LinkBufs solo_L{};
-    int solo_grid = 0;
-    int solo_nt = 256;   // threads per block of its own linker launch
-    int solo_pool = 0;   // and that launch's shared-memory pool
 };
 
 struct BatchShared {
     LinkBufs* d_L = nullptr;
-    int* d_mem = nullptr;
-    int* d_fstart = nullptr;
-    int* d_ndirty = nullptr;
+    unsigned long long* d_stat = nullptr;
     int* d_passes = nullptr;
     int* d_status = nullptr;  // 8 ints per movie: err[0..3], nrows
     int nlink = 0, max_passes = 0, link_grid = 0;
-    int nsolo = 0, solo_grid = 0;
     int launches = 0;
 };
 
@@ -1103,10 +1048,7 @@ int enqueue_front(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t 
     scan_frames_kernel<<<1, 1024, 0, s>>>(w.npart, w.off, T);
     CK(cudaGetLastError());
     *launches += 3;
-    if (P.link) {
-        CK(cudaMemsetAsync(w.mcount, 0, sizeof(int) * T, s));
-        CK(cudaMemsetAsync(w.dirty, 0, sizeof(int) * T, s));
-    }
+    if (P.link) return link_prepare(ctx, w, s);
     return GT_OK;
 }
 
@@ -1154,30 +1096,9 @@ int enqueue_batch(gt_ctx* ctx, std::vector<BatchMovie>& B, gt_movie* mv, int n, 
         CK(cudaStreamWaitEvent(st, ctx->bev[1 + k], 0));
     }
     if (S.nlink > 0) {
-        CK(cudaMemsetAsync(S.d_ndirty, 0, sizeof(int) * (size_t)(S.max_passes + 2) * S.nlink, st));
-        const LinkBufs* Ls = S.d_L;
-        const int* mem = S.d_mem;
-        const int* fst = S.d_fstart;
-        int nm = S.nlink, mp = S.max_passes;
-        int* nd = S.d_ndirty;
-        int* ps = S.d_passes;
-        void* args[] = {(void*)&Ls, (void*)&mem, (void*)&fst, &nm, &mp, &nd, &ps};
-        CK(cudaLaunchCooperativeKernel((const void*)link_fixpoint_multi_kernel, dim3(S.link_grid), dim3(256), args,
-                                       LINK_POOL_BYTES, st));
-        S.launches += 1;
-    }
-    for (int i = 0; i < n; ++i) {
-        if (!B[i].solo) continue;
-        BatchMovie& bm = B[i];
-        CK(cudaMemsetAsync(bm.w.ndirty, 0, sizeof(int) * (bm.P.T + 2), st));
-        CK(cudaMemsetAsync(bm.w.phase_ns, 0, sizeof(unsigned long long) * 4, st));
-        LinkBufs L = bm.solo_L;
-        int memory = (int)bm.P.r.memory, max_passes = bm.P.T + 1, rounds = 0;
-        int* nd = bm.w.ndirty;
-        int* ps = bm.w.err + 1;
-        unsigned long long* ph = bm.w.phase_ns;
-        void* args[] = {&L, &memory, &max_passes, &rounds, &nd, &ps, &ph};
-        CK(launch_link_fixpoint(bm.solo_nt, bm.solo_grid, args, bm.solo_pool, st));
+        CK(cudaMemsetAsync(S.d_passes, 0, sizeof(int), st));
+        CK(cudaMemsetAsync(S.d_stat, 0, sizeof(unsigned long long) * 12, st));
+        CK(launch_link_multi(S.d_L, S.nlink, S.max_passes, S.d_passes, S.d_stat, S.link_grid, st));
         S.launches += 1;
     }
     CK(cudaEventRecord(ctx->bev[9], st));
@@ -1246,53 +1167,22 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         if (!ctx->ev[i]) CK(cudaEventCreate(&ctx->ev[i]));
     // kernel choice
     for (int i = 0; i < n; ++i) B[i].fast = B[i].P.fast != 0;
-    // linked movies: a movie whose per-block scratch would cap the linker
-    // grid below full residency is linked by its own launch (as in the
-    // one-movie path); the others share one launch whose blocks share one
-    // scratch pool (slot strides of the largest of them)
+    // all linked movies share one linker launch and its scratch slots (a
+    // block resolves one large component at a time)
     BatchShared S;
-    const size_t budget = (size_t)6 << 30;
-    auto slot_bytes = [](long long s_, long long s1, long long p1, long long n_, long long e_, long long h_) {
-        return (size_t)(4 * (3 * s_ + s1) + 8 * e_ * 2 + 4 * p1 + 4 * 4 * n_ + n_ + 16 * n_ + 4 + 8 * h_);
-    };
-    int per_sm_multi = 0, per_sm_solo = 0;
-    CK(cudaFuncSetAttribute(link_fixpoint_multi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LINK_POOL_BYTES));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_multi, link_fixpoint_multi_kernel, 256, LINK_POOL_BYTES));
-    CK(link_fixpoint_occupancy(256, LINK_POOL_BYTES, &per_sm_solo));
-    const size_t full_grid = (size_t)std::max(1, per_sm_multi) * ctx->num_sms;
-    long long st_s = 1, st_s1 = 1, st_p1 = 1, st_n = 1, st_e = 1, st_h = 64;        // shared launch
-    long long bt_s = 1, bt_s1 = 1, bt_p1 = 1, bt_n = 1, bt_e = 1, bt_h = 64;        // solo launches
+    int rc_g = link_grid(ctx, 1, &S.link_grid);
+    if (rc_g) return rc_g;
+    Plan big;
     for (int i = 0; i < n; ++i) {
         const Plan& P = B[i].P;
         if (!P.link) continue;
-        const size_t own = slot_bytes(P.cap_s, (long long)P.cap_s + 1, (long long)P.cap_p + 1,
-                                      (long long)P.cap_s + P.cap_p, P.cap_e, P.hsize);
-        if (budget / own < full_grid) {
-            B[i].solo = true;
-            ++S.nsolo;
-            bt_s = std::max<long long>(bt_s, P.cap_s);
-            bt_s1 = std::max<long long>(bt_s1, (long long)P.cap_s + 1);
-            bt_p1 = std::max<long long>(bt_p1, (long long)P.cap_p + 1);
-            bt_n = std::max<long long>(bt_n, (long long)P.cap_s + P.cap_p);
-            bt_e = std::max<long long>(bt_e, P.cap_e);
-            bt_h = std::max<long long>(bt_h, P.hsize);
-            continue;
-        }
         B[i].link_slot = S.nlink++;
-        st_s = std::max<long long>(st_s, P.cap_s);
-        st_s1 = std::max<long long>(st_s1, (long long)P.cap_s + 1);
-        st_p1 = std::max<long long>(st_p1, (long long)P.cap_p + 1);
-        st_n = std::max<long long>(st_n, (long long)P.cap_s + P.cap_p);
-        st_e = std::max<long long>(st_e, P.cap_e);
-        st_h = std::max<long long>(st_h, P.hsize);
         S.max_passes = std::max(S.max_passes, P.T + 1);
+        big.nslot = std::max(big.nslot, P.nslot);
+        big.big_d = std::max(big.big_d, P.big_d);
+        big.big_s = std::max(big.big_s, P.big_s);
+        big.big_e = std::max(big.big_e, P.big_e);
     }
-    if (S.nlink > 0)
-        S.link_grid = (int)std::max<size_t>(1, std::min<size_t>(full_grid,
-                                                                budget / slot_bytes(st_s, st_s1, st_p1, st_n, st_e, st_h)));
-    if (S.nsolo > 0)
-        S.solo_grid = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::max(1, per_sm_solo) * ctx->num_sms,
-                                                                budget / slot_bytes(bt_s, bt_s1, bt_p1, bt_n, bt_e, bt_h)));
     // arena layout: movies, link pool, shared arrays
     size_t total = 0;
     for (int i = 0; i < n; ++i) {
@@ -1303,52 +1193,16 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         total += carve(Pc, nullptr, &w, 0, true, false);
         total = (total + 255) / 256 * 256;
     }
-    const size_t G = S.link_grid, GB = S.solo_grid;
     Carver pc{nullptr};
-    auto slots = [](Carver& c, Work& pw, size_t g, long long s_, long long s1, long long p1, long long n_,
-                    long long e_, long long h_) {
-        pw.s_y = c.take<float>(g * s_); pw.s_x = c.take<float>(g * s_); pw.s_h = c.take<int>(g * s_);
-        pw.s_deg = c.take<int>(g * s1); pw.e_dst = c.take<int>(g * e_); pw.e_w = c.take<float>(g * e_);
-        pw.d_cnt = c.take<int>(g * p1); pw.d_src = c.take<int>(g * e_); pw.d_w = c.take<float>(g * e_);
-        pw.uf = c.take<int>(g * n_); pw.c_nd = c.take<int>(g * n_); pw.c_ns = c.take<int>(g * n_);
-        pw.c_min = c.take<int>(g * n_); pw.vis = c.take<unsigned char>(g * n_);
-        pw.work = c.take<int>(g * 4 * n_); pw.bump = c.take<int>(g); pw.hkey = c.take<int>(g * h_);
-        pw.hval = c.take<int>(g * h_);
-    };
-    // solo launches run one after another: each lays out its own grid of
-    // slots with its own strides at the start of one shared region
-    size_t big_bytes = 0;
-    for (int i = 0; i < n; ++i) {
-        if (!B[i].solo) continue;
-        const Plan& P = B[i].P;
-        const size_t own = slot_bytes(P.cap_s, (long long)P.cap_s + 1, (long long)P.cap_p + 1,
-                                      (long long)P.cap_s + P.cap_p, P.cap_e, P.hsize);
-        int per_sm_own = 1;
-        int rc_s = link_shape(ctx, (long long)P.H * P.W, &B[i].solo_nt, &per_sm_own, &B[i].solo_pool);
-        if (rc_s) return rc_s;
-        B[i].solo_grid = (int)std::max<size_t>(1, std::min<size_t>({(size_t)P.T,
-                                                                   (size_t)per_sm_own * ctx->num_sms,
-                                                                   budget / own}));
-        Carver dry{nullptr};
-        Work wd{};
-        slots(dry, wd, B[i].solo_grid, P.cap_s, (long long)P.cap_s + 1, (long long)P.cap_p + 1,
-              (long long)P.cap_s + P.cap_p, P.cap_e, P.hsize);
-        big_bytes = std::max(big_bytes, dry.off);
-    }
-    char* big_base = nullptr;
-    (void)GB;
-    auto pool_layout = [&](Carver& c, Work& pw) {
-        slots(c, pw, G, st_s, st_s1, st_p1, st_n, st_e, st_h);
-        big_base = c.take<char>(big_bytes);
+    int* big_pool = nullptr;
+    auto pool_layout = [&](Carver& c) {
+        big_pool = c.take<int>((size_t)big.nslot * big_ints(big));
         S.d_L = c.take<LinkBufs>(std::max(1, S.nlink));
-        S.d_mem = c.take<int>(std::max(1, S.nlink));
-        S.d_fstart = c.take<int>(std::max(1, S.nlink));
-        S.d_ndirty = c.take<int>((size_t)(S.max_passes + 2) * std::max(1, S.nlink));
+        S.d_stat = c.take<unsigned long long>(12);
         S.d_passes = c.take<int>(1);
         S.d_status = c.take<int>(8 * (size_t)n);
     };
-    Work pool{};
-    pool_layout(pc, pool);
+    pool_layout(pc);
     const size_t pool_bytes = pc.off + 256;
     const size_t need = total + pool_bytes;
     {
@@ -1382,7 +1236,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         carve(Pc, ctx->arena + B[i].off, &B[i].w, 0, true, false);
     }
     Carver c2{ctx->arena + total};
-    pool_layout(c2, pool);
+    pool_layout(c2);
     const bool replay = ctx->batch_exec && key == ctx->batch_key;
     // constant tables and linker descriptors (other calls may have reused
     // the arena since the graph was built)
@@ -1391,44 +1245,15 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         if (rc) return rc;
     }
     std::vector<LinkBufs> hL(std::max(1, S.nlink));
-    std::vector<int> hm(std::max(1, S.nlink)), hf(std::max(1, S.nlink));
     if (S.nlink > 0) {
-        int fs = 0;
         for (int i = 0; i < n; ++i) {
             if (B[i].link_slot < 0) continue;
             LinkBufs L = link_bufs(B[i].P, B[i].w, ctx->subnet_budget);
-            L.nslot = (int)G;
-            L.s_y = pool.s_y; L.s_x = pool.s_x; L.s_h = pool.s_h; L.s_deg = pool.s_deg;
-            L.e_dst = pool.e_dst; L.e_w = pool.e_w; L.d_cnt = pool.d_cnt; L.d_src = pool.d_src; L.d_w = pool.d_w;
-            L.uf = pool.uf; L.c_nd = pool.c_nd; L.c_ns = pool.c_ns; L.c_min = pool.c_min; L.vis = pool.vis;
-            L.work = pool.work; L.bump = pool.bump; L.hkey = pool.hkey; L.hval = pool.hval;
-            L.st_s = st_s; L.st_s1 = st_s1; L.st_p1 = st_p1; L.st_n = st_n; L.st_e = st_e; L.st_h = st_h;
-            L.lsm_bytes = LINK_POOL_BYTES;
+            L.nslot = big.nslot; L.big_d = big.big_d; L.big_s = big.big_s; L.big_e = big.big_e;
+            L.big_ints = big_ints(big); L.big = big_pool;
             hL[B[i].link_slot] = L;
-            hm[B[i].link_slot] = (int)B[i].P.r.memory;
-            hf[B[i].link_slot] = fs;
-            fs += B[i].P.T;
         }
         CK(cudaMemcpyAsync(S.d_L, hL.data(), sizeof(LinkBufs) * S.nlink, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(S.d_mem, hm.data(), sizeof(int) * S.nlink, cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(S.d_fstart, hf.data(), sizeof(int) * S.nlink, cudaMemcpyHostToDevice, st));
-    }
-    for (int i = 0; i < n; ++i) {
-        if (!B[i].solo) continue;
-        const Plan& P = B[i].P;
-        Work pool_big{};
-        Carver cb{big_base};
-        slots(cb, pool_big, B[i].solo_grid, P.cap_s, (long long)P.cap_s + 1, (long long)P.cap_p + 1,
-              (long long)P.cap_s + P.cap_p, P.cap_e, P.hsize);
-        LinkBufs L = link_bufs(B[i].P, B[i].w, ctx->subnet_budget);
-        L.nslot = B[i].solo_grid;
-        L.s_y = pool_big.s_y; L.s_x = pool_big.s_x; L.s_h = pool_big.s_h; L.s_deg = pool_big.s_deg;
-        L.e_dst = pool_big.e_dst; L.e_w = pool_big.e_w; L.d_cnt = pool_big.d_cnt; L.d_src = pool_big.d_src;
-        L.d_w = pool_big.d_w; L.uf = pool_big.uf; L.c_nd = pool_big.c_nd; L.c_ns = pool_big.c_ns;
-        L.c_min = pool_big.c_min; L.vis = pool_big.vis; L.work = pool_big.work; L.bump = pool_big.bump;
-        L.hkey = pool_big.hkey; L.hval = pool_big.hval;
-        L.lsm_bytes = B[i].solo_pool;  // slot strides: the movie's own (link_bufs)
-        B[i].solo_L = L;
     }
     if (!replay) {
         if (ctx->batch_exec) { cudaGraphExecDestroy(ctx->batch_exec); ctx->batch_exec = nullptr; }
@@ -1490,7 +1315,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
             const Plan& P = B[i].P;
             cnt += (P.T + 65534) / 65535 + 3 + (P.link ? 2 : 0) + 1;
         }
-        S.launches = cnt + (S.nlink > 0 ? 1 : 0) + S.nsolo;
+        S.launches = cnt + (S.nlink > 0 ? 1 : 0);
     }
     CK(cudaEventRecord(ctx->ev[1], st));
     CK(cudaStreamSynchronize(st));
@@ -1501,8 +1326,6 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         CK(cudaMemcpy(&passes, S.d_passes, sizeof(int), cudaMemcpyDeviceToHost));
         ctx->stats.link_iterations = passes;
     }
-    for (int i = 0; i < n; ++i)
-        if (B[i].solo) ctx->stats.link_iterations = std::max(ctx->stats.link_iterations, ctx->h_status[8 * i + 1]);
     // per-movie status; capacity overflows are rerun through the plain path
     std::vector<int> status(ctx->h_status, ctx->h_status + 8 * (size_t)n);
     gt_stats keep = ctx->stats;
@@ -2108,9 +1931,6 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         P.r.search_range = search_range;
         P.r.memory = mem;
         P.cap_p = maxg;
-        P.cap_m = (int)std::max<long long>(1, (long long)mem * P.cap_p);
-        P.cap_s = P.cap_p + P.cap_m;
-        P.cap_e = (int)std::min<long long>((long long)P.cap_s * std::min(16 * scale, P.cap_p), 1LL << 30);
         // grid over the positions' bounding box, shifted to start at 0
         // cells of absolute positions; negative coordinates clamp into the
         // first cell (clamping is monotone, so neighbours stay adjacent)
@@ -2119,12 +1939,7 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         P.ncy = (int)(std::max(ymax, 0.0f) / P.G) + 1;
         P.ncx = (int)(std::max(xmax, 0.0f) / P.G) + 1;
         (void)ymin; (void)xmin;
-        P.hsize = 2 * next_pow2(2LL * std::max({P.cap_p, P.cap_m, 32}));
-        const size_t nn = (size_t)P.cap_s + P.cap_p;
-        const size_t per_slot = 4 * (3 * (size_t)P.cap_s + 1) + 8 * (size_t)P.cap_e * 2 +
-                                4 * ((size_t)P.cap_p + 1) + 4 * 4 * nn + nn + 16 * nn + 4 + 8 * (size_t)P.hsize;
-        P.nslot = (int)std::max<size_t>(1, std::min<size_t>({(size_t)T, (size_t)ctx->num_sms * 4,
-                                                             ((size_t)6 << 30) / per_slot}));
+        link_scratch(&P, scale);
         P.cap_c = 1;
         Work w{};
         const size_t need = carve(P, nullptr, &w, 0, false);
@@ -2146,7 +1961,7 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         CK(cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(sizeof(int) * (size_t)P.ncx * P.ncy)));
         grid_kernel<<<T, 512, sizeof(int) * (size_t)P.ncx * P.ncy, st>>>(w.py, w.px, w.npart, P.cap_p, P.G,
-                                                                        P.ncy, P.ncx, w.gstart, w.gidx);
+                                                                        P.ncy, P.ncx, w.gstart, w.gidx, w.gpos);
         CK(cudaGetLastError());
         scan_frames_kernel<<<1, 1024, 0, st>>>(w.npart, w.off, T);
         rc = run_link(ctx, P, w, st);

@@ -11,6 +11,8 @@
 //   grid_*     cell starts (T*(ncell+1)) and indices (T*cap_p) for linking
 //   pred       int, T*cap_p  (global index of the linked source, -1 = new)
 #pragma once
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 #define GT_MAX_TAPS 64
@@ -78,7 +80,7 @@ enum ErrBits {
 struct MovieBufs {
     const void* frames;
     int T;
-    int cap_c, cap_p, cap_m, cap_e;
+    int cap_c, cap_p;
     Cand* cand;
     int* fcount;
     int* rowcnt;
@@ -92,6 +94,7 @@ struct MovieBufs {
     int G, ncx, ncy;      // link/separation grid: cell size and counts
     int* gstart;          // T*(ncx*ncy+1)
     int* gidx;            // T*cap_p
+    float2* gpos;         // T*cap_p (y, x) of gidx's particles
     int* cperm;           // T*cap_c finalize scratch (raster permutation)
     float* cy;            // T*cap_c emitted candidates in raster order
     float* cx;
@@ -107,53 +110,46 @@ struct MovieBufs {
 };
 
 struct LinkBufs {
-    int T, cap_p, cap_m, cap_e, cap_s;
+    int T, cap_p, memory;
     int tb, te;           // frames linked by this launch; earlier frames are final
     float r;              // search range
-    int G, ncx, ncy;
+    float inv_g;          // 1 / cell size
+    int ncx, ncy;
     const float* py;
     const float* px;
     const int* npart;
     const int* off;       // exclusive prefix of npart (compact particle index)
     const int* gstart;
     const int* gidx;
+    const float2* gpos;   // slab: (y, x) of gidx's particles
+    // per particle, by compact index
+    size_t np;            // stride of the membership words: T * cap_p
     int* pred;            // compact index of the linked source, -1 = new
-    unsigned char* lnext; // slab: particle linked by the next frame
-    int* mlist;           // T*cap_m slab handles
-    int* mcount;          // T
-    int* dirty;           // T
-    int* ndirty;
-    int* newrank;         // compact: rank among new particles of its frame
+    unsigned* lnk;        // bit j: linked by the frame j + 1 later (j = 0, 1)
+    unsigned* mm;         // word w, bit b: memory entry of the frame 2 + 32 w + b later
+    int* stamp;           // last pass in which the particle was a seed
+    int* rstamp;          // last pass that listed it for a membership check
+    int* seedq;           // slab handles of the pass's seeds
+    int* recq;            // particles whose linked bits the pass changed
+    int* deferq;          // seeds whose component is resolved in scratch
+    int* newrank;         // rank among new particles of its frame
+    int* root;
+    int* lroot;           // where the pred chain enters the particle's chunk
+    // memory >= 3
+    int* gframe;          // frame
+    int* head;            // by root: list of its unused particles
+    int* nextc;
+    unsigned* pres;       // as mm: the id is present in the frame 1 + 32 w + b later
     int* newcount;        // T
-    int* root;            // compact
-    int* lroot;           // compact: where the pred chain enters the particle's chunk
+    int* fstamp;          // T: last pass with a seed in the frame
+    int* ctr;             // 4 passes x {seeds, membership checks, deferred, frames}
     int* err;
     long long budget;     // branch-and-bound option trials per subnet
-    // per-CTA scratch, `nslot` slots of these sizes
-    int nslot;
-    float* s_y;           // cap_s
-    float* s_x;
-    int* s_h;             // slab handle of each source
-    int* s_deg;           // cap_s + 1
-    int* e_dst;           // cap_e
-    float* e_w;
-    int* d_cnt;           // cap_p + 1
-    int* d_src;           // cap_e
-    float* d_w;
-    int* uf;              // cap_s + cap_p
-    int* c_nd;            // cap_s + cap_p
-    int* c_ns;
-    int* c_min;
-    unsigned char* vis;   // cap_s + cap_p
-    int* work;            // 4 * (cap_s + cap_p): stacks, paths, choices
-    int* bump;            // 1 per slot
-    int* hkey;            // hash tables, hsize per slot
-    int* hval;
-    int hsize;
-    int lsm_bytes;        // dynamic shared memory pool of the linker blocks
-    // slot strides of the scratch arrays (>= the capacities above; equal to
-    // the largest movie's when several movies share one pool)
-    long long st_s, st_s1, st_p1, st_n, st_e, st_h;
+    // scratch of the components beyond a thread's own arrays: nslot slots of
+    // big_ints for big_d destinations, big_s sources and big_e edges
+    int nslot, big_d, big_s, big_e;
+    size_t big_ints;
+    int* big;
 };
 
 // Adjoint of bandpass + refine at fixed peaks.  The forward arithmetic uses

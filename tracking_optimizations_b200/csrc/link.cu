@@ -11,10 +11,26 @@
 // Parallel structure.  Frame t's assignment depends only on the positions of
 // frames t-1 and t and on the memory entries M(t) (unlinked particles of the
 // previous `memory` frames, deduplicated by trajectory).  All frames are
-// linked at once for a guessed M; M is then recomputed from the result, and
-// only frames whose M changed are linked again, until M is a fixed point.
+// linked at once with M = {}; M is then evaluated from the result, and links
+// and M are updated in turn until no M changes in reach of a destination.
 // M(t) depends on frames < t only, so iteration k settles frame k at the
 // latest and the fixed point is the sequential result.
+//
+// What bounds it: latency.  A pass changes little (the benchmark movie of
+// 1000 x 400 particles: 178k of its destinations in pass 1, a few hundred from
+// pass 6 on), so a pass touches what changed and nothing else:
+//   - membership in M is a bit per (particle, frame distance), and a
+//     component whose memory entries did not change keeps its links: adding
+//     or removing entries alters exactly the components that hold a
+//     destination in reach of one (every piece that a removed entry leaves
+//     behind was next to it), so those destinations are the pass's seeds;
+//   - a thread explores one seed's component through the frames' cell grids
+//     and resolves it; of the seeds of a component the smallest does it.
+//     There is no per-frame state, so the work spreads over the whole grid
+//     whatever the frames' sizes.
+// Relinking whole frames instead, a block per changed frame with the graph in
+// shared memory, took 0.99 ms for that movie, 64 ms for 200 frames of 15k
+// particles with memory 3 and 9.2 ms for a table of 500 frames of 760.
 #include <cooperative_groups.h>
 
 #include "gt_device.cuh"
@@ -23,11 +39,8 @@ namespace cg = cooperative_groups;
 
 namespace gt {
 
-
-
 namespace {
-constexpr int NTL = 256;   // threads of a linker block for small frames
-constexpr int NTL_BIG = 1024;  // for large frames: one block per SM, 32 warps per frame
+constexpr int NTL = 256;  // threads of a linker block
 
 __device__ __forceinline__ bool within_r(float qy, float qx, float iy, float ix, float r, float* dist) {
     // kd-tree box pre-filter + linking.rs:91-100 distance (dest - source)
@@ -41,555 +54,415 @@ __device__ __forceinline__ bool within_r(float qy, float qx, float iy, float ix,
     return dd < r * r;
 }
 
-__device__ __forceinline__ int cell_of(float y, float x, float G, int ncy, int ncx) {
-    int cy = (int)floorf(y / G), cx = (int)floorf(x / G);
-    cy = clampi(cy, 0, ncy - 1);
-    cx = clampi(cx, 0, ncx - 1);
-    return cy * ncx + cx;
-}
-
-__device__ int uf_find(int* uf, int x) {
-    while (true) {
-        int p = uf[x];
-        if (p == x) return x;
-        int gp = uf[p];
-        if (gp != p) atomicCAS(&uf[x], p, gp);  // path halving
-        x = p;
+// The frame of compact particle index g, in [lo, hi).
+__device__ __forceinline__ int frame_of(const LinkBufs& L, int g, int lo, int hi) {
+    --hi;
+    while (lo < hi) {
+        const int m = (lo + hi + 1) >> 1;
+        if (__ldg(L.off + m) <= g) lo = m;
+        else hi = m - 1;
     }
+    return lo;
 }
 
-__device__ void uf_union(int* uf, int a, int b) {
-    while (true) {
-        a = uf_find(uf, a);
-        b = uf_find(uf, b);
-        if (a == b) return;
-        if (a < b) { int t = a; a = b; b = t; }
-        if (atomicCAS(&uf[a], a, b) == a) return;
+// fn(index, y, x) for the particles of frame f in the 3 x 3 cells around
+// (qy, qx): a row of cells is one range of the cell-ordered positions.  The
+// cells are at least search_range + 1 wide, so rounding of the cell number
+// cannot lose a pair.  Stops when fn returns false.
+template <class F>
+__device__ __forceinline__ bool near(const LinkBufs& L, int f, float qy, float qx, F&& fn) {
+    const float ig = L.inv_g;
+    const int cy = clampi((int)floorf(qy * ig), 0, L.ncy - 1), cx = clampi((int)floorf(qx * ig), 0, L.ncx - 1);
+    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, L.ncx - 1) + 1;
+    const int* gs = L.gstart + (size_t)f * ((size_t)L.ncx * L.ncy + 1);
+    int a[3], n[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const int yy = cy + q - 1;
+        const bool in = yy >= 0 && yy < L.ncy;
+        a[q] = in ? __ldg(gs + yy * L.ncx + x0) : 0;
+        n[q] = in ? __ldg(gs + yy * L.ncx + x1) - a[q] : 0;
     }
+    const size_t base = (size_t)f * L.cap_p;
+    const int n01 = n[0] + n[1], total = n01 + n[2];
+    for (int s = 0; s < total; ++s) {
+        const size_t at = base + (s < n[0] ? a[0] + s : s < n01 ? a[1] + (s - n[0]) : a[2] + (s - n01));
+        const float2 p = __ldg(L.gpos + at);
+        if (!fn(__ldg(L.gidx + at), p.x, p.y)) return false;
+    }
+    return true;
 }
 
-template <int NT>
-__device__ int block_scan_inplace_l(int* data, int n, int* warp_tot, int* s_total) {
-    const int chunk = (n + NT - 1) / NT;
-    const int q0 = threadIdx.x * chunk, q1 = min(q0 + chunk, n);
-    int mine = 0;
-    for (int q = q0; q < q1; ++q) mine += data[q];
-    int pos = block_excl_scan<NT>(mine, warp_tot, s_total);
-    for (int q = q0; q < q1; ++q) { int v = data[q]; data[q] = pos; pos += v; }
-    __syncthreads();
-    return *s_total;
+// *ctr += 1: one atomic for the lanes that call together with the same
+// counter (lanes of a warp may be at different movies of a batch).
+__device__ __forceinline__ int push_slot(int* ctr) {
+    const unsigned same = __match_any_sync(__activemask(), (unsigned long long)ctr);
+    const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
+    int base = 0;
+    if (lane == leader) base = atomicAdd(ctr, __popc(same));
+    return __shfl_sync(same, base, leader) + __popc(same & ((1u << lane) - 1u));
 }
 
-// Exhaustive search of one subnet (linking.rs:390-452) by one thread.
-// dests: destination indices in DFS order; sources are chosen through the
-// per-destination lists d_src/d_w (ascending source index); null costs r^2.
-// Returns false when the option-trial budget is exhausted.
-__device__ bool solve_subnet(const LinkBufs& L, const int* dests, int nd, const int* d_off,
-                             const int* d_src, const float* d_w, unsigned char* used, int* oi,
-                             int* cur, int* best_choice, float null_cost) {
+// One component: destinations (index in frame t), sources (keys that order
+// them as linking.rs:244-259 does: frame t-1 by index, then the memory
+// entries by (frame, index): cap_p + slab handle) and their edges.  Most
+// components fit the thread's own arrays; larger ones are resolved by one
+// thread per block with arrays in global memory (LinkBufs::big).
+struct SmallComp {
+    static constexpr int MD = 16, MS = 16, ME = 48;
+    int D[MD];
+    unsigned S[MS];
+    float ew[ME], dw[ME];
+    unsigned char ed[ME], es[ME], dsrc[ME];
+    unsigned char doff[MD + 1], path[MD], oi[MD], used[MS], vis[MD], stk[MD + MS];
+    signed char cur[MD], best[MD];
+    __device__ int md() const { return MD; }
+    __device__ int ms() const { return MS; }
+    __device__ int me() const { return ME; }
+};
+
+struct BigComp {
+    int* D;
+    unsigned* S;
+    float *ew, *dw;
+    int *ed, *es, *dsrc, *doff, *path, *oi, *used, *vis, *stk, *cur, *best;
+    int cd, cs, ce;
+    __device__ int md() const { return cd; }
+    __device__ int ms() const { return cs; }
+    __device__ int me() const { return ce; }
+};
+
+__device__ __forceinline__ BigComp big_comp(const LinkBufs& L, int slot) {
+    BigComp b;
+    int* p = L.big + (size_t)slot * L.big_ints;
+    auto take = [&](int n) { int* q = p; p += n; return q; };
+    const int nd = L.big_d, ns = L.big_s, ne = L.big_e;
+    b.cd = nd; b.cs = ns; b.ce = ne;
+    b.D = take(nd); b.S = (unsigned*)take(ns);
+    b.ew = (float*)take(ne); b.dw = (float*)take(ne);
+    b.ed = take(ne); b.es = take(ne); b.dsrc = take(ne);
+    b.doff = take(nd + 1); b.path = take(nd); b.oi = take(nd); b.used = take(ns); b.vis = take(nd);
+    b.stk = take(nd + ns); b.cur = take(nd); b.best = take(nd);
+    return b;
+}
+
+// Exhaustive search of one subnet (linking.rs:390-452): destinations in DFS
+// order (path); sources are chosen through the per-destination lists
+// (ascending source order), null costs r^2.  Returns false when the
+// option-trial budget is exhausted.
+template <class C>
+__device__ bool solve_subnet(C& c, int nd, long long budget, float null_cost) {
     float score = 0.f, best = CUDART_INF_F;
     long long trials = 0;
     int l = 0;
-    oi[0] = 0;
+    c.oi[0] = 0;
     bool after_child = false;
     while (true) {
-        const int d = dests[l];
-        const int nopt = d_off[d + 1] - d_off[d] + 1;
+        const int d = c.path[l];
+        const int d0 = c.doff[d];
+        const int nopt = c.doff[d + 1] - d0 + 1;
         if (after_child) {
             // child returned: undo this level's option and advance
-            const int o = oi[l];
-            const float c = (o == nopt - 1) ? null_cost : d_w[d_off[d] + o];
-            if (o != nopt - 1) used[d_src[d_off[d] + o]] = 0;
-            score -= c;
-            oi[l] = o + 1;
+            const int o = c.oi[l];
+            const float w = (o == nopt - 1) ? null_cost : c.dw[d0 + o];
+            if (o != nopt - 1) c.used[c.dsrc[d0 + o]] = 0;
+            score -= w;
+            c.oi[l] = o + 1;
             after_child = false;
             continue;
         }
-        const int o = oi[l];
+        const int o = c.oi[l];
         if (o >= nopt || score > best) {  // loop exhausted, or early return
             if (l == 0) break;
             --l;
             after_child = true;
             continue;
         }
-        if (++trials > L.budget) {
-            // give back the sources the open levels hold
-            for (int q = 0; q < l; ++q)
-                if (cur[q] >= 0) used[cur[q]] = 0;
-            return false;
-        }
+        if (++trials > budget) return false;
         const bool is_null = (o == nopt - 1);
-        const float c = is_null ? null_cost : d_w[d_off[d] + o];
-        score += c;
+        const float w = is_null ? null_cost : c.dw[d0 + o];
+        score += w;
         if (!is_null) {
-            const int s = d_src[d_off[d] + o];
-            if (used[s]) { score -= c; oi[l] = o + 1; continue; }
-            used[s] = 1;
-            cur[l] = s;
+            const int s = c.dsrc[d0 + o];
+            if (c.used[s]) { score -= w; c.oi[l] = o + 1; continue; }
+            c.used[s] = 1;
+            c.cur[l] = s;
         } else {
-            cur[l] = -1;
+            c.cur[l] = -1;
         }
         if (l == nd - 1) {
             if (score < best) {
                 best = score;
-                for (int q = 0; q < nd; ++q) best_choice[q] = cur[q];
+                for (int q = 0; q < nd; ++q) c.best[q] = c.cur[q];
             }
-            if (!is_null) used[cur[l]] = 0;
-            score -= c;
-            oi[l] = o + 1;
+            if (!is_null) c.used[c.cur[l]] = 0;
+            score -= w;
+            c.oi[l] = o + 1;
         } else {
             ++l;
-            oi[l] = 0;
+            c.oi[l] = 0;
         }
     }
     return true;
 }
-}  // namespace
 
-// One CTA per frame (grid-stride); frame t >= 1 links P(t-1) + M(t) to P(t).
-template <int NT>
-// only_dirty: 0 = every frame, else the dirty bit of the pass (frames whose
-// memory entries that pass changed).
-__device__ void link_frames_body(const LinkBufs& L, int only_dirty, int t0, int tstride) {
-    __shared__ int warp_tot[NT / 32];
-    __shared__ int s_total;
-    __shared__ int s_bump;
-    extern __shared__ __align__(16) int lsm[];  // per-frame scratch pool
-    const int slot = blockIdx.x;
-    const int cap_p = L.cap_p;
+enum CompResult { COMP_DONE = 0, COMP_SKIP = 1, COMP_BIG = 2 };
+
+__device__ __forceinline__ bool in_memory(const LinkBufs& L, int g, int dist) {
+    return (__ldcg(L.mm + (size_t)((dist - 1) >> 5) * L.np + g) >> ((dist - 1) & 31)) & 1u;
+}
+
+// Writes the link of destination g (frame t): pred, the linked bits of the
+// old and the new source, and (pass > 0) both sources for the next pass's
+// membership check.  Bit j of L.lnk: linked by the frame j + 1 later.
+__device__ __forceinline__ void mark_linked(const LinkBufs& L, int src, int fs, int t, int k, bool set) {
+    const int j = t - fs - 1;
+    if (j < 2) {
+        if (set) atomicOr(L.lnk + src, 1u << j);
+        else atomicAnd(L.lnk + src, ~(1u << j));
+        if (k > 0 && L.memory <= 2 && atomicExch(L.rstamp + src, k) != k)
+            L.recq[push_slot(L.ctr + (k & 3) * 4 + 1)] = src;
+    }
+}
+
+// Explores the component of destination d of frame t and resolves it.
+// k = 0: every destination is a seed and there are no memory entries.
+// COMP_SKIP: a smaller seed of the same component does it; COMP_BIG: it does
+// not fit c (nothing is written).
+template <class C>
+__device__ int link_component(const LinkBufs& L, C& c, int t, int d, int k) {
     const float r = L.r;
-    const float G = (float)L.G;
-    const int ncell = L.ncx * L.ncy;
-    const int pool = L.lsm_bytes / 4;
-
-    for (int t = L.tb + t0; t < L.te; t += tstride) {
-        if (only_dirty && !(__ldcg(L.dirty + t) & only_dirty)) continue;
-        const int nd = L.npart[t];
-        int* pred = L.pred + L.off[t];
-        if (t == 0) {
-            for (int i = threadIdx.x; i < nd; i += NT) pred[i] = -1;
-            __syncthreads();
+    const int offt = __ldg(L.off + t);
+    const size_t bt = (size_t)t * L.cap_p;
+    int nd = 1, ns = 0, ne = 0, qd = 0, qs = 0, res = COMP_DONE;
+    c.D[0] = d;
+    while (true) {
+        if (qd < nd) {
+            const int di = qd++;
+            const float y = __ldg(L.py + bt + c.D[di]), x = __ldg(L.px + bt + c.D[di]);
+            auto edge = [&](unsigned key, float w) {
+                int s = 0;
+                while (s < ns && c.S[s] != key) ++s;
+                if (s == ns) {
+                    if (ns == c.ms()) { res = COMP_BIG; return false; }
+                    c.S[ns++] = key;
+                }
+                if (ne == c.me()) { res = COMP_BIG; return false; }
+                c.ed[ne] = di;
+                c.es[ne] = s;
+                c.ew[ne++] = w;
+                return true;
+            };
+            bool go = true;
+            if (t > 0)
+                go = near(L, t - 1, y, x, [&](int i, float sy, float sx) {
+                    float w;
+                    return !within_r(sy, sx, y, x, r, &w) || edge((unsigned)i, w);
+                });
+            if (k > 0)
+                for (int j = 1; go && j <= L.memory && t - 1 - j >= 0; ++j) {
+                    const int f = t - 1 - j, of = __ldg(L.off + f);
+                    go = near(L, f, y, x, [&](int i, float sy, float sx) {
+                        float w;
+                        if (!within_r(sy, sx, y, x, r, &w) || !in_memory(L, of + i, j)) return true;
+                        return edge((unsigned)L.cap_p + (unsigned)(f * L.cap_p + i), w);
+                    });
+                }
+            if (!go) return res;
+        } else if (qs < ns) {
+            const unsigned key = c.S[qs++];
+            const size_t h = key < (unsigned)L.cap_p ? (size_t)(t - 1) * L.cap_p + key : (size_t)(key - (unsigned)L.cap_p);
+            const float sy = __ldg(L.py + h), sx = __ldg(L.px + h);
+            const bool go = near(L, t, sy, sx, [&](int i, float y, float x) {
+                float w;
+                if (!within_r(sy, sx, y, x, r, &w)) return true;
+                int q = 0;
+                while (q < nd && c.D[q] != i) ++q;
+                if (q < nd) return true;
+                if (i < d && (k == 0 || __ldcg(L.stamp + offt + i) == k)) { res = COMP_SKIP; return false; }
+                if (nd == c.md()) { res = COMP_BIG; return false; }
+                c.D[nd++] = i;
+                return true;
+            });
+            if (!go) return res;
         } else {
-            const int n1 = L.npart[t - 1];
-            const int nm = __ldcg(L.mcount + t);
-            const int ns = n1 + nm;
-            const int nnode = ns + nd;
-            // the frame's particles, grid and scratch live in shared memory
-            // when they fit (latency), else in this block's global slot
-            // the cell index is staged too when it fits beside the rest
-            const int need_rest = 3 * nd + 4 * ns + 1 + nd + 1 + 8 * nnode + (nnode + 3) / 4;
-            const bool sm = need_rest <= pool;
-            const bool grid_sm = sm && need_rest + ncell + 1 <= pool;
-            const int need = need_rest + (grid_sm ? ncell + 1 : 0);
-            int* o = lsm;
-            auto take = [&](int n) { int* q = o; o += n; return q; };
-            const float* dy;
-            const float* dx;
-            const int* gs;
-            const int* gi;
-            float *sy, *sx;
-            int *sh, *sdeg, *dcnt, *uf, *cnd, *cns, *cmin, *work;
-            unsigned char* vis;
-            if (sm) {
-                float* ddy = (float*)take(nd);
-                float* ddx = (float*)take(nd);
-                int* ggi = take(nd);
-                const float* py_t = L.py + (size_t)t * cap_p;
-                const float* px_t = L.px + (size_t)t * cap_p;
-                const int* gs_t = L.gstart + (size_t)t * (ncell + 1);
-                const int* gi_t = L.gidx + (size_t)t * cap_p;
-                for (int i = threadIdx.x; i < nd; i += NT) { ddy[i] = py_t[i]; ddx[i] = px_t[i]; ggi[i] = gi_t[i]; }
-                if (grid_sm) {
-                    int* ggs = take(ncell + 1);
-                    for (int i = threadIdx.x; i <= ncell; i += NT) ggs[i] = gs_t[i];
-                    gs = ggs;
-                } else {
-                    gs = gs_t;
-                }
-                dy = ddy; dx = ddx; gi = ggi;
-                sy = (float*)take(ns); sx = (float*)take(ns); sh = take(ns); sdeg = take(ns + 1);
-                dcnt = take(nd + 1);
-                uf = take(nnode); cnd = take(nnode); cns = take(nnode); cmin = take(nnode);
-                work = take(4 * nnode);
-                vis = (unsigned char*)take((nnode + 3) / 4);
-            } else {
-                dy = L.py + (size_t)t * cap_p;
-                dx = L.px + (size_t)t * cap_p;
-                gs = L.gstart + (size_t)t * (ncell + 1);
-                gi = L.gidx + (size_t)t * cap_p;
-                sy = L.s_y + (size_t)slot * L.st_s;
-                sx = L.s_x + (size_t)slot * L.st_s;
-                sh = L.s_h + (size_t)slot * L.st_s;
-                sdeg = L.s_deg + (size_t)slot * L.st_s1;
-                dcnt = L.d_cnt + (size_t)slot * L.st_p1;
-                uf = L.uf + (size_t)slot * L.st_n;
-                cnd = L.c_nd + (size_t)slot * L.st_n;
-                cns = L.c_ns + (size_t)slot * L.st_n;
-                cmin = L.c_min + (size_t)slot * L.st_n;
-                vis = L.vis + (size_t)slot * L.st_n;
-                work = L.work + (size_t)slot * 4 * L.st_n;
-            }
-            int* bump = &s_bump;
-            if (threadIdx.x == 0) *bump = 0;
-            // sources: P(t-1) then M(t) (linking.rs:244-259 order)
-            for (int s = threadIdx.x; s < ns; s += NT) {
-                int h;
-                if (s < n1) h = (t - 1) * cap_p + s;
-                else h = __ldcg(L.mlist + (size_t)t * L.cap_m + (s - n1));
-                sh[s] = h;
-                sy[s] = L.py[h];
-                sx[s] = L.px[h];
-            }
-            for (int s = threadIdx.x; s < n1; s += NT) L.lnext[(size_t)(t - 1) * cap_p + s] = 0;
-            __syncthreads();
-            // candidate pairs: degree pass
-            for (int s = threadIdx.x; s < ns; s += NT) {
-                const float qy = sy[s], qx = sx[s];
-                const int c = cell_of(qy, qx, G, L.ncy, L.ncx);
-                const int cy0 = c / L.ncx, cx0 = c - cy0 * L.ncx;
-                int deg = 0;
-                for (int ddy = -1; ddy <= 1; ++ddy) {
-                    const int yy = cy0 + ddy;
-                    if (yy < 0 || yy >= L.ncy) continue;
-                    for (int ddx = -1; ddx <= 1; ++ddx) {
-                        const int xx = cx0 + ddx;
-                        if (xx < 0 || xx >= L.ncx) continue;
-                        const int cc = yy * L.ncx + xx;
-                        for (int k = gs[cc]; k < gs[cc + 1]; ++k) {
-                            const int d = gi[k];
-                            float dist;
-                            if (within_r(qy, qx, dy[d], dx[d], r, &dist)) ++deg;
-                        }
-                    }
-                }
-                sdeg[s] = deg;
-            }
-            __syncthreads();
-            const int ne = block_scan_inplace_l<NT>(sdeg, ns, warp_tot, &s_total);
-            if (threadIdx.x == 0) sdeg[ns] = ne;
-            int *edst, *dsrc;
-            float *ew, *dw;
-            if (sm && need + 4 * ne <= pool) {
-                edst = take(ne); ew = (float*)take(ne); dsrc = take(ne); dw = (float*)take(ne);
-            } else {
-                edst = L.e_dst + (size_t)slot * L.st_e;
-                ew = L.e_w + (size_t)slot * L.st_e;
-                dsrc = L.d_src + (size_t)slot * L.st_e;
-                dw = L.d_w + (size_t)slot * L.st_e;
-            }
-            if (ne > L.cap_e) {
-                if (threadIdx.x == 0) atomicOr(L.err, ERR_EDGE_OVERFLOW);
-                for (int i = threadIdx.x; i < nd; i += NT) pred[i] = -1;
-                __syncthreads();
-                continue;
-            }
-            for (int i = threadIdx.x; i <= nd; i += NT) dcnt[i] = 0;
-            __syncthreads();
-            // fill, then order each source's list by destination index
-            for (int s = threadIdx.x; s < ns; s += NT) {
-                const float qy = sy[s], qx = sx[s];
-                const int c = cell_of(qy, qx, G, L.ncy, L.ncx);
-                const int cy0 = c / L.ncx, cx0 = c - cy0 * L.ncx;
-                int w = sdeg[s];
-                const int w0 = w;
-                for (int ddy = -1; ddy <= 1; ++ddy) {
-                    const int yy = cy0 + ddy;
-                    if (yy < 0 || yy >= L.ncy) continue;
-                    for (int ddx = -1; ddx <= 1; ++ddx) {
-                        const int xx = cx0 + ddx;
-                        if (xx < 0 || xx >= L.ncx) continue;
-                        const int cc = yy * L.ncx + xx;
-                        for (int k = gs[cc]; k < gs[cc + 1]; ++k) {
-                            const int d = gi[k];
-                            float dist;
-                            if (within_r(qy, qx, dy[d], dx[d], r, &dist)) {
-                                int q = w++;
-                                while (q > w0 && edst[q - 1] > d) { edst[q] = edst[q - 1]; ew[q] = ew[q - 1]; --q; }
-                                edst[q] = d; ew[q] = dist;
-                            }
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-            // per-destination counts in a pass of their own: atomics inside
-            // the neighbour search above stall it several-fold
-            for (int q = threadIdx.x; q < ne; q += NT) atomicAdd(&dcnt[edst[q]], 1);
-            __syncthreads();
-            block_scan_inplace_l<NT>(dcnt, nd + 1, warp_tot, &s_total);
-            // destination lists, ascending source index (linking.rs:310-315)
-            int* dcur = cmin;  // reuse: cursors per destination
-            for (int d = threadIdx.x; d < nd; d += NT) dcur[d] = dcnt[d];
-            __syncthreads();
-            for (int s = threadIdx.x; s < ns; s += NT) {
-                for (int q = sdeg[s]; q < sdeg[s + 1]; ++q) {
-                    const int d = edst[q];
-                    const int k = atomicAdd(&dcur[d], 1);
-                    dsrc[k] = s;
-                    dw[k] = ew[q];
-                }
-            }
-            __syncthreads();
-            for (int d = threadIdx.x; d < nd; d += NT) {
-                const int a = dcnt[d], e = dcnt[d + 1];
-                for (int q = a + 1; q < e; ++q) {
-                    const int ks = dsrc[q];
-                    const float kw = dw[q];
-                    int z = q;
-                    while (z > a && dsrc[z - 1] > ks) { dsrc[z] = dsrc[z - 1]; dw[z] = dw[z - 1]; --z; }
-                    dsrc[z] = ks; dw[z] = kw;
-                }
-            }
-            // union-find over sources [0, ns) and destinations [ns, ns + nd)
-            for (int i = threadIdx.x; i < nnode; i += NT) {
-                uf[i] = i; cnd[i] = 0; cns[i] = 0; vis[i] = 0;
-            }
-            __syncthreads();
-            for (int s = threadIdx.x; s < ns; s += NT)
-                for (int q = sdeg[s]; q < sdeg[s + 1]; ++q) uf_union(uf, s, ns + edst[q]);
-            __syncthreads();
-            for (int i = threadIdx.x; i < nnode; i += NT) uf[i] = uf_find(uf, i);
-            __syncthreads();
-            for (int i = threadIdx.x; i < nnode; i += NT) cmin[i] = 0x7fffffff;
-            __syncthreads();
-            for (int s = threadIdx.x; s < ns; s += NT)
-                if (sdeg[s + 1] > sdeg[s]) atomicAdd(&cns[uf[s]], 1);
-            for (int d = threadIdx.x; d < nd; d += NT) {
-                const int rt = uf[ns + d];
-                atomicAdd(&cnd[rt], 1);
-                atomicMin(&cmin[rt], d);
-            }
-            __syncthreads();
-            // components, each resolved by the thread of its first destination
-            const float null_cost = r * r;
-            for (int d = threadIdx.x; d < nd; d += NT) {
-                const int rt = uf[ns + d];
-                if (cmin[rt] != d) continue;
-                const int cd = cnd[rt], cs = cns[rt];
-                if (cd == 1 && cs == 0) { pred[d] = -1; continue; }
-                if (cd == 1 && cs == 1) {
-                    const int s = dsrc[dcnt[d]];
-                    const int h = sh[s];
-                    pred[d] = L.off[h / cap_p] + (h % cap_p);
-                    if (s < n1) L.lnext[(size_t)(t - 1) * cap_p + s] = 1;
-                    continue;
-                }
-                // subnet: DFS preorder from d (linking.rs:316-342)
-                const int sz = cd + cs;
-                const int base = atomicAdd(bump, 4 * sz);
-                int* stk_n = work + base;          // node ids (dest: ns + d)
-                int* stk_p = stk_n + sz;           // next neighbour position
-                int* path = stk_p + sz;            // destinations in DFS order
-                int* choice = path + sz;           // per level: cur | best
-                int top = 0, npath = 0;
-                stk_n[0] = ns + d; stk_p[0] = 0; vis[ns + d] = 1; path[npath++] = d;
-                top = 1;
-                while (top > 0) {
-                    const int node = stk_n[top - 1];
-                    int pos = stk_p[top - 1];
-                    int next = -1;
-                    if (node >= ns) {
-                        const int dd2 = node - ns;
-                        if (dcnt[dd2] + pos < dcnt[dd2 + 1]) next = dsrc[dcnt[dd2] + pos];
-                    } else {
-                        if (sdeg[node] + pos < sdeg[node + 1]) next = ns + edst[sdeg[node] + pos];
-                    }
-                    if (next < 0) { --top; continue; }
-                    stk_p[top - 1] = pos + 1;
-                    if (vis[next]) continue;
-                    vis[next] = 1;
-                    if (next >= ns) path[npath++] = next - ns;
-                    stk_n[top] = next; stk_p[top] = 0; ++top;
-                }
-                // branch and bound; `vis` bytes of sources double as `used`
-                // flags: reset them first (all sources of the subnet were
-                // visited above)
-                for (int q = 0; q < npath; ++q) {
-                    const int dd2 = path[q];
-                    for (int z = dcnt[dd2]; z < dcnt[dd2 + 1]; ++z) vis[dsrc[z]] = 0;
-                }
-                int* oi = stk_n;                     // reuse the DFS stack
-                int* cur = stk_p;
-                int* bestc = choice;
-                for (int q = 0; q < npath; ++q) bestc[q] = -1;
-                const bool ok = solve_subnet(L, path, npath, dcnt, dsrc, dw, vis, oi, cur, bestc, null_cost);
-                if (!ok) atomicOr(L.err, ERR_SUBNET_BUDGET);
-                for (int q = 0; q < npath; ++q) {
-                    const int s = bestc[q];
-                    if (s < 0) { pred[path[q]] = -1; continue; }
-                    const int h = sh[s];
-                    pred[path[q]] = L.off[h / cap_p] + (h % cap_p);
-                    if (s < n1) L.lnext[(size_t)(t - 1) * cap_p + s] = 1;
-                }
-            }
-            __syncthreads();
+            break;
         }
-        // rank of each new particle within the frame (linking.rs:470)
-        int* nr = L.newrank + L.off[t];
-        const int chunk = (nd + NT - 1) / NT;
-        const int q0 = threadIdx.x * chunk, q1 = min(q0 + chunk, nd);
-        int mine = 0;
-        for (int q = q0; q < q1; ++q) mine += (pred[q] < 0);
-        int pos = block_excl_scan<NT>(mine, warp_tot, &s_total);
-        for (int q = q0; q < q1; ++q) nr[q] = pred[q] < 0 ? pos++ : -1;
-        if (threadIdx.x == 0) L.newcount[t] = s_total;
-        __syncthreads();
+    }
+    int np = nd;
+    if (nd == 1 && ns <= 1) {
+        c.path[0] = 0;
+        c.best[0] = ns - 1;  // the only source, or none
+    } else {
+        // per-destination lists, ascending source order (linking.rs:310-315)
+        for (int q = 0; q <= nd; ++q) c.doff[q] = 0;
+        for (int e = 0; e < ne; ++e) ++c.doff[c.ed[e] + 1];
+        for (int q = 0; q < nd; ++q) c.doff[q + 1] = c.doff[q + 1] + c.doff[q];
+        for (int q = 0; q < nd; ++q) c.vis[q] = 0;
+        for (int e = 0; e < ne; ++e) {
+            const int q = c.ed[e];
+            const int s = c.es[e];
+            const float w = c.ew[e];
+            int z = c.doff[q] + c.vis[q];
+            c.vis[q] = c.vis[q] + 1;
+            while (z > c.doff[q] && c.S[c.dsrc[z - 1]] > c.S[s]) {
+                c.dsrc[z] = c.dsrc[z - 1];
+                c.dw[z] = c.dw[z - 1];
+                --z;
+            }
+            c.dsrc[z] = s;
+            c.dw[z] = w;
+        }
+        // DFS preorder from the smallest destination (linking.rs:316-342):
+        // neighbours in ascending order, so the next node is the smallest
+        // one not yet visited
+        int first = 0;
+        for (int q = 0; q < nd; ++q) {
+            c.vis[q] = 0;
+            if (c.D[q] < c.D[first]) first = q;
+        }
+        for (int s = 0; s < ns; ++s) c.used[s] = 0;
+        int top = 1;
+        np = 0;
+        c.stk[0] = first;
+        c.vis[first] = 1;
+        c.path[np++] = first;
+        while (top > 0) {
+            const int node = c.stk[top - 1];
+            int next = -1;
+            if (node < nd) {
+                for (int z = c.doff[node]; z < c.doff[node + 1]; ++z)
+                    if (!c.used[c.dsrc[z]]) { next = c.dsrc[z]; break; }
+                if (next >= 0) {
+                    c.used[next] = 1;
+                    next += nd;
+                }
+            } else {
+                const int s = node - nd;
+                for (int e = 0; e < ne; ++e)
+                    if (c.es[e] == s && !c.vis[c.ed[e]] && (next < 0 || c.D[c.ed[e]] < c.D[next])) next = c.ed[e];
+                if (next >= 0) {
+                    c.vis[next] = 1;
+                    c.path[np++] = next;
+                }
+            }
+            if (next < 0) --top;
+            else c.stk[top++] = next;
+        }
+        for (int s = 0; s < ns; ++s) c.used[s] = 0;
+        for (int q = 0; q < np; ++q) c.best[q] = -1;
+        if (!solve_subnet(c, np, L.budget, r * r)) atomicOr(L.err, ERR_SUBNET_BUDGET);
+    }
+    // the links: first every source given up, then every source taken (a
+    // source that changes destination ends up linked)
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 0 && k == 0) continue;
+        for (int q = 0; q < np; ++q) {
+            const int g = offt + c.D[c.path[q]];
+            const int s = c.best[q];
+            int fs = t - 1, src = -1;
+            if (s >= 0) {
+                unsigned h = c.S[s];
+                if (h >= (unsigned)L.cap_p) {
+                    h -= (unsigned)L.cap_p;
+                    fs = (int)(h / (unsigned)L.cap_p);
+                    h -= (unsigned)(fs * L.cap_p);
+                }
+                src = __ldg(L.off + fs) + (int)h;
+            }
+            if (pass == 0) {
+                const int old = __ldcg(L.pred + g);
+                if (old < 0 || old == src) continue;
+                int fo = t - 1;
+                while (__ldg(L.off + fo) > old) --fo;
+                mark_linked(L, old, fo, t, k, false);
+            } else {
+                if (k > 0 && __ldcg(L.pred + g) == src) continue;
+                L.pred[g] = src;
+                if (src >= 0 && L.memory > 0) mark_linked(L, src, fs, t, k, true);
+            }
+        }
+    }
+    return COMP_DONE;
+}
+
+// Links every destination of the window with M = {}.
+__device__ void link_all(const LinkBufs& L, int tid, int nthr) {
+    const int g1 = __ldg(L.off + L.te);
+    for (int g = __ldg(L.off + L.tb) + tid; g < g1; g += nthr) {
+        const int t = frame_of(L, g, L.tb, L.te);
+        const int d = g - __ldg(L.off + t);
+        SmallComp c;
+        if (link_component(L, c, t, d, 0) == COMP_BIG) L.deferq[push_slot(L.ctr + 2)] = t * L.cap_p + d;
     }
 }
 
-// Memory entries M(t) (linking.rs:244-259): particles of frames
-// [t-1-memory, t-2] that the next frame did not link (the `unused` lists of
-// linking.rs:479-485, oldest list first, index order within a list),
-// skipping trajectories present in frame t-1 and keeping the first entry of
-// each trajectory.  Marks frames whose M changed.
-template <int NT>
-__device__ void memory_body(const LinkBufs& L, int memory, int* ndirty, int wbit, int t0, int tstride) {
-    __shared__ int warp_tot[NT / 32];
-    __shared__ int s_total;
-    __shared__ int s_diff;
-    __shared__ int s_red;
-    extern __shared__ __align__(16) int lsm[];
-    const int slot = blockIdx.x;
-    const int cap_p = L.cap_p;
-    const int nn = L.cap_s + cap_p;
-    const int pool = L.lsm_bytes / 4;
-    for (int t = L.tb + t0; t < L.te; t += tstride) {
-        const int fbeg = max(0, t - 1 - memory), fend = t - 2;
-        if (fend < fbeg) continue;
-        // number of candidates, to place the scratch
-        if (threadIdx.x == 0) s_red = 0;
-        __syncthreads();
-        {
-            int cnt = 0;
-            for (int f = fbeg; f <= fend; ++f) {
-                const int n = L.npart[f];
-                const unsigned char* ln = L.lnext + (size_t)f * cap_p;
-                for (int i = threadIdx.x; i < n; i += NT) cnt += __ldcg(ln + i) ? 0 : 1;
-            }
-            atomicAdd(&s_red, cnt);
-        }
-        __syncthreads();
-        const int ncnt = s_red;
-        const int n1 = L.npart[t - 1];
-        int hs1 = 64;
-        while (hs1 < 2 * n1) hs1 <<= 1;
-        int hs2 = 64;
-        while (hs2 < 2 * ncnt) hs2 <<= 1;
-        int nmax = 0;
-        for (int f = fbeg; f <= fend; ++f) nmax = max(nmax, L.npart[f]);
-        const int cn = max(ncnt, nmax) + 1;
-        const bool sm = 3 * cn + 2 * (hs1 + hs2) <= pool;
-        int *ch, *cr, *cpos, *hk, *hv;
-        int lim;
-        if (sm) {
-            ch = lsm; cr = ch + cn; cpos = cr + cn; hk = cpos + cn; hv = hk + hs1 + hs2;
-            lim = cn;
-        } else {
-            ch = L.work + (size_t)slot * 4 * L.st_n;
-            cr = ch + nn;
-            cpos = cr + nn;
-            hk = L.hkey + (size_t)slot * L.st_h;
-            hv = L.hval + (size_t)slot * L.st_h;
-            lim = nn;
-        }
-        // candidates in (frame, index) order
-        int nc = 0;
-        for (int f = fbeg; f <= fend; ++f) {
-            const int n = L.npart[f];
-            const unsigned char* ln = L.lnext + (size_t)f * cap_p;
-            for (int i = threadIdx.x; i < n; i += NT) cpos[i] = __ldcg(ln + i) ? 0 : 1;
-            __syncthreads();
-            const int k = block_scan_inplace_l<NT>(cpos, n, warp_tot, &s_total);
-            for (int i = threadIdx.x; i < n; i += NT) {
-                if (__ldcg(ln + i)) continue;
-                const int j = nc + cpos[i];
-                if (j < lim) {
-                    ch[j] = f * cap_p + i;
-                    cr[j] = __ldcg(L.root + L.off[f] + i);
-                }
-            }
-            nc += k;
-            __syncthreads();
-        }
-        if (nc > lim) { if (threadIdx.x == 0) atomicOr(L.err, ERR_MEM_OVERFLOW); nc = lim; }
-        if (!sm && hs1 + hs2 > L.hsize) { if (threadIdx.x == 0) atomicOr(L.err, ERR_SCRATCH_OVERFLOW); continue; }
-        int* k1 = hk;
-        int* k2 = hk + hs1;
-        int* v2 = hv + hs1;
-        for (int i = threadIdx.x; i < hs1 + hs2; i += NT) { hk[i] = -1; hv[i] = 0x7fffffff; }
-        __syncthreads();
-        // trajectories present in frame t-1
-        for (int i = threadIdx.x; i < n1; i += NT) {
-            const int key = __ldcg(L.root + L.off[t - 1] + i);
-            unsigned hsh = ((unsigned)key * 2654435761u) & (hs1 - 1);
-            while (true) {
-                const int prev = atomicCAS(&k1[hsh], -1, key);
-                if (prev == -1 || prev == key) break;
-                hsh = (hsh + 1) & (hs1 - 1);
-            }
-        }
-        // first candidate of each trajectory
-        for (int j = threadIdx.x; j < nc; j += NT) {
-            const int key = cr[j];
-            unsigned hsh = ((unsigned)key * 2654435761u) & (hs2 - 1);
-            while (true) {
-                const int prev = atomicCAS(&k2[hsh], -1, key);
-                if (prev == -1 || prev == key) break;
-                hsh = (hsh + 1) & (hs2 - 1);
-            }
-            atomicMin(&v2[hsh], j);
-        }
-        __syncthreads();
-        for (int j = threadIdx.x; j < nc; j += NT) {
-            const int key = cr[j];
-            bool keep = true;
-            unsigned hsh = ((unsigned)key * 2654435761u) & (hs1 - 1);
-            while (true) {
-                const int kk = k1[hsh];
-                if (kk == -1) break;
-                if (kk == key) { keep = false; break; }
-                hsh = (hsh + 1) & (hs1 - 1);
-            }
-            if (keep) {
-                hsh = ((unsigned)key * 2654435761u) & (hs2 - 1);
-                while (k2[hsh] != key) hsh = (hsh + 1) & (hs2 - 1);
-                keep = v2[hsh] == j;
-            }
-            cpos[j] = keep ? 1 : 0;
-        }
-        if (threadIdx.x == 0) s_diff = 0;
-        __syncthreads();
-        const int nk = block_scan_inplace_l<NT>(cpos, nc, warp_tot, &s_total);
-        int* ml = L.mlist + (size_t)t * L.cap_m;
-        const int old = __ldcg(L.mcount + t);
-        if (nk > L.cap_m) { if (threadIdx.x == 0) atomicOr(L.err, ERR_MEM_OVERFLOW); continue; }
-        if (old != nk && threadIdx.x == 0) s_diff = 1;
-        __syncthreads();
-        for (int j = threadIdx.x; j < nc; j += NT) {
-            const int a = cpos[j];
-            const int nxt = (j + 1 < nc) ? cpos[j + 1] : nk;
-            if (nxt > a && __ldcg(ml + a) != ch[j]) s_diff = 1;
-        }
-        __syncthreads();
-        if (s_diff) {
-            for (int j = threadIdx.x; j < nc; j += NT) {
-                const int a = cpos[j];
-                const int nxt = (j + 1 < nc) ? cpos[j + 1] : nk;
-                if (nxt > a) ml[a] = ch[j];
-            }
-            if (threadIdx.x == 0) {
-                L.mcount[t] = nk;
-                atomicOr(L.dirty + t, wbit);
-                atomicAdd(ndirty, 1);
-            }
-        } else if (threadIdx.x == 0) {
-            atomicAnd(L.dirty + t, ~wbit);
-        }
-        __syncthreads();
+// Resolves the components of pass k's seeds.
+__device__ void link_seeds(const LinkBufs& L, int k, int vt, int nthr) {
+    int* ctr = L.ctr + (k & 3) * 4;
+    const int n = __ldcg(ctr);
+    for (int q = vt; q < n; q += nthr) {
+        const int h = __ldcg(L.seedq + q);
+        const int t = h / L.cap_p;
+        SmallComp c;
+        if (link_component(L, c, t, h - t * L.cap_p, k) == COMP_BIG) L.deferq[push_slot(ctr + 2)] = h;
     }
 }
 
-// Memory entries M(t) for memory 1 or 2, without trajectory roots.
+// The components that do not fit a thread's arrays, one thread per block and
+// scratch slot.
+__device__ void link_deferred(const LinkBufs& L, int k) {
+    const int n = __ldcg(L.ctr + (k & 3) * 4 + 2);
+    if (threadIdx.x != 0 || (int)blockIdx.x >= L.nslot) return;
+    for (int q = blockIdx.x; q < n; q += min((int)gridDim.x, L.nslot)) {
+        const int h = __ldcg(L.deferq + q);
+        const int t = h / L.cap_p;
+        BigComp c = big_comp(L, blockIdx.x);
+        if (link_component(L, c, t, h - t * L.cap_p, k) == COMP_BIG) {
+            // the host retries with larger slots; until the launch ends every
+            // link of the frame must be a valid index
+            atomicOr(L.err, ERR_EDGE_OVERFLOW);
+            if (k == 0)
+                for (int g = __ldg(L.off + t); g < __ldg(L.off + t + 1); ++g) L.pred[g] = -1;
+        }
+    }
+}
+
+// Every destination of frame t within reach of (y, x) becomes a seed of
+// pass k.
+__device__ __forceinline__ void seed_around(const LinkBufs& L, float y, float x, int t, int k) {
+    const int offt = __ldg(L.off + t);
+    near(L, t, y, x, [&](int i, float dy, float dx) {
+        float w;
+        if (within_r(y, x, dy, dx, L.r, &w) && atomicExch(L.stamp + offt + i, k) != k) {
+            L.seedq[push_slot(L.ctr + (k & 3) * 4)] = t * L.cap_p + i;
+            if (__ldcg(L.fstamp + t) != k && atomicExch(L.fstamp + t, k) != k) atomicAdd(L.ctr + (k & 3) * 4 + 3, 1);
+        }
+        return true;
+    });
+}
+
+// Replaces the bits `wm` of word w of particle g's membership (frame f) by
+// `bits` and seeds pass k around it in the frames where they changed.
+__device__ __forceinline__ void set_members(const LinkBufs& L, int g, int f, int w, unsigned wm, unsigned bits, int k) {
+    unsigned* m = L.mm + (size_t)w * L.np + g;
+    const unsigned old = __ldcg(m);
+    unsigned diff = (old ^ bits) & wm;
+    if (!diff) return;
+    *m = old ^ diff;
+    const size_t h = (size_t)f * L.cap_p + (g - __ldg(L.off + f));
+    const float y = __ldg(L.py + h), x = __ldg(L.px + h);
+    while (diff) {
+        const int b = __ffs(diff) - 1;
+        diff &= diff - 1;
+        seed_around(L, y, x, f + 2 + 32 * w + b, k);
+    }
+}
+
+// Frames whose particles can be memory entries of the window start here.
+__device__ __forceinline__ int first_member(const LinkBufs& L) { return max(0, L.tb - 1 - L.memory); }
+
+// Membership for memory 1 or 2, without trajectory roots.
 //
 // With at most two memory lists no trajectory branches: a particle left
 // unused by the next frame is a memory candidate for the next two frames
@@ -604,89 +477,130 @@ __device__ void memory_body(const LinkBufs& L, int memory, int* ndirty, int wbit
 //     t-1 particle exactly when that particle's pred is it (it was linked
 //     into t-1 as a memory entry): it has no descendant in t-2.
 // linking.rs:244-259 (unused lists oldest first, index order within a
-// list, dedupe by id against prev and among the entries) thus gives:
-// M(t) = the frame t-3 particles unused by t-2 and not the pred of a
-// frame t-1 particle, then the frame t-2 particles unused by t-1 (memory 1:
-// the latter only).  Marks frames whose M changed.
-// M(t) reads lnext of frames t-3 and t-2 and pred of frame t-1, which only
-// relinking frames t-2 and t-1 writes (lnext of a frame is written by the
-// link into the next frame), so from the second pass on (k > 1) a frame
-// whose frames t-1 and t-2 (memory 1: t-1) the previous pass did not relink
-// keeps its M.  Pass k marks with wbit = 1 << (k & 1) and reads the previous
-// pass's bit, so that concurrent marks never touch the bit being read.
-template <int NT>
-__device__ void memory_body_short(const LinkBufs& L, int memory, int* ndirty, int k, int t0, int tstride) {
-    __shared__ int warp_tot[NT / 32];
-    __shared__ int s_total;
-    __shared__ int s_diff;
-    extern __shared__ __align__(16) int lsm[];
-    const int slot = blockIdx.x;
-    const int cap_p = L.cap_p;
-    const int pool = L.lsm_bytes / 4;
-    const int wbit = 1 << (k & 1), pbit = 1 << ((k - 1) & 1);
-    for (int t = L.tb + t0; t < L.te; t += tstride) {
-        const int fbeg = max(0, t - 1 - memory), fend = t - 2;
-        if (fend < fbeg) continue;
-        if (k > 1 && !(__ldcg(L.dirty + t - 1) & pbit) && !(memory == 2 && (__ldcg(L.dirty + t - 2) & pbit))) {
-            if (threadIdx.x == 0) atomicAnd(L.dirty + t, ~wbit);
+// list, dedupe by id against prev and among the entries) thus makes a
+// particle an entry of the frame 2 later when the next frame does not link
+// it, and of the frame 3 later when the one between does not either.
+// Pass 1 checks every particle, later passes those whose linked bits the
+// pass before changed.
+__device__ void members_short(const LinkBufs& L, int k, int tid, int nthr) {
+    const int fb = first_member(L);
+    auto check = [&](int g, int f) {
+        const unsigned l = __ldcg(L.lnk + g);
+        unsigned wm = 0, bits = 0;
+        if (f + 2 >= L.tb && f + 2 < L.te) {
+            wm |= 1u;
+            if (!(l & 1u)) bits |= 1u;
+        }
+        if (L.memory == 2 && f + 3 >= L.tb && f + 3 < L.te) {
+            wm |= 2u;
+            if (!(l & 3u)) bits |= 2u;
+        }
+        set_members(L, g, f, 0, wm, bits, k);
+    };
+    if (k == 1) {
+        const int g1 = __ldg(L.off + L.te);
+        for (int g = __ldg(L.off + fb) + tid; g < g1; g += nthr) check(g, frame_of(L, g, fb, L.te));
+    } else {
+        const int n = __ldcg(L.ctr + ((k - 1) & 3) * 4 + 1);
+        for (int q = tid; q < n; q += nthr) {
+            const int g = __ldcg(L.recq + q);
+            check(g, frame_of(L, g, fb, L.te));
+        }
+    }
+}
+
+// Membership for memory >= 3.  Trajectories can branch (a particle relinked
+// from an older memory entry), so ids are compared by trajectory root.  A
+// particle unused by the next frame is an entry of frame t unless its id is
+// present in frame t-1 or an older frame of the window holds an unused
+// particle of the same id (linking.rs:244-259).  In steps, a grid barrier
+// between them: roots, then
+//   members_chain    the unused particles of each root as a list;
+//   members_present  every particle marks, in the entries of its root's list
+//                    at most `memory` frames before it, that their id is
+//                    present in its frame;
+//   members_long     the membership bits of every particle;
+//   members_clear    the lists emptied for the next pass.
+__device__ void members_chain(const LinkBufs& L, int tid, int nthr) {
+    const int g1 = __ldg(L.off + max(L.te - 2, first_member(L)));
+    const int nw = (L.memory + 31) >> 5;
+    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr) {
+        if (__ldcg(L.lnk + g) & 1u) continue;
+        for (int w = 0; w < nw; ++w) L.pres[(size_t)w * L.np + g] = 0u;
+        L.nextc[g] = atomicExch(L.head + __ldcg(L.root + g), g);
+    }
+}
+
+__device__ void members_present(const LinkBufs& L, int tid, int nthr) {
+    const int g1 = __ldg(L.off + max(L.te - 1, first_member(L)));
+    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr) {
+        const int f = __ldcg(L.gframe + g);
+        for (int c = __ldcg(L.head + __ldcg(L.root + g)); c >= 0; c = __ldcg(L.nextc + c)) {
+            const int dist = f - __ldcg(L.gframe + c);
+            if (dist > 0 && dist <= L.memory)
+                atomicOr(L.pres + (size_t)((dist - 1) >> 5) * L.np + c, 1u << ((dist - 1) & 31));
+        }
+    }
+}
+
+__device__ void members_long(const LinkBufs& L, int k, int tid, int nthr) {
+    const int g1 = __ldg(L.off + max(L.te - 2, first_member(L)));
+    const int nw = (L.memory + 31) >> 5;
+    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr) {
+        const int f = __ldcg(L.gframe + g);
+        const bool cand = !(__ldcg(L.lnk + g) & 1u);
+        // distances j (frame f + 1 + j) inside the window
+        const int j0 = max(1, L.tb - 1 - f);
+        int j1 = min(L.memory, L.te - 2 - f);
+        int fo = -1;  // latest older unused particle of the same id
+        if (cand)
+            for (int c = __ldcg(L.head + __ldcg(L.root + g)); c >= 0; c = __ldcg(L.nextc + c)) {
+                const int fc = __ldcg(L.gframe + c);
+                if (fc < f) fo = max(fo, fc);
+            }
+        // frame f + 1 + j's entries reach back to frame f + j - memory
+        const int jmin = fo < 0 ? 0 : fo - f + L.memory + 1;
+        for (int w = 0; w < nw; ++w) {
+            unsigned wm = 0, bits = 0;
+            for (int b = 0; b < 32; ++b) {
+                const int j = 32 * w + b + 1;
+                if (j < j0 || j > j1) continue;
+                wm |= 1u << b;
+                if (cand && j >= jmin) bits |= 1u << b;
+            }
+            if (!wm) continue;
+            if (bits) bits &= ~__ldcg(L.pres + (size_t)w * L.np + g);
+            set_members(L, g, f, w, wm, bits, k);
+        }
+    }
+}
+
+__device__ void members_clear(const LinkBufs& L, int tid, int nthr) {
+    const int g1 = __ldg(L.off + max(L.te - 2, first_member(L)));
+    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr) L.head[__ldcg(L.root + g)] = -1;
+}
+
+// State of the window's particles before the first pass (earlier windows'
+// is kept; their rstamp may hold a pass number of their own).
+__device__ void window_begin(const LinkBufs& L, int tid, int nthr) {
+    const int nw = (L.memory + 31) >> 5;
+    const int fb = first_member(L);
+    const int gb = __ldg(L.off + L.tb), g1 = __ldg(L.off + L.te);
+    for (int g = __ldg(L.off + fb) + tid; g < g1; g += nthr) {
+        L.rstamp[g] = 0;
+        if (g < gb) {
+            if (L.memory > 2) L.head[__ldcg(L.root + g)] = -1;  // earlier windows' roots are final
             continue;
         }
-        const int fo = (fend > fbeg) ? fbeg : -1;  // frame t-3 (memory 2)
-        const int no = fo >= 0 ? L.npart[fo] : 0;
-        const int nb = L.npart[fbeg], ne = L.npart[fend];
-        const int nmax = max(nb, ne);
-        const int ccap = nb + (fo >= 0 ? ne : 0);
-        int *taken, *cpos, *ch;
-        if (no + nmax + ccap + 1 <= pool) {
-            taken = lsm; cpos = taken + no; ch = cpos + nmax;
-        } else {
-            int* w = L.work + (size_t)slot * 4 * L.st_n;
-            taken = w; cpos = w + L.st_n; ch = w + 2 * L.st_n;
+        L.lnk[g] = 0u;
+        L.stamp[g] = 0;
+        for (int w = 0; w < nw; ++w) L.mm[(size_t)w * L.np + g] = 0u;
+        if (L.memory > 2) {
+            L.head[g] = -1;
+            L.gframe[g] = frame_of(L, g, L.tb, L.te);
         }
-        for (int i = threadIdx.x; i < no; i += NT) taken[i] = 0;
-        if (threadIdx.x == 0) s_diff = 0;
-        __syncthreads();
-        if (fo >= 0) {
-            const int o0 = L.off[fo], n1 = L.npart[t - 1];
-            const int* pr = L.pred + L.off[t - 1];
-            for (int x = threadIdx.x; x < n1; x += NT) {
-                const int p = __ldcg(pr + x);
-                if (p >= o0 && p < o0 + no) taken[p - o0] = 1;
-            }
-        }
-        __syncthreads();
-        int nc = 0;
-        for (int f = fbeg; f <= fend; ++f) {
-            const int n = L.npart[f];
-            const unsigned char* ln = L.lnext + (size_t)f * cap_p;
-            const bool old = f == fo;
-            for (int i = threadIdx.x; i < n; i += NT) cpos[i] = (__ldcg(ln + i) || (old && taken[i])) ? 0 : 1;
-            __syncthreads();
-            const int k = block_scan_inplace_l<NT>(cpos, n, warp_tot, &s_total);
-            for (int i = threadIdx.x; i < n; i += NT)
-                if (!(__ldcg(ln + i) || (old && taken[i]))) ch[nc + cpos[i]] = f * cap_p + i;
-            nc += k;
-            __syncthreads();
-        }
-        int* ml = L.mlist + (size_t)t * L.cap_m;
-        const int oldn = __ldcg(L.mcount + t);
-        if (nc > L.cap_m) { if (threadIdx.x == 0) atomicOr(L.err, ERR_MEM_OVERFLOW); continue; }
-        if (oldn != nc && threadIdx.x == 0) s_diff = 1;
-        for (int j = threadIdx.x; j < nc; j += NT)
-            if (__ldcg(ml + j) != ch[j]) s_diff = 1;
-        __syncthreads();
-        if (s_diff) {
-            for (int j = threadIdx.x; j < nc; j += NT) ml[j] = ch[j];
-            if (threadIdx.x == 0) {
-                L.mcount[t] = nc;
-                atomicOr(L.dirty + t, wbit);
-                atomicAdd(ndirty, 1);
-            }
-        } else if (threadIdx.x == 0) {
-            atomicAnd(L.dirty + t, ~wbit);
-        }
-        __syncthreads();
     }
+    for (int t = L.tb + tid; t < L.te; t += nthr) L.fstamp[t] = 0;
 }
 
 // Trajectory roots (the first particle of each trajectory, compact index),
@@ -746,142 +660,192 @@ __device__ void roots_global(const LinkBufs& L) {
     }
 }
 
-__device__ void roots_body(const LinkBufs& L, cg::grid_group& grid) {
-    roots_local(L);
-    grid.sync();
-    roots_global(L);
+// rank of each new particle within its frame (linking.rs:470), a block per
+// frame
+__device__ void new_ranks(const LinkBufs& L) {
+    __shared__ int warp_tot[NTL / 32];
+    __shared__ int s_total;
+    for (int t = L.tb + blockIdx.x; t < L.te; t += gridDim.x) {
+        const int o = __ldg(L.off + t), n = __ldg(L.off + t + 1) - o;
+        int base = 0;
+        for (int i0 = 0; i0 < n; i0 += NTL) {
+            const int i = i0 + threadIdx.x;
+            const bool fresh = i < n && __ldcg(L.pred + o + i) < 0;
+            const int pos = block_excl_scan<NTL>(fresh ? 1 : 0, warp_tot, &s_total);
+            if (i < n) L.newrank[o + i] = fresh ? base + pos : -1;
+            base += s_total;
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) L.newcount[t] = base;
+    }
 }
 
-// The whole linker in one cooperative launch: link every frame with M = {},
-// then alternate {trajectory roots, memory entries M(t), relink frames whose
-// M changed} until no M changes (at most T + 1 passes).  ndirty[k] counts
-// the frames changed by pass k (zeroed by the host).
-namespace {
 __device__ __forceinline__ unsigned long long gtimer() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-}  // namespace
 
-// phase_ns: [0] first linking, [1] roots, [2] memory entries, [3] relinking
-// (nanoseconds summed over passes, stamped by block 0 after each barrier).
-// The memory entries of every frame are computed from one consistent state
-// (a grid barrier before and after): a frame read while another block
-// relinks its neighbour could see that neighbour's links half rewritten,
-// which inflates the entries and the subnetworks they form.
-template <int NT>
-__global__ void __launch_bounds__(NT, NT == NTL ? 4 : 1) link_fixpoint_kernel(LinkBufs L, int memory, int max_passes, int rounds,
-                                                               int* ndirty, int* passes,
-                                                               unsigned long long* phase_ns) {
+// The linker over movies 0 .. nm - 1 (movie(m) gives the buffers): one grid
+// barrier per phase serves them all.  A movie without seeds in a pass is at
+// its fixed point (movies are independent) and later passes skip it.
+// stat: [0..3] nanoseconds of the first linking, roots, memory entries and
+// relinking (summed over passes, stamped by block 0 after each barrier);
+// [4 + k - 1] frames with seeds in pass k <= 8.
+template <class M>
+__device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_passes, int* passes,
+                                              unsigned long long* stat) {
     cg::grid_group grid = cg::this_grid();
+    const int nthr = gridDim.x * NTL;
+    const int tid0 = blockIdx.x * NTL + threadIdx.x;
+    // few items: lane 0 of a warp in every block first
+    const int vt0 = ((threadIdx.x & 31) * (NTL / 32) + (threadIdx.x >> 5)) * gridDim.x + blockIdx.x;
     const bool stamp = blockIdx.x == 0 && threadIdx.x == 0;
     unsigned long long t0 = stamp ? gtimer() : 0, acc[4] = {0, 0, 0, 0};
-    link_frames_body<NT>(L, 0, blockIdx.x, gridDim.x);
-    int k = 0;
-    if (memory > 0 && L.te > 2) {
-        // memory 1 or 2: the entries need no trajectory roots
-        // (memory_body_short), so the roots are computed once, at the end
-        const bool short_mem = memory <= 2;
-        for (k = 1; k <= max_passes; ++k) {
-            grid.sync();
-            if (stamp) { const unsigned long long t = gtimer(); acc[k == 1 ? 0 : 3] += t - t0; t0 = t; }
-            if (!short_mem) {
-                roots_body(L, grid);
-                grid.sync();
-            }
-            if (stamp) { const unsigned long long t = gtimer(); acc[1] += t - t0; t0 = t; }
-            if (short_mem) memory_body_short<NT>(L, memory, ndirty + k, k, blockIdx.x, gridDim.x);
-            else memory_body<NT>(L, memory, ndirty + k, 1 << (k & 1), blockIdx.x, gridDim.x);
-            grid.sync();
-            if (stamp) { const unsigned long long t = gtimer(); acc[2] += t - t0; t0 = t; }
-            if (*(volatile int*)(ndirty + k) == 0) break;
-            link_frames_body<NT>(L, 1 << (k & 1), blockIdx.x, gridDim.x);
+    auto tick = [&](int i) {
+        if (stamp) { const unsigned long long t = gtimer(); acc[i] += t - t0; t0 = t; }
+    };
+    // a movie's items start on the threads after the previous movie's
+    auto rot = [&](int id, int& r, const LinkBufs& L) {
+        const int v = id - r < 0 ? id - r + nthr : id - r;
+        r = (int)(((long long)r + __ldg(L.off + L.te) - __ldg(L.off + L.tb)) % nthr);
+        return v;
+    };
+    bool any_mem = false, any_long = false;
+    for (int m = 0; m < nm; ++m) {
+        const int mem = movie(m).memory;
+        any_mem |= mem > 0;
+        any_long |= mem > 2;
+    }
+    if (any_mem) {
+        int r = 0;
+        for (int m = 0; m < nm; ++m) {
+            const LinkBufs L = movie(m);
+            const int id = rot(tid0, r, L);
+            if (L.memory > 0) window_begin(L, id, nthr);
+        }
+        grid.sync();
+    }
+    {
+        int r = 0;
+        for (int m = 0; m < nm; ++m) {
+            const LinkBufs L = movie(m);
+            link_all(L, rot(tid0, r, L), nthr);
         }
     }
     grid.sync();
-    if (stamp) { const unsigned long long t = gtimer(); acc[k <= 1 ? 0 : 3] += t - t0; t0 = t; }
-    roots_body(L, grid);
-    grid.sync();  // so that the last stamp covers every block's walk
-    if (stamp) {
-        acc[1] += gtimer() - t0;
-        *passes = max(*passes, k);  // several launches (frame windows) add up
-        for (int i = 0; i < 4; ++i) phase_ns[i] += acc[i];
-    }
-    (void)rounds;
-}
-
-template __global__ void link_fixpoint_kernel<NTL>(LinkBufs, int, int, int, int*, int*, unsigned long long*);
-template __global__ void link_fixpoint_kernel<NTL_BIG>(LinkBufs, int, int, int, int*, int*, unsigned long long*);
-
-// Host side: the kernel for `nt` threads per block (256 or 1024), its
-// resident blocks per SM, and a cooperative launch of it.
-static const void* link_fixpoint_fn(int nt) {
-    return nt == NTL_BIG ? (const void*)link_fixpoint_kernel<NTL_BIG> : (const void*)link_fixpoint_kernel<NTL>;
-}
-
-cudaError_t link_fixpoint_occupancy(int nt, int smem, int* per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(link_fixpoint_fn(nt), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, link_fixpoint_fn(nt), nt, smem);
-}
-
-cudaError_t launch_link_fixpoint(int nt, int grid, void** args, int smem, cudaStream_t st) {
-    return cudaLaunchCooperativeKernel(link_fixpoint_fn(nt), dim3(grid), dim3(nt), args, smem, st);
-}
-
-// Several movies in one cooperative launch (the batched path): every phase
-// of link_fixpoint_kernel runs over the frames of all movies, movie m's
-// frame t on block (fstart[m] + t) mod gridDim.x so that short movies spread
-// over the grid; one grid barrier per phase serves all movies, and the
-// fixed point ends when no movie's memory entries change.  Ls[m] share one
-// per-block scratch pool (slot strides st_*), since a block links one frame
-// at a time.
-__global__ void __launch_bounds__(NTL, 4) link_fixpoint_multi_kernel(const LinkBufs* Ls, const int* memory,
-                                                                     const int* fstart, int nm, int max_passes,
-                                                                     int* ndirty, int* passes) {
-    cg::grid_group grid = cg::this_grid();
-    const int G = gridDim.x;
-    auto t0_of = [&](int m) { const int s = fstart[m] % G; return ((int)blockIdx.x - s + G) % G; };
-    bool any_mem = false;
-    for (int m = 0; m < nm; ++m) {
-        link_frames_body<NTL>(Ls[m], 0, t0_of(m), G);
-        any_mem |= memory[m] > 0 && Ls[m].T > 2;
-    }
-    // ndirty[k * nm + m]: frames of movie m changed by pass k.  A movie
-    // whose memory entries did not change in a pass is at its fixed point
-    // (movies are independent): later passes skip it.
-    auto active = [&](int m, int k) {
-        return memory[m] > 0 && Ls[m].T > 2 && (k == 1 || *(volatile int*)(ndirty + (k - 1) * nm + m) > 0);
+    auto deferred = [&](int k) {
+        bool any = false;
+        for (int m = 0; m < nm; ++m) any |= __ldcg(movie(m).ctr + (k & 3) * 4 + 2) > 0;
+        if (!any) return;
+        for (int m = 0; m < nm; ++m) link_deferred(movie(m), k);
+        grid.sync();
     };
+    deferred(0);
+    tick(0);
     int k = 0;
     if (any_mem) {
+        auto active = [&](const LinkBufs& L, int kk) {
+            return L.memory > 0 && L.te > 2 && (kk == 1 || __ldcg(L.ctr + ((kk - 1) & 3) * 4) > 0);
+        };
         for (k = 1; k <= max_passes; ++k) {
-            grid.sync();
-            for (int m = 0; m < nm; ++m)
-                if (active(m, k) && memory[m] > 2) roots_local(Ls[m]);
-            grid.sync();
-            for (int m = 0; m < nm; ++m)
-                if (active(m, k) && memory[m] > 2) roots_global(Ls[m]);
-            grid.sync();
+            bool longs = false;
+            if (any_long)
+                for (int m = 0; m < nm; ++m) {
+                    const LinkBufs L = movie(m);
+                    longs |= L.memory > 2 && active(L, k);
+                }
+            if (longs) {
+                auto each = [&](auto&& fn) {
+                    for (int m = 0; m < nm; ++m) {
+                        const LinkBufs L = movie(m);
+                        if (L.memory > 2 && active(L, k)) fn(L);
+                    }
+                    grid.sync();
+                };
+                each([&](const LinkBufs& L) { roots_local(L); });
+                each([&](const LinkBufs& L) { roots_global(L); });
+                tick(1);
+                each([&](const LinkBufs& L) { members_chain(L, tid0, nthr); });
+                each([&](const LinkBufs& L) { members_present(L, tid0, nthr); });
+            }
+            int r = 0;
             for (int m = 0; m < nm; ++m) {
-                if (!active(m, k)) continue;
-                if (memory[m] <= 2) memory_body_short<NTL>(Ls[m], memory[m], ndirty + k * nm + m, k, t0_of(m), G);
-                else memory_body<NTL>(Ls[m], memory[m], ndirty + k * nm + m, 1 << (k & 1), t0_of(m), G);
+                const LinkBufs L = movie(m);
+                const int id = rot(vt0, r, L);
+                // the counters of pass k + 1 were last read in pass k - 2
+                if (stamp)
+                    for (int q = 0; q < 4; ++q) L.ctr[((k + 1) & 3) * 4 + q] = 0;
+                if (!active(L, k)) continue;
+                if (L.memory <= 2) members_short(L, k, k == 1 ? tid0 : id, nthr);
+                else members_long(L, k, tid0, nthr);
             }
             grid.sync();
             int total = 0;
-            for (int m = 0; m < nm; ++m) total += *(volatile int*)(ndirty + k * nm + m);
+            for (int m = 0; m < nm; ++m) total += __ldcg(movie(m).ctr + (k & 3) * 4);
+            tick(2);
+            if (stamp && k <= 8) {
+                unsigned long long nf = 0;
+                for (int m = 0; m < nm; ++m) nf += (unsigned)__ldcg(movie(m).ctr + (k & 3) * 4 + 3);
+                stat[4 + k - 1] += nf;
+            }
             if (total == 0) break;
-            for (int m = 0; m < nm; ++m)
-                if (*(volatile int*)(ndirty + k * nm + m) > 0) link_frames_body<NTL>(Ls[m], 1 << (k & 1), t0_of(m), G);
+            r = 0;
+            for (int m = 0; m < nm; ++m) {
+                const LinkBufs L = movie(m);
+                const int id = rot(vt0, r, L);
+                if (!active(L, k)) continue;
+                if (L.memory > 2) members_clear(L, tid0, nthr);
+                link_seeds(L, k, id, nthr);
+            }
+            grid.sync();
+            deferred(k);
+            tick(3);
         }
     }
+    for (int m = 0; m < nm; ++m) {
+        const LinkBufs L = movie(m);
+        roots_local(L);
+        new_ranks(L);
+    }
     grid.sync();
-    for (int m = 0; m < nm; ++m) roots_local(Ls[m]);
-    grid.sync();
-    for (int m = 0; m < nm; ++m) roots_global(Ls[m]);
-    if (blockIdx.x == 0 && threadIdx.x == 0) *passes = k;
+    for (int m = 0; m < nm; ++m) roots_global(movie(m));
+    if (stamp) {
+        acc[1] += gtimer() - t0;
+        *passes = max(*passes, k);  // several launches (frame windows) add up
+        for (int i = 0; i < 4; ++i) stat[i] += acc[i];
+    }
+}
+}  // namespace
+
+// One movie (or one frame window of it) in one cooperative launch.
+__global__ void __launch_bounds__(NTL, 4) link_fixpoint_kernel(const __grid_constant__ LinkBufs L, int max_passes,
+                                                               int* passes, unsigned long long* stat) {
+    link_fixpoint([&](int) -> const LinkBufs& { return L; }, 1, max_passes, passes, stat);
+}
+
+// Several movies in one cooperative launch (the batched path).
+__global__ void __launch_bounds__(NTL, 4) link_fixpoint_multi_kernel(const LinkBufs* Ls, int nm, int max_passes,
+                                                                     int* passes, unsigned long long* stat) {
+    link_fixpoint([&](int m) { return Ls[m]; }, nm, max_passes, passes, stat);
+}
+
+cudaError_t link_blocks_per_sm(bool multi, int* per_sm) {
+    const void* fn = multi ? (const void*)link_fixpoint_multi_kernel : (const void*)link_fixpoint_kernel;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, NTL, 0);
+}
+
+cudaError_t launch_link(const LinkBufs& L, int max_passes, int* passes, unsigned long long* stat, int grid,
+                        cudaStream_t st) {
+    LinkBufs a = L;
+    void* args[] = {&a, &max_passes, &passes, &stat};
+    return cudaLaunchCooperativeKernel((const void*)link_fixpoint_kernel, dim3(grid), dim3(NTL), args, 0, st);
+}
+
+cudaError_t launch_link_multi(const LinkBufs* d_L, int nm, int max_passes, int* passes, unsigned long long* stat,
+                              int grid, cudaStream_t st) {
+    void* args[] = {&d_L, &nm, &max_passes, &passes, &stat};
+    return cudaLaunchCooperativeKernel((const void*)link_fixpoint_multi_kernel, dim3(grid), dim3(NTL), args, 0, st);
 }
 
 }  // namespace gt

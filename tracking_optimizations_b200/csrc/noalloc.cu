@@ -242,7 +242,7 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
     std::memset(&b, 0, sizeof(b));
     b.frames = d_frame;
     b.T = 1;
-    b.cap_c = cap_c; b.cap_p = cap_c; b.cap_m = 1; b.cap_e = 1;
+    b.cap_c = cap_c; b.cap_p = cap_c;
     b.cand = c.take<Cand>(cap_c);
     b.fcount = c.take<int>(1);
     b.rowcnt = c.take<int>((size_t)H * lp.ntx);
