@@ -380,7 +380,8 @@ struct Work {
     // linker (LinkBufs)
     float2* gpos;
     unsigned *lnk, *mm, *pres;
-    int *stamp, *rstamp, *seedq, *recq, *deferq, *gframe, *head, *nextc, *fstamp, *big;
+    int *stamp, *rstamp, *seedq, *recq, *deferq, *gframe, *cstamp, *head, *fstamp, *big;
+    int4* ent;
     unsigned long long* lstat;  // 4 phase times, 8 frame counts, then the linker's counters (16 ints)
     float* out;
 };
@@ -451,8 +452,11 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->recq = c.take<int>(nm);
     w->deferq = c.take<int>(np);
     w->gframe = c.take<int>(nl);
-    w->head = c.take<int>(nl);
-    w->nextc = c.take<int>(nl);
+    w->cstamp = c.take<int>(nl);
+    size_t nh = 1;
+    while (nh < nl) nh <<= 1;
+    w->head = c.take<int>(nh);
+    w->ent = c.take<int4>(nl);
     w->pres = c.take<unsigned>(nl * nw);
     w->fstamp = c.take<int>(T);
     w->lstat = c.take<unsigned long long>(12 + 8);
@@ -492,7 +496,8 @@ LinkBufs link_bufs(const Plan& P, const Work& w, long long budget) {
     L.pred = w.pred; L.lnk = w.lnk; L.mm = w.mm; L.stamp = w.stamp; L.rstamp = w.rstamp;
     L.seedq = w.seedq; L.recq = w.recq; L.deferq = w.deferq;
     L.newrank = w.newrank; L.newcount = w.newcount; L.root = w.root; L.lroot = w.lroot;
-    L.gframe = w.gframe; L.head = w.head; L.nextc = w.nextc; L.pres = w.pres;
+    L.gframe = w.gframe; L.cstamp = w.cstamp; L.head = w.head; L.ent = w.ent; L.pres = w.pres;
+    while ((1 << L.fshift) < L.memory) ++L.fshift;
     L.fstamp = w.fstamp; L.ctr = (int*)(w.lstat + 12); L.err = w.err;
     L.budget = budget;
     L.nslot = P.nslot; L.big_d = P.big_d; L.big_s = P.big_s; L.big_e = P.big_e;

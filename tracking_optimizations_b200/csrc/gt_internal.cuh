@@ -130,15 +130,18 @@ struct LinkBufs {
     int* stamp;           // last pass in which the particle was a seed
     int* rstamp;          // last pass that listed it for a membership check
     int* seedq;           // slab handles of the pass's seeds
-    int* recq;            // particles whose linked bits the pass changed
+    int* recq;            // particles whose linked bits the pass changed (memory 1, 2),
+                          // or those of the trajectories that it changed
     int* deferq;          // seeds whose component is resolved in scratch
     int* newrank;         // rank among new particles of its frame
     int* root;
     int* lroot;           // where the pred chain enters the particle's chunk
     // memory >= 3
     int* gframe;          // frame
-    int* head;            // by root: list of its unused particles
-    int* nextc;
+    int* cstamp;          // by root: pass that evaluates the trajectory again
+    int* head;            // lists of unused particles, hashed by (root, frame >> fshift)
+    int4* ent;            // their entries: root, frame, next
+    int fshift;           // 2^fshift >= memory frames
     unsigned* pres;       // as mm: the id is present in the frame 1 + 32 w + b later
     int* newcount;        // T
     int* fstamp;          // T: last pass with a seed in the frame

@@ -41,6 +41,8 @@ namespace gt {
 
 namespace {
 constexpr int NTL = 256;  // threads of a linker block
+constexpr int NEAR = 2;   // candidates loaded at once by a thread
+
 
 __device__ __forceinline__ bool within_r(float qy, float qx, float iy, float ix, float r, float* dist) {
     // kd-tree box pre-filter + linking.rs:91-100 distance (dest - source)
@@ -85,10 +87,20 @@ __device__ __forceinline__ bool near(const LinkBufs& L, int f, float qy, float q
     }
     const size_t base = (size_t)f * L.cap_p;
     const int n01 = n[0] + n[1], total = n01 + n[2];
-    for (int s = 0; s < total; ++s) {
-        const size_t at = base + (s < n[0] ? a[0] + s : s < n01 ? a[1] + (s - n[0]) : a[2] + (s - n01));
-        const float2 p = __ldg(L.gpos + at);
-        if (!fn(__ldg(L.gidx + at), p.x, p.y)) return false;
+    // a few candidates' loads in flight at once
+    for (int s = 0; s < total; s += NEAR) {
+        float2 p[NEAR];
+        int id[NEAR];
+#pragma unroll
+        for (int u = 0; u < NEAR; ++u) {
+            const int q = min(s + u, total - 1);
+            const size_t at = base + (q < n[0] ? a[0] + q : q < n01 ? a[1] + (q - n[0]) : a[2] + (q - n01));
+            p[u] = __ldg(L.gpos + at);
+            id[u] = __ldg(L.gidx + at);
+        }
+#pragma unroll
+        for (int u = 0; u < NEAR; ++u)
+            if (s + u < total && !fn(id[u], p[u].x, p[u].y)) return false;
     }
     return true;
 }
@@ -105,20 +117,43 @@ __device__ __forceinline__ int push_slot(int* ctr) {
 
 // One component: destinations (index in frame t), sources (keys that order
 // them as linking.rs:244-259 does: frame t-1 by index, then the memory
-// entries by (frame, index): cap_p + slab handle) and their edges.  Most
-// components fit the thread's own arrays; larger ones are resolved by one
-// thread per block with arrays in global memory (LinkBufs::big).
+// entries by (frame, index): cap_p + slab handle) and their edges.  At most 32
+// destinations and 32 sources fit a thread's local arrays (SmallComp, the first
+// linking) or a warp (WarpComp, the passes); larger components are resolved by
+// one thread per block with arrays in global memory (LinkBufs::big).
+constexpr int CAP_N = 32, CAP_E = 112;
+
+// Set of at most 32 sources or destinations.
+struct BitSet {
+    unsigned m = 0;
+    __device__ bool has(int i) const { return (m >> i) & 1u; }
+    __device__ void add(int i) { m |= 1u << i; }
+    __device__ void del(int i) { m &= ~(1u << i); }
+    __device__ void clear(int) { m = 0; }
+};
+
+struct ArraySet {
+    int* p;
+    __device__ bool has(int i) const { return p[i] != 0; }
+    __device__ void add(int i) { p[i] = 1; }
+    __device__ void del(int i) { p[i] = 0; }
+    __device__ void clear(int n) {
+        for (int i = 0; i < n; ++i) p[i] = 0;
+    }
+};
+
 struct SmallComp {
-    static constexpr int MD = 16, MS = 16, ME = 48;
-    int D[MD];
-    unsigned S[MS];
-    float ew[ME], dw[ME];
-    unsigned char ed[ME], es[ME], dsrc[ME];
-    unsigned char doff[MD + 1], path[MD], oi[MD], used[MS], vis[MD], stk[MD + MS];
-    signed char cur[MD], best[MD];
-    __device__ int md() const { return MD; }
-    __device__ int ms() const { return MS; }
-    __device__ int me() const { return ME; }
+    int D[CAP_N];
+    unsigned S[CAP_N];
+    float ew[CAP_E], dw[CAP_E];
+    unsigned char ed[CAP_E], es[CAP_E], dsrc[CAP_E];
+    unsigned char doff[CAP_N + 1], path[CAP_N], oi[CAP_N], stk[2 * CAP_N];
+    signed char cur[CAP_N], best[CAP_N];
+    __device__ int md() const { return CAP_N; }
+    __device__ int ms() const { return CAP_N; }
+    __device__ int me() const { return CAP_E; }
+    __device__ BitSet dset() { return BitSet(); }
+    __device__ BitSet sset() { return BitSet(); }
 };
 
 struct BigComp {
@@ -130,6 +165,8 @@ struct BigComp {
     __device__ int md() const { return cd; }
     __device__ int ms() const { return cs; }
     __device__ int me() const { return ce; }
+    __device__ ArraySet dset() { return ArraySet{vis}; }
+    __device__ ArraySet sset() { return ArraySet{used}; }
 };
 
 __device__ __forceinline__ BigComp big_comp(const LinkBufs& L, int slot) {
@@ -146,61 +183,101 @@ __device__ __forceinline__ BigComp big_comp(const LinkBufs& L, int slot) {
     return b;
 }
 
+// DFS preorder of the destinations from `first` (linking.rs:316-342) over
+// the per-destination lists: neighbours in ascending order, so the next node
+// is the smallest one not yet visited.  Returns the number of destinations.
+template <class C>
+__device__ int dfs_order(C& c, int first, int nd, int ns, int ne) {
+    auto vis = c.dset();
+    auto used = c.sset();
+    vis.clear(nd);
+    used.clear(ns);
+    int top = 1, np = 0;
+    c.stk[0] = first;
+    vis.add(first);
+    c.path[np++] = first;
+    while (top > 0) {
+        const int node = c.stk[top - 1];
+        int next = -1;
+        if (node < nd) {
+            for (int z = c.doff[node]; z < c.doff[node + 1]; ++z)
+                if (!used.has(c.dsrc[z])) { next = c.dsrc[z]; break; }
+            if (next >= 0) {
+                used.add(next);
+                next += nd;
+            }
+        } else {
+            const int s = node - nd;
+            for (int e = 0; e < ne; ++e)
+                if (c.es[e] == s && !vis.has(c.ed[e]) && (next < 0 || c.D[c.ed[e]] < c.D[next])) next = c.ed[e];
+            if (next >= 0) {
+                vis.add(next);
+                c.path[np++] = next;
+            }
+        }
+        if (next < 0) --top;
+        else c.stk[top++] = next;
+    }
+    return np;
+}
+
 // Exhaustive search of one subnet (linking.rs:390-452): destinations in DFS
 // order (path); sources are chosen through the per-destination lists
 // (ascending source order), null costs r^2.  Returns false when the
 // option-trial budget is exhausted.
 template <class C>
-__device__ bool solve_subnet(C& c, int nd, long long budget, float null_cost) {
+__device__ bool solve_subnet(C& c, int nd, int ns, long long budget, float null_cost) {
+    auto used = c.sset();
+    used.clear(ns);
     float score = 0.f, best = CUDART_INF_F;
     long long trials = 0;
-    int l = 0;
-    c.oi[0] = 0;
-    bool after_child = false;
+    int l = 0, o = 0, d0 = 0, nreal = 0;  // level, its option, its list
+    auto level = [&](int q) {
+        const int d = c.path[q];
+        d0 = c.doff[d];
+        nreal = c.doff[d + 1] - d0;
+    };
+    level(0);
     while (true) {
-        const int d = c.path[l];
-        const int d0 = c.doff[d];
-        const int nopt = c.doff[d + 1] - d0 + 1;
-        if (after_child) {
-            // child returned: undo this level's option and advance
-            const int o = c.oi[l];
-            const float w = (o == nopt - 1) ? null_cost : c.dw[d0 + o];
-            if (o != nopt - 1) c.used[c.dsrc[d0 + o]] = 0;
-            score -= w;
-            c.oi[l] = o + 1;
-            after_child = false;
-            continue;
-        }
-        const int o = c.oi[l];
-        if (o >= nopt || score > best) {  // loop exhausted, or early return
+        if (o > nreal || score > best) {  // options exhausted, or early return
             if (l == 0) break;
-            --l;
-            after_child = true;
+            level(--l);
+            // child returned: undo this level's option and advance
+            o = c.oi[l];
+            float w = null_cost;
+            if (o < nreal) {
+                w = c.dw[d0 + o];
+                used.del(c.dsrc[d0 + o]);
+            }
+            score -= w;
+            ++o;
             continue;
         }
         if (++trials > budget) return false;
-        const bool is_null = (o == nopt - 1);
-        const float w = is_null ? null_cost : c.dw[d0 + o];
-        score += w;
-        if (!is_null) {
-            const int s = c.dsrc[d0 + o];
-            if (c.used[s]) { score -= w; c.oi[l] = o + 1; continue; }
-            c.used[s] = 1;
-            c.cur[l] = s;
-        } else {
-            c.cur[l] = -1;
+        float w = null_cost;
+        int s = -1;
+        if (o < nreal) {
+            w = c.dw[d0 + o];
+            s = c.dsrc[d0 + o];
         }
+        score += w;
+        if (s >= 0) {
+            if (used.has(s)) { score -= w; ++o; continue; }
+            used.add(s);
+        }
+        c.cur[l] = s;
         if (l == nd - 1) {
             if (score < best) {
                 best = score;
                 for (int q = 0; q < nd; ++q) c.best[q] = c.cur[q];
             }
-            if (!is_null) c.used[c.cur[l]] = 0;
+            if (s >= 0) used.del(s);
             score -= w;
-            c.oi[l] = o + 1;
+            ++o;
         } else {
-            ++l;
-            c.oi[l] = 0;
+            c.oi[l] = o;
+            level(++l);
+            o = 0;
         }
     }
     return true;
@@ -223,6 +300,43 @@ __device__ __forceinline__ void mark_linked(const LinkBufs& L, int src, int fs, 
         if (k > 0 && L.memory <= 2 && atomicExch(L.rstamp + src, k) != k)
             L.recq[push_slot(L.ctr + (k & 3) * 4 + 1)] = src;
     }
+}
+
+// The compact index of source `key` (-1: none) of frame t and its frame.
+__device__ __forceinline__ int source_of(const LinkBufs& L, long long key, int t, int* fs) {
+    *fs = t - 1;
+    if (key < 0) return -1;
+    unsigned h = (unsigned)key;
+    if (h >= (unsigned)L.cap_p) {
+        h -= (unsigned)L.cap_p;
+        *fs = (int)(h / (unsigned)L.cap_p);
+        h -= (unsigned)(*fs * L.cap_p);
+    }
+    return __ldg(L.off + *fs) + (int)h;
+}
+
+// Destination g (frame t) gets source `key`: give_up releases its former
+// source if that is another, take_up writes the link.
+__device__ __forceinline__ void give_up(const LinkBufs& L, long long key, int g, int t, int k) {
+    int fs;
+    const int src = source_of(L, key, t, &fs);
+    const int old = __ldcg(L.pred + g);
+    if (old < 0 || old == src) return;
+    int fo = t - 1;
+    while (__ldg(L.off + fo) > old) --fo;
+    mark_linked(L, old, fo, t, k, false);
+}
+
+__device__ __forceinline__ void take_up(const LinkBufs& L, long long key, int g, int t, int k) {
+    int fs;
+    const int src = source_of(L, key, t, &fs);
+    if (k > 0 && __ldcg(L.pred + g) == src) return;
+    L.pred[g] = src;
+    if (k > 0 && L.memory > 2) {  // the trajectories that the change touches
+        L.cstamp[__ldcg(L.root + g)] = k + 1;
+        if (src >= 0) L.cstamp[__ldcg(L.root + src)] = k + 1;
+    }
+    if (src >= 0 && L.memory > 0) mark_linked(L, src, fs, t, k, true);
 }
 
 // Explores the component of destination d of frame t and resolves it.
@@ -298,13 +412,13 @@ __device__ int link_component(const LinkBufs& L, C& c, int t, int d, int k) {
         for (int q = 0; q <= nd; ++q) c.doff[q] = 0;
         for (int e = 0; e < ne; ++e) ++c.doff[c.ed[e] + 1];
         for (int q = 0; q < nd; ++q) c.doff[q + 1] = c.doff[q + 1] + c.doff[q];
-        for (int q = 0; q < nd; ++q) c.vis[q] = 0;
+        for (int q = 0; q < nd; ++q) c.path[q] = 0;  // entries so far
         for (int e = 0; e < ne; ++e) {
             const int q = c.ed[e];
             const int s = c.es[e];
             const float w = c.ew[e];
-            int z = c.doff[q] + c.vis[q];
-            c.vis[q] = c.vis[q] + 1;
+            int z = c.doff[q] + c.path[q];
+            c.path[q] = c.path[q] + 1;
             while (z > c.doff[q] && c.S[c.dsrc[z - 1]] > c.S[s]) {
                 c.dsrc[z] = c.dsrc[z - 1];
                 c.dw[z] = c.dw[z - 1];
@@ -313,76 +427,327 @@ __device__ int link_component(const LinkBufs& L, C& c, int t, int d, int k) {
             c.dsrc[z] = s;
             c.dw[z] = w;
         }
-        // DFS preorder from the smallest destination (linking.rs:316-342):
-        // neighbours in ascending order, so the next node is the smallest
-        // one not yet visited
         int first = 0;
-        for (int q = 0; q < nd; ++q) {
-            c.vis[q] = 0;
+        for (int q = 1; q < nd; ++q)
             if (c.D[q] < c.D[first]) first = q;
-        }
-        for (int s = 0; s < ns; ++s) c.used[s] = 0;
-        int top = 1;
-        np = 0;
-        c.stk[0] = first;
-        c.vis[first] = 1;
-        c.path[np++] = first;
-        while (top > 0) {
-            const int node = c.stk[top - 1];
-            int next = -1;
-            if (node < nd) {
-                for (int z = c.doff[node]; z < c.doff[node + 1]; ++z)
-                    if (!c.used[c.dsrc[z]]) { next = c.dsrc[z]; break; }
-                if (next >= 0) {
-                    c.used[next] = 1;
-                    next += nd;
-                }
-            } else {
-                const int s = node - nd;
-                for (int e = 0; e < ne; ++e)
-                    if (c.es[e] == s && !c.vis[c.ed[e]] && (next < 0 || c.D[c.ed[e]] < c.D[next])) next = c.ed[e];
-                if (next >= 0) {
-                    c.vis[next] = 1;
-                    c.path[np++] = next;
-                }
-            }
-            if (next < 0) --top;
-            else c.stk[top++] = next;
-        }
-        for (int s = 0; s < ns; ++s) c.used[s] = 0;
+        np = dfs_order(c, first, nd, ns, ne);
         for (int q = 0; q < np; ++q) c.best[q] = -1;
-        if (!solve_subnet(c, np, L.budget, r * r)) atomicOr(L.err, ERR_SUBNET_BUDGET);
+        if (!solve_subnet(c, np, ns, L.budget, r * r)) atomicOr(L.err, ERR_SUBNET_BUDGET);
     }
     // the links: first every source given up, then every source taken (a
     // source that changes destination ends up linked)
-    for (int pass = 0; pass < 2; ++pass) {
-        if (pass == 0 && k == 0) continue;
-        for (int q = 0; q < np; ++q) {
-            const int g = offt + c.D[c.path[q]];
-            const int s = c.best[q];
-            int fs = t - 1, src = -1;
-            if (s >= 0) {
-                unsigned h = c.S[s];
-                if (h >= (unsigned)L.cap_p) {
-                    h -= (unsigned)L.cap_p;
-                    fs = (int)(h / (unsigned)L.cap_p);
-                    h -= (unsigned)(fs * L.cap_p);
+    if (k > 0)
+        for (int q = 0; q < np; ++q) give_up(L, c.best[q] < 0 ? -1 : (long long)c.S[c.best[q]], offt + c.D[c.path[q]], t, k);
+    for (int q = 0; q < np; ++q) take_up(L, c.best[q] < 0 ? -1 : (long long)c.S[c.best[q]], offt + c.D[c.path[q]], t, k);
+    return COMP_DONE;
+}
+
+// A pass's seeds are resolved by a warp each: what a thread does one
+// dependent load after the other (up to 100k cycles for a component of 3
+// destinations and 5 sources with memory 3) the lanes do side by side.  The
+// nodes of a search level are expanded together: their cell ranges in all
+// frames, then the ranges' particles, then the membership bits.  Lane i holds
+// destination i and source i; edges go through shared memory.
+struct WarpComp {
+    float ew[CAP_E], w[CAP_E];  // edges as found, then by search level
+    unsigned char ed[CAP_E], es[CAP_E], s[CAP_E];
+};
+
+// Row q of the 3 x 3 cells around (y, x) in frame f: its first slab index and
+// particle count (0 for rows outside the grid).
+__device__ __forceinline__ void cell_row(const LinkBufs& L, int f, int q, float y, float x, unsigned* a, int* n) {
+    const int cy = clampi((int)floorf(y * L.inv_g), 0, L.ncy - 1) + q - 1;
+    const int cx = clampi((int)floorf(x * L.inv_g), 0, L.ncx - 1);
+    *a = 0;
+    *n = 0;
+    if (cy < 0 || cy >= L.ncy) return;
+    const int* gs = L.gstart + (size_t)f * ((size_t)L.ncx * L.ncy + 1) + (size_t)cy * L.ncx;
+    const int a0 = __ldg(gs + max(cx - 1, 0)), a1 = __ldg(gs + min(cx + 1, L.ncx - 1) + 1);
+    *a = (unsigned)(f * L.cap_p + a0);
+    *n = a1 - a0;
+}
+
+// fn(row, slab index in cell order) for the particles of the rows held by
+// lanes [0, nrows) (first index a, count n), 32 particles at a time; row is -1
+// on lanes without one.  Stops when fn (uniform) returns false.
+template <class F>
+__device__ __forceinline__ bool each_in_rows(unsigned a, int n, int nrows, F&& fn) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int incl = lane < nrows ? n : 0;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(full, incl, d);
+        if (lane >= d) incl += v;
+    }
+    const int total = __shfl_sync(full, incl, 31);
+    for (int base = 0; base < total; base += 32) {
+        // the row of particle idx: the first whose inclusive sum exceeds it
+        // (binary search over the lanes)
+        const int idx = base + lane;
+        int row = 0;
+#pragma unroll
+        for (int b = 16; b > 0; b >>= 1)
+            if (__shfl_sync(full, incl, row + b - 1) <= idx) row += b;
+        row = min(row, nrows - 1);
+        const unsigned first = __shfl_sync(full, a, row);
+        const int before = __shfl_sync(full, incl - n, row);
+        if (!fn(idx < total ? row : -1, first + (unsigned)(idx - before))) return false;
+    }
+    return true;
+}
+
+// The component of seed d of frame t (t >= 1) in pass k >= 1; as
+// link_component.
+__device__ int link_component_warp(const LinkBufs& L, WarpComp& c, int t, int d, int k) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const float r = L.r;
+    const int offt = __ldg(L.off + t);
+    int myD = d;  // lane i: destination i, its position, source i, its position
+    float dy = __ldg(L.py + (size_t)t * L.cap_p + d), dx = __ldg(L.px + (size_t)t * L.cap_p + d);
+    unsigned myS = 0;
+    float sy = 0.f, sx = 0.f;
+    int nd = 1, ns = 0, ne = 0, qd = 0, qs = 0, res = COMP_DONE;
+    const int ngr = min(L.memory, t - 1) + 1;  // source frames t-1, t-2, ...
+    while (true) {
+        if (qd < nd) {
+            // 3 rows of cells in each source frame; several destinations at
+            // once while their rows fit the warp
+            const int nb = 3 * ngr <= 16 ? min(nd - qd, 32 / (3 * ngr)) : 1;
+            for (int j0 = 0; j0 < ngr; j0 += 10) {
+                const int per = 3 * min(10, ngr - j0);
+                const int mine = qd + min(lane / per, nb - 1);
+                const float y = __shfl_sync(full, dy, mine), x = __shfl_sync(full, dx, mine);
+                const int q = lane - (mine - qd) * per;
+                unsigned a = 0;
+                int n = 0;
+                if (lane < nb * per) cell_row(L, t - 1 - j0 - q / 3, q % 3, y, x, &a, &n);
+                const bool go = each_in_rows(a, n, nb * per, [&](int row, unsigned at) {
+                    const int node = max(row, 0) / per;
+                    const float y = __shfl_sync(full, dy, qd + node), x = __shfl_sync(full, dx, qd + node);
+                    unsigned key = 0;
+                    float w = 0.f;
+                    float2 p = make_float2(0.f, 0.f);
+                    bool hit = false;
+                    if (row >= 0) {
+                        const int j = j0 + (row - node * per) / 3, f = t - 1 - j;
+                        p = __ldg(L.gpos + at);
+                        const int i = __ldg(L.gidx + at);
+                        hit = within_r(p.x, p.y, y, x, r, &w);
+                        if (hit && j > 0) hit = in_memory(L, __ldg(L.off + f) + i, j);
+                        key = j == 0 ? (unsigned)i : (unsigned)L.cap_p + (unsigned)(f * L.cap_p + i);
+                    }
+                    for (unsigned m = __ballot_sync(full, hit); m; m &= m - 1) {
+                        const int b = __ffs(m) - 1;
+                        const unsigned kb = __shfl_sync(full, key, b);
+                        const float yb = __shfl_sync(full, p.x, b), xb = __shfl_sync(full, p.y, b);
+                        const unsigned same = __ballot_sync(full, lane < ns && myS == kb);
+                        int s = __ffs(same) - 1;
+                        if (!same) {
+                            if (ns == CAP_N) { res = COMP_BIG; return false; }
+                            s = ns++;
+                            if (lane == s) { myS = kb; sy = yb; sx = xb; }
+                        }
+                        if (ne == CAP_E) { res = COMP_BIG; return false; }
+                        if (lane == b) {
+                            c.ed[ne] = (unsigned char)(qd + node);
+                            c.es[ne] = (unsigned char)s;
+                            c.ew[ne] = w;
+                        }
+                        ++ne;
+                    }
+                    return true;
+                });
+                if (!go) return res;
+            }
+            qd += nb;
+        } else if (qs < ns) {
+            const int nb = min(ns - qs, 10);
+            const int mine = qs + min(lane / 3, nb - 1);
+            const float y = __shfl_sync(full, sy, mine), x = __shfl_sync(full, sx, mine);
+            unsigned a = 0;
+            int n = 0;
+            if (lane < 3 * nb) cell_row(L, t, lane % 3, y, x, &a, &n);
+            const bool go = each_in_rows(a, n, 3 * nb, [&](int row, unsigned at) {
+                const int node = qs + max(row, 0) / 3;
+                const float y = __shfl_sync(full, sy, node), x = __shfl_sync(full, sx, node);
+                int i = -1;
+                bool hit = false, smaller = false;
+                float2 p = make_float2(0.f, 0.f);
+                if (row >= 0) {
+                    p = __ldg(L.gpos + at);
+                    i = __ldg(L.gidx + at);
+                    float w;
+                    hit = within_r(y, x, p.x, p.y, r, &w);
+                    smaller = hit && i < d && __ldcg(L.stamp + offt + i) == k;
                 }
-                src = __ldg(L.off + fs) + (int)h;
-            }
-            if (pass == 0) {
-                const int old = __ldcg(L.pred + g);
-                if (old < 0 || old == src) continue;
-                int fo = t - 1;
-                while (__ldg(L.off + fo) > old) --fo;
-                mark_linked(L, old, fo, t, k, false);
-            } else {
-                if (k > 0 && __ldcg(L.pred + g) == src) continue;
-                L.pred[g] = src;
-                if (src >= 0 && L.memory > 0) mark_linked(L, src, fs, t, k, true);
-            }
+                if (__any_sync(full, smaller)) { res = COMP_SKIP; return false; }
+                for (unsigned m = __ballot_sync(full, hit); m; m &= m - 1) {
+                    const int b = __ffs(m) - 1;
+                    const int ib = __shfl_sync(full, i, b);
+                    const float yb = __shfl_sync(full, p.x, b), xb = __shfl_sync(full, p.y, b);
+                    if (__any_sync(full, lane < nd && myD == ib)) continue;
+                    if (nd == CAP_N) { res = COMP_BIG; return false; }
+                    if (lane == nd) { myD = ib; dy = yb; dx = xb; }
+                    ++nd;
+                }
+                return true;
+            });
+            if (!go) return res;
+            qs += nb;
+        } else {
+            break;
         }
     }
+    long long key = -1;  // lane i < nd: the source that destination mine gets
+    int mine = myD;
+    if (nd == 1 && ns <= 1) {
+        if (ns == 1) key = __shfl_sync(full, myS, 0);
+    } else {
+        // ranks: destinations by index, sources by key, so that the search's
+        // "ascending" is the order of bits
+        int rd = 0, rs = 0;
+        for (int q = 0; q < nd; ++q) rd += __shfl_sync(full, myD, q) < myD;
+        for (int q = 0; q < ns; ++q) rs += __shfl_sync(full, myS, q) < myS;
+        unsigned srcs = 0, dsts = 0;  // lane i: neighbours of destination i, of source i (ranks)
+        int sortD = 0, sortS = 0;     // the destination and the source of rank i
+        for (int q = 0; q < nd; ++q)
+            if (__shfl_sync(full, rd, q) == lane) sortD = q;
+        for (int q = 0; q < ns; ++q)
+            if (__shfl_sync(full, rs, q) == lane) sortS = q;
+        mine = __shfl_sync(full, myD, sortD);
+        const unsigned keyS = __shfl_sync(full, myS, sortS);
+        __syncwarp();
+        for (int e0 = 0; e0 < ne; e0 += 32) {
+            const int e = e0 + lane;
+            const int q = __shfl_sync(full, rd, e < ne ? c.ed[e] : 0), s = __shfl_sync(full, rs, e < ne ? c.es[e] : 0);
+            const int cnt = min(32, ne - e0);
+            for (int b = 0; b < cnt; ++b) {
+                const int qb = __shfl_sync(full, q, b), sb = __shfl_sync(full, s, b);
+                if (lane == qb) srcs |= 1u << sb;
+                if (lane == sb) dsts |= 1u << qb;
+            }
+        }
+        // DFS preorder from the smallest destination (linking.rs:316-342)
+        unsigned vd = 1u, vs = 0u;
+        int level = lane == 0 ? 0 : -1;  // lane i: level of destination i in the order
+        int np = 1, node = 0, top = 0;   // node < 32: destination, else source + 32
+        int stk = 0;                     // lane q: entry q of the stack (entries 32.. in stk2)
+        int stk2 = 0;
+        while (true) {
+            const bool isd = node < 32;
+            const unsigned nb = __shfl_sync(full, isd ? srcs : dsts, node & 31) & ~(isd ? vs : vd);
+            if (nb) {
+                const int x = __ffs(nb) - 1;
+                if (lane == (top & 31)) {
+                    if (top < 32) stk = node;
+                    else stk2 = node;
+                }
+                ++top;
+                if (isd) {
+                    vs |= 1u << x;
+                    node = x + 32;
+                } else {
+                    vd |= 1u << x;
+                    if (lane == x) level = np;
+                    ++np;
+                    node = x;
+                }
+            } else {
+                if (top == 0) break;
+                --top;
+                node = __shfl_sync(full, top < 32 ? stk : stk2, top & 31);
+            }
+        }
+        // the search's option lists: lane l holds level l's destination, the
+        // start of its list and its length
+        int dest = 0;
+        for (int q = 0; q < nd; ++q)
+            if (__shfl_sync(full, level, q) == lane) dest = q;
+        const unsigned lsrcs = __shfl_sync(full, srcs, dest);
+        const int deg = lane < nd ? __popc(lsrcs) : 0;
+        int start = deg;
+#pragma unroll
+        for (int q = 1; q < 32; q <<= 1) {
+            const int v = __shfl_up_sync(full, start, q);
+            if (lane >= q) start += v;
+        }
+        start -= deg;
+        for (int e0 = 0; e0 < ne; e0 += 32) {
+            const int e = e0 + lane;
+            const bool in = e < ne;
+            const int q = __shfl_sync(full, rd, in ? c.ed[e] : 0), s = __shfl_sync(full, rs, in ? c.es[e] : 0);
+            const int at = __shfl_sync(full, start, __shfl_sync(full, level, q));
+            const unsigned before = __shfl_sync(full, srcs, q) & ((1u << s) - 1u);
+            if (in) {
+                c.w[at + __popc(before)] = c.ew[e];
+                c.s[at + __popc(before)] = (unsigned char)s;
+            }
+        }
+        __syncwarp();
+        // exhaustive search (solve_subnet), every lane in step; lane l keeps
+        // level l's option
+        const float null_cost = r * r;
+        float score = 0.f, best = CUDART_INF_F;
+        unsigned used = 0;
+        int l = 0, o = 0, opt = -1, bopt = -1;
+        int l0 = __shfl_sync(full, start, 0), nreal = __shfl_sync(full, deg, 0);
+        long long trials = 0;
+        while (true) {
+            if (o > nreal || score > best) {
+                if (l == 0) break;
+                --l;
+                l0 = __shfl_sync(full, start, l);
+                nreal = __shfl_sync(full, deg, l);
+                o = __shfl_sync(full, opt, l);
+                float w = null_cost;
+                if (o < nreal) {
+                    w = c.w[l0 + o];
+                    used &= ~(1u << c.s[l0 + o]);
+                }
+                score -= w;
+                ++o;
+                continue;
+            }
+            if (++trials > L.budget) {
+                if (lane == 0) atomicOr(L.err, ERR_SUBNET_BUDGET);
+                break;
+            }
+            float w = null_cost;
+            unsigned bit = 0;
+            if (o < nreal) {
+                w = c.w[l0 + o];
+                bit = 1u << c.s[l0 + o];
+            }
+            score += w;
+            if (used & bit) { score -= w; ++o; continue; }
+            if (lane == l) opt = o;
+            if (l == nd - 1) {
+                if (score < best) {
+                    best = score;
+                    bopt = opt;
+                }
+                score -= w;
+                ++o;
+            } else {
+                used |= bit;
+                ++l;
+                l0 = __shfl_sync(full, start, l);
+                nreal = __shfl_sync(full, deg, l);
+                o = 0;
+            }
+        }
+        const bool real = lane < nd && bopt >= 0 && bopt < deg;
+        const unsigned got = __shfl_sync(full, keyS, real ? c.s[start + bopt] : 0);
+        if (real) key = got;
+        mine = __shfl_sync(full, mine, dest);
+    }
+    // every source given up before any is taken
+    if (lane < nd) give_up(L, key, offt + mine, t, k);
+    __syncwarp();
+    if (lane < nd) take_up(L, key, offt + mine, t, k);
+    __syncwarp();
     return COMP_DONE;
 }
 
@@ -397,15 +762,17 @@ __device__ void link_all(const LinkBufs& L, int tid, int nthr) {
     }
 }
 
-// Resolves the components of pass k's seeds.
-__device__ void link_seeds(const LinkBufs& L, int k, int vt, int nthr) {
+// Resolves the components of pass k's seeds, starting with a warp per block.
+__device__ void link_seeds(const LinkBufs& L, int k, int vw, int nwarp) {
+    __shared__ WarpComp wc[NTL / 32];
     int* ctr = L.ctr + (k & 3) * 4;
     const int n = __ldcg(ctr);
-    for (int q = vt; q < n; q += nthr) {
+    for (int q = vw; q < n; q += nwarp) {
         const int h = __ldcg(L.seedq + q);
         const int t = h / L.cap_p;
-        SmallComp c;
-        if (link_component(L, c, t, h - t * L.cap_p, k) == COMP_BIG) L.deferq[push_slot(ctr + 2)] = h;
+        if (link_component_warp(L, wc[threadIdx.x >> 5], t, h - t * L.cap_p, k) == COMP_BIG && (threadIdx.x & 31) == 0)
+            L.deferq[push_slot(ctr + 2)] = h;
+        __syncwarp();
     }
 }
 
@@ -513,53 +880,98 @@ __device__ void members_short(const LinkBufs& L, int k, int tid, int nthr) {
 // from an older memory entry), so ids are compared by trajectory root.  A
 // particle unused by the next frame is an entry of frame t unless its id is
 // present in frame t-1 or an older frame of the window holds an unused
-// particle of the same id (linking.rs:244-259).  In steps, a grid barrier
-// between them: roots, then
-//   members_chain    the unused particles of each root as a list;
-//   members_present  every particle marks, in the entries of its root's list
-//                    at most `memory` frames before it, that their id is
-//                    present in its frame;
+// particle of the same id (linking.rs:244-259).  Pass 1 evaluates all
+// particles.  Later passes take those of the trajectories that the pass
+// before changed (the former root of every relinked destination and of its new
+// source): a root, a membership or a list can only change within them, and
+// they are complete, since every particle of a new trajectory comes from one
+// of them.  In steps, a grid barrier between them:
+//   members_find     the particles of those trajectories (from pass 2 on);
+//   roots_local, roots_global  their roots;
+//   members_chain    the unused particles in lists hashed by (root, block of
+//                    2^fshift >= memory frames), so that a lookup meets only
+//                    its own stretch of a trajectory (lists by root alone grow
+//                    with the trajectories: 480 us a pass instead of 130 for
+//                    200 frames of 15k particles);
+//   members_present  every particle marks, in the list entries of its id at
+//                    most `memory` frames before it, that the id is present
+//                    in its frame;
 //   members_long     the membership bits of every particle;
 //   members_clear    the lists emptied for the next pass.
-__device__ void members_chain(const LinkBufs& L, int tid, int nthr) {
-    const int g1 = __ldg(L.off + max(L.te - 2, first_member(L)));
-    const int nw = (L.memory + 31) >> 5;
-    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr) {
-        if (__ldcg(L.lnk + g) & 1u) continue;
+__device__ __forceinline__ int list_mask(const LinkBufs& L) {
+    const int n = __ldg(L.off + L.te) - __ldg(L.off + first_member(L));
+    return n <= 1 ? 0 : (1 << (32 - __clz(n - 1))) - 1;
+}
+
+__device__ __forceinline__ unsigned list_of(int root, int block) {
+    return ((unsigned)root * 2654435761u + (unsigned)block * 0x9E3779B1u) >> 3;
+}
+
+// fn(frame, index) for the unused particles of id `root` in frames [f0, f1].
+template <class F>
+__device__ __forceinline__ void each_unused(const LinkBufs& L, int mask, int root, int f0, int f1, F&& fn) {
+    for (int b = max(f0, 0) >> L.fshift; b <= f1 >> L.fshift; ++b)
+        for (int c = __ldcg(L.head + (list_of(root, b) & mask)); c >= 0;) {
+            const int4 e = __ldcg(L.ent + c);  // root, frame, next
+            if (e.x == root && e.y >= f0 && e.y <= f1) fn(e.y, c);
+            c = e.z;
+        }
+}
+
+// The particles that pass k evaluates: number, and the i-th.
+__device__ __forceinline__ int find_count(const LinkBufs& L, int k) {
+    return k == 1 ? __ldg(L.off + L.te) - __ldg(L.off + first_member(L)) : __ldcg(L.ctr + (k & 3) * 4 + 1);
+}
+
+__device__ __forceinline__ int find_item(const LinkBufs& L, int k, int i) {
+    return k == 1 ? __ldg(L.off + first_member(L)) + i : __ldcg(L.recq + i);
+}
+
+__device__ void members_find(const LinkBufs& L, int k, int tid, int nthr) {
+    const int g1 = __ldg(L.off + L.te);
+    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr)
+        if (__ldcg(L.cstamp + __ldcg(L.root + g)) == k) L.recq[push_slot(L.ctr + (k & 3) * 4 + 1)] = g;
+}
+
+__device__ void members_chain(const LinkBufs& L, int k, int tid, int nthr) {
+    const int n = find_count(L, k), nw = (L.memory + 31) >> 5, mask = list_mask(L);
+    for (int i = tid; i < n; i += nthr) {
+        const int g = find_item(L, k, i), f = __ldcg(L.gframe + g);
+        if (f > L.te - 3 || (__ldcg(L.lnk + g) & 1u)) continue;
         for (int w = 0; w < nw; ++w) L.pres[(size_t)w * L.np + g] = 0u;
-        L.nextc[g] = atomicExch(L.head + __ldcg(L.root + g), g);
+        const int root = __ldcg(L.root + g);
+        const int next = atomicExch(L.head + (list_of(root, f >> L.fshift) & mask), g);
+        L.ent[g] = make_int4(root, f, next, 0);
     }
 }
 
-__device__ void members_present(const LinkBufs& L, int tid, int nthr) {
-    const int g1 = __ldg(L.off + max(L.te - 1, first_member(L)));
-    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr) {
-        const int f = __ldcg(L.gframe + g);
-        for (int c = __ldcg(L.head + __ldcg(L.root + g)); c >= 0; c = __ldcg(L.nextc + c)) {
-            const int dist = f - __ldcg(L.gframe + c);
-            if (dist > 0 && dist <= L.memory)
-                atomicOr(L.pres + (size_t)((dist - 1) >> 5) * L.np + c, 1u << ((dist - 1) & 31));
-        }
+__device__ void members_present(const LinkBufs& L, int k, int tid, int nthr) {
+    const int n = find_count(L, k), mask = list_mask(L);
+    for (int i = tid; i < n; i += nthr) {
+        const int g = find_item(L, k, i), f = __ldcg(L.gframe + g);
+        if (f > L.te - 2) continue;
+        each_unused(L, mask, __ldcg(L.root + g), f - L.memory, f - 1, [&](int fc, int c) {
+            const int b = f - fc - 1;
+            atomicOr(L.pres + (size_t)(b >> 5) * L.np + c, 1u << (b & 31));
+        });
     }
 }
 
 __device__ void members_long(const LinkBufs& L, int k, int tid, int nthr) {
-    const int g1 = __ldg(L.off + max(L.te - 2, first_member(L)));
-    const int nw = (L.memory + 31) >> 5;
-    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr) {
-        const int f = __ldcg(L.gframe + g);
+    const int n = find_count(L, k), nw = (L.memory + 31) >> 5, mask = list_mask(L);
+    for (int i = tid; i < n; i += nthr) {
+        const int g = find_item(L, k, i), f = __ldcg(L.gframe + g);
+        if (f > L.te - 3) continue;
         const bool cand = !(__ldcg(L.lnk + g) & 1u);
         // distances j (frame f + 1 + j) inside the window
         const int j0 = max(1, L.tb - 1 - f);
-        int j1 = min(L.memory, L.te - 2 - f);
-        int fo = -1;  // latest older unused particle of the same id
+        const int j1 = min(L.memory, L.te - 2 - f);
+        // frame f + 1 + j's entries reach back to frame f + j - memory: an
+        // older unused particle of the same id in them goes first
+        int jmin = 0;
         if (cand)
-            for (int c = __ldcg(L.head + __ldcg(L.root + g)); c >= 0; c = __ldcg(L.nextc + c)) {
-                const int fc = __ldcg(L.gframe + c);
-                if (fc < f) fo = max(fo, fc);
-            }
-        // frame f + 1 + j's entries reach back to frame f + j - memory
-        const int jmin = fo < 0 ? 0 : fo - f + L.memory + 1;
+            each_unused(L, mask, __ldcg(L.root + g), f + 1 - L.memory, f - 1,
+                        [&](int fc, int) { jmin = max(jmin, fc - f + L.memory + 1); });
         for (int w = 0; w < nw; ++w) {
             unsigned wm = 0, bits = 0;
             for (int b = 0; b < 32; ++b) {
@@ -575,9 +987,12 @@ __device__ void members_long(const LinkBufs& L, int k, int tid, int nthr) {
     }
 }
 
-__device__ void members_clear(const LinkBufs& L, int tid, int nthr) {
-    const int g1 = __ldg(L.off + max(L.te - 2, first_member(L)));
-    for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr) L.head[__ldcg(L.root + g)] = -1;
+__device__ void members_clear(const LinkBufs& L, int k, int tid, int nthr) {
+    const int n = find_count(L, k), mask = list_mask(L);
+    for (int i = tid; i < n; i += nthr) {
+        const int g = find_item(L, k, i);
+        L.head[list_of(__ldcg(L.root + g), __ldcg(L.gframe + g) >> L.fshift) & mask] = -1;
+    }
 }
 
 // State of the window's particles before the first pass (earlier windows'
@@ -588,18 +1003,15 @@ __device__ void window_begin(const LinkBufs& L, int tid, int nthr) {
     const int gb = __ldg(L.off + L.tb), g1 = __ldg(L.off + L.te);
     for (int g = __ldg(L.off + fb) + tid; g < g1; g += nthr) {
         L.rstamp[g] = 0;
-        if (g < gb) {
-            if (L.memory > 2) L.head[__ldcg(L.root + g)] = -1;  // earlier windows' roots are final
-            continue;
-        }
+        if (L.memory > 2) L.cstamp[g < gb ? __ldcg(L.root + g) : g] = 0;  // earlier windows' roots are final
+        if (g < gb) continue;
         L.lnk[g] = 0u;
         L.stamp[g] = 0;
         for (int w = 0; w < nw; ++w) L.mm[(size_t)w * L.np + g] = 0u;
-        if (L.memory > 2) {
-            L.head[g] = -1;
-            L.gframe[g] = frame_of(L, g, L.tb, L.te);
-        }
+        if (L.memory > 2) L.gframe[g] = frame_of(L, g, L.tb, L.te);
     }
+    if (L.memory > 2)
+        for (int h = tid; h <= list_mask(L); h += nthr) L.head[h] = -1;
     for (int t = L.tb + tid; t < L.te; t += nthr) L.fstamp[t] = 0;
 }
 
@@ -625,11 +1037,15 @@ __device__ __forceinline__ int root_chunk(const LinkBufs& L) {
     return max(1, (n + nc - 1) / nc);
 }
 
-__device__ void roots_local(const LinkBufs& L) {
-    const int g0 = L.off[L.tb], n = L.off[L.te];
+// fn(i) gives the i-th of n particles to resolve (those before the window
+// are skipped); a particle's whole chain inside the window must be among them.
+template <class F>
+__device__ __forceinline__ void roots_local(const LinkBufs& L, int n, int tid, int nthr, F&& item) {
+    const int g0 = __ldg(L.off + L.tb);
     const int cs = root_chunk(L);
-    const int stride = gridDim.x * blockDim.x;
-    for (int g = g0 + blockIdx.x * blockDim.x + threadIdx.x; g < n; g += stride) {
+    for (int i = tid; i < n; i += nthr) {
+        const int g = item(i);
+        if (g < g0) continue;
         const int cbeg = g0 + (g - g0) / cs * cs;
         int r = g;
         while (true) {
@@ -642,11 +1058,13 @@ __device__ void roots_local(const LinkBufs& L) {
     }
 }
 
-__device__ void roots_global(const LinkBufs& L) {
-    const int g0 = L.off[L.tb], n = L.off[L.te];
-    const int stride = gridDim.x * blockDim.x;
+template <class F>
+__device__ __forceinline__ void roots_global(const LinkBufs& L, int n, int tid, int nthr, F&& item) {
+    const int g0 = __ldg(L.off + L.tb);
     volatile int* root = L.root;
-    for (int g = g0 + blockIdx.x * blockDim.x + threadIdx.x; g < n; g += stride) {
+    for (int i = tid; i < n; i += nthr) {
+        const int g = item(i);
+        if (g < g0) continue;
         int r = __ldcg(L.lroot + g);
         while (true) {
             const int known = root[r];
@@ -700,6 +1118,7 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
     const int tid0 = blockIdx.x * NTL + threadIdx.x;
     // few items: lane 0 of a warp in every block first
     const int vt0 = ((threadIdx.x & 31) * (NTL / 32) + (threadIdx.x >> 5)) * gridDim.x + blockIdx.x;
+    const int vw0 = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;  // the same for warps
     const bool stamp = blockIdx.x == 0 && threadIdx.x == 0;
     unsigned long long t0 = stamp ? gtimer() : 0, acc[4] = {0, 0, 0, 0};
     auto tick = [&](int i) {
@@ -763,11 +1182,16 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
                     }
                     grid.sync();
                 };
-                each([&](const LinkBufs& L) { roots_local(L); });
-                each([&](const LinkBufs& L) { roots_global(L); });
+                if (k > 1) each([&](const LinkBufs& L) { members_find(L, k, tid0, nthr); });
+                each([&](const LinkBufs& L) {
+                    roots_local(L, find_count(L, k), tid0, nthr, [&](int i) { return find_item(L, k, i); });
+                });
+                each([&](const LinkBufs& L) {
+                    roots_global(L, find_count(L, k), tid0, nthr, [&](int i) { return find_item(L, k, i); });
+                });
                 tick(1);
-                each([&](const LinkBufs& L) { members_chain(L, tid0, nthr); });
-                each([&](const LinkBufs& L) { members_present(L, tid0, nthr); });
+                each([&](const LinkBufs& L) { members_chain(L, k, tid0, nthr); });
+                each([&](const LinkBufs& L) { members_present(L, k, tid0, nthr); });
             }
             int r = 0;
             for (int m = 0; m < nm; ++m) {
@@ -793,10 +1217,10 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
             r = 0;
             for (int m = 0; m < nm; ++m) {
                 const LinkBufs L = movie(m);
-                const int id = rot(vt0, r, L);
+                const int id = rot(vw0 * 32, r, L) >> 5;
                 if (!active(L, k)) continue;
-                if (L.memory > 2) members_clear(L, tid0, nthr);
-                link_seeds(L, k, id, nthr);
+                if (L.memory > 2) members_clear(L, k, tid0, nthr);
+                link_seeds(L, k, id, nthr >> 5);
             }
             grid.sync();
             deferred(k);
@@ -805,11 +1229,16 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
     }
     for (int m = 0; m < nm; ++m) {
         const LinkBufs L = movie(m);
-        roots_local(L);
+        const int g0 = __ldg(L.off + L.tb);
+        roots_local(L, __ldg(L.off + L.te) - g0, tid0, nthr, [&](int i) { return g0 + i; });
         new_ranks(L);
     }
     grid.sync();
-    for (int m = 0; m < nm; ++m) roots_global(movie(m));
+    for (int m = 0; m < nm; ++m) {
+        const LinkBufs L = movie(m);
+        const int g0 = __ldg(L.off + L.tb);
+        roots_global(L, __ldg(L.off + L.te) - g0, tid0, nthr, [&](int i) { return g0 + i; });
+    }
     if (stamp) {
         acc[1] += gtimer() - t0;
         *passes = max(*passes, k);  // several launches (frame windows) add up
