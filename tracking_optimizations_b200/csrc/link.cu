@@ -795,34 +795,87 @@ __device__ void link_deferred(const LinkBufs& L, int k) {
     }
 }
 
-// Every destination of frame t within reach of (y, x) becomes a seed of
-// pass k.
-__device__ __forceinline__ void seed_around(const LinkBufs& L, float y, float x, int t, int k) {
-    const int offt = __ldg(L.off + t);
-    near(L, t, y, x, [&](int i, float dy, float dx) {
-        float w;
-        if (within_r(y, x, dy, dx, L.r, &w) && atomicExch(L.stamp + offt + i, k) != k) {
-            L.seedq[push_slot(L.ctr + (k & 3) * 4)] = t * L.cap_p + i;
-            if (__ldcg(L.fstamp + t) != k && atomicExch(L.fstamp + t, k) != k) atomicAdd(L.ctr + (k & 3) * 4 + 3, 1);
-        }
-        return true;
-    });
+// A block's seeds on their way to the queue: one global atomic per block
+// instead of one per few lanes (a million pushes to one counter took 0.6 ms).
+constexpr int SEED_BUF = 1024;
+struct SeedBuf {
+    int n;
+    int h[SEED_BUF];
+};
+
+// Empties the block's buffer into the movie's queue; every thread calls it.
+__device__ __forceinline__ void flush_seeds(const LinkBufs& L, SeedBuf& sb, int k) {
+    __shared__ int s_base;
+    __syncthreads();
+    const int n = min(sb.n, SEED_BUF);
+    if (n > 0) {
+        if (threadIdx.x == 0) s_base = atomicAdd(L.ctr + (k & 3) * 4, n);
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += NTL) L.seedq[s_base + i] = sb.h[i];
+        __syncthreads();
+        if (threadIdx.x == 0) sb.n = 0;
+        __syncthreads();
+    }
 }
 
-// Replaces the bits `wm` of word w of particle g's membership (frame f) by
-// `bits` and seeds pass k around it in the frames where they changed.
-__device__ __forceinline__ void set_members(const LinkBufs& L, int g, int f, int w, unsigned wm, unsigned bits, int k) {
-    unsigned* m = L.mm + (size_t)w * L.np + g;
-    const unsigned old = __ldcg(m);
-    unsigned diff = (old ^ bits) & wm;
-    if (!diff) return;
-    *m = old ^ diff;
-    const size_t h = (size_t)f * L.cap_p + (g - __ldg(L.off + f));
-    const float y = __ldg(L.py + h), x = __ldg(L.px + h);
-    while (diff) {
-        const int b = __ffs(diff) - 1;
-        diff &= diff - 1;
-        seed_around(L, y, x, f + 2 + 32 * w + b, k);
+// Sets the bits `wm` of word w of the lanes' particles' membership (particle
+// g of frame f; wm 0: none) to `bits`, and makes every destination in reach of
+// a particle whose bits changed, in the frames where they did, a seed of pass
+// k.  The warp takes one changed particle after the other, its cell rows in up
+// to ten frames at once: neighbour searches and the stamps' atomics by single
+// lanes left the others waiting (1.0 ms of the dense movie's pass 1).  Every
+// lane calls it.
+__device__ __forceinline__ void set_members(const LinkBufs& L, SeedBuf& sb, int g, int f, int w, unsigned wm,
+                                            unsigned bits, int k) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned diff = 0;
+    float gy = 0.f, gx = 0.f;
+    if (wm) {
+        unsigned* m = L.mm + (size_t)w * L.np + g;
+        const unsigned old = __ldcg(m);
+        diff = (old ^ bits) & wm;
+        if (diff) {
+            *m = old ^ diff;
+            const size_t h = (size_t)f * L.cap_p + (g - __ldg(L.off + f));
+            gy = __ldg(L.py + h);
+            gx = __ldg(L.px + h);
+        }
+    }
+    for (unsigned todo = __ballot_sync(full, diff != 0); todo; todo &= todo - 1) {
+        const int b = __ffs(todo) - 1;
+        const float y = __shfl_sync(full, gy, b), x = __shfl_sync(full, gx, b);
+        const int t0 = __shfl_sync(full, f, b) + 2 + 32 * w;
+        for (unsigned d = __shfl_sync(full, diff, b); d;) {
+            // lanes 3 i .. 3 i + 2: the rows of the i-th changed frame
+            const int nf = min(__popc(d), 10);
+            unsigned rest = d;
+            for (int q = 0; q < lane / 3 && rest; ++q) rest &= rest - 1;
+            const int t = t0 + __ffs(rest) - 1;
+            unsigned a = 0;
+            int n = 0;
+            if (lane < 3 * nf) cell_row(L, t, lane % 3, y, x, &a, &n);
+            each_in_rows(a, n, 3 * nf, [&](int row, unsigned at) {
+                const int tt = __shfl_sync(full, t, max(row, 0));
+                if (row >= 0) {
+                    const float2 p = __ldg(L.gpos + at);
+                    float dist;
+                    if (within_r(y, x, p.x, p.y, L.r, &dist)) {
+                        const int i = __ldg(L.gidx + at), h = tt * L.cap_p + i;
+                        if (atomicExch(L.stamp + __ldg(L.off + tt) + i, k) != k) {
+                            const int slot = atomicAdd(&sb.n, 1);
+                            if (slot < SEED_BUF) sb.h[slot] = h;
+                            else L.seedq[push_slot(L.ctr + (k & 3) * 4)] = h;
+                            if (__ldcg(L.fstamp + tt) != k && atomicExch(L.fstamp + tt, k) != k)
+                                atomicAdd(L.ctr + (k & 3) * 4 + 3, 1);
+                        }
+                    }
+                }
+                __syncwarp();
+                return true;
+            });
+            for (int q = 0; q < nf; ++q) d &= d - 1;
+        }
     }
 }
 
@@ -849,30 +902,28 @@ __device__ __forceinline__ int first_member(const LinkBufs& L) { return max(0, L
 // it, and of the frame 3 later when the one between does not either.
 // Pass 1 checks every particle, later passes those whose linked bits the
 // pass before changed.
-__device__ void members_short(const LinkBufs& L, int k, int tid, int nthr) {
+__device__ void members_short(const LinkBufs& L, SeedBuf& sb, int k, int tid, int nthr) {
     const int fb = first_member(L);
-    auto check = [&](int g, int f) {
-        const unsigned l = __ldcg(L.lnk + g);
+    const int g0 = __ldg(L.off + fb);
+    // pass 1: all, in order; later: spread over the grid's warps
+    const int n = k == 1 ? __ldg(L.off + L.te) - g0 : __ldcg(L.ctr + ((k - 1) & 3) * 4 + 1);
+    for (int i = tid; __any_sync(0xffffffffu, i < n); i += nthr) {
+        int g = 0, f = 0;
         unsigned wm = 0, bits = 0;
-        if (f + 2 >= L.tb && f + 2 < L.te) {
-            wm |= 1u;
-            if (!(l & 1u)) bits |= 1u;
+        if (i < n) {
+            g = k == 1 ? g0 + i : __ldcg(L.recq + i);
+            f = frame_of(L, g, fb, L.te);
+            const unsigned l = __ldcg(L.lnk + g);
+            if (f + 2 >= L.tb && f + 2 < L.te) {
+                wm |= 1u;
+                if (!(l & 1u)) bits |= 1u;
+            }
+            if (L.memory == 2 && f + 3 >= L.tb && f + 3 < L.te) {
+                wm |= 2u;
+                if (!(l & 3u)) bits |= 2u;
+            }
         }
-        if (L.memory == 2 && f + 3 >= L.tb && f + 3 < L.te) {
-            wm |= 2u;
-            if (!(l & 3u)) bits |= 2u;
-        }
-        set_members(L, g, f, 0, wm, bits, k);
-    };
-    if (k == 1) {
-        const int g1 = __ldg(L.off + L.te);
-        for (int g = __ldg(L.off + fb) + tid; g < g1; g += nthr) check(g, frame_of(L, g, fb, L.te));
-    } else {
-        const int n = __ldcg(L.ctr + ((k - 1) & 3) * 4 + 1);
-        for (int q = tid; q < n; q += nthr) {
-            const int g = __ldcg(L.recq + q);
-            check(g, frame_of(L, g, fb, L.te));
-        }
+        set_members(L, sb, g, f, 0, wm, bits, k);
     }
 }
 
@@ -957,12 +1008,12 @@ __device__ void members_present(const LinkBufs& L, int k, int tid, int nthr) {
     }
 }
 
-__device__ void members_long(const LinkBufs& L, int k, int tid, int nthr) {
+__device__ void members_long(const LinkBufs& L, SeedBuf& sb, int k, int tid, int nthr) {
     const int n = find_count(L, k), nw = (L.memory + 31) >> 5, mask = list_mask(L);
-    for (int i = tid; i < n; i += nthr) {
-        const int g = find_item(L, k, i), f = __ldcg(L.gframe + g);
-        if (f > L.te - 3) continue;
-        const bool cand = !(__ldcg(L.lnk + g) & 1u);
+    for (int i = tid; __any_sync(0xffffffffu, i < n); i += nthr) {
+        const int g = i < n ? find_item(L, k, i) : 0;
+        const int f = i < n ? __ldcg(L.gframe + g) : L.te;
+        const bool cand = f <= L.te - 3 && !(__ldcg(L.lnk + g) & 1u);
         // distances j (frame f + 1 + j) inside the window
         const int j0 = max(1, L.tb - 1 - f);
         const int j1 = min(L.memory, L.te - 2 - f);
@@ -973,16 +1024,13 @@ __device__ void members_long(const LinkBufs& L, int k, int tid, int nthr) {
             each_unused(L, mask, __ldcg(L.root + g), f + 1 - L.memory, f - 1,
                         [&](int fc, int) { jmin = max(jmin, fc - f + L.memory + 1); });
         for (int w = 0; w < nw; ++w) {
-            unsigned wm = 0, bits = 0;
-            for (int b = 0; b < 32; ++b) {
-                const int j = 32 * w + b + 1;
-                if (j < j0 || j > j1) continue;
-                wm |= 1u << b;
-                if (cand && j >= jmin) bits |= 1u << b;
-            }
-            if (!wm) continue;
+            // bits of the distances lo .. hi of this word
+            const int lo = max(j0 - 32 * w - 1, 0), hi = min(j1 - 32 * w - 1, 31);
+            const unsigned wm = lo <= hi ? (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo) : 0u;
+            const int lom = max(jmin - 32 * w - 1, 0);
+            unsigned bits = cand && lom < 32 ? wm & (0xffffffffu << lom) : 0u;
             if (bits) bits &= ~__ldcg(L.pres + (size_t)w * L.np + g);
-            set_members(L, g, f, w, wm, bits, k);
+            set_members(L, sb, g, f, w, wm, bits, k);
         }
     }
 }
@@ -1113,6 +1161,8 @@ __device__ __forceinline__ unsigned long long gtimer() {
 template <class M>
 __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_passes, int* passes,
                                               unsigned long long* stat) {
+    __shared__ SeedBuf sb;
+    if (threadIdx.x == 0) sb.n = 0;
     cg::grid_group grid = cg::this_grid();
     const int nthr = gridDim.x * NTL;
     const int tid0 = blockIdx.x * NTL + threadIdx.x;
@@ -1182,16 +1232,18 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
                     }
                     grid.sync();
                 };
+                // many items in order (neighbours share cache lines), few spread
+                auto order = [&](const LinkBufs& L) { return find_count(L, k) > nthr / 8 ? tid0 : vt0; };
                 if (k > 1) each([&](const LinkBufs& L) { members_find(L, k, tid0, nthr); });
                 each([&](const LinkBufs& L) {
-                    roots_local(L, find_count(L, k), tid0, nthr, [&](int i) { return find_item(L, k, i); });
+                    roots_local(L, find_count(L, k), order(L), nthr, [&](int i) { return find_item(L, k, i); });
                 });
                 each([&](const LinkBufs& L) {
-                    roots_global(L, find_count(L, k), tid0, nthr, [&](int i) { return find_item(L, k, i); });
+                    roots_global(L, find_count(L, k), order(L), nthr, [&](int i) { return find_item(L, k, i); });
                 });
                 tick(1);
-                each([&](const LinkBufs& L) { members_chain(L, k, tid0, nthr); });
-                each([&](const LinkBufs& L) { members_present(L, k, tid0, nthr); });
+                each([&](const LinkBufs& L) { members_chain(L, k, order(L), nthr); });
+                each([&](const LinkBufs& L) { members_present(L, k, order(L), nthr); });
             }
             int r = 0;
             for (int m = 0; m < nm; ++m) {
@@ -1201,8 +1253,9 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
                 if (stamp)
                     for (int q = 0; q < 4; ++q) L.ctr[((k + 1) & 3) * 4 + q] = 0;
                 if (!active(L, k)) continue;
-                if (L.memory <= 2) members_short(L, k, k == 1 ? tid0 : id, nthr);
-                else members_long(L, k, tid0, nthr);
+                if (L.memory <= 2) members_short(L, sb, k, k == 1 ? tid0 : id, nthr);
+                else members_long(L, sb, k, find_count(L, k) > nthr / 8 ? tid0 : id, nthr);
+                flush_seeds(L, sb, k);
             }
             grid.sync();
             int total = 0;
