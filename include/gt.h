@@ -325,7 +325,9 @@ typedef struct gt_stats {
     float ms_link;             /* linking incl. fixed-point passes and ids */
     float ms_assemble;         /* output table */
     float ms_total;            /* first to last kernel of the call */
-    int32_t locate_kernel;     /* 0 generic, 1 specialised, 2 specialised with TMA staging */
+    int32_t locate_kernel;     /* dilation size: 0 at run time (generic kernel, or the specialised one for
+                                * float frames and other separations), 1 specialised, 2 specialised with
+                                * TMA staging */
     float link_phase_ms[4];    /* linker: first pass, roots, memory entries, relinking */
     int32_t link_dirty[8];     /* frames relinked by fixed-point passes 1..8 */
     float ms_adjoint_particles; /* gt_adjoint_*: per-particle kernel */

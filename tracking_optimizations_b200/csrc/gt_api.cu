@@ -42,7 +42,7 @@ __global__ void newid_kernel(const int* newrank, const int* newbase, const int* 
 __global__ void assemble_kernel(AsmArgs a);
 __global__ void grid_kernel(const float* py, const float* px, const int* npart, int cap_p, int G,
                             int ncy, int ncx, int* gstart, int* gidx, float2* gpos);
-bool fast_supported(int kr, int dd, int rc, int diameter);
+int fast_supported(int kr, int dd, int rc, int diameter, int dtype);
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, int T, int frame0, int* used_tma);
 void gauss_taps(int smoothing_size, float noise_size, int normalized, float* w, float* norm, float* rn);
@@ -315,16 +315,16 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     lp.tma_spin = 1 << 22;
     lp.tma_withhold = 0;
     P.fast = 0;
-    const bool want_fast = dtype == GT_U16 && fast_supported(lp.krad, lp.D, lp.rint_c, lp.d) && !force_generic_flag;
+    const int want_fast = force_generic_flag ? 0 : fast_supported(lp.krad, lp.D, lp.rint_c, lp.d, dtype);
     P.char_tab.clear(); P.char_off.clear(); P.gchar_tab.clear();
     circle_tables(lp.char_r, P.char_tab, &P.char_off, 1);
     circle_tables(lp.rint_c, P.gchar_tab, nullptr, 0);
     lp.n_char = (int)P.char_off.size() / 2;
     lp.n_gchar = (int)P.gchar_tab.size() / 2;
     if (want_fast) {
-        P.fast = 1;
-        P.fast_th = fast_tile_rows;
-        lp.TH = fast_tile_rows;
+        P.fast = want_fast;
+        P.fast_th = want_fast == 2 ? 64 : fast_tile_rows;
+        lp.TH = P.fast_th;
         lp.TW = 64;
         lp.ntx = (W + lp.TW - 1) / lp.TW;
         lp.nty = (H + lp.TH - 1) / lp.TH;
@@ -613,7 +613,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
         if (!ctx->ev[i]) CK(cudaEventCreate(&ctx->ev[i]));
     const int ntiles = P.lp.ntx * P.lp.nty;
     const bool fast = P.fast != 0;
-    ctx->stats.locate_kernel = fast ? 1 : 0;
+    ctx->stats.locate_kernel = P.fast == 1 ? 1 : 0;
     // frame chunks: up to 16 for host frames (copy/locate overlap; the
     // locate of the last chunk is what remains after the copy), else as
     // large as the grid allows
@@ -683,7 +683,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
             int used_tma = 0;
             CK(launch_locate_fast(P.lp.krad, P.lp.D, P.lp.rint_c, P.fast_th, grid, st, P.lp, b, T, f0, &used_tma));
             ctx->stats.launches += 1;
-            ctx->stats.locate_kernel = used_tma ? 2 : 1;
+            if (P.fast == 1) ctx->stats.locate_kernel = used_tma ? 2 : 1;
             if (chunked && (rc = post(f0, nf))) return rc;
         }
     } else {
@@ -1265,7 +1265,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         ctx->batch_key.clear();
         // autotuned tile rows (timed on this movie's frames and workspace)
         for (int i = 0; i < n; ++i)
-            if (B[i].fast) {
+            if (B[i].P.fast == 1) {
                 rc = tune_tile_rows(ctx, B[i], mv[i].frames, st);
                 if (rc) return rc;
             }

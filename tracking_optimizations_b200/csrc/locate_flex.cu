@@ -1,0 +1,34 @@
+// locate_flex.cu -- the specialised locate kernel with a run-time dilation
+// size: float frames, diameters 13 and 15, and separations beside the default
+// diameter + 1.
+#include "locate_fast.cuh"
+
+namespace gt {
+
+namespace {
+// (radius, dilation size of separation = diameter + 1); tiles of 64 rows
+#define GT_FLEX_LIST(X) X(2, 8) X(3, 11) X(4, 14) X(5, 16) X(6, 19) X(7, 22)
+}  // namespace
+
+// The largest dilation size of radius rc's instance, 0 without one.
+int flex_dilation(int rc, int dtype) {
+#define GT_FLEX_CASE(R, DD) if (rc == R) return DD;
+    GT_FLEX_LIST(GT_FLEX_CASE)
+#undef GT_FLEX_CASE
+    (void)dtype;
+    return 0;
+}
+
+cudaError_t launch_locate_flex(int kr, int rc, int dtype, dim3 grid, cudaStream_t st, const LocParams& p,
+                               const MovieBufs& b, int T, int frame0, int* used_tma) {
+    if (kr != rc || p.D < FM || p.D > flex_dilation(rc, dtype)) return cudaErrorInvalidValue;
+#define GT_FLEX_CASE(R, DD)                                                                                   \
+    if (rc == R)                                                                                              \
+        return dtype == 0 ? launch_instance<R, DD, 64, R, unsigned short, true>(grid, st, p, b, T, frame0, used_tma) \
+                          : launch_instance<R, DD, 64, R, float, true>(grid, st, p, b, T, frame0, used_tma);
+    GT_FLEX_LIST(GT_FLEX_CASE)
+#undef GT_FLEX_CASE
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace gt

@@ -32,7 +32,7 @@ __global__ void fallback_walk_kernel(const LocParams p, const MovieBufs b, int w
 __global__ void finalize_kernel(const LocParams p, MovieBufs b, float sep, int link_grid, int frame0);
 __global__ void scan_frames_kernel(const int* in, int* out, int n);
 __global__ void assemble_kernel(AsmArgs a);
-bool fast_supported(int kr, int dd, int rc, int diameter);
+int fast_supported(int kr, int dd, int rc, int diameter, int dtype);
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, int T, int frame0, int* used_tma);
 void gauss_taps(int smoothing_size, float noise_size, int normalized, float* w, float* norm, float* rn);
@@ -224,7 +224,7 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
     const int n_sig = sig ? circle_f(pr->sig_radius, sig_off) : 0;
     const int n_bg = bg ? annulus_f(pr->bg_radius, pr->sig_radius + gap, bg_off) : 0;
 
-    const bool fast = dtype == GT_U16 && fast_supported(lp.krad, lp.D, lp.rint_c, lp.d);
+    const bool fast = fast_supported(lp.krad, lp.D, lp.rint_c, lp.d, dtype) != 0;
     const int th = fast ? 64 : 32;
     lp.TH = th;
     lp.TW = 64;
