@@ -29,7 +29,8 @@
 namespace gt {
 __global__ void locate_tiles_kernel(const LocParams p, const MovieBufs b, int frame0);
 __global__ void fallback_walk_kernel(const LocParams p, const MovieBufs b, int win, const int* pbeg);
-__global__ void finalize_kernel(const LocParams p, MovieBufs b, float sep, int link_grid, int frame0);
+cudaError_t launch_finalize(const LocParams& p, const MovieBufs& b, float sep, int link_grid, int frame0, int nf,
+                            size_t smem, cudaStream_t st);
 cudaError_t link_blocks_per_sm(bool multi, int* per_sm);
 cudaError_t launch_link(const LinkBufs& L, int max_passes, int* passes, unsigned long long* stat, int grid,
                         cudaStream_t st);
@@ -39,7 +40,7 @@ __global__ void scan_frames_kernel(const int* in, int* out, int n);
 __global__ void scan_frames_from_kernel(const int* in, int* out, int f0, int n);
 __global__ void newid_kernel(const int* newrank, const int* newbase, const int* off, const int* npart,
                              int* newid, int T);
-__global__ void assemble_kernel(AsmArgs a);
+cudaError_t launch_assemble(const AsmArgs& a, int num_sms, cudaStream_t st);
 __global__ void grid_kernel(const float* py, const float* px, const int* npart, int cap_p, int G,
                             int ncy, int ncx, int* gstart, int* gidx, float2* gpos);
 int fast_supported(int kr, int dd, int rc, int diameter, int dtype);
@@ -223,7 +224,8 @@ struct Plan {
     float sep = 0.f;
     int link = 0;
     int cap_c = 0, cap_p = 0;
-    int G = 8, ncx = 1, ncy = 1;
+    int G = 8, ncx = 1, ncy = 1;      // separation grid
+    int LG = 8, lncx = 1, lncy = 1;  // linker's grid
     // linker scratch for components beyond a thread's own arrays
     int nslot = 0, big_d = 1, big_s = 1, big_e = 1;
     size_t smem_loc = 0, smem_fb = 0, smem_fin = 0;
@@ -352,11 +354,18 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     const double ext_h = H + 2.0 * lp.rint_c + s, ext_w = W + 2.0 * lp.rint_c + s;
     long long pack = (long long)(ext_h * ext_w / (0.785 * s * s)) + 16;
     P.cap_p = (int)std::min<long long>(P.cap_c, pack * scale);
-    P.G = std::max({(int)std::ceil(P.sep) + 1, P.link ? (int)std::ceil(r.search_range) + 1 : 0, 8,
-                    (int)std::ceil(std::sqrt((double)HW / 16384.0))});
+    // cells at least separation + 1 and at most 16384 of them; the linker's at
+    // least search_range + 1 and at most 40960: its neighbour searches read
+    // 3 x 3 cells of several frames (200 frames of 15k particles, range 7: cells
+    // of 10 instead of 16 pixels halve what they read), and a frame's cell
+    // counts fit shared memory
+    P.G = std::max({(int)std::ceil(P.sep) + 1, 8, (int)std::ceil(std::sqrt((double)HW / 16384.0))});
+    P.LG = std::max({P.link ? (int)std::ceil(r.search_range) + 1 : 0, 8, (int)std::ceil(std::sqrt((double)HW / 40960.0))});
+    P.lncy = (H + P.LG - 1) / P.LG;
+    P.lncx = (W + P.LG - 1) / P.LG;
     P.ncy = (H + P.G - 1) / P.G;
     P.ncx = (W + P.G - 1) / P.G;
-    P.smem_fin = sizeof(int) * (size_t)P.ncx * P.ncy;
+    P.smem_fin = sizeof(int) * std::max((size_t)P.ncx * P.ncy, P.link ? (size_t)P.lncx * P.lncy : 0);
     if (P.smem_fin > 200 * 1024) { *msg = "grid too fine"; return GT_ERR_ARG; }
     link_scratch(&P, scale);
     column_list(r, P.names, P.types);
@@ -401,7 +410,7 @@ struct Carver {
 size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_locate, bool own_out = true) {
     Carver c{base};
     const size_t T = P.T;
-    const size_t ncell = (size_t)P.ncx * P.ncy;
+    const size_t ncell = (size_t)P.ncx * P.ncy, lcell = (size_t)P.lncx * P.lncy;
     w->frames = c.take<char>(frame_bytes);
     const size_t cc = need_locate ? T * P.cap_c : 1;
     w->cand = c.take<Cand>(cc);
@@ -414,7 +423,7 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->pm = c.take<float>(T * P.cap_p);
     w->prec = c.take<int>(T * P.cap_p);
     w->npart = c.take<int>(T);
-    w->gstart = c.take<int>(T * (ncell + 1));
+    w->gstart = c.take<int>(T * (lcell + 1));
     w->gidx = c.take<int>(T * P.cap_p);
     w->cperm = c.take<int>(cc);
     w->crec = c.take<int>(cc);
@@ -489,8 +498,8 @@ LinkBufs link_bufs(const Plan& P, const Work& w, long long budget) {
     L.te = P.T;
     L.T = P.T; L.cap_p = P.cap_p; L.memory = (int)P.r.memory;
     L.r = P.r.search_range;
-    L.inv_g = 1.0f / (float)P.G;
-    L.ncx = P.ncx; L.ncy = P.ncy;
+    L.inv_g = 1.0f / (float)P.LG;
+    L.ncx = P.lncx; L.ncy = P.lncy;
     L.py = w.py; L.px = w.px; L.npart = w.npart; L.off = w.off; L.gstart = w.gstart; L.gidx = w.gidx; L.gpos = w.gpos;
     L.np = (size_t)P.T * P.cap_p;
     L.pred = w.pred; L.lnk = w.lnk; L.mm = w.mm; L.stamp = w.stamp; L.rstamp = w.rstamp;
@@ -583,7 +592,7 @@ MovieBufs movie_bufs(const Plan& P, const Work& w, const void* frames) {
     b.cap_c = P.cap_c; b.cap_p = P.cap_p;
     b.cand = w.cand; b.fcount = w.fcount; b.rowcnt = w.rowcnt; b.pend = w.pend; b.npend = w.npend;
     b.py = w.py; b.px = w.px; b.pm = w.pm; b.prec = w.prec; b.npart = w.npart;
-    b.G = P.G; b.ncx = P.ncx; b.ncy = P.ncy; b.gstart = w.gstart; b.gidx = w.gidx; b.gpos = w.gpos;
+    b.G = P.G; b.ncx = P.ncx; b.ncy = P.ncy; b.LG = P.LG; b.lncx = P.lncx; b.lncy = P.lncy; b.gstart = w.gstart; b.gidx = w.gidx; b.gpos = w.gpos;
     b.cperm = w.cperm; b.cy = w.cy; b.cx = w.cx; b.cm = w.cm; b.crec = w.crec; b.ccell = w.ccell;
     b.cstart = w.cstart; b.cidx = w.cidx;
     b.char_tab = w.char_tab; b.char_off = w.char_off; b.gchar_tab = w.gchar_tab;
@@ -652,11 +661,10 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     }
     CK(cudaMemsetAsync(w.pbeg, 0, sizeof(int) * LINK_WINDOWS, st));
     CK(cudaFuncSetAttribute(fallback_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem_fb));
-    CK(cudaFuncSetAttribute(finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem_fin));
     int wi = 0;
     auto post = [&](int f0, int nf) -> int {
         fallback_walk_kernel<<<ctx->num_sms * 4, 128, P.smem_fb, st>>>(P.lp, b, P.fb_win, w.pbeg + wi);
-        finalize_kernel<<<nf, 512, P.smem_fin, st>>>(P.lp, b, P.sep, P.link, f0);
+        CK(launch_finalize(P.lp, b, P.sep, P.link, f0, nf, P.smem_fin, st));
         scan_frames_from_kernel<<<1, 1024, 0, st>>>(w.npart, w.off, f0, nf);
         CK(cudaGetLastError());
         ctx->stats.launches += 3;
@@ -709,7 +717,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     if (!chunked) {
         // the whole movie as one window: finalize, then link
         fallback_walk_kernel<<<ctx->num_sms * 4, 128, P.smem_fb, st>>>(P.lp, b, P.fb_win, w.pbeg);
-        finalize_kernel<<<T, 512, P.smem_fin, st>>>(P.lp, b, P.sep, P.link, 0);
+        CK(launch_finalize(P.lp, b, P.sep, P.link, 0, T, P.smem_fin, st));
         scan_frames_from_kernel<<<1, 1024, 0, st>>>(w.npart, w.off, 0, T);
         CK(cudaGetLastError());
         ctx->stats.launches += 3;
@@ -736,8 +744,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     a.out_rows = d_out ? out_rows : LLONG_MAX;
     a.walk = d_walk;
     a.walk_rows = walk_rows;
-    assemble_kernel<<<T, 256, 0, st>>>(a);
-    CK(cudaGetLastError());
+    CK(launch_assemble(a, ctx->num_sms, st));
     ctx->stats.launches += 1;
     CK(cudaEventRecord(ctx->ev[4], st));
     // every statistic of the call in one readback: error words, row count,
@@ -1049,7 +1056,7 @@ int enqueue_front(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t 
     }
     CK(cudaGetLastError());
     fallback_walk_kernel<<<ctx->num_sms, 128, P.smem_fb, s>>>(P.lp, b, P.fb_win, nullptr);
-    finalize_kernel<<<T, 512, P.smem_fin, s>>>(P.lp, b, P.sep, P.link, 0);
+    CK(launch_finalize(P.lp, b, P.sep, P.link, 0, T, P.smem_fin, s));
     scan_frames_kernel<<<1, 1024, 0, s>>>(w.npart, w.off, T);
     CK(cudaGetLastError());
     *launches += 3;
@@ -1078,8 +1085,7 @@ int enqueue_back(gt_ctx* ctx, BatchMovie& bm, const gt_movie& mv, int* d_status,
     a.bg_off = w.bg_off; a.n_bg = (int)P.bg_off.size() / 2;
     a.out = mv.out;
     a.out_rows = mv.out ? mv.out_rows : 0;
-    assemble_kernel<<<T, 256, 0, s>>>(a);
-    CK(cudaGetLastError());
+    CK(launch_assemble(a, ctx->num_sms, s));
     *launches += 1;
     CK(cudaMemcpyAsync(d_status, w.err, sizeof(int) * 4, cudaMemcpyDeviceToDevice, s));
     CK(cudaMemcpyAsync(d_status + 4, w.off + T, sizeof(int), cudaMemcpyDeviceToDevice, s));
@@ -1269,15 +1275,13 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
                 rc = tune_tile_rows(ctx, B[i], mv[i].frames, st);
                 if (rc) return rc;
             }
-        size_t sl = 0, sf = 0, sn = 0;
+        size_t sl = 0, sf = 0;
         for (int i = 0; i < n; ++i) {
             sl = std::max(sl, B[i].P.smem_loc);
             sf = std::max(sf, B[i].P.smem_fb);
-            sn = std::max(sn, B[i].P.smem_fin);
         }
         CK(cudaFuncSetAttribute(locate_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl));
         CK(cudaFuncSetAttribute(fallback_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf));
-        CK(cudaFuncSetAttribute(finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sn));
         CK(cudaStreamSynchronize(st));
         // capture; where capture is refused, run the same sequence directly
         cudaGraph_t graph = nullptr;
@@ -1940,9 +1944,9 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         // cells of absolute positions; negative coordinates clamp into the
         // first cell (clamping is monotone, so neighbours stay adjacent)
         const double ext = std::max({(double)ymax, (double)xmax, 0.0}) + 1.0;
-        P.G = std::max({(int)std::ceil(search_range) + 1, 8, (int)std::ceil(ext / 128.0)});
-        P.ncy = (int)(std::max(ymax, 0.0f) / P.G) + 1;
-        P.ncx = (int)(std::max(xmax, 0.0f) / P.G) + 1;
+        P.LG = std::max({(int)std::ceil(search_range) + 1, 8, (int)std::ceil(ext / 200.0)});
+        P.lncy = (int)(std::max(ymax, 0.0f) / P.LG) + 1;
+        P.lncx = (int)(std::max(xmax, 0.0f) / P.LG) + 1;
         (void)ymin; (void)xmin;
         link_scratch(&P, scale);
         P.cap_c = 1;
@@ -1964,9 +1968,9 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         CK(cudaMemcpyAsync(w.npart, gsize.data(), sizeof(int) * T, cudaMemcpyHostToDevice, st));
         CK(cudaMemsetAsync(w.err, 0, sizeof(int) * 4, st));
         CK(cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(int) * (size_t)P.ncx * P.ncy)));
-        grid_kernel<<<T, 512, sizeof(int) * (size_t)P.ncx * P.ncy, st>>>(w.py, w.px, w.npart, P.cap_p, P.G,
-                                                                        P.ncy, P.ncx, w.gstart, w.gidx, w.gpos);
+                                (int)(sizeof(int) * (size_t)P.lncx * P.lncy)));
+        grid_kernel<<<T, 512, sizeof(int) * (size_t)P.lncx * P.lncy, st>>>(w.py, w.px, w.npart, P.cap_p, P.LG,
+                                                                        P.lncy, P.lncx, w.gstart, w.gidx, w.gpos);
         CK(cudaGetLastError());
         scan_frames_kernel<<<1, 1024, 0, st>>>(w.npart, w.off, T);
         rc = run_link(ctx, P, w, st);

@@ -91,8 +91,9 @@ struct MovieBufs {
     float* pm;
     int* prec;
     int* npart;
-    int G, ncx, ncy;      // link/separation grid: cell size and counts
-    int* gstart;          // T*(ncx*ncy+1)
+    int G, ncx, ncy;      // separation grid: cell size and counts
+    int LG, lncx, lncy;   // linker's grid
+    int* gstart;          // T*(lncx*lncy+1)
     int* gidx;            // T*cap_p
     float2* gpos;         // T*cap_p (y, x) of gidx's particles
     int* cperm;           // T*cap_c finalize scratch (raster permutation)

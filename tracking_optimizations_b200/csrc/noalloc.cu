@@ -29,9 +29,10 @@
 namespace gt {
 __global__ void locate_tiles_kernel(const LocParams p, const MovieBufs b, int frame0);
 __global__ void fallback_walk_kernel(const LocParams p, const MovieBufs b, int win, const int* pbeg);
-__global__ void finalize_kernel(const LocParams p, MovieBufs b, float sep, int link_grid, int frame0);
+cudaError_t launch_finalize(const LocParams& p, const MovieBufs& b, float sep, int link_grid, int frame0, int nf,
+                            size_t smem, cudaStream_t st);
 __global__ void scan_frames_kernel(const int* in, int* out, int n);
-__global__ void assemble_kernel(AsmArgs a);
+cudaError_t launch_assemble(const AsmArgs& a, int num_sms, cudaStream_t st);
 int fast_supported(int kr, int dd, int rc, int diameter, int dtype);
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, int T, int frame0, int* used_tma);
@@ -307,8 +308,7 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
     SCK(cudaFuncSetAttribute(fallback_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fb));
     fallback_walk_kernel<<<ds.num_sms * 4, 128, smem_fb, st>>>(lp, b, fb_win, nullptr);
     SCK(cudaGetLastError());
-    SCK(cudaFuncSetAttribute(finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(4 * ncell)));
-    finalize_kernel<<<1, 512, 4 * ncell, st>>>(lp, b, (float)sep, 0, 0);
+    SCK(launch_finalize(lp, b, (float)sep, 0, 0, 1, 4 * (size_t)ncell, st));
     scan_frames_kernel<<<1, 1024, 0, st>>>(b.npart, off, 1);
     AsmArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -320,7 +320,7 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
     a.sig_off = d_sig_off; a.n_sig = n_sig; a.bg_off = d_bg_off; a.n_bg = n_bg;
     a.out = stage;
     a.out_rows = LLONG_MAX;
-    assemble_kernel<<<1, 256, 0, st>>>(a);
+    SCK(launch_assemble(a, 148, st));
     SCK(cudaGetLastError());
     int hb[2] = {0, 0};
     SCK(cudaMemcpyAsync(&hb[0], b.err, sizeof(int), cudaMemcpyDeviceToHost, st));
