@@ -17,8 +17,13 @@
 // at the circle pixels with the locate kernels' exact operation order, so
 // its (y, x, mass) equal the located rows bit for bit.  The backward pass
 // recomputes the same bandpass values (nothing from the forward is stored),
-// scatters dL/dR onto a zeroed plane and applies the transposed bandpass as
-// one dense stencil pass.  The clip has subgradient 0 at R == 0.
+// stores each peak's dL/dR (K values) and links the peak to the output tiles
+// in its reach; the transposed bandpass then sums each tile's dL/dR in shared
+// memory and filters it there, so that HBM sees the frames once and the
+// gradient once (a plane of dL/dR in HBM, zeroed, added to and read back, took
+// 128 of 895 us for 256 x 512x512 frames with 102k peaks, and bandpass values
+// evaluated tap by tap per circle pixel 520 us; now 70 + 80 + 90 us).  The
+// clip has subgradient 0 at R == 0.
 //
 // Parameter derivatives: noise_size is the Gaussian variance s, and
 // dG/ds = (da (x) a + a (x) da) * I with a_i = w_i / sum(w).  smoothing_size
@@ -27,14 +32,19 @@
 // held fixed): dR/dk = 2 B / k.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <math_constants.h>
+
 #include "gt_internal.cuh"
+#include "gt_simd.cuh"
 
 namespace gt {
 
 namespace {
 
 constexpr int ADJ_NT = 128;
-constexpr int TR_TH = 32, TR_TW = 64, TR_NT = 256;
+constexpr int TR_TW = 64, TR_NT = 256;
+// rows of a transpose tile: 64 with a compile-time radius, else 32
+__host__ __device__ constexpr int tr_th(int krt) { return krt > 0 ? 64 : 32; }
 
 struct BpTerms {
     float r;      // bandpass before the clip
@@ -100,27 +110,96 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 enum AdjMode { ADJ_FORWARD = 0, ADJ_BACKWARD = 1, ADJ_UNCERTAINTY = 2 };
 
+// Shared floats of a warp: R, B, dG/ds at the circle pixels and 3K of the
+// uncertainty; with a compile-time radius also the raw window and the row
+// pass's sums over it.
+__host__ __device__ constexpr int adj_window(int r) { return (4 * r + 1) * (4 * r + 1); }
+__host__ __device__ constexpr int adj_rows(int r) { return (4 * r + 1) * (2 * r + 1); }
+__host__ __device__ constexpr int adj_warp_floats(int mode, int r, int K) {
+    return 6 * K + (r > 0 ? adj_window(r) + adj_rows(r) * (mode == 1 ? 4 : 2) : 0);
+}
+
+// The bandpass at the circle pixels of a peak whose whole window lies inside
+// the frame (smoothing radius = circle radius = R): the raw window once into
+// shared memory, the row sums once per (row, circle column), the column sums
+// per circle pixel -- the values of bandpass_terms in the same order.
+template <int MODE, int R>
+__device__ __forceinline__ void window_terms(const AdjParams& p, const float* fr, int ul, int vl, int K, const int* sci,
+                                             float* win, float* sR, float* sB, float* sD) {
+    constexpr int WS = 4 * R + 1, CW = 2 * R + 1, NP = WS * CW;
+    const int lane = threadIdx.x & 31;
+    float* rg = win + WS * WS;
+    float* rb = rg + NP;
+    float* ra = rb + NP;
+    float* rd = ra + NP;
+    const float* src = fr + (size_t)(ul - 2 * R) * p.W + (vl - 2 * R);
+    for (int q = lane; q < WS * WS; q += 32) win[q] = __ldg(src + (size_t)(q / WS) * p.W + q % WS);
+    __syncwarp();
+    for (int q = lane; q < NP; q += 32) {
+        const float* w = win + (q / CW) * WS + q % CW;
+        float g = 0.f, b = 0.f, a = 0.f, d = 0.f;
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+            const float v = w[j];
+            g = fmaf(p.w[j], v, g);
+            b = b + v;
+            if (MODE == 1) {
+                a = fmaf(p.a[j], v, a);
+                d = fmaf(p.da[j], v, d);
+            }
+        }
+        rg[q] = g * p.rn;
+        rb[q] = b;
+        if (MODE == 1) {
+            ra[q] = a;
+            rd[q] = d;
+        }
+    }
+    __syncwarp();
+    for (int c = lane; c < K; c += 32) {
+        const int q0 = (sci[2 * c] + R) * CW + sci[2 * c + 1] + R;
+        float gs = 0.f, cs = 0.f, dg = 0.f;
+#pragma unroll
+        for (int i = 0; i < CW; ++i) {
+            const int q = q0 + i * CW;
+            gs = fmaf(p.w[i], rg[q], gs);
+            cs = cs + rb[q];
+            if (MODE == 1) {
+                dg = fmaf(p.da[i], ra[q], dg);
+                dg = fmaf(p.a[i], rd[q], dg);
+            }
+        }
+        sR[c] = fmaf(-cs, p.rkk, gs * p.rn);
+        if (MODE == 1) {
+            sB[c] = cs * p.rkk;
+            sD[c] = dg;
+        }
+    }
+}
+
 // One warp per particle (grid-stride over warps), ADJ_NT / 32 warps per
 // CTA sharing the circle table.  walk rows: {frame, ul, vl, up, vp}.
-// FORWARD writes yxm (n x 3).  BACKWARD reads grad (n x 3), adds dL/dR into
-// the zeroed plane gR (T x H x W) and dL/d{noise_size, smoothing_size} into
-// gpar.  UNCERTAINTY writes the standard deviations of (y, x, mass) under
+// FORWARD writes yxm (n x 3).  BACKWARD reads grad (n x 3), writes dL/dR at the
+// circle pixels to tl.g (n x K), links the peak to the tiles whose output it
+// reaches and writes the block's dL/d{noise_size, smoothing_size} to gpar.
+// R: smoothing and circle radius where they are equal and at most 7, else 0.  UNCERTAINTY writes the standard deviations of (y, x, mass) under
 // var(I) = gain * max(I, 0) + read_var by linear propagation (n x 3).
-template <int MODE>
+template <int MODE, int R>
 __global__ void __launch_bounds__(ADJ_NT) adjoint_particle_kernel(AdjParams p, const float* __restrict__ frames,
                                                                   const int* __restrict__ walk, long long n,
                                                                   const int* __restrict__ circ,
                                                                   const float* __restrict__ grad, float* yxm,
-                                                                  float* gR, double* gpar, int* err) {
+                                                                  AdjTiles tl, double* gpar, int* err) {
     extern __shared__ __align__(16) float asm_[];
     constexpr int NW = ADJ_NT / 32;
     const int K = p.K;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int* sci = (int*)asm_;                      // 2K circle offsets {i, j}, shared
-    float* sR = asm_ + 2 * K + wid * 6 * K;     // this warp's R at the circle pixels
+    float* sR = asm_ + 2 * K + wid * adj_warp_floats(MODE, R, K);  // this warp's R at the circle pixels
     float* sB = sR + K;                         // B
     float* sD = sB + K;                         // dG/ds
     float* sJ = sD + K;                         // 3K: dy/dR, dx/dR, dm/dR (uncertainty)
+    float* win = sJ + 3 * K;
     for (int q = threadIdx.x; q < 2 * K; q += ADJ_NT) sci[q] = circ[q];
     __syncthreads();
     const int H = p.H, W = p.W, kr = p.krad, b = p.border;
@@ -150,30 +229,28 @@ __global__ void __launch_bounds__(ADJ_NT) adjoint_particle_kernel(AdjParams p, c
         }
         const float* fr = frames + (size_t)t * H * W;
         __syncwarp();  // the previous particle's reads of this warp's arrays are done
-        for (int c = lane; c < K; c += 32) {
-            const BpTerms bt = bandpass_terms(p, fr, ul + sci[2 * c], vl + sci[2 * c + 1]);
-            sR[c] = bt.r;
-            sB[c] = bt.bmean;
-            sD[c] = bt.dg;
+        if (R > 0 && ul - 2 * R >= 0 && ul + 2 * R < H && vl - 2 * R >= 0 && vl + 2 * R < W) {
+            window_terms<MODE, R>(p, fr, ul, vl, K, sci, win, sR, sB, sD);
+        } else {
+            for (int c = lane; c < K; c += 32) {
+                const BpTerms bt = bandpass_terms(p, fr, ul + sci[2 * c], vl + sci[2 * c + 1]);
+                sR[c] = bt.r;
+                sB[c] = bt.bmean;
+                sD[c] = bt.dg;
+            }
         }
         __syncwarp();
-        float c0 = 0.f, c1 = 0.f, m = 0.f;
-        if (lane == 0) {
-            // centers.wgsl:23-109 accumulation order (i outer, j inner)
-            float a0 = 0.f, a1 = 0.f, mm = 0.f;
-            for (int c = 0; c < K; ++c) {
-                const float data = sR[c] < 0.f ? 0.f : sR[c];
-                a0 = fmaf(data, (float)sci[2 * c], a0);
-                a1 = fmaf(data, (float)sci[2 * c + 1], a1);
-                mm = mm + data;
-            }
-            c0 = __fmul_rn(a0, __frcp_rn(mm));  // centers.wgsl:82-83, a shader division
-            c1 = __fmul_rn(a1, __frcp_rn(mm));
-            m = mm;
+        // centers.wgsl:23-109 accumulation order (i outer, j inner): lane 0
+        // sums i P, lane 1 j P, the others P (fma(P, 1, m) is m + P)
+        float sum = 0.f;
+        for (int c = 0; c < K; ++c) {
+            const float data = sR[c] < 0.f ? 0.f : sR[c];
+            sum = fmaf(data, lane < 2 ? (float)sci[2 * c + lane] : 1.f, sum);
         }
-        c0 = __shfl_sync(0xffffffffu, c0, 0);
-        c1 = __shfl_sync(0xffffffffu, c1, 0);
-        m = __shfl_sync(0xffffffffu, m, 0);
+        const float m = __shfl_sync(0xffffffffu, sum, 2);
+        // centers.wgsl:82-83, a shader division
+        const float c0 = __fmul_rn(__shfl_sync(0xffffffffu, sum, 0), __frcp_rn(m));
+        const float c1 = __fmul_rn(__shfl_sync(0xffffffffu, sum, 1), __frcp_rn(m));
         if constexpr (MODE == ADJ_FORWARD) {
             if (lane == 0) {
                 yxm[3 * k] = (float)up + c0;
@@ -194,12 +271,24 @@ __global__ void __launch_bounds__(ADJ_NT) adjoint_particle_kernel(AdjParams p, c
         if constexpr (MODE == ADJ_BACKWARD) {
             const float gy = __ldg(grad + 3 * k), gx = __ldg(grad + 3 * k + 1), gm = __ldg(grad + 3 * k + 2);
             float ds = 0.f, dk = 0.f;
-            float* plane = gR + (size_t)t * H * W;
+            // link the peak to the tiles that its circle, widened by kr, meets
+            const int reach = p.rc + kr;
+            const int ty0 = max(ul - reach, 0) / tl.th, tx0 = max(vl - reach, 0) / TR_TW;
+            const int ny = min(ul + reach, H - 1) / tl.th - ty0 + 1, nx = min(vl + reach, W - 1) / TR_TW - tx0 + 1;
+            for (int q = lane; q < ny * nx; q += 32) {
+                const int entry = (int)(k * tl.slots) + q;
+                const int tile = (t * tl.nty + ty0 + q / nx) * tl.ntx + tx0 + q % nx;
+                tl.next[entry] = atomicExch(tl.head + tile, entry);
+            }
             for (int c = lane; c < K; c += 32) {
-                if (!(sR[c] > 0.f)) continue;
+                float* gc = tl.g + (size_t)k * K + c;
+                if (!(sR[c] > 0.f)) {
+                    *gc = 0.f;
+                    continue;
+                }
                 const float ic = (float)sci[2 * c], jc = (float)sci[2 * c + 1];
                 const float g = gm + (gy * (ic - c0) + gx * (jc - c1)) * inv_m;
-                atomicAdd(plane + (size_t)(ul + sci[2 * c]) * W + (vl + sci[2 * c + 1]), g);
+                *gc = g;
                 ds = fmaf(g, sD[c], ds);
                 dk = fmaf(g, 2.f * sB[c] / p.k, dk);
             }
@@ -267,7 +356,9 @@ __global__ void __launch_bounds__(ADJ_NT) adjoint_particle_kernel(AdjParams p, c
 
 // out[0..1] = the sums of part[2b], part[2b + 1] over blocks b in a fixed
 // order: thread i takes blocks i, i + 256, ... in order, then a fixed tree.
-__global__ void __launch_bounds__(256) adjoint_param_reduce_kernel(const double* part, int nblocks, double* out) {
+// `add`: onto the sums of earlier chunks of peaks.
+__global__ void __launch_bounds__(256) adjoint_param_reduce_kernel(const double* part, int nblocks, double* out,
+                                                                   int add) {
     __shared__ double sa[256], sc[256];
     double a = 0.0, c = 0.0;
     for (int b = threadIdx.x; b < nblocks; b += 256) {
@@ -285,209 +376,271 @@ __global__ void __launch_bounds__(256) adjoint_param_reduce_kernel(const double*
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        out[0] = sa[0];
-        out[1] = sc[0];
+        out[0] = add ? out[0] + sa[0] : sa[0];
+        out[1] = add ? out[1] + sc[0] : sc[0];
     }
 }
 
 // Transposed bandpass of dL/dR:  dL/dI = G^T gR - B^T gR.  G is separable,
 // symmetric and zero padded, so G^T is the same Gaussian pass; B^T weights
 // each tap by the number of reflect-padded window positions that land on it
-// (box_count), all of which lie within +-kr of the output pixel.  One CTA per
-// 32 x 64 output tile, gR staged with a kr halo (zero outside the frame).
+// (box_count), all of which lie within +-kr of the output pixel: 1 away from
+// the frame edges.  One CTA per tile of tr_th x 64 output pixels: the peaks
+// linked to it add their dL/dR to a shared plane with a kr halo, which two
+// separable passes over row pairs (packed FP32x2, 8 outputs per item) filter;
+// a tile without peaks is zero.  Bound by the arithmetic and shared memory
+// traffic of the passes, then by the gradient's write.
 template <int KRT>  // smoothing half window; 0 = taken from p.krad at run time
-__global__ void __launch_bounds__(TR_NT) adjoint_transpose_kernel(AdjParams p, const float* __restrict__ gR,
-                                                                  float* __restrict__ gI) {
+__global__ void __launch_bounds__(TR_NT) adjoint_transpose_kernel(AdjParams p, AdjTiles tl, const int* __restrict__ walk,
+                                                                  const int* __restrict__ circ,
+                                                                  float* __restrict__ gI, int frame0, int add) {
     extern __shared__ __align__(16) float tsm[];
+    constexpr int TH = tr_th(KRT), LIST = 256;
+    __shared__ int s_list[LIST];
+    __shared__ int s_n, s_more;
     const int kr = KRT > 0 ? KRT : p.krad;
-    const int H = p.H, W = p.W;
-    const int SH = TR_TH + 2 * kr, SW = TR_TW + 2 * kr;
-    constexpr int RS = TR_TW + 1;  // row stride of the row-pass planes (odd: conflict-free column reads)
-    float* S = tsm;               // SH x SW
-    float* RG = S + SH * SW;      // SH x RS, Gaussian row pass
-    float* RB = RG + SH * RS;     // SH x RS, box row pass
-    const int ntx = (W + TR_TW - 1) / TR_TW;
-    const int u0 = (blockIdx.x / ntx) * TR_TH, v0 = (blockIdx.x % ntx) * TR_TW;
-    const int t = blockIdx.y;
-    const float* src = gR + (size_t)t * H * W;
-    for (int q = threadIdx.x; q < SH * SW; q += TR_NT) {
-        const int r = q / SW, c = q - r * SW;
-        const int gu = u0 - kr + r, gv = v0 - kr + c;
-        S[q] = (gu >= 0 && gu < H && gv >= 0 && gv < W) ? __ldg(src + (size_t)gu * W + gv) : 0.f;
-    }
-    __syncthreads();
-    // away from the frame edges every box tap counts once
-    const bool cols_inner = v0 >= kr && v0 + TR_TW <= W - kr;
-    const bool rows_inner = u0 >= kr && u0 + TR_TH <= H - kr;
-    if (KRT > 0 && cols_inner) {
-        // 8 outputs of one row per item (taps loaded once), rows fastest
-        // across the lanes
-        constexpr int TP = 2 * KRT + 1, RF = 8, NCH = TR_TW / RF;
-        float a[TP];
-#pragma unroll
-        for (int j = 0; j < TP; ++j) a[j] = p.a[j];
-        for (int it = threadIdx.x; it < SH * NCH; it += TR_NT) {
-            const int ch = it / SH, r = it - ch * SH;
-            const int c0 = ch * RF;
-            const float* srow = S + r * SW + c0;
-            float v[RF + TP - 1];
-#pragma unroll
-            for (int i = 0; i < RF + TP - 1; ++i) v[i] = srow[i];
-            float* rg = RG + r * RS + c0;
-            float* rb = RB + r * RS + c0;
-#pragma unroll
-            for (int m = 0; m < RF; ++m) {
-                float g = 0.f;
-#pragma unroll
-                for (int j = 0; j < TP; ++j) g = fmaf(a[j], v[m + j], g);
-                rg[m] = g;
+    const int H = p.H, W = p.W, K = p.K;
+    const int SH = TH + 2 * kr, SW = TR_TW + 2 * kr;
+    const int SS = SW | 1;            // row pair strides, odd: conflict-free column of pairs
+    constexpr int RS = TR_TW | 1;
+    float2* S = (float2*)tsm;         // SH / 2 x SS
+    float2* RG = S + (SH / 2) * SS;   // SH / 2 x RS, Gaussian row pass
+    float2* RB = RG + (SH / 2) * RS;  // SH / 2 x RS, box row pass
+    const int u0 = (blockIdx.x / tl.ntx) * TH, v0 = (blockIdx.x % tl.ntx) * TR_TW;
+    const int t = frame0 + blockIdx.y;
+    float* dst = gI + (size_t)t * H * W;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // a scalar of the pair planes
+    auto at = [](float2* plane, int stride, int r, int c) -> float& {
+        return ((float*)plane)[(((r >> 1) * stride + c) << 1) + (r & 1)];
+    };
+    int entry = threadIdx.x == 0 ? tl.head[((size_t)t * tl.nty + blockIdx.x / tl.ntx) * tl.ntx + blockIdx.x % tl.ntx] : -1;
+    bool any = false;
+    while (true) {
+        if (threadIdx.x == 0) {
+            int n = 0;
+            for (; entry >= 0 && n < LIST; entry = __ldg(tl.next + entry)) s_list[n++] = entry / tl.slots;
+            s_n = n;
+            s_more = entry >= 0;
+        }
+        __syncthreads();
+        const int n = s_n;
+        if (n > 0 && !any) {
+            for (int q = threadIdx.x; q < (SH / 2) * SS; q += TR_NT) S[q] = make_float2(0.f, 0.f);
+            __syncthreads();
+            any = true;
+        }
+        for (int e = warp; e < n; e += TR_NT / 32) {
+            const long long k = s_list[e];
+            const int ru = __ldg(walk + 5 * k + 1) - u0 + kr, rv = __ldg(walk + 5 * k + 2) - v0 + kr;
+            for (int c = lane; c < K; c += 32) {
+                const float g = __ldg(tl.g + (size_t)k * K + c);
+                const int r = ru + __ldg(circ + 2 * c), x = rv + __ldg(circ + 2 * c + 1);
+                if (g != 0.f && r >= 0 && r < SH && x >= 0 && x < SW) atomicAdd(&at(S, SS, r, x), g);
             }
-            // direct sums, not a running difference: a window of zeros
-            // must give exactly zero (no gradient outside the particles)
+        }
+        const bool more = s_more != 0;
+        __syncthreads();
+        if (!more) break;
+    }
+    if (!any) {
+        if (add) return;
+        for (int q = threadIdx.x; q < TH * TR_TW; q += TR_NT) {
+            const int qu = u0 + q / TR_TW, qv = v0 + q % TR_TW;
+            if (qu < H && qv < W) dst[(size_t)qu * W + qv] = 0.f;
+        }
+        return;
+    }
+    auto put = [&](int qu, int qv, float v) {
+        float* d = dst + (size_t)qu * W + qv;
+        *d = add ? *d + v : v;
+    };
+    const float ikk = 1.f / p.kk;
+    // box sums along a row or column of length n whose outputs near its ends
+    // count reflected taps: tap(q) is the value at position q, 0 <= q < n
+    auto edge_box = [&](int q, int n, auto&& tap) {
+        float bx = 0.f;
+        for (int j = -kr; j <= kr; ++j) {
+            const int pp = q + j;
+            if (pp >= 0 && pp < n) bx = fmaf((float)box_count(pp, q, n, kr), tap(j), bx);
+        }
+        return bx;
+    };
+    if constexpr (KRT > 0) {
+        constexpr int TP = 2 * KRT + 1, F = 8;
+        float2 a2[TP];
 #pragma unroll
-            for (int m = 0; m < RF; ++m) {
-                float bs = 0.f;
+        for (int j = 0; j < TP; ++j) a2[j] = make_float2(p.a[j], p.a[j]);
+        // row pass: 8 outputs of a row pair per item, pairs fastest across the
+        // lanes.  Sums direct, not running: a window of zeros must give zero
+        constexpr int NPR = (TH + 2 * KRT) / 2;
+        for (int it = threadIdx.x; it < NPR * (TR_TW / F); it += TR_NT) {
+            const int c0 = it / NPR * F, pr = it % NPR;
+            const float2* srow = S + pr * SS + c0;
+            float2 v[F + TP - 1];
 #pragma unroll
-                for (int j = 0; j < TP; ++j) bs = bs + v[m + j];
-                rb[m] = bs;
+            for (int i = 0; i < F + TP - 1; ++i) v[i] = srow[i];
+#pragma unroll
+            for (int m = 0; m < F; ++m) {
+                float2 g = make_float2(0.f, 0.f), bs = v[m];
+#pragma unroll
+                for (int j = 0; j < TP; ++j) g = fma2(a2[j], v[m + j], g);
+#pragma unroll
+                for (int j = 1; j < TP; ++j) bs = add2(bs, v[m + j]);
+                RG[pr * RS + c0 + m] = g;
+                RB[pr * RS + c0 + m] = bs;
+            }
+        }
+        __syncthreads();
+        if (v0 < KRT || v0 + TR_TW > W - KRT) {
+            // columns within kr of the left or right frame edge
+            const int le = max(0, min(KRT, W) - v0), r0 = max(max(0, W - KRT - v0), le), r1 = min(TR_TW, W - v0);
+            const int ncol = le + max(0, r1 - r0);
+            for (int it = threadIdx.x; it < ncol * SH; it += TR_NT) {
+                const int q = it / SH, r = it - q * SH;
+                const int c = q < le ? q : r0 + (q - le);
+                at(RB, RS, r, c) = edge_box(v0 + c, W, [&](int j) { return at(S, SS, r, c + KRT + j); });
+            }
+            __syncthreads();
+        }
+        // column pass: 8 rows of one column per item, columns fastest
+        const bool rows_inner = u0 >= KRT && u0 + TH <= H - KRT;
+        for (int it = threadIdx.x; it < TR_TW * (TH / F); it += TR_NT) {
+            const int c = it % TR_TW, r0 = it / TR_TW * F;
+            if (u0 + r0 >= H || v0 + c >= W) continue;
+            float2 l[F / 2 + KRT], ml[F / 2 + KRT - 1];
+            float2 gs[F / 2], bs[F / 2];
+#pragma unroll
+            for (int i = 0; i < F / 2 + KRT; ++i) l[i] = RG[(r0 / 2 + i) * RS + c];
+#pragma unroll
+            for (int i = 0; i < F / 2 + KRT - 1; ++i) ml[i] = make_float2(l[i].y, l[i + 1].x);
+#pragma unroll
+            for (int m = 0; m < F / 2; ++m) {
+                gs[m] = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int j = 0; j < TP; ++j) gs[m] = fma2(a2[j], (j & 1) ? ml[m + (j >> 1)] : l[m + (j >> 1)], gs[m]);
+            }
+#pragma unroll
+            for (int i = 0; i < F / 2 + KRT; ++i) l[i] = RB[(r0 / 2 + i) * RS + c];
+#pragma unroll
+            for (int i = 0; i < F / 2 + KRT - 1; ++i) ml[i] = make_float2(l[i].y, l[i + 1].x);
+#pragma unroll
+            for (int m = 0; m < F / 2; ++m) {
+                bs[m] = l[m];
+#pragma unroll
+                for (int j = 1; j < TP; ++j) bs[m] = add2(bs[m], (j & 1) ? ml[m + (j >> 1)] : l[m + (j >> 1)]);
+            }
+#pragma unroll
+            for (int m = 0; m < F; ++m) {
+                const int qu = u0 + r0 + m;
+                if (qu >= H) break;
+                float bx = (m & 1) ? bs[m / 2].y : bs[m / 2].x;
+                if (!rows_inner && (qu < KRT || qu >= H - KRT))
+                    bx = edge_box(qu, H, [&](int j) { return at(RB, RS, r0 + m + KRT + j, c); });
+                put(qu, v0 + c, fmaf(-bx, ikk, (m & 1) ? gs[m / 2].y : gs[m / 2].x));
             }
         }
     } else {
         for (int q = threadIdx.x; q < SH * TR_TW; q += TR_NT) {
             const int r = q / TR_TW, c = q % TR_TW;
-            const int qv = v0 + c;
-            float g = 0.f, bx = 0.f;
-            const float* srow = S + r * SW + c + kr;
-            if (qv < W) {
-                for (int j = -kr; j <= kr; ++j) {
-                    const float v = srow[j];
-                    g = fmaf(p.a[j + kr], v, g);
-                    const int pv = qv + j;
-                    if (pv >= 0 && pv < W) bx = fmaf((float)box_count(pv, qv, W, kr), v, bx);
-                }
-            }
-            RG[r * RS + c] = g;
-            RB[r * RS + c] = bx;
+            if (v0 + c >= W) continue;
+            float g = 0.f;
+            for (int j = 0; j <= 2 * kr; ++j) g = fmaf(p.a[j], at(S, SS, r, c + j), g);
+            at(RG, RS, r, c) = g;
+            at(RB, RS, r, c) = edge_box(v0 + c, W, [&](int j) { return at(S, SS, r, c + kr + j); });
         }
-    }
-    __syncthreads();
-    float* dst = gI + (size_t)t * H * W;
-    const float ikk = 1.f / p.kk;
-    if (KRT > 0 && rows_inner && v0 + TR_TW <= W) {
-        // 8 outputs of one column per item, columns fastest across the lanes
-        constexpr int TP = 2 * KRT + 1, CF = 8;
-        float a[TP];
-#pragma unroll
-        for (int j = 0; j < TP; ++j) a[j] = p.a[j];
-        for (int it = threadIdx.x; it < TR_TW * (TR_TH / CF); it += TR_NT) {
-            const int c = it % TR_TW, r0 = (it / TR_TW) * CF;
-            float g[CF + TP - 1], b[CF + TP - 1];
-#pragma unroll
-            for (int i = 0; i < CF + TP - 1; ++i) {
-                g[i] = RG[(r0 + i) * RS + c];
-                b[i] = RB[(r0 + i) * RS + c];
-            }
-#pragma unroll
-            for (int m = 0; m < CF; ++m) {
-                float bs = 0.f;
-#pragma unroll
-                for (int i = 0; i < TP; ++i) bs = bs + b[m + i];
-                float gs = 0.f;
-#pragma unroll
-                for (int i = 0; i < TP; ++i) gs = fmaf(a[i], g[m + i], gs);
-                dst[(size_t)(u0 + r0 + m) * W + (v0 + c)] = fmaf(-bs, ikk, gs);
-            }
-        }
-    } else {
-        for (int q = threadIdx.x; q < TR_TH * TR_TW; q += TR_NT) {
+        __syncthreads();
+        for (int q = threadIdx.x; q < TH * TR_TW; q += TR_NT) {
             const int r = q / TR_TW, c = q % TR_TW;
-            const int qu = u0 + r, qv = v0 + c;
-            if (qu >= H || qv >= W) continue;
-            float g = 0.f, bx = 0.f;
-            for (int i = -kr; i <= kr; ++i) {
-                const int rr = (r + kr + i) * RS + c;
-                g = fmaf(p.a[i + kr], RG[rr], g);
-                const int pu = qu + i;
-                if (pu >= 0 && pu < H) bx = fmaf((float)box_count(pu, qu, H, kr), RB[rr], bx);
-            }
-            dst[(size_t)qu * W + qv] = fmaf(-bx, ikk, g);
+            if (u0 + r >= H || v0 + c >= W) continue;
+            float g = 0.f;
+            for (int i = 0; i <= 2 * kr; ++i) g = fmaf(p.a[i], at(RG, RS, r + i, c), g);
+            const float bx = edge_box(u0 + r, H, [&](int j) { return at(RB, RS, r + kr + j, c); });
+            put(u0 + r, v0 + c, fmaf(-bx, ikk, g));
         }
     }
 }
 
-size_t adjoint_particle_smem(int K) { return sizeof(float) * (size_t)(2 * K + (ADJ_NT / 32) * 6 * K); }
-
-size_t adjoint_transpose_smem(int kr) {
-    const int SH = TR_TH + 2 * kr, SW = TR_TW + 2 * kr;
-    return sizeof(float) * (size_t)(SH * SW + 2 * SH * (TR_TW + 1));
-}
+namespace {
+int adj_radius(const AdjParams& p) { return p.rc == p.krad && p.krad <= 7 ? p.krad : 0; }
+}  // namespace
 
 // Upper bound of the particle kernel's grid (partial sums of the backward
 // pass: two doubles per block).
 int adjoint_particle_blocks_max(int num_sms) { return num_sms * 16; }
 
+// Tile lists of the backward pass: tiles per frame and the most tiles that a
+// peak reaches (its circle widened by the smoothing radius).
+void adjoint_tiles(const AdjParams& p, AdjTiles* tl) {
+    tl->th = tr_th(p.krad >= 1 && p.krad <= 7 ? p.krad : 0);
+    tl->nty = (p.H + tl->th - 1) / tl->th;
+    tl->ntx = (p.W + TR_TW - 1) / TR_TW;
+    const int ext = 2 * (p.rc + p.krad);
+    tl->slots = (ext / tl->th + 2) * (ext / TR_TW + 2);
+}
+
+template <int MODE, int R>
+cudaError_t particles_launch(const AdjParams& p, const float* frames, const int* walk, long long n, const int* circ,
+                             const float* grad, float* yxm, const AdjTiles& tl, double* gpar, int* err, int grid,
+                             cudaStream_t st) {
+    const size_t smem = sizeof(float) * (size_t)(2 * p.K + (ADJ_NT / 32) * adj_warp_floats(MODE, R, p.K));
+    const auto fn = adjoint_particle_kernel<MODE, R>;
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e) return e;
+    fn<<<grid, ADJ_NT, smem, st>>>(p, frames, walk, n, circ, grad, yxm, tl, gpar, err);
+    return cudaGetLastError();
+}
+
+// BACKWARD: `add` keeps the parameter gradients of earlier chunks of peaks.
 cudaError_t launch_adjoint_particles(int mode, const AdjParams& p, const float* frames, const int* walk, long long n,
-                                     const int* circ, const float* grad, float* yxm, float* gR, double* gpar,
-                                     double* gpart, int* err, int num_sms, cudaStream_t st) {
+                                     const int* circ, const float* grad, float* yxm, const AdjTiles& tl, double* gpar,
+                                     double* gpart, int* err, int add, int num_sms, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const size_t smem = adjoint_particle_smem(p.K);
     const int grid = (int)std::min<long long>((n + ADJ_NT / 32 - 1) / (ADJ_NT / 32), (long long)num_sms * 16);
-    cudaError_t e = cudaSuccess;
-    switch (mode) {
-        case ADJ_FORWARD:
-            e = cudaFuncSetAttribute(adjoint_particle_kernel<ADJ_FORWARD>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e) return e;
-            adjoint_particle_kernel<ADJ_FORWARD><<<grid, ADJ_NT, smem, st>>>(p, frames, walk, n, circ, grad, yxm,
-                                                                             gR, gpar, err);
-            break;
-        case ADJ_BACKWARD:
-            e = cudaFuncSetAttribute(adjoint_particle_kernel<ADJ_BACKWARD>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e) return e;
-            adjoint_particle_kernel<ADJ_BACKWARD><<<grid, ADJ_NT, smem, st>>>(p, frames, walk, n, circ, grad, yxm,
-                                                                              gR, gpart, err);
-            e = cudaGetLastError();
-            if (e) return e;
-            adjoint_param_reduce_kernel<<<1, 256, 0, st>>>(gpart, grid, gpar);
-            break;
-        default:
-            e = cudaFuncSetAttribute(adjoint_particle_kernel<ADJ_UNCERTAINTY>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e) return e;
-            adjoint_particle_kernel<ADJ_UNCERTAINTY><<<grid, ADJ_NT, smem, st>>>(p, frames, walk, n, circ, grad,
-                                                                                 yxm, gR, gpar, err);
-            break;
+    double* out = mode == ADJ_BACKWARD ? gpart : gpar;
+    cudaError_t e = cudaErrorInvalidValue;
+#define ADJ_CASE(R)                                                                                               \
+    case R:                                                                                                       \
+        e = mode == ADJ_FORWARD                                                                                   \
+                ? particles_launch<ADJ_FORWARD, R>(p, frames, walk, n, circ, grad, yxm, tl, out, err, grid, st)   \
+            : mode == ADJ_BACKWARD                                                                                \
+                ? particles_launch<ADJ_BACKWARD, R>(p, frames, walk, n, circ, grad, yxm, tl, out, err, grid, st)  \
+                : particles_launch<ADJ_UNCERTAINTY, R>(p, frames, walk, n, circ, grad, yxm, tl, out, err, grid, st); \
+        break;
+    switch (adj_radius(p)) {
+        ADJ_CASE(0) ADJ_CASE(1) ADJ_CASE(2) ADJ_CASE(3) ADJ_CASE(4) ADJ_CASE(5) ADJ_CASE(6) ADJ_CASE(7)
     }
+#undef ADJ_CASE
+    if (e || mode != ADJ_BACKWARD) return e;
+    adjoint_param_reduce_kernel<<<1, 256, 0, st>>>(gpart, grid, gpar, add);
     return cudaGetLastError();
 }
 
 template <int KRT>
-cudaError_t transpose_launch(const AdjParams& p, const float* gR, float* gI, size_t smem, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(adjoint_transpose_kernel<KRT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+cudaError_t transpose_launch(const AdjParams& p, const AdjTiles& tl, const int* walk, const int* circ, float* gI, int add,
+                             cudaStream_t st) {
+    const int SH = tl.th + 2 * p.krad, SW = TR_TW + 2 * p.krad;
+    const size_t smem = sizeof(float2) * (size_t)(SH / 2) * ((SW | 1) + 2 * (TR_TW | 1));
+    const auto fn = adjoint_transpose_kernel<KRT>;
+    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e) return e;
-    const int ntx = (p.W + TR_TW - 1) / TR_TW, nty = (p.H + TR_TH - 1) / TR_TH;
-    for (int f0 = 0; f0 < p.T; f0 += 65535) {
-        const int nf = std::min(65535, p.T - f0);
-        dim3 grid(ntx * nty, nf);
-        adjoint_transpose_kernel<KRT><<<grid, TR_NT, smem, st>>>(p, gR + (size_t)f0 * p.H * p.W,
-                                                                 gI + (size_t)f0 * p.H * p.W);
-    }
+    for (int f0 = 0; f0 < p.T; f0 += 65535)
+        fn<<<dim3(tl.ntx * tl.nty, std::min(65535, p.T - f0)), TR_NT, smem, st>>>(p, tl, walk, circ, gI, f0, add);
     return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_transpose(const AdjParams& p, const float* gR, float* gI, cudaStream_t st) {
-    const size_t smem = adjoint_transpose_smem(p.krad);
+// `add`: onto the gradient of earlier chunks of peaks.
+cudaError_t launch_adjoint_transpose(const AdjParams& p, const AdjTiles& tl, const int* walk, const int* circ, float* gI,
+                                     int add, cudaStream_t st) {
     switch (p.krad) {
-        case 1: return transpose_launch<1>(p, gR, gI, smem, st);
-        case 2: return transpose_launch<2>(p, gR, gI, smem, st);
-        case 3: return transpose_launch<3>(p, gR, gI, smem, st);
-        case 4: return transpose_launch<4>(p, gR, gI, smem, st);
-        case 5: return transpose_launch<5>(p, gR, gI, smem, st);
-        case 6: return transpose_launch<6>(p, gR, gI, smem, st);
-        case 7: return transpose_launch<7>(p, gR, gI, smem, st);
-        default: return transpose_launch<0>(p, gR, gI, smem, st);
+        case 1: return transpose_launch<1>(p, tl, walk, circ, gI, add, st);
+        case 2: return transpose_launch<2>(p, tl, walk, circ, gI, add, st);
+        case 3: return transpose_launch<3>(p, tl, walk, circ, gI, add, st);
+        case 4: return transpose_launch<4>(p, tl, walk, circ, gI, add, st);
+        case 5: return transpose_launch<5>(p, tl, walk, circ, gI, add, st);
+        case 6: return transpose_launch<6>(p, tl, walk, circ, gI, add, st);
+        case 7: return transpose_launch<7>(p, tl, walk, circ, gI, add, st);
+        default: return transpose_launch<0>(p, tl, walk, circ, gI, add, st);
     }
 }
 

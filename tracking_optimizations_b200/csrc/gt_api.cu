@@ -48,10 +48,12 @@ cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaSt
                                const MovieBufs& b, int T, int frame0, int* used_tma);
 void gauss_taps(int smoothing_size, float noise_size, int normalized, float* w, float* norm, float* rn);
 cudaError_t launch_adjoint_particles(int mode, const AdjParams& p, const float* frames, const int* walk, long long n,
-                                     const int* circ, const float* grad, float* yxm, float* gR, double* gpar,
-                                     double* gpart, int* err, int num_sms, cudaStream_t st);
+                                     const int* circ, const float* grad, float* yxm, const AdjTiles& tl, double* gpar,
+                                     double* gpart, int* err, int add, int num_sms, cudaStream_t st);
+void adjoint_tiles(const AdjParams& p, AdjTiles* tl);
 int adjoint_particle_blocks_max(int num_sms);
-cudaError_t launch_adjoint_transpose(const AdjParams& p, const float* gR, float* gI, cudaStream_t st);
+cudaError_t launch_adjoint_transpose(const AdjParams& p, const AdjTiles& tl, const int* walk, const int* circ, float* gI,
+                                     int add, cudaStream_t st);
 int traj_filter_stubs(const int64_t* h_ids, int64_t n, int64_t threshold, uint8_t* h_keep, int64_t* h_count,
                       int64_t* nkept, cudaStream_t st, int num_sms, std::string* msg);
 int traj_steps(const int64_t* h_ids, const float* h_x, const float* h_y, int64_t n, float mppf, float* h_xs,
@@ -1433,27 +1435,37 @@ int adjoint_setup(gt_ctx* ctx, const float* d_frames, int T, int H, int W, const
 }
 
 // Scratch of the gt_adjoint_* calls in the context arena: the error word,
-// the circle table and (backward only) the dL/dR plane.
+// the circle table and (backward only) the partial parameter gradients and the
+// tile lists of a chunk of peaks.
 struct AdjWork {
     int* err;
     int* circ;
-    float* plane;
-    double* gpart;  // per-block partial parameter gradients (backward only)
+    double* gpart;
+    AdjTiles tl{};
+    int64_t chunk = 0;  // peaks per chunk
 };
 
-int adjoint_work(gt_ctx* ctx, const AdjParams& ap, const std::vector<int>& circ, bool plane, AdjWork* aw,
+int adjoint_work(gt_ctx* ctx, const AdjParams& ap, const std::vector<int>& circ, int64_t n_back, AdjWork* aw,
                  cudaStream_t st) {
-    const size_t off_circ = 256;
-    const size_t off_part = off_circ + ((sizeof(int) * circ.size() + 255) / 256) * 256;
-    const size_t n_part = 2 * (size_t)adjoint_particle_blocks_max(ctx->num_sms);
-    const size_t off_plane = off_part + ((sizeof(double) * n_part + 255) / 256) * 256;
-    const size_t need = off_plane + (plane ? sizeof(float) * (size_t)ap.T * ap.H * ap.W : 0);
-    int rc = ensure_arena(ctx, need);
+    auto layout = [&](char* base) {
+        Carver c{base};
+        aw->err = c.take<int>(1);
+        aw->circ = c.take<int>(circ.size());
+        aw->gpart = c.take<double>(2 * (size_t)adjoint_particle_blocks_max(ctx->num_sms));
+        if (n_back >= 0) {
+            adjoint_tiles(ap, &aw->tl);
+            // up to 2^23 peaks and 1 GB of dL/dR at a time
+            aw->chunk = std::min<int64_t>({std::max<int64_t>(n_back, 1), (int64_t)1 << 23,
+                                           std::max<int64_t>(1, ((int64_t)1 << 28) / ap.K)});
+            aw->tl.g = c.take<float>((size_t)aw->chunk * ap.K);
+            aw->tl.next = c.take<int>((size_t)aw->chunk * aw->tl.slots);
+            aw->tl.head = c.take<int>((size_t)ap.T * aw->tl.nty * aw->tl.ntx);
+        }
+        return c.off + 256;
+    };
+    const int rc = ensure_arena(ctx, layout(nullptr));
     if (rc) return rc;
-    aw->err = (int*)ctx->arena;
-    aw->circ = (int*)(ctx->arena + off_circ);
-    aw->gpart = (double*)(ctx->arena + off_part);
-    aw->plane = plane ? (float*)(ctx->arena + off_plane) : nullptr;
+    layout(ctx->arena);
     CK(cudaMemsetAsync(aw->err, 0, sizeof(int), st));
     CK(cudaMemcpyAsync(aw->circ, circ.data(), sizeof(int) * circ.size(), cudaMemcpyHostToDevice, st));
     for (int i = 0; i < 3; ++i)
@@ -1686,10 +1698,10 @@ int gt_adjoint_forward(gt_ctx* ctx, const float* d_frames, int T, int H, int W, 
     if (n > 0 && !d_yxm) { ctx->err = "null output"; return GT_ERR_ARG; }
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     AdjWork aw;
-    rc = adjoint_work(ctx, ap, circ, false, &aw, st);
+    rc = adjoint_work(ctx, ap, circ, -1, &aw, st);
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[0], st));
-    CK(launch_adjoint_particles(0, ap, d_frames, d_walk, n, aw.circ, nullptr, d_yxm, nullptr, nullptr, nullptr, aw.err,
+    CK(launch_adjoint_particles(0, ap, d_frames, d_walk, n, aw.circ, nullptr, d_yxm, aw.tl, nullptr, nullptr, aw.err, 0,
                                 ctx->num_sms, st));
     CK(cudaEventRecord(ctx->ev[1], st));
     ctx->stats.launches = n > 0 ? 1 : 0;
@@ -1709,20 +1721,30 @@ int gt_adjoint_backward(gt_ctx* ctx, const float* d_frames, int T, int H, int W,
     if (!d_grad_frames || !d_grad_params || (n > 0 && !d_grad_yxm)) { ctx->err = "null output"; return GT_ERR_ARG; }
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     AdjWork aw;
-    rc = adjoint_work(ctx, ap, circ, true, &aw, st);
+    rc = adjoint_work(ctx, ap, circ, n, &aw, st);
     if (rc) return rc;
+    for (int i = 0; i < 4; ++i)
+        if (!ctx->ev[i]) CK(cudaEventCreate(&ctx->ev[i]));
     if (n == 0) CK(cudaMemsetAsync(d_grad_params, 0, 2 * sizeof(double), st));
-    CK(cudaEventRecord(ctx->ev[0], st));
-    CK(cudaMemsetAsync(aw.plane, 0, sizeof(float) * (size_t)T * H * W, st));
-    CK(cudaEventRecord(ctx->ev[1], st));
-    CK(launch_adjoint_particles(1, ap, d_frames, d_walk, n, aw.circ, d_grad_yxm, nullptr, aw.plane, d_grad_params,
-                                aw.gpart, aw.err, ctx->num_sms, st));
-    CK(cudaEventRecord(ctx->ev[2], st));
-    CK(launch_adjoint_transpose(ap, aw.plane, d_grad_frames, st));
-    ctx->stats.launches = (n > 0 ? 2 : 0) + (T + 65534) / 65535;
-    // the dense part is the zeroing plus the transposed bandpass
-    if (!ctx->ev[3]) CK(cudaEventCreate(&ctx->ev[3]));
-    CK(cudaEventRecord(ctx->ev[3], st));
+    const size_t heads = sizeof(int) * (size_t)T * aw.tl.nty * aw.tl.ntx;
+    ctx->stats.launches = 0;
+    // the peaks in chunks (one, unless there are millions); the dense part is
+    // the empty lists plus the transposed bandpass.  Times: the last chunk's
+    int64_t k0 = 0;
+    do {
+        const int64_t nk = std::min<int64_t>(aw.chunk, n - k0);
+        const int add = k0 > 0;
+        CK(cudaEventRecord(ctx->ev[0], st));
+        CK(cudaMemsetAsync(aw.tl.head, 0xff, heads, st));
+        CK(cudaEventRecord(ctx->ev[1], st));
+        CK(launch_adjoint_particles(1, ap, d_frames, d_walk + 5 * k0, nk, aw.circ, d_grad_yxm + 3 * k0, nullptr, aw.tl,
+                                    d_grad_params, aw.gpart, aw.err, add, ctx->num_sms, st));
+        CK(cudaEventRecord(ctx->ev[2], st));
+        CK(launch_adjoint_transpose(ap, aw.tl, d_walk + 5 * k0, aw.circ, d_grad_frames, add, st));
+        CK(cudaEventRecord(ctx->ev[3], st));
+        ctx->stats.launches += (nk > 0 ? 2 : 0) + (T + 65534) / 65535;
+        k0 += nk;
+    } while (k0 < n);
     rc = adjoint_finish(ctx, aw, st);
     cudaEventElapsedTime(&ctx->stats.ms_adjoint_particles, ctx->ev[1], ctx->ev[2]);
     float tz = 0.f, tt = 0.f;
@@ -1749,10 +1771,10 @@ int gt_adjoint_uncertainty(gt_ctx* ctx, const float* d_frames, int T, int H, int
     ap.read_var = read_noise * read_noise;
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     AdjWork aw;
-    rc = adjoint_work(ctx, ap, circ, false, &aw, st);
+    rc = adjoint_work(ctx, ap, circ, -1, &aw, st);
     if (rc) return rc;
     CK(cudaEventRecord(ctx->ev[0], st));
-    CK(launch_adjoint_particles(2, ap, d_frames, d_walk, n, aw.circ, nullptr, d_sd, nullptr, nullptr, nullptr, aw.err,
+    CK(launch_adjoint_particles(2, ap, d_frames, d_walk, n, aw.circ, nullptr, d_sd, aw.tl, nullptr, nullptr, aw.err, 0,
                                 ctx->num_sms, st));
     CK(cudaEventRecord(ctx->ev[1], st));
     ctx->stats.launches = n > 0 ? 1 : 0;

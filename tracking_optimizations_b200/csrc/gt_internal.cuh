@@ -175,6 +175,17 @@ struct AdjParams {
     float gain, read_var;    // noise model of the uncertainty kernel
 };
 
+// The backward pass's dL/dR: K values per peak of the chunk, and per output
+// tile (frame, tile row, tile column) a list of the peaks that reach it, entry
+// = peak * slots + one of its tiles.
+struct AdjTiles {
+    float* g;
+    int* head;  // -1: no peak
+    int* next;
+    int slots;
+    int th, nty, ntx;  // tile rows (columns: 64) and tiles per frame
+};
+
 struct AsmArgs {
     int T, H, W, cap_p, cap_c, ncols;
     int has_link, cpu_processed, characterize, sig, bg;
