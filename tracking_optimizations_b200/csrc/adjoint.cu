@@ -110,53 +110,84 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 enum AdjMode { ADJ_FORWARD = 0, ADJ_BACKWARD = 1, ADJ_UNCERTAINTY = 2 };
 
-// Shared floats of a warp: R, B, dG/ds at the circle pixels and 3K of the
-// uncertainty; with a compile-time radius also the raw window and the row
-// pass's sums over it.
-__host__ __device__ constexpr int adj_window(int r) { return (4 * r + 1) * (4 * r + 1); }
+// Circle pixels of radius R (i * i + j * j <= R * R), in table order.
+__host__ __device__ constexpr int circle_size(int R) {
+    int k = 0;
+    for (int i = -R; i <= R; ++i)
+        for (int j = -R; j <= R; ++j) k += i * i + j * j <= R * R;
+    return k;
+}
+
+// Shared floats of a warp, a multiple of 4: R, B, dG/ds at the circle pixels
+// and 3K of the uncertainty; with a compile-time radius also the clipped
+// values, the raw window and the row pass's sums over it.
+__host__ __device__ constexpr int round4(int x) { return (x + 3) / 4 * 4; }
 __host__ __device__ constexpr int adj_rows(int r) { return (4 * r + 1) * (2 * r + 1); }
 __host__ __device__ constexpr int adj_warp_floats(int mode, int r, int K) {
-    return 6 * K + (r > 0 ? adj_window(r) + adj_rows(r) * (mode == 1 ? 4 : 2) : 0);
+    return r > 0 ? round4(K) + round4(6 * K + (4 * r + 1) * (4 * r + 1) + adj_rows(r) * (mode == 1 ? 4 : 2)) : round4(6 * K);
 }
 
 // The bandpass at the circle pixels of a peak whose whole window lies inside
 // the frame (smoothing radius = circle radius = R): the raw window once into
 // shared memory, the row sums once per (row, circle column), the column sums
-// per circle pixel -- the values of bandpass_terms in the same order.
+// per circle pixel -- the values of bandpass_terms in the same order.  Bound
+// by instructions issued, so lanes map to rows and columns without divisions.
 template <int MODE, int R>
-__device__ __forceinline__ void window_terms(const AdjParams& p, const float* fr, int ul, int vl, int K, const int* sci,
+__device__ __forceinline__ void window_terms(const AdjParams& p, const float* fr, int ul, int vl, const int* sci,
                                              float* win, float* sR, float* sB, float* sD) {
-    constexpr int WS = 4 * R + 1, CW = 2 * R + 1, NP = WS * CW;
+    constexpr int WS = 4 * R + 1, CW = 2 * R + 1, NP = WS * CW, K = circle_size(R);
+    constexpr int LW = WS <= 8 ? 8 : WS <= 16 ? 16 : 32, LC = CW <= 4 ? 4 : CW <= 8 ? 8 : 16;  // lanes per row
     const int lane = threadIdx.x & 31;
     float* rg = win + WS * WS;
     float* rb = rg + NP;
     float* ra = rb + NP;
     float* rd = ra + NP;
-    const float* src = fr + (size_t)(ul - 2 * R) * p.W + (vl - 2 * R);
-    for (int q = lane; q < WS * WS; q += 32) win[q] = __ldg(src + (size_t)(q / WS) * p.W + q % WS);
-    __syncwarp();
-    for (int q = lane; q < NP; q += 32) {
-        const float* w = win + (q / CW) * WS + q % CW;
-        float g = 0.f, b = 0.f, a = 0.f, d = 0.f;
+    {
+        const int r0 = lane / LW, c = lane % LW;
+        const float* src = fr + (size_t)(ul - 2 * R + r0) * p.W + (vl - 2 * R + c);
+        const size_t step = (size_t)(32 / LW) * p.W;
+        if (c < WS) {
 #pragma unroll
-        for (int j = 0; j < CW; ++j) {
-            const float v = w[j];
-            g = fmaf(p.w[j], v, g);
-            b = b + v;
-            if (MODE == 1) {
-                a = fmaf(p.a[j], v, a);
-                d = fmaf(p.da[j], v, d);
+            for (int r = 0; r < WS; r += 32 / LW) {
+                if (r + r0 < WS) win[(r + r0) * WS + c] = __ldg(src);
+                src += step;
             }
-        }
-        rg[q] = g * p.rn;
-        rb[q] = b;
-        if (MODE == 1) {
-            ra[q] = a;
-            rd[q] = d;
         }
     }
     __syncwarp();
-    for (int c = lane; c < K; c += 32) {
+    {
+        const int r0 = lane / LC, c = lane % LC;
+        if (c < CW) {
+#pragma unroll
+            for (int r = 0; r < WS; r += 32 / LC) {
+                if (r + r0 >= WS) break;
+                const float* w = win + (r + r0) * WS + c;
+                float g = 0.f, b = 0.f, a = 0.f, d = 0.f;
+#pragma unroll
+                for (int j = 0; j < CW; ++j) {
+                    const float v = w[j];
+                    g = fmaf(p.w[j], v, g);
+                    b = b + v;
+                    if (MODE == 1) {
+                        a = fmaf(p.a[j], v, a);
+                        d = fmaf(p.da[j], v, d);
+                    }
+                }
+                const int q = (r + r0) * CW + c;
+                rg[q] = g * p.rn;
+                rb[q] = b;
+                if (MODE == 1) {
+                    ra[q] = a;
+                    rd[q] = d;
+                }
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c0 = 0; c0 < K; c0 += 32) {
+        const int c = c0 + lane;
+        if (c >= K) break;
         const int q0 = (sci[2 * c] + R) * CW + sci[2 * c + 1] + R;
         float gs = 0.f, cs = 0.f, dg = 0.f;
 #pragma unroll
@@ -177,6 +208,31 @@ __device__ __forceinline__ void window_terms(const AdjParams& p, const float* fr
     }
 }
 
+// Centroid sums over the clipped circle values P (16-byte aligned) in
+// centers.wgsl:23-109 order (i outer, j inner), every lane alike.
+template <int R>
+__device__ __forceinline__ void circle_sums(const float* P, float& a0, float& a1, float& mm) {
+    constexpr int K = circle_size(R);
+    float v[round4(K)];
+#pragma unroll
+    for (int q = 0; q < K; q += 4) {
+        const float4 z = *(const float4*)(P + q);
+        v[q] = z.x; v[q + 1] = z.y; v[q + 2] = z.z; v[q + 3] = z.w;
+    }
+    a0 = a1 = mm = 0.f;
+    int q = 0;
+#pragma unroll
+    for (int i = -R; i <= R; ++i)
+#pragma unroll
+        for (int j = -R; j <= R; ++j) {
+            if (i * i + j * j > R * R) continue;
+            a0 = fmaf(v[q], (float)i, a0);
+            a1 = fmaf(v[q], (float)j, a1);
+            mm = mm + v[q];
+            ++q;
+        }
+}
+
 // One warp per particle (grid-stride over warps), ADJ_NT / 32 warps per
 // CTA sharing the circle table.  walk rows: {frame, ul, vl, up, vp}.
 // FORWARD writes yxm (n x 3).  BACKWARD reads grad (n x 3), writes dL/dR at the
@@ -192,10 +248,11 @@ __global__ void __launch_bounds__(ADJ_NT) adjoint_particle_kernel(AdjParams p, c
                                                                   AdjTiles tl, double* gpar, int* err) {
     extern __shared__ __align__(16) float asm_[];
     constexpr int NW = ADJ_NT / 32;
-    const int K = p.K;
+    const int K = R > 0 ? circle_size(R) : p.K;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int* sci = (int*)asm_;                      // 2K circle offsets {i, j}, shared
-    float* sR = asm_ + 2 * K + wid * adj_warp_floats(MODE, R, K);  // this warp's R at the circle pixels
+    float* sP = asm_ + round4(2 * K) + wid * adj_warp_floats(MODE, R, K);
+    float* sR = sP + (R > 0 ? round4(K) : 0);   // this warp's R at the circle pixels
     float* sB = sR + K;                         // B
     float* sD = sB + K;                         // dG/ds
     float* sJ = sD + K;                         // 3K: dy/dR, dx/dR, dm/dR (uncertainty)
@@ -230,7 +287,7 @@ __global__ void __launch_bounds__(ADJ_NT) adjoint_particle_kernel(AdjParams p, c
         const float* fr = frames + (size_t)t * H * W;
         __syncwarp();  // the previous particle's reads of this warp's arrays are done
         if (R > 0 && ul - 2 * R >= 0 && ul + 2 * R < H && vl - 2 * R >= 0 && vl + 2 * R < W) {
-            window_terms<MODE, R>(p, fr, ul, vl, K, sci, win, sR, sB, sD);
+            window_terms<MODE, R>(p, fr, ul, vl, sci, win, sR, sB, sD);
         } else {
             for (int c = lane; c < K; c += 32) {
                 const BpTerms bt = bandpass_terms(p, fr, ul + sci[2 * c], vl + sci[2 * c + 1]);
@@ -240,17 +297,25 @@ __global__ void __launch_bounds__(ADJ_NT) adjoint_particle_kernel(AdjParams p, c
             }
         }
         __syncwarp();
-        // centers.wgsl:23-109 accumulation order (i outer, j inner): lane 0
-        // sums i P, lane 1 j P, the others P (fma(P, 1, m) is m + P)
-        float sum = 0.f;
-        for (int c = 0; c < K; ++c) {
-            const float data = sR[c] < 0.f ? 0.f : sR[c];
-            sum = fmaf(data, lane < 2 ? (float)sci[2 * c + lane] : 1.f, sum);
+        float c0, c1, m;
+        if constexpr (R > 0) {
+            for (int c = lane; c < K; c += 32) sP[c] = sR[c] < 0.f ? 0.f : sR[c];
+            __syncwarp();
+            circle_sums<R>(sP, c0, c1, m);
+        } else {
+            // centers.wgsl:23-109 accumulation order (i outer, j inner): lane 0
+            // sums i P, lane 1 j P, the others P (fma(P, 1, m) is m + P)
+            float sum = 0.f;
+            for (int c = 0; c < K; ++c) {
+                const float data = sR[c] < 0.f ? 0.f : sR[c];
+                sum = fmaf(data, lane < 2 ? (float)sci[2 * c + lane] : 1.f, sum);
+            }
+            c0 = __shfl_sync(0xffffffffu, sum, 0);
+            c1 = __shfl_sync(0xffffffffu, sum, 1);
+            m = __shfl_sync(0xffffffffu, sum, 2);
         }
-        const float m = __shfl_sync(0xffffffffu, sum, 2);
-        // centers.wgsl:82-83, a shader division
-        const float c0 = __fmul_rn(__shfl_sync(0xffffffffu, sum, 0), __frcp_rn(m));
-        const float c1 = __fmul_rn(__shfl_sync(0xffffffffu, sum, 1), __frcp_rn(m));
+        c0 = __fmul_rn(c0, __frcp_rn(m));  // centers.wgsl:82-83, a shader division
+        c1 = __fmul_rn(c1, __frcp_rn(m));
         if constexpr (MODE == ADJ_FORWARD) {
             if (lane == 0) {
                 yxm[3 * k] = (float)up + c0;
@@ -276,9 +341,14 @@ __global__ void __launch_bounds__(ADJ_NT) adjoint_particle_kernel(AdjParams p, c
             const int ty0 = max(ul - reach, 0) / tl.th, tx0 = max(vl - reach, 0) / TR_TW;
             const int ny = min(ul + reach, H - 1) / tl.th - ty0 + 1, nx = min(vl + reach, W - 1) / TR_TW - tx0 + 1;
             for (int q = lane; q < ny * nx; q += 32) {
-                const int entry = (int)(k * tl.slots) + q;
                 const int tile = (t * tl.nty + ty0 + q / nx) * tl.ntx + tx0 + q % nx;
-                tl.next[entry] = atomicExch(tl.head + tile, entry);
+                const int at = atomicAdd(tl.count + tile, 1);
+                if (at < TILE_PEAKS) {
+                    tl.peaks[(size_t)tile * TILE_PEAKS + at] = (int)k;
+                } else {
+                    const int entry = (int)(k * tl.slots) + q;
+                    tl.next[entry] = atomicExch(tl.head + tile, entry + 1);
+                }
             }
             for (int c = lane; c < K; c += 32) {
                 float* gc = tl.g + (size_t)k * K + c;
@@ -397,7 +467,7 @@ __global__ void __launch_bounds__(TR_NT) adjoint_transpose_kernel(AdjParams p, A
     extern __shared__ __align__(16) float tsm[];
     constexpr int TH = tr_th(KRT), LIST = 256;
     __shared__ int s_list[LIST];
-    __shared__ int s_n, s_more;
+    __shared__ int s_n, s_entry;
     const int kr = KRT > 0 ? KRT : p.krad;
     const int H = p.H, W = p.W, K = p.K;
     const int SH = TH + 2 * kr, SW = TR_TW + 2 * kr;
@@ -414,22 +484,23 @@ __global__ void __launch_bounds__(TR_NT) adjoint_transpose_kernel(AdjParams p, A
     auto at = [](float2* plane, int stride, int r, int c) -> float& {
         return ((float*)plane)[(((r >> 1) * stride + c) << 1) + (r & 1)];
     };
-    int entry = threadIdx.x == 0 ? tl.head[((size_t)t * tl.nty + blockIdx.x / tl.ntx) * tl.ntx + blockIdx.x % tl.ntx] : -1;
-    bool any = false;
+    const size_t tile = ((size_t)t * tl.nty + blockIdx.x / tl.ntx) * tl.ntx + blockIdx.x % tl.ntx;
+    const int count = __ldg(tl.count + tile);
+    if (count == 0) {
+        if (add) return;
+        for (int q = threadIdx.x; q < TH * TR_TW; q += TR_NT) {
+            const int qu = u0 + q / TR_TW, qv = v0 + q % TR_TW;
+            if (qu < H && qv < W) dst[(size_t)qu * W + qv] = 0.f;
+        }
+        return;
+    }
+    // the tile's peaks: the first TILE_PEAKS from its array, then the list
+    int n = min(count, TILE_PEAKS);
+    if (threadIdx.x < n) s_list[threadIdx.x] = __ldg(tl.peaks + tile * TILE_PEAKS + threadIdx.x);
+    if (threadIdx.x == 0) s_entry = count > TILE_PEAKS ? __ldg(tl.head + tile) : 0;
+    for (int q = threadIdx.x; q < (SH / 2) * SS; q += TR_NT) S[q] = make_float2(0.f, 0.f);
+    __syncthreads();
     while (true) {
-        if (threadIdx.x == 0) {
-            int n = 0;
-            for (; entry >= 0 && n < LIST; entry = __ldg(tl.next + entry)) s_list[n++] = entry / tl.slots;
-            s_n = n;
-            s_more = entry >= 0;
-        }
-        __syncthreads();
-        const int n = s_n;
-        if (n > 0 && !any) {
-            for (int q = threadIdx.x; q < (SH / 2) * SS; q += TR_NT) S[q] = make_float2(0.f, 0.f);
-            __syncthreads();
-            any = true;
-        }
         for (int e = warp; e < n; e += TR_NT / 32) {
             const long long k = s_list[e];
             const int ru = __ldg(walk + 5 * k + 1) - u0 + kr, rv = __ldg(walk + 5 * k + 2) - v0 + kr;
@@ -439,22 +510,17 @@ __global__ void __launch_bounds__(TR_NT) adjoint_transpose_kernel(AdjParams p, A
                 if (g != 0.f && r >= 0 && r < SH && x >= 0 && x < SW) atomicAdd(&at(S, SS, r, x), g);
             }
         }
-        const bool more = s_more != 0;
         __syncthreads();
-        if (!more) break;
-    }
-    if (!any) {
-        if (add) return;
-        for (int q = threadIdx.x; q < TH * TR_TW; q += TR_NT) {
-            const int qu = u0 + q / TR_TW, qv = v0 + q % TR_TW;
-            if (qu < H && qv < W) dst[(size_t)qu * W + qv] = 0.f;
+        if (s_entry == 0) break;
+        if (threadIdx.x == 0) {
+            int entry = s_entry, q = 0;
+            for (; entry > 0 && q < LIST; entry = __ldg(tl.next + entry - 1)) s_list[q++] = (entry - 1) / tl.slots;
+            s_n = q;
+            s_entry = entry;
         }
-        return;
+        __syncthreads();
+        n = s_n;
     }
-    auto put = [&](int qu, int qv, float v) {
-        float* d = dst + (size_t)qu * W + qv;
-        *d = add ? *d + v : v;
-    };
     const float ikk = 1.f / p.kk;
     // box sums along a row or column of length n whose outputs near its ends
     // count reflected taps: tap(q) is the value at position q, 0 <= q < n
@@ -530,14 +596,27 @@ __global__ void __launch_bounds__(TR_NT) adjoint_transpose_kernel(AdjParams p, A
 #pragma unroll
                 for (int j = 1; j < TP; ++j) bs[m] = add2(bs[m], (j & 1) ? ml[m + (j >> 1)] : l[m + (j >> 1)]);
             }
+            float o[F];
 #pragma unroll
-            for (int m = 0; m < F; ++m) {
-                const int qu = u0 + r0 + m;
-                if (qu >= H) break;
-                float bx = (m & 1) ? bs[m / 2].y : bs[m / 2].x;
-                if (!rows_inner && (qu < KRT || qu >= H - KRT))
-                    bx = edge_box(qu, H, [&](int j) { return at(RB, RS, r0 + m + KRT + j, c); });
-                put(qu, v0 + c, fmaf(-bx, ikk, (m & 1) ? gs[m / 2].y : gs[m / 2].x));
+            for (int m = 0; m < F / 2; ++m) {
+                o[2 * m] = fmaf(-bs[m].x, ikk, gs[m].x);
+                o[2 * m + 1] = fmaf(-bs[m].y, ikk, gs[m].y);
+            }
+            float* d = dst + (size_t)(u0 + r0) * W + (v0 + c);
+            if (rows_inner && !add) {
+#pragma unroll
+                for (int m = 0; m < F; ++m) d[(size_t)m * W] = o[m];
+            } else {
+#pragma unroll
+                for (int m = 0; m < F; ++m) {
+                    const int qu = u0 + r0 + m;
+                    if (qu >= H) break;
+                    if (qu < KRT || qu >= H - KRT) {
+                        const float bx = edge_box(qu, H, [&](int j) { return at(RB, RS, r0 + m + KRT + j, c); });
+                        o[m] = fmaf(-bx, ikk, (m & 1) ? gs[m / 2].y : gs[m / 2].x);
+                    }
+                    d[(size_t)m * W] = add ? d[(size_t)m * W] + o[m] : o[m];
+                }
             }
         }
     } else {
@@ -556,7 +635,9 @@ __global__ void __launch_bounds__(TR_NT) adjoint_transpose_kernel(AdjParams p, A
             float g = 0.f;
             for (int i = 0; i <= 2 * kr; ++i) g = fmaf(p.a[i], at(RG, RS, r + i, c), g);
             const float bx = edge_box(u0 + r, H, [&](int j) { return at(RB, RS, r + kr + j, c); });
-            put(u0 + r, v0 + c, fmaf(-bx, ikk, g));
+            float* d = dst + (size_t)(u0 + r) * W + (v0 + c);
+            const float o = fmaf(-bx, ikk, g);
+            *d = add ? *d + o : o;
         }
     }
 }
@@ -583,7 +664,7 @@ template <int MODE, int R>
 cudaError_t particles_launch(const AdjParams& p, const float* frames, const int* walk, long long n, const int* circ,
                              const float* grad, float* yxm, const AdjTiles& tl, double* gpar, int* err, int grid,
                              cudaStream_t st) {
-    const size_t smem = sizeof(float) * (size_t)(2 * p.K + (ADJ_NT / 32) * adj_warp_floats(MODE, R, p.K));
+    const size_t smem = sizeof(float) * (size_t)(round4(2 * p.K) + (ADJ_NT / 32) * adj_warp_floats(MODE, R, p.K));
     const auto fn = adjoint_particle_kernel<MODE, R>;
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e) return e;

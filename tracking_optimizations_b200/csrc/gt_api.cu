@@ -1459,7 +1459,10 @@ int adjoint_work(gt_ctx* ctx, const AdjParams& ap, const std::vector<int>& circ,
                                            std::max<int64_t>(1, ((int64_t)1 << 28) / ap.K)});
             aw->tl.g = c.take<float>((size_t)aw->chunk * ap.K);
             aw->tl.next = c.take<int>((size_t)aw->chunk * aw->tl.slots);
-            aw->tl.head = c.take<int>((size_t)ap.T * aw->tl.nty * aw->tl.ntx);
+            const size_t tiles = (size_t)ap.T * aw->tl.nty * aw->tl.ntx;
+            aw->tl.count = c.take<int>(2 * tiles);  // and the lists' heads
+            aw->tl.head = aw->tl.count + tiles;
+            aw->tl.peaks = c.take<int>(tiles * TILE_PEAKS);
         }
         return c.off + 256;
     };
@@ -1726,7 +1729,7 @@ int gt_adjoint_backward(gt_ctx* ctx, const float* d_frames, int T, int H, int W,
     for (int i = 0; i < 4; ++i)
         if (!ctx->ev[i]) CK(cudaEventCreate(&ctx->ev[i]));
     if (n == 0) CK(cudaMemsetAsync(d_grad_params, 0, 2 * sizeof(double), st));
-    const size_t heads = sizeof(int) * (size_t)T * aw.tl.nty * aw.tl.ntx;
+    const size_t heads = 2 * sizeof(int) * (size_t)T * aw.tl.nty * aw.tl.ntx;
     ctx->stats.launches = 0;
     // the peaks in chunks (one, unless there are millions); the dense part is
     // the empty lists plus the transposed bandpass.  Times: the last chunk's
@@ -1735,7 +1738,7 @@ int gt_adjoint_backward(gt_ctx* ctx, const float* d_frames, int T, int H, int W,
         const int64_t nk = std::min<int64_t>(aw.chunk, n - k0);
         const int add = k0 > 0;
         CK(cudaEventRecord(ctx->ev[0], st));
-        CK(cudaMemsetAsync(aw.tl.head, 0xff, heads, st));
+        CK(cudaMemsetAsync(aw.tl.count, 0, heads, st));
         CK(cudaEventRecord(ctx->ev[1], st));
         CK(launch_adjoint_particles(1, ap, d_frames, d_walk + 5 * k0, nk, aw.circ, d_grad_yxm + 3 * k0, nullptr, aw.tl,
                                     d_grad_params, aw.gpart, aw.err, add, ctx->num_sms, st));

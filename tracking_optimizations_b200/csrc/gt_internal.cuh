@@ -175,12 +175,16 @@ struct AdjParams {
     float gain, read_var;    // noise model of the uncertainty kernel
 };
 
-// The backward pass's dL/dR: K values per peak of the chunk, and per output
-// tile (frame, tile row, tile column) a list of the peaks that reach it, entry
-// = peak * slots + one of its tiles.
+// The backward pass's dL/dR: K values per peak of the chunk, and the peaks that
+// reach an output tile (frame, tile row, tile column): the first TILE_PEAKS in
+// an array, the others in a list of entries peak * slots + one of its tiles,
+// numbered from 1.
+constexpr int TILE_PEAKS = 16;
 struct AdjTiles {
     float* g;
-    int* head;  // -1: no peak
+    int* count;  // peaks of the tile
+    int* head;   // 0: no list
+    int* peaks;
     int* next;
     int slots;
     int th, nty, ntx;  // tile rows (columns: 64) and tiles per frame
