@@ -24,7 +24,9 @@
 
 #include "gt.h"
 #include "gt_internal.cuh"
+#include "hostcopy.h"
 #include "ingest.h"
+#include "traj.h"
 
 namespace gt {
 __global__ void locate_tiles_kernel(const LocParams p, const MovieBufs b, int frame0);
@@ -55,13 +57,13 @@ int adjoint_particle_blocks_max(int num_sms);
 cudaError_t launch_adjoint_transpose(const AdjParams& p, const AdjTiles& tl, const int* walk, const int* circ, float* gI,
                                      int add, cudaStream_t st);
 int traj_filter_stubs(const int64_t* h_ids, int64_t n, int64_t threshold, uint8_t* h_keep, int64_t* h_count,
-                      int64_t* nkept, cudaStream_t st, int num_sms, std::string* msg);
+                      int64_t* nkept, TrajMem& M, cudaStream_t st, int num_sms, std::string* msg);
 int traj_steps(const int64_t* h_ids, const float* h_x, const float* h_y, int64_t n, float mppf, float* h_xs,
-               float* h_ys, double* h_xstep, double* h_ystep, double* h_len, int64_t* h_order, cudaStream_t st,
-               int num_sms, std::string* msg);
+               float* h_ys, double* h_xstep, double* h_ystep, double* h_len, int64_t* h_order, TrajMem& M,
+               cudaStream_t st, int num_sms, std::string* msg);
 int traj_imsd(const int64_t* h_ids, const int64_t* h_frames, const float* h_x, const float* h_y, int64_t n,
               float mppf, int64_t max_lagtime, float* (*alloc)(size_t), float** out, int64_t* nout, float* ms_msd,
-              cudaStream_t st, int num_sms, std::string* msg);
+              TrajMem& M, cudaStream_t st, int num_sms, std::string* msg);
 
 // preprocess_rows.wgsl:44-45: taps exp(-i^2 / (2 * noise_size)) for
 // i = -k/2..k/2 and their running sum; the passes multiply by the
@@ -121,6 +123,8 @@ struct gt_ctx {
     int tune_disabled = 0;
     int batch_cap_div = 64;           // first candidate capacity of batched movies: H*W / this
     cudaStream_t copy_stream = nullptr;  // host->device frame chunks
+    HostCopy hc;                         // pageable host arrays
+    TrajMem traj;                        // scratch of the trajectory calls
     cudaEvent_t cev[9] = {};
 };
 
@@ -645,8 +649,8 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
             const int rr = (*ready)(f0, nf);
             if (rr) return rr;
         }
-        CK(cudaMemcpyAsync((char*)d_frames + (size_t)f0 * fbytes, (const char*)h_frames + (size_t)f0 * fbytes,
-                           (size_t)nf * fbytes, cudaMemcpyHostToDevice, ctx->copy_stream));
+        CK(ctx->hc.upload((char*)d_frames + (size_t)f0 * fbytes, (const char*)h_frames + (size_t)f0 * fbytes,
+                          (size_t)nf * fbytes, ctx->copy_stream));
         CK(cudaEventRecord(ctx->cev[ci & 7], ctx->copy_stream));
         CK(cudaStreamWaitEvent(st, ctx->cev[ci & 7], 0));
         ++ci;
@@ -1855,7 +1859,8 @@ int gt_filter_stubs(gt_ctx* ctx, const int64_t* ids, int64_t n, int64_t threshol
     if (rc || !nkept) return rc ? rc : GT_ERR_ARG;
     *nkept = 0;
     if (n == 0) return GT_OK;
-    return traj_filter_stubs(ids, n, threshold, keep, count, nkept, ctx->stream, ctx->num_sms, &ctx->err);
+    ctx->traj.hc = &ctx->hc;
+    return traj_filter_stubs(ids, n, threshold, keep, count, nkept, ctx->traj, ctx->stream, ctx->num_sms, &ctx->err);
 }
 
 int gt_steps(gt_ctx* ctx, const int64_t* ids, const float* x, const float* y, int64_t n, double mpp, float* xs,
@@ -1863,7 +1868,8 @@ int gt_steps(gt_ctx* ctx, const int64_t* ids, const float* x, const float* y, in
     int rc = traj_begin(ctx, n, ids && x && y && xs && ys && x_step && y_step && steplength && order);
     if (rc) return rc;
     if (n == 0) return GT_OK;
-    return traj_steps(ids, x, y, n, (float)mpp, xs, ys, x_step, y_step, steplength, order, ctx->stream,
+    ctx->traj.hc = &ctx->hc;
+    return traj_steps(ids, x, y, n, (float)mpp, xs, ys, x_step, y_step, steplength, order, ctx->traj, ctx->stream,
                       ctx->num_sms, &ctx->err);
 }
 
@@ -1879,7 +1885,8 @@ int gt_imsd(gt_ctx* ctx, const int64_t* ids, const int64_t* frames, const float*
     int64_t m = 0;
     float ms = 0.f;
     if (n > 0) {
-        rc = traj_imsd(ids, frames, x, y, n, (float)mpp, max_lagtime, table_alloc, &data, &m, &ms, ctx->stream,
+        ctx->traj.hc = &ctx->hc;
+        rc = traj_imsd(ids, frames, x, y, n, (float)mpp, max_lagtime, table_alloc, &data, &m, &ms, ctx->traj, ctx->stream,
                        ctx->num_sms, &ctx->err);
         if (rc) {
             if (data) table_release(data);

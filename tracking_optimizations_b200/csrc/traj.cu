@@ -6,8 +6,13 @@
 // (hatzakis_lab_tracking.py:199-214).
 //
 // Rows are grouped by particle with a stable order: keys (particle - min id)
-// << 32 | row are radix-sorted, which gives exactly pandas' groupby order
+// << 32 | row, in row order, are radix-sorted by their particle bits (a stable
+// sort keeps the rows in order), which gives exactly pandas' groupby order
 // (ascending particle, rows of a particle in table order).
+//
+// Scratch comes from the context's TrajMem, which keeps its memory: stream-
+// ordered allocations, whose pool gives everything back at each
+// synchronisation, took 5 of 8 ms of the three calls on a 360k-row table.
 //
 // MSD of one particle (trackpy.msd's definition): positions p = xy * mpp in
 // float32, placed on the frame axis from the particle's first to its last
@@ -28,6 +33,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "gt.h"
+#include "traj.h"
 
 namespace gt {
 
@@ -63,27 +69,33 @@ __global__ void heads_kernel(const unsigned long long* keys, int64_t n, int64_t*
         heads[j] = (j == 0 || gkey(keys[j - 1]) != gkey(keys[j])) ? 1 : 0;
 }
 
-// gstart[g] = first sorted position of group g (groups in particle order)
+// gstart[g] = first sorted position of group g (groups in particle order),
+// gstart[number of groups] = n
 __global__ void gstart_kernel(const unsigned long long* keys, int64_t n, const int64_t* gid, int64_t* gstart) {
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x)
-        if (j == 0 || gkey(keys[j - 1]) != gkey(keys[j])) gstart[gid[j]] = j;
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
+        const bool head = j == 0 || gkey(keys[j - 1]) != gkey(keys[j]);
+        if (head) gstart[gid[j]] = j;
+        if (j == n - 1) gstart[gid[j] + head] = n;
+    }
 }
 
 // keep[row] for every row of groups with at least `threshold` rows;
-// count[row] = rows of the row's group
-__global__ void stubs_kernel(const unsigned long long* keys, int64_t n, const int64_t* gstart, int64_t G,
+// count[row] = rows of the row's group.  gid[j] counts the heads before j.
+__global__ void stubs_kernel(const unsigned long long* keys, int64_t n, const int64_t* gid, const int64_t* gstart,
                              int64_t threshold, uint8_t* keep, int64_t* count, unsigned long long* nkept) {
-    unsigned long long mine = 0;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < G; g += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = gstart[g], e = g + 1 < G ? gstart[g + 1] : n;
-        const uint8_t k = (e - j) >= threshold ? 1 : 0;
-        for (int64_t q = j; q < e; ++q) {
-            keep[keys[q] & 0xffffffffu] = k;
-            count[keys[q] & 0xffffffffu] = e - j;
-        }
-        if (k) mine += (unsigned long long)(e - j);
+    unsigned mine = 0;
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x) {
+        const bool head = j == 0 || gkey(keys[j - 1]) != gkey(keys[j]);
+        const int64_t g = gid[j] + head - 1;
+        const int64_t rows = gstart[g + 1] - gstart[g];
+        const int64_t row = (int64_t)(keys[j] & 0xffffffffu);
+        const bool k = rows >= threshold;
+        keep[row] = k;
+        count[row] = rows;
+        mine += k;
     }
-    if (mine) atomicAdd(nkept, mine);
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(nkept, (unsigned long long)mine);
 }
 // step_tracker: scaled positions per row (float32), steps in group order
 // (float64: the lab code takes the float32 values as Python floats)
@@ -109,52 +121,61 @@ __global__ void steps_kernel(const unsigned long long* keys, int64_t n, const fl
     }
 }
 
-// per group: first frame, span and number of lags
-__global__ void msd_groups_kernel(const unsigned long long* keys, int64_t n, const int64_t* frames,
-                                  const int64_t* gstart, int64_t G, int64_t max_lagtime, int64_t* gfirst,
-                                  int64_t* gspan, int64_t* glags, int* err) {
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < G; g += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = gstart[g], e = g + 1 < G ? gstart[g + 1] : n;
-        int64_t fmin = LLONG_MAX, fmax = LLONG_MIN;
-        for (int64_t q = j; q < e; ++q) {
-            const int64_t f = frames[keys[q] & 0xffffffffu];
+// one block per (group, chunk of MSD_LAGS lags), threads over the lags:
+// the lags of a long-lived particle spread over several blocks
+constexpr int MSD_LAGS = 128;
+
+// per group, a warp each: first frame, span, number of lags and of lag chunks;
+// stat[0] error bits, stat[1] the longest lag
+__global__ void msd_groups_kernel(const unsigned long long* keys, const int64_t* frames, const int64_t* gstart, int64_t G,
+                                  int64_t max_lagtime, int64_t* gfirst, int64_t* gspan, int64_t* glags, int64_t* gchunks,
+                                  unsigned long long* stat) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = (int64_t)gridDim.x * blockDim.x / 32;
+    for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; g < G; g += nw) {
+        const int64_t e = gstart[g + 1];
+        long long fmin = LLONG_MAX, fmax = LLONG_MIN;
+        for (int64_t q = gstart[g] + lane; q < e; q += 32) {
+            const long long f = (long long)frames[keys[q] & 0xffffffffu];
             fmin = min(fmin, f);
             fmax = max(fmax, f);
         }
-        int64_t span = fmax - fmin + 1;
-        if (span > ((int64_t)1 << 31) || span < 1) {
-            atomicOr(err, 2);
-            span = 1;
+        for (int o = 16; o > 0; o >>= 1) {
+            fmin = min(fmin, __shfl_xor_sync(0xffffffffu, fmin, o));
+            fmax = max(fmax, __shfl_xor_sync(0xffffffffu, fmax, o));
         }
-        gfirst[g] = fmin;
-        gspan[g] = span;
-        glags[g] = min(max_lagtime, span - 1);
+        if (lane == 0) {
+            int64_t span = fmax - fmin + 1;
+            if (span > ((int64_t)1 << 31) || span < 1) {
+                atomicOr(stat, 2ull);
+                span = 1;
+            }
+            const int64_t lags = min(max_lagtime, span - 1);
+            gfirst[g] = fmin;
+            gspan[g] = span;
+            glags[g] = lags;
+            gchunks[g] = (lags + MSD_LAGS - 1) / MSD_LAGS;
+            if (lags > 0) atomicMax(stat + 1, (unsigned long long)lags);
+        }
     }
 }
 
 // positions of the groups on their frame axes (NaN = gap); a frame taken
 // twice by one particle is an error (trackpy: "more than one trajectory
 // per particle")
-__global__ void msd_scatter_kernel(const unsigned long long* keys, int64_t n, const int64_t* frames, const float* x,
+__global__ void msd_scatter_kernel(const unsigned long long* keys, const int64_t* frames, const float* x,
                                    const float* y, float mppf, const int64_t* gstart, const int64_t* gfirst,
-                                   const int64_t* gbase, int64_t ngroups, float2* pos, int* taken, int* err) {
+                                   const int64_t* gbase, int64_t ngroups, float2* pos, int* taken,
+                                   unsigned long long* stat) {
     for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
-        const int64_t e = g + 1 < ngroups ? gstart[g + 1] : n;
+        const int64_t e = gstart[g + 1];
         for (int64_t q = gstart[g] + threadIdx.x; q < e; q += blockDim.x) {
             const int64_t r = (int64_t)(keys[q] & 0xffffffffu);
             const int64_t s = gbase[g] + (frames[r] - gfirst[g]);
-            if (atomicExch(taken + s, 1) != 0) atomicOr(err, 1);
+            if (atomicExch(taken + s, 1) != 0) atomicOr(stat, 1ull);
             pos[s] = make_float2(__fmul_rn(x[r], mppf), __fmul_rn(y[r], mppf));
         }
     }
-}
-
-// one block per (group, chunk of MSD_LAGS lags), threads over the lags:
-// the lags of a long-lived particle spread over several blocks
-constexpr int MSD_LAGS = 128;
-__global__ void msd_chunks_kernel(const int64_t* glags, int64_t ngroups, int64_t* gchunks) {
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += (int64_t)gridDim.x * blockDim.x)
-        gchunks[g] = (glags[g] + MSD_LAGS - 1) / MSD_LAGS;
 }
 
 __global__ void msd_kernel(const float2* pos, const int* taken, const int64_t* gbase, const int64_t* gspan,
@@ -192,36 +213,33 @@ __global__ void msd_kernel(const float2* pos, const int* taken, const int64_t* g
     }
 }
 
-// (lag, particle) sort keys of the entries; entries without a pair last
-__global__ void msd_keys_kernel(const float* msd, const int64_t* gout, const int64_t* glags,
-                                const unsigned long long* keys, const int64_t* gstart, int64_t ngroups,
-                                unsigned long long* ekeys, int64_t* eidx) {
+// (lag, group) sort keys of the entries, (lag - 1) * groups + group: the order
+// of lags, then particles, in as few bits as it takes; entries without a pair
+// get the key `last`
+__global__ void msd_keys_kernel(const float* msd, const int64_t* gout, const int64_t* glags, int64_t ngroups,
+                                unsigned long long last, unsigned long long* ekeys, int* eidx) {
     for (int64_t g = blockIdx.x; g < ngroups; g += gridDim.x) {
-        const unsigned int pid = gkey(keys[gstart[g]]);
         for (int64_t L = 1 + threadIdx.x; L <= glags[g]; L += blockDim.x) {
             const int64_t e = gout[g] + L - 1;
-            ekeys[e] = isnan(msd[e]) ? ~0ull : (((unsigned long long)L << 32) | pid);
-            eidx[e] = e;
+            ekeys[e] = isnan(msd[e]) ? last : (unsigned long long)(L - 1) * ngroups + g;
+            eidx[e] = (int)e;
         }
     }
 }
 
-__global__ void msd_table_kernel(const unsigned long long* ekeys, const int64_t* eidx, const float* msd,
-                                 int64_t nvalid, long long idmin, float* out) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < nvalid; e += (int64_t)gridDim.x * blockDim.x) {
+__global__ void msd_table_kernel(const unsigned long long* ekeys, const int* eidx, const float* msd, int64_t ne,
+                                 int64_t ngroups, unsigned long long last, const unsigned long long* keys,
+                                 const int64_t* gstart, long long idmin, float* out, unsigned long long* nvalid) {
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x) {
         const unsigned long long k = ekeys[e];
-        out[3 * e + 0] = (float)(k >> 32);
-        out[3 * e + 1] = (float)((long long)(k & 0xffffffffu) + idmin);
+        if (k == last) continue;
+        if (e == ne - 1 || ekeys[e + 1] == last) *nvalid = (unsigned long long)(e + 1);
+        const unsigned long long L = k / ngroups;
+        const unsigned int pid = gkey(keys[gstart[k - L * ngroups]]);
+        out[3 * e + 0] = (float)(L + 1);
+        out[3 * e + 1] = (float)((long long)pid + idmin);
         out[3 * e + 2] = msd[eidx[e]];
     }
-}
-
-__global__ void count_valid_kernel(const unsigned long long* ekeys, int64_t ne, unsigned long long* nvalid) {
-    unsigned long long mine = 0;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (int64_t)gridDim.x * blockDim.x)
-        mine += ekeys[e] != ~0ull;
-    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(nvalid, mine);
 }
 
 int bits_for(unsigned long long v) {
@@ -229,23 +247,6 @@ int bits_for(unsigned long long v) {
     while (b < 64 && (v >> b)) ++b;
     return b;
 }
-
-// Stream-ordered device buffers, freed when the object goes out of scope.
-struct DevBuf {
-    cudaStream_t st;
-    std::vector<void*> ptrs;
-    explicit DevBuf(cudaStream_t s) : st(s) {}
-    template <class X>
-    X* get(size_t n) {
-        void* p = nullptr;
-        if (cudaMallocAsync(&p, sizeof(X) * (n ? n : 1), st) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
-        return (X*)p;
-    }
-    ~DevBuf() {
-        for (void* p : ptrs) cudaFreeAsync(p, st);
-    }
-};
 
 #define TK(x)                              \
     do {                                   \
@@ -263,26 +264,20 @@ struct DevBuf {
         }                                      \
     } while (0)
 
-// Grouping of the rows by particle: the keys sorted in pandas' groupby
-// order and the first sorted position of every group.
-struct Groups {
+// Rows in pandas' groupby order: the sorted keys.
+struct Sorted {
     unsigned long long* keys = nullptr;
-    int64_t* gstart = nullptr;
-    int64_t G = 0;
     long long idmin = 0;
     unsigned long long range = 0;
 };
 
-int make_groups(const int64_t* h_ids, int64_t n, DevBuf& B, cudaStream_t st, int grid, Groups* out,
-                std::string* msg) {
-    int64_t* ids = B.get<int64_t>(n);
-    unsigned long long* lohi = B.get<unsigned long long>(2);
-    unsigned long long* k0 = B.get<unsigned long long>(n);
-    unsigned long long* k1 = B.get<unsigned long long>(n);
-    int64_t* heads = B.get<int64_t>(n);
-    int64_t* gid = B.get<int64_t>(n);
-    TA(ids && lohi && k0 && k1 && heads && gid);
-    TK(cudaMemcpyAsync(ids, h_ids, sizeof(int64_t) * n, cudaMemcpyHostToDevice, st));
+int sort_rows(const int64_t* h_ids, int64_t n, TrajMem& M, cudaStream_t st, int grid, Sorted* out, std::string* msg) {
+    int64_t* ids = M.get<int64_t>(n);
+    unsigned long long* lohi = M.get<unsigned long long>(2);
+    unsigned long long* k0 = M.get<unsigned long long>(n);
+    unsigned long long* k1 = M.get<unsigned long long>(n);
+    TA(ids && lohi && k0 && k1);
+    TK(M.hc->upload(ids, h_ids, sizeof(int64_t) * n, st));
     const unsigned long long init[2] = {(unsigned long long)LLONG_MAX, (unsigned long long)LLONG_MIN};
     TK(cudaMemcpyAsync(lohi, init, sizeof(init), cudaMemcpyHostToDevice, st));
     id_range_kernel<<<grid, 256, 0, st>>>(ids, n, lohi);
@@ -299,96 +294,93 @@ int make_groups(const int64_t* h_ids, int64_t n, DevBuf& B, cudaStream_t st, int
     out->range = (unsigned long long)(idmax - out->idmin);
     group_keys_kernel<<<grid, 256, 0, st>>>(ids, n, out->idmin, k0);
     TK(cudaGetLastError());
+    out->keys = k0;
+    if (out->range == 0) return GT_OK;  // one particle: in order
     const int end_bit = 32 + bits_for(out->range);
     cub::DoubleBuffer<unsigned long long> db(k0, k1);
-    size_t tmp = 0, tmp2 = 0;
-    TK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, db, (int)n, 0, end_bit, st));
-    TK(cub::DeviceScan::ExclusiveSum(nullptr, tmp2, heads, gid, (int)n, st));
-    void* t = B.get<char>(std::max(tmp, tmp2));
+    size_t tmp = 0;
+    TK(cub::DeviceRadixSort::SortKeys(nullptr, tmp, db, (int)n, 32, end_bit, st));
+    void* t = M.get<char>(tmp);
     TA(t);
-    TK(cub::DeviceRadixSort::SortKeys(t, tmp, db, (int)n, 0, end_bit, st));
+    TK(cub::DeviceRadixSort::SortKeys(t, tmp, db, (int)n, 32, end_bit, st));
     out->keys = db.Current();
-    heads_kernel<<<grid, 256, 0, st>>>(out->keys, n, heads);
-    TK(cudaGetLastError());
-    TK(cub::DeviceScan::ExclusiveSum(t, tmp2, heads, gid, (int)n, st));
-    int64_t last[2];
-    TK(cudaMemcpyAsync(&last[0], gid + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    TK(cudaMemcpyAsync(&last[1], heads + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    TK(cudaStreamSynchronize(st));
-    out->G = last[0] + last[1];
-    out->gstart = B.get<int64_t>(out->G);
-    TA(out->gstart);
-    gstart_kernel<<<grid, 256, 0, st>>>(out->keys, n, gid, out->gstart);
-    TK(cudaGetLastError());
     return GT_OK;
 }
 
-// exclusive prefix sum of v[0..G) into o, total returned in *tot
-int exclusive_sum(const int64_t* v, int64_t* o, int64_t G, DevBuf& B, cudaStream_t st, int64_t* tot,
-                  std::string* msg) {
+// gid[j]: heads of groups before sorted position j; gstart as gstart_kernel
+// (room for n + 1); *total (may be NULL) receives {gid, head} of the last row.
+int find_groups(const Sorted& S, int64_t n, TrajMem& M, cudaStream_t st, int grid, int64_t** gid, int64_t** gstart,
+                int64_t* total, std::string* msg) {
+    int64_t* heads = M.get<int64_t>(n);
+    *gid = M.get<int64_t>(n);
+    *gstart = M.get<int64_t>(n + 1);
     size_t tmp = 0;
-    TK(cub::DeviceScan::ExclusiveSum(nullptr, tmp, v, o, (int)G, st));
-    void* t = B.get<char>(tmp);
-    TA(t);
-    TK(cub::DeviceScan::ExclusiveSum(t, tmp, v, o, (int)G, st));
-    int64_t a = 0, b = 0;
-    TK(cudaMemcpyAsync(&a, o + G - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    TK(cudaMemcpyAsync(&b, v + G - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    TK(cudaStreamSynchronize(st));
-    *tot = a + b;
+    TK(cub::DeviceScan::ExclusiveSum(nullptr, tmp, heads, *gid, (int)n, st));
+    void* t = M.get<char>(tmp);
+    TA(heads && *gid && *gstart && t);
+    heads_kernel<<<grid, 256, 0, st>>>(S.keys, n, heads);
+    TK(cudaGetLastError());
+    TK(cub::DeviceScan::ExclusiveSum(t, tmp, heads, *gid, (int)n, st));
+    gstart_kernel<<<grid, 256, 0, st>>>(S.keys, n, *gid, *gstart);
+    TK(cudaGetLastError());
+    if (total) {
+        TK(cudaMemcpyAsync(&total[0], *gid + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        TK(cudaMemcpyAsync(&total[1], heads + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        TK(cudaStreamSynchronize(st));
+    }
     return GT_OK;
 }
 
 }  // namespace
 
 int traj_filter_stubs(const int64_t* h_ids, int64_t n, int64_t threshold, uint8_t* h_keep, int64_t* h_count,
-                      int64_t* nkept, cudaStream_t st, int num_sms, std::string* msg) {
-    DevBuf B(st);
+                      int64_t* nkept, TrajMem& M, cudaStream_t st, int num_sms, std::string* msg) {
     const int grid = num_sms * 8;
-    Groups Gr;
-    int rc = make_groups(h_ids, n, B, st, grid, &Gr, msg);
+    TK(M.begin());
+    Sorted S;
+    int rc = sort_rows(h_ids, n, M, st, grid, &S, msg);
+    int64_t *gid, *gstart;
+    if (!rc) rc = find_groups(S, n, M, st, grid, &gid, &gstart, nullptr, msg);
     if (rc) return rc;
-    uint8_t* keep = B.get<uint8_t>(n);
-    int64_t* count = B.get<int64_t>(n);
-    unsigned long long* cnt = B.get<unsigned long long>(1);
+    uint8_t* keep = M.get<uint8_t>(n);
+    int64_t* count = M.get<int64_t>(n);
+    unsigned long long* cnt = M.get<unsigned long long>(1);
     TA(keep && count && cnt);
     TK(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), st));
-    stubs_kernel<<<grid, 256, 0, st>>>(Gr.keys, n, Gr.gstart, Gr.G, threshold, keep, count, cnt);
+    stubs_kernel<<<grid, 256, 0, st>>>(S.keys, n, gid, gstart, threshold, keep, count, cnt);
     TK(cudaGetLastError());
     unsigned long long hk = 0;
-    TK(cudaMemcpyAsync(h_keep, keep, n, cudaMemcpyDeviceToHost, st));
-    if (h_count) TK(cudaMemcpyAsync(h_count, count, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st));
     TK(cudaMemcpyAsync(&hk, cnt, sizeof(hk), cudaMemcpyDeviceToHost, st));
+    TK(M.hc->download(h_keep, keep, n, st));
+    if (h_count) TK(M.hc->download(h_count, count, sizeof(int64_t) * n, st));
     TK(cudaStreamSynchronize(st));
     *nkept = (int64_t)hk;
     return GT_OK;
 }
 
 int traj_steps(const int64_t* h_ids, const float* h_x, const float* h_y, int64_t n, float mppf, float* h_xs,
-               float* h_ys, double* h_xstep, double* h_ystep, double* h_len, int64_t* h_order, cudaStream_t st,
-               int num_sms, std::string* msg) {
-    DevBuf B(st);
+               float* h_ys, double* h_xstep, double* h_ystep, double* h_len, int64_t* h_order, TrajMem& M,
+               cudaStream_t st, int num_sms, std::string* msg) {
     const int grid = num_sms * 8;
-    Groups Gr;
-    int rc = make_groups(h_ids, n, B, st, grid, &Gr, msg);
+    TK(M.begin());
+    Sorted S;
+    int rc = sort_rows(h_ids, n, M, st, grid, &S, msg);
     if (rc) return rc;
-    float* x = B.get<float>(n);
-    float* y = B.get<float>(n);
-    float* sxy = B.get<float>(2 * (size_t)n);
-    double* st3 = B.get<double>(3 * (size_t)n);
-    int64_t* order = B.get<int64_t>(n);
+    float* x = M.get<float>(n);
+    float* y = M.get<float>(n);
+    float* sxy = M.get<float>(2 * (size_t)n);
+    double* st3 = M.get<double>(3 * (size_t)n);
+    int64_t* order = M.get<int64_t>(n);
     TA(x && y && sxy && st3 && order);
-    TK(cudaMemcpyAsync(x, h_x, sizeof(float) * n, cudaMemcpyHostToDevice, st));
-    TK(cudaMemcpyAsync(y, h_y, sizeof(float) * n, cudaMemcpyHostToDevice, st));
-    steps_kernel<<<grid, 256, 0, st>>>(Gr.keys, n, x, y, mppf, sxy, sxy + n, st3, st3 + n, st3 + 2 * n, order);
+    TK(M.hc->upload(x, h_x, sizeof(float) * n, st));
+    TK(M.hc->upload(y, h_y, sizeof(float) * n, st));
+    steps_kernel<<<grid, 256, 0, st>>>(S.keys, n, x, y, mppf, sxy, sxy + n, st3, st3 + n, st3 + 2 * n, order);
     TK(cudaGetLastError());
-    TK(cudaMemcpyAsync(h_xs, sxy, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
-    TK(cudaMemcpyAsync(h_ys, sxy + n, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
+    TK(M.hc->download(h_xs, sxy, sizeof(float) * n, st));
+    TK(M.hc->download(h_ys, sxy + n, sizeof(float) * n, st));
     double* dst[3] = {h_xstep, h_ystep, h_len};
-    for (int i = 0; i < 3; ++i)
-        TK(cudaMemcpyAsync(dst[i], st3 + (size_t)i * n, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
-    TK(cudaMemcpyAsync(h_order, order, sizeof(int64_t) * n, cudaMemcpyDeviceToHost, st));
-    TK(cudaStreamSynchronize(st));
+    for (int i = 0; i < 3; ++i) TK(M.hc->download(dst[i], st3 + (size_t)i * n, sizeof(double) * n, st));
+    TK(M.hc->download(h_order, order, sizeof(int64_t) * n, st));
     return GT_OK;
 }
 
@@ -397,40 +389,53 @@ int traj_steps(const int64_t* h_ids, const float* h_x, const float* h_y, int64_t
 // alloc(bytes).  *ms_msd: device time of the MSD kernel.
 int traj_imsd(const int64_t* h_ids, const int64_t* h_frames, const float* h_x, const float* h_y, int64_t n,
               float mppf, int64_t max_lagtime, float* (*alloc)(size_t), float** out, int64_t* nout, float* ms_msd,
-              cudaStream_t st, int num_sms, std::string* msg) {
-    DevBuf B(st);
+              TrajMem& M, cudaStream_t st, int num_sms, std::string* msg) {
     const int grid = num_sms * 8;
-    Groups Gr;
-    int rc = make_groups(h_ids, n, B, st, grid, &Gr, msg);
+    TK(M.begin());
+    Sorted S;
+    int rc = sort_rows(h_ids, n, M, st, grid, &S, msg);
     if (rc) return rc;
-    if (Gr.idmin < 0 || Gr.idmin + (long long)Gr.range >= (1LL << 24)) {
+    if (S.idmin < 0 || S.idmin + (long long)S.range >= (1LL << 24)) {
         *msg = "particle ids must lie in [0, 2^24) for the float32 result table";
         return GT_ERR_ARG;
     }
-    const int64_t G = Gr.G;
-    int64_t* frames = B.get<int64_t>(n);
-    float* x = B.get<float>(n);
-    float* y = B.get<float>(n);
-    int64_t* g5 = B.get<int64_t>(5 * (size_t)G);  // first, span, lags, base, out offset per group
-    int* err = B.get<int>(1);
-    TA(frames && x && y && g5 && err);
-    int64_t *gfirst = g5, *gspan = g5 + G, *glags = g5 + 2 * G, *gbase = g5 + 3 * G, *gout = g5 + 4 * G;
-    TK(cudaMemcpyAsync(frames, h_frames, sizeof(int64_t) * n, cudaMemcpyHostToDevice, st));
-    TK(cudaMemcpyAsync(x, h_x, sizeof(float) * n, cudaMemcpyHostToDevice, st));
-    TK(cudaMemcpyAsync(y, h_y, sizeof(float) * n, cudaMemcpyHostToDevice, st));
-    TK(cudaMemsetAsync(err, 0, sizeof(int), st));
+    int64_t *gid, *gstart, last2[2];
+    rc = find_groups(S, n, M, st, grid, &gid, &gstart, last2, msg);
+    if (rc) return rc;
+    const int64_t G = last2[0] + last2[1];
+    int64_t* frames = M.get<int64_t>(n);
+    float* x = M.get<float>(n);
+    float* y = M.get<float>(n);
+    // per group: first, then span, lags, chunks, each with a spare entry so
+    // that its exclusive sums (base, out offset, chunk start) end in the total
+    const int64_t G1 = G + 1;
+    int64_t* g7 = M.get<int64_t>(7 * (size_t)G1);
+    unsigned long long* stat = M.get<unsigned long long>(3);  // error bits, longest lag, valid entries
+    TA(frames && x && y && g7 && stat);
+    int64_t *gfirst = g7, *gspan = g7 + G1, *glags = g7 + 2 * G1, *gchunks = g7 + 3 * G1;
+    int64_t *gbase = g7 + 4 * G1, *gout = g7 + 5 * G1, *cstart = g7 + 6 * G1;
+    TK(M.hc->upload(frames, h_frames, sizeof(int64_t) * n, st));
+    TK(M.hc->upload(x, h_x, sizeof(float) * n, st));
+    TK(M.hc->upload(y, h_y, sizeof(float) * n, st));
+    TK(cudaMemsetAsync(stat, 0, 3 * sizeof(unsigned long long), st));
     if (max_lagtime < 0) max_lagtime = 0;
-    msd_groups_kernel<<<grid, 256, 0, st>>>(Gr.keys, n, frames, Gr.gstart, G, max_lagtime, gfirst, gspan, glags, err);
+    msd_groups_kernel<<<grid, 256, 0, st>>>(S.keys, frames, gstart, G, max_lagtime, gfirst, gspan, glags, gchunks, stat);
     TK(cudaGetLastError());
-    int64_t tot_span = 0, tot_out = 0;
-    rc = exclusive_sum(gspan, gbase, G, B, st, &tot_span, msg);
-    if (rc) return rc;
-    rc = exclusive_sum(glags, gout, G, B, st, &tot_out, msg);
-    if (rc) return rc;
-    int h_err = 0;
-    TK(cudaMemcpyAsync(&h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st));
+    size_t tmp = 0;
+    TK(cub::DeviceScan::ExclusiveSum(nullptr, tmp, gspan, gbase, (int)G1, st));
+    void* t = M.get<char>(tmp);
+    TA(t);
+    TK(cub::DeviceScan::ExclusiveSum(t, tmp, gspan, gbase, (int)G1, st));
+    TK(cub::DeviceScan::ExclusiveSum(t, tmp, glags, gout, (int)G1, st));
+    TK(cub::DeviceScan::ExclusiveSum(t, tmp, gchunks, cstart, (int)G1, st));
+    int64_t tot_span = 0, tot_out = 0, nchunks = 0;
+    unsigned long long hs[3] = {0, 0, 0};
+    TK(cudaMemcpyAsync(&tot_span, gbase + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    TK(cudaMemcpyAsync(&tot_out, gout + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    TK(cudaMemcpyAsync(&nchunks, cstart + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    TK(cudaMemcpyAsync(hs, stat, sizeof(hs), cudaMemcpyDeviceToHost, st));
     TK(cudaStreamSynchronize(st));
-    if (h_err) {
+    if (hs[0]) {
         *msg = "a particle spans more than 2^31 frames";
         return GT_ERR_ARG;
     }
@@ -438,72 +443,51 @@ int traj_imsd(const int64_t* h_ids, const int64_t* h_frames, const float* h_x, c
         *msg = "trajectories span too many frames in total";
         return GT_ERR_ARG;
     }
-    float2* pos = B.get<float2>(tot_span);
-    int* taken = B.get<int>(tot_span);
+    float2* pos = M.get<float2>(tot_span);
+    int* taken = M.get<int>(tot_span);
     TA(pos && taken);
     TK(cudaMemsetAsync(taken, 0, sizeof(int) * tot_span, st));
     const int gg = (int)std::min<int64_t>(std::max<int64_t>(G, 1), (int64_t)num_sms * 64);
-    msd_scatter_kernel<<<gg, 128, 0, st>>>(Gr.keys, n, frames, x, y, mppf, Gr.gstart, gfirst, gbase, G, pos, taken,
-                                           err);
+    msd_scatter_kernel<<<gg, 128, 0, st>>>(S.keys, frames, x, y, mppf, gstart, gfirst, gbase, G, pos, taken, stat);
     TK(cudaGetLastError());
-    TK(cudaMemcpyAsync(&h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st));
+    *ms_msd = 0.f;
+    float* tab = nullptr;
+    const bool timed = tot_out > 0;
+    if (timed) {
+        float* msd = M.get<float>(tot_out);
+        unsigned long long* ekeys = M.get<unsigned long long>(tot_out);
+        unsigned long long* ekeys2 = M.get<unsigned long long>(tot_out);
+        int* eidx = M.get<int>(tot_out);
+        int* eidx2 = M.get<int>(tot_out);
+        tab = M.get<float>(3 * (size_t)tot_out);
+        TA(msd && ekeys && ekeys2 && eidx && eidx2 && tab);
+        const int gc = (int)std::min<int64_t>(std::max<int64_t>(nchunks, 1), (int64_t)num_sms * 64);
+        TK(cudaEventRecord(M.ev[0], st));
+        msd_kernel<<<gc, MSD_LAGS, 0, st>>>(pos, taken, gbase, gspan, glags, gout, cstart, G, nchunks, msd);
+        TK(cudaEventRecord(M.ev[1], st));
+        TK(cudaGetLastError());
+        const unsigned long long last = hs[1] * (unsigned long long)G;
+        msd_keys_kernel<<<gg, 128, 0, st>>>(msd, gout, glags, G, last, ekeys, eidx);
+        TK(cudaGetLastError());
+        cub::DoubleBuffer<unsigned long long> dk(ekeys, ekeys2);
+        cub::DoubleBuffer<int> dv(eidx, eidx2);
+        const int bits = bits_for(last);
+        TK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, dk, dv, (int)tot_out, 0, bits, st));
+        t = M.get<char>(tmp);
+        TA(t);
+        TK(cub::DeviceRadixSort::SortPairs(t, tmp, dk, dv, (int)tot_out, 0, bits, st));
+        msd_table_kernel<<<grid, 256, 0, st>>>(dk.Current(), dv.Current(), msd, tot_out, G, last, S.keys, gstart, S.idmin,
+                                               tab, stat + 2);
+        TK(cudaGetLastError());
+    }
+    TK(cudaMemcpyAsync(hs, stat, sizeof(hs), cudaMemcpyDeviceToHost, st));
     TK(cudaStreamSynchronize(st));
-    if (h_err) {
+    if (hs[0]) {
         *msg = "more than one position for a particle in one frame (one trajectory per particle expected)";
         return GT_ERR_ARG;
     }
-    int64_t nvalid = 0;
-    *ms_msd = 0.f;
-    float* tab = nullptr;
-    if (tot_out > 0) {
-        float* msd = B.get<float>(tot_out);
-        unsigned long long* ekeys = B.get<unsigned long long>(tot_out);
-        unsigned long long* ekeys2 = B.get<unsigned long long>(tot_out);
-        int64_t* eidx = B.get<int64_t>(tot_out);
-        int64_t* eidx2 = B.get<int64_t>(tot_out);
-        unsigned long long* nv = B.get<unsigned long long>(1);
-        TA(msd && ekeys && ekeys2 && eidx && eidx2 && nv);
-        int64_t* gch = B.get<int64_t>(2 * (size_t)G);
-        TA(gch);
-        msd_chunks_kernel<<<grid, 256, 0, st>>>(glags, G, gch);
-        TK(cudaGetLastError());
-        int64_t nchunks = 0;
-        rc = exclusive_sum(gch, gch + G, G, B, st, &nchunks, msg);
-        if (rc) return rc;
-        const int gc = (int)std::min<int64_t>(std::max<int64_t>(nchunks, 1), (int64_t)num_sms * 64);
-        cudaEvent_t e0, e1;
-        TK(cudaEventCreate(&e0));
-        TK(cudaEventCreate(&e1));
-        TK(cudaEventRecord(e0, st));
-        msd_kernel<<<gc, MSD_LAGS, 0, st>>>(pos, taken, gbase, gspan, glags, gout, gch + G, G, nchunks, msd);
-        TK(cudaEventRecord(e1, st));
-        TK(cudaGetLastError());
-        msd_keys_kernel<<<gg, 128, 0, st>>>(msd, gout, glags, Gr.keys, Gr.gstart, G, ekeys, eidx);
-        TK(cudaGetLastError());
-        cub::DoubleBuffer<unsigned long long> dk(ekeys, ekeys2);
-        cub::DoubleBuffer<int64_t> dv(eidx, eidx2);
-        size_t tmp = 0;
-        TK(cub::DeviceRadixSort::SortPairs(nullptr, tmp, dk, dv, (int)tot_out, 0, 64, st));
-        void* t = B.get<char>(tmp);
-        TA(t);
-        TK(cub::DeviceRadixSort::SortPairs(t, tmp, dk, dv, (int)tot_out, 0, 64, st));
-        TK(cudaMemsetAsync(nv, 0, sizeof(unsigned long long), st));
-        count_valid_kernel<<<grid, 256, 0, st>>>(dk.Current(), tot_out, nv);
-        TK(cudaGetLastError());
-        unsigned long long hv = 0;
-        TK(cudaMemcpyAsync(&hv, nv, sizeof(hv), cudaMemcpyDeviceToHost, st));
-        TK(cudaStreamSynchronize(st));
-        cudaEventElapsedTime(ms_msd, e0, e1);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        nvalid = (int64_t)hv;
-        tab = B.get<float>(3 * (size_t)std::max<int64_t>(nvalid, 1));
-        TA(tab);
-        if (nvalid > 0) {
-            msd_table_kernel<<<grid, 256, 0, st>>>(dk.Current(), dv.Current(), msd, nvalid, Gr.idmin, tab);
-            TK(cudaGetLastError());
-        }
-    }
+    if (timed) cudaEventElapsedTime(ms_msd, M.ev[0], M.ev[1]);
+    const int64_t nvalid = (int64_t)hs[2];
     *out = alloc(sizeof(float) * 3 * (size_t)std::max<int64_t>(nvalid, 1));
     if (!*out) {
         *msg = "host allocation failed";

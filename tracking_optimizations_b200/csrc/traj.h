@@ -1,0 +1,78 @@
+// traj.h -- device scratch of the trajectory calls, kept by the context.
+#pragma once
+#include <cuda_runtime.h>
+#include <stddef.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "hostcopy.h"
+
+namespace gt {
+
+// Scratch handed out piece by piece and taken back as a whole by the next
+// call's begin() (every call ends with its stream synchronised).  What a call
+// needed is one block for the next call.
+struct TrajMem {
+    HostCopy* hc = nullptr;
+    cudaEvent_t ev[2] = {nullptr, nullptr};
+
+    cudaError_t begin() {
+        for (auto& e : ev)
+            if (!e) {
+                const cudaError_t r = cudaEventCreate(&e);
+                if (r != cudaSuccess) return r;
+            }
+        if (blocks_.size() > 1) {
+            size_t sum = 0;
+            for (auto& b : blocks_) sum += b.size;
+            release();
+            add(sum);  // a failure shows at the first get()
+        }
+        used_ = 0;
+        return cudaSuccess;
+    }
+
+    template <class X>
+    X* get(size_t n) {
+        const size_t bytes = (sizeof(X) * std::max<size_t>(n, 1) + 255) / 256 * 256;
+        if (blocks_.empty() || used_ + bytes > blocks_.back().size) {
+            if (!add(std::max(bytes, (size_t)16 << 20))) return nullptr;
+            used_ = 0;
+        }
+        char* p = blocks_.back().p + used_;
+        used_ += bytes;
+        return (X*)p;
+    }
+
+    void release() {
+        for (auto& b : blocks_) cudaFree(b.p);
+        blocks_.clear();
+        used_ = 0;
+    }
+
+    ~TrajMem() {
+        release();
+        for (auto& e : ev)
+            if (e) cudaEventDestroy(e);
+    }
+
+  private:
+    struct Block {
+        char* p;
+        size_t size;
+    };
+    bool add(size_t bytes) {
+        void* q = nullptr;
+        if (cudaMalloc(&q, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        blocks_.push_back({(char*)q, bytes});
+        return true;
+    }
+    std::vector<Block> blocks_;
+    size_t used_ = 0;
+};
+
+}  // namespace gt

@@ -109,7 +109,8 @@ def imsd(ids, frames, x, y, mpp, fps, max_lagtime=100, device=0):
     finally:
         lib.gt_table_free(ctypes.byref(tab))
     lag = a[:, 0].astype(np.float64)
-    return lag / float(fps), a[:, 1].astype(np.int64), a[:, 2]
+    lag /= float(fps)
+    return lag, a[:, 1].astype(np.int64), a[:, 2]
 
 
 def postprocess(df, params):
