@@ -11,7 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgt.so")
-SOURCES = ["gt_api.cu", "locate.cu", "locate_fast.cu", "locate_flex.cu", "finalize.cu", "link.cu", "assemble.cu", "noalloc.cu",
+SOURCES = ["gt_api.cu", "locate.cu", "locate_fast.cu", "locate_flex.cu", "finalize.cu", "link.cu", "linktable.cu", "assemble.cu", "noalloc.cu",
            "adjoint.cu", "synth.cu", "traj.cu", "ingest.cpp", "hostcopy.cpp"]
 
 # --fmad=false: the only fused multiply-adds are explicit fmaf() calls, so the

@@ -65,6 +65,11 @@ int traj_imsd(const int64_t* h_ids, const int64_t* h_frames, const float* h_x, c
               float mppf, int64_t max_lagtime, float* (*alloc)(size_t), float** out, int64_t* nout, float* ms_msd,
               TrajMem& M, cudaStream_t st, int num_sms, std::string* msg);
 
+int table_load(const float* h_rows, int n, int ncols, TrajMem& M, cudaStream_t st, int num_sms, LinkTable* t,
+               std::string* msg);
+cudaError_t table_slabs(const LinkTable& t, int cap, float* py, float* px, int* npart, int num_sms, cudaStream_t st);
+cudaError_t table_ids(const LinkTable& t, const int* root, const int* newid, int num_sms, cudaStream_t st);
+
 // preprocess_rows.wgsl:44-45: taps exp(-i^2 / (2 * noise_size)) for
 // i = -k/2..k/2 and their running sum; the passes multiply by the
 // reciprocal of that sum (a shader division).  With `normalized` the taps
@@ -502,7 +507,7 @@ LinkBufs link_bufs(const Plan& P, const Work& w, long long budget) {
     LinkBufs L{};
     L.tb = 0;
     L.te = P.T;
-    L.T = P.T; L.cap_p = P.cap_p; L.memory = (int)P.r.memory;
+    L.T = P.T; L.cap_p = P.cap_p; L.memory = (int)std::min<uint32_t>(P.r.memory, (uint32_t)P.T);
     L.r = P.r.search_range;
     L.inv_g = 1.0f / (float)P.LG;
     L.ncx = P.lncx; L.ncy = P.lncy;
@@ -1926,43 +1931,13 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
     if (n == 0) return GT_OK;
     if (n > (1LL << 30)) { ctx->err = "table too large"; return GT_ERR_ARG; }
     const uint32_t mem = has_memory ? memory : 0;
-    // FrameSubsetter (linking.rs:33-61): runs of equal column-0 values; the
-    // iterator starts with cur_frame = 0, so a first value != 0 yields a
-    // leading empty group.
-    std::vector<int64_t> gstart;
-    std::vector<int> gsize;
-    {
-        int64_t idx = 0;
-        float cur = 0.0f;
-        while (true) {
-            int64_t s = idx;
-            bool end = false;
-            while (true) {
-                if (idx >= n) { end = true; break; }
-                const float fr = rows[idx * ncols];
-                if (fr != cur) { cur = fr; break; }
-                ++idx;
-            }
-            if (end && idx == s) break;
-            gstart.push_back(s);
-            gsize.push_back((int)(idx - s));
-            if (end) break;
-        }
-    }
-    const int T = (int)gstart.size();
-    int maxg = 1;
-    float ymin = 0.f, ymax = 1.f, xmin = 0.f, xmax = 1.f;
-    bool first = true;
-    for (int64_t i = 0; i < n; ++i) {
-        const float y = rows[i * ncols + 2], x = rows[i * ncols + 3];
-        if (!std::isfinite(y) || !std::isfinite(x)) { ctx->err = "non-finite position"; return GT_ERR_ARG; }
-        if (first) { ymin = ymax = y; xmin = xmax = x; first = false; }
-        ymin = std::min(ymin, y); ymax = std::max(ymax, y);
-        xmin = std::min(xmin, x); xmax = std::max(xmax, x);
-    }
-    for (int g : gsize) maxg = std::max(maxg, g);
     CK(cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
+    LinkTable tab;
+    ctx->traj.hc = &ctx->hc;
+    int rc = table_load(rows, (int)n, ncols, ctx->traj, st, ctx->num_sms, &tab, &ctx->err);
+    if (rc) return rc;
+    const int T = tab.T;
     for (int scale = 1; scale <= 64; scale *= 4) {
         Plan P;
         P.T = T;
@@ -1970,34 +1945,22 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         P.r = Resolved{};
         P.r.has_search_range = 1;
         P.r.search_range = search_range;
-        P.r.memory = mem;
-        P.cap_p = maxg;
-        // grid over the positions' bounding box, shifted to start at 0
+        P.r.memory = std::min<uint32_t>(mem, (uint32_t)T);  // no entry is older than the table
+        P.cap_p = tab.largest;
         // cells of absolute positions; negative coordinates clamp into the
         // first cell (clamping is monotone, so neighbours stay adjacent)
-        const double ext = std::max({(double)ymax, (double)xmax, 0.0}) + 1.0;
+        const double ext = (double)std::max(tab.ymax, tab.xmax) + 1.0;
         P.LG = std::max({(int)std::ceil(search_range) + 1, 8, (int)std::ceil(ext / 200.0)});
-        P.lncy = (int)(std::max(ymax, 0.0f) / P.LG) + 1;
-        P.lncx = (int)(std::max(xmax, 0.0f) / P.LG) + 1;
-        (void)ymin; (void)xmin;
+        P.lncy = (int)(tab.ymax / P.LG) + 1;
+        P.lncx = (int)(tab.xmax / P.LG) + 1;
         link_scratch(&P, scale);
         P.cap_c = 1;
         Work w{};
         const size_t need = carve(P, nullptr, &w, 0, false);
-        int rc = ensure_arena(ctx, need);
+        rc = ensure_arena(ctx, need);
         if (rc) return rc;
         carve(P, ctx->arena, &w, 0, false);
-        // particle slabs, positions shifted so the grid starts at the origin
-        std::vector<float> hy((size_t)T * P.cap_p, 0.f), hx((size_t)T * P.cap_p, 0.f);
-        for (int t = 0; t < T; ++t)
-            for (int i = 0; i < gsize[t]; ++i) {
-                const int64_t rr = gstart[t] + i;
-                hy[(size_t)t * P.cap_p + i] = rows[rr * ncols + 2];
-                hx[(size_t)t * P.cap_p + i] = rows[rr * ncols + 3];
-            }
-        CK(cudaMemcpyAsync(w.py, hy.data(), sizeof(float) * hy.size(), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(w.px, hx.data(), sizeof(float) * hx.size(), cudaMemcpyHostToDevice, st));
-        CK(cudaMemcpyAsync(w.npart, gsize.data(), sizeof(int) * T, cudaMemcpyHostToDevice, st));
+        CK(table_slabs(tab, P.cap_p, w.py, w.px, w.npart, ctx->num_sms, st));
         CK(cudaMemsetAsync(w.err, 0, sizeof(int) * 4, st));
         CK(cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(sizeof(int) * (size_t)P.lncx * P.lncy)));
@@ -2008,9 +1971,7 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         rc = run_link(ctx, P, w, st);
         if (rc) return rc;
         // ids in row order: compact index g == row index
-        std::vector<int> root(n), newid(n);
-        CK(cudaMemcpyAsync(root.data(), w.root, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(newid.data(), w.newid, sizeof(int) * n, cudaMemcpyDeviceToHost, st));
+        CK(table_ids(tab, w.root, w.newid, ctx->num_sms, st));
         int bits = 0;
         CK(cudaMemcpyAsync(&bits, w.err, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -2018,7 +1979,7 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         rc = err_status(ctx, bits, &retry);
         if (rc && retry && scale < 64) continue;
         if (rc) return rc;
-        for (int64_t i = 0; i < n; ++i) ids[i] = (uint64_t)newid[root[i]];
+        CK(ctx->hc.download(ids, tab.ids, sizeof(uint64_t) * (size_t)n, st));
         ctx->stats.particles = n;
         return GT_OK;
     }

@@ -1,4 +1,4 @@
-// traj.h -- device scratch of the trajectory calls, kept by the context.
+// traj.h -- device scratch of the calls on host tables, kept by the context.
 #pragma once
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -73,6 +73,17 @@ struct TrajMem {
     }
     std::vector<Block> blocks_;
     size_t used_ = 0;
+};
+
+// A position table on the device and its frames (linktable.cu).
+struct LinkTable {
+    const float* rows = nullptr;
+    int n = 0, ncols = 0, T = 0;
+    int* frame = nullptr;  // per row
+    int* off = nullptr;    // first row of each frame; off[T] = n
+    int largest = 1;       // rows of the largest frame
+    float ymax = 0.f, xmax = 0.f;  // at least 0
+    unsigned long long* ids = nullptr;
 };
 
 }  // namespace gt
