@@ -141,6 +141,7 @@ constexpr int LOC_CMAX = 512;
 constexpr int FB_WIN_MAX = 100;
 constexpr long long SUBNET_BUDGET = 1LL << 26;  // option trials per subnet
 constexpr int LINK_WINDOWS = 16;  // upload chunks of the host-frames path, at most
+constexpr int LINK_RUNS = 4;      // linker launches over them, at most
 
 struct Resolved {
     // lib.rs:77-91 defaults
@@ -662,8 +663,9 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
         return GT_OK;
     };
     // With host frames and linking, each uploaded chunk is also finalized
-    // (pending walks, ordering, separation filter, offsets) and linked
-    // behind its copy, so only the last chunk's work follows the upload.
+    // (pending walks, ordering, separation filter, offsets) behind its copy,
+    // and every few chunks are linked, so only the last ones' work follows the
+    // upload.
     const int nchunks = (T + chunk - 1) / chunk;
     const bool chunked = h_frames && P.link && nchunks > 1 && nchunks <= LINK_WINDOWS;
     if (P.link) {
@@ -672,18 +674,21 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     }
     CK(cudaMemsetAsync(w.pbeg, 0, sizeof(int) * LINK_WINDOWS, st));
     CK(cudaFuncSetAttribute(fallback_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem_fb));
-    int wi = 0;
+    int wi = 0, linked = 0;
     auto post = [&](int f0, int nf) -> int {
         fallback_walk_kernel<<<ctx->num_sms * 4, 128, P.smem_fb, st>>>(P.lp, b, P.fb_win, w.pbeg + wi);
         CK(launch_finalize(P.lp, b, P.sep, P.link, f0, nf, P.smem_fin, st));
         scan_frames_from_kernel<<<1, 1024, 0, st>>>(w.npart, w.off, f0, nf);
         CK(cudaGetLastError());
         ctx->stats.launches += 3;
-        if (P.link) {
-            const int r2 = link_window(ctx, P, w, st, f0, f0 + nf);
-            if (r2) return r2;
-        }
         ++wi;
+        // linked in LINK_RUNS runs of chunks: a run costs its passes (about 15
+        // us each) whatever its frames, 13 runs 2.0 ms of a 200-frame movie
+        if (P.link && (f0 + nf == T || wi % ((nchunks + LINK_RUNS - 1) / LINK_RUNS) == 0)) {
+            const int r2 = link_window(ctx, P, w, st, linked, f0 + nf);
+            if (r2) return r2;
+            linked = f0 + nf;
+        }
         return GT_OK;
     };
     // the fallback list position where chunk wi's entries begin

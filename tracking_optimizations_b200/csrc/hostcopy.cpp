@@ -4,6 +4,10 @@
 #include <algorithm>
 #include <cstring>
 
+#ifdef __SSE2__
+#include <emmintrin.h>
+#endif
+
 namespace gt {
 
 namespace {
@@ -37,6 +41,28 @@ void CopyPool::start() {
     }
 }
 
+// memcpy for data that the device reads next: stores past the caches.  A
+// transfer that finds its lines dirty in eight cores' caches ran at 7 GB/s.
+static void stream_copy(char* d, const char* s, size_t n) {
+#ifdef __SSE2__
+    const size_t head = std::min(n, (size_t)(-(intptr_t)d & 63));
+    std::memcpy(d, s, head);
+    d += head; s += head; n -= head;
+    for (; n >= 64; n -= 64, d += 64, s += 64) {
+        const __m128i a = _mm_loadu_si128((const __m128i*)s), b = _mm_loadu_si128((const __m128i*)(s + 16));
+        const __m128i c = _mm_loadu_si128((const __m128i*)(s + 32)), e = _mm_loadu_si128((const __m128i*)(s + 48));
+        _mm_stream_si128((__m128i*)d, a);
+        _mm_stream_si128((__m128i*)(d + 16), b);
+        _mm_stream_si128((__m128i*)(d + 32), c);
+        _mm_stream_si128((__m128i*)(d + 48), e);
+    }
+    std::memcpy(d, s, n);
+    _mm_sfence();
+#else
+    std::memcpy(d, s, n);
+#endif
+}
+
 // Worker `part` copies its share of every job.
 void CopyPool::work(unsigned part) {
     unsigned long long seen = 0;
@@ -50,20 +76,21 @@ void CopyPool::work(unsigned part) {
         char* d = dst_;
         const char* s = src_;
         lk.unlock();
-        if (b1 > b0) std::memcpy(d + b0, s + b0, b1 - b0);
+        if (b1 > b0) (to_device_ ? stream_copy(d + b0, s + b0, b1 - b0) : (void)std::memcpy(d + b0, s + b0, b1 - b0));
         lk.lock();
         if (--left_ == 0) done_.notify_one();
     }
 }
 
-void CopyPool::copy(void* dst, const void* src, size_t bytes) {
+void CopyPool::copy(void* dst, const void* src, size_t bytes, bool to_device) {
+    const auto own = [&](size_t n) { to_device ? stream_copy((char*)dst, (const char*)src, n) : (void)std::memcpy(dst, src, n); };
     if (bytes < 2 * PART_MIN) {
-        std::memcpy(dst, src, bytes);
+        own(bytes);
         return;
     }
     if (threads_.empty()) start();
     if (threads_.empty()) {
-        std::memcpy(dst, src, bytes);
+        own(bytes);
         return;
     }
     size_t mine;
@@ -72,12 +99,13 @@ void CopyPool::copy(void* dst, const void* src, size_t bytes) {
         dst_ = (char*)dst;
         src_ = (const char*)src;
         bytes_ = bytes;
+        to_device_ = to_device;
         left_ = (unsigned)threads_.size();
         ++job_;
         mine = std::min(bytes, (bytes / (threads_.size() + 1) + 63) / 64 * 64);
     }
     go_.notify_all();
-    std::memcpy(dst, src, mine);
+    own(mine);
     std::unique_lock<std::mutex> lk(m_);
     done_.wait(lk, [&] { return left_ == 0; });
 }
@@ -120,7 +148,7 @@ cudaError_t HostCopy::upload(void* dst, const void* src, size_t bytes, cudaStrea
         next_ = (next_ + 1) % SLOTS;
         cudaError_t e = cudaEventSynchronize(ev_[s]);  // the slot's last transfer, on whatever stream
         if (e != cudaSuccess) return e;
-        pool_.copy(slot_[s], (const char*)src + at, n);
+        pool_.copy(slot_[s], (const char*)src + at, n, true);
         e = cudaMemcpyAsync((char*)dst + at, slot_[s], n, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaEventRecord(ev_[s], st);
         if (e != cudaSuccess) return e;
@@ -154,7 +182,7 @@ cudaError_t HostCopy::download(void* dst, const void* src, size_t bytes, cudaStr
         const int s = (int)((first + i) % SLOTS);
         const cudaError_t e = cudaEventSynchronize(ev_[s]);
         if (e != cudaSuccess) return e;
-        pool_.copy((char*)dst + i * SLOT, slot_[s], std::min(SLOT, bytes - i * SLOT));
+        pool_.copy((char*)dst + i * SLOT, slot_[s], std::min(SLOT, bytes - i * SLOT), false);
     }
     next_ = (int)((first + parts) % SLOTS);
     return cudaSuccess;

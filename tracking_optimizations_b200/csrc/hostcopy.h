@@ -22,7 +22,7 @@ namespace gt {
 class CopyPool {
   public:
     ~CopyPool();
-    void copy(void* dst, const void* src, size_t bytes);
+    void copy(void* dst, const void* src, size_t bytes, bool to_device);
 
   private:
     void start();
@@ -36,6 +36,7 @@ class CopyPool {
     char* dst_ = nullptr;
     const char* src_ = nullptr;
     size_t bytes_ = 0;
+    bool to_device_ = false;
 };
 
 // Owned by one context and used by one call at a time, as the context is.

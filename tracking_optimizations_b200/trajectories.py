@@ -16,6 +16,7 @@ import ctypes
 import numpy as np
 
 from . import _native
+from .gpu_tracking import _adopt_table as adopt_table
 
 
 def _i64(a):
@@ -104,10 +105,10 @@ def imsd(ids, frames, x, y, mpp, fps, max_lagtime=100, device=0):
     _native.check(lib.gt_imsd(ctx, _ptr(ids), _ptr(frames), _ptr(x), _ptr(y), n, float(mpp), int(max_lagtime),
                               ctypes.byref(tab)), ctx)
     try:
-        m = tab.nrows
-        a = np.ctypeslib.as_array(tab.data, shape=(max(m, 1) * 3,))[: m * 3].reshape(m, 3).copy()
-    finally:
+        a = adopt_table(lib, tab, tab.nrows, 3)
+    except BaseException:
         lib.gt_table_free(ctypes.byref(tab))
+        raise
     lag = a[:, 0].astype(np.float64)
     lag /= float(fps)
     return lag, a[:, 1].astype(np.int64), a[:, 2]
