@@ -114,11 +114,8 @@ __device__ __forceinline__ bool within_r(float qy, float qx, float iy, float ix,
 }  // namespace
 
 template <int NTF>
-__global__ void __launch_bounds__(NTF) finalize_kernel(const LocParams p, MovieBufs b, float sep,
-                                                       int link_grid, int frame0) {
-    __shared__ int warp_tot[NTF / 32];
-    __shared__ int s_total;
-    extern __shared__ int cnt_s[];  // cells of the larger grid
+__device__ __forceinline__ void finalize_frame(const LocParams& p, const MovieBufs& b, float sep, int link_grid,
+                                               int frame0, int* cnt_s, int* warp_tot, int& s_total) {
     const int t = frame0 + blockIdx.x;
     const int cap_c = b.cap_c;
     const int nrc = p.H * p.ntx;
@@ -230,12 +227,46 @@ __global__ void __launch_bounds__(NTF) finalize_kernel(const LocParams p, MovieB
     }
 }
 
+template <int NTF>
+__global__ void __launch_bounds__(NTF) finalize_kernel(const LocParams p, MovieBufs b, float sep,
+                                                       int link_grid, int frame0) {
+    __shared__ int warp_tot[NTF / 32];
+    __shared__ int s_total, s_last;
+    extern __shared__ int cnt_s[];  // cells of the larger grid
+    finalize_frame<NTF>(p, b, sep, link_grid, frame0, cnt_s, warp_tot, s_total);
+    if (!b.done) return;
+    // the last block done: offsets of the launch's frames (a launch of its own
+    // costs a short movie more than the sums)
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(b.done, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const int n = gridDim.x;
+    int carry = frame0 > 0 ? b.off[frame0] : 0;
+    for (int b0 = 0; b0 < n; b0 += NTF) {
+        const int i = b0 + threadIdx.x;
+        const int v = i < n ? __ldcg(b.npart + frame0 + i) : 0;
+        const int e = block_excl_scan<NTF>(v, warp_tot, &s_total);
+        if (i < n) b.off[frame0 + i] = carry + e;
+        carry += s_total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        b.off[frame0 + n] = carry;
+        *b.nrows = carry;
+        *b.done = 0;
+    }
+}
+
 // Frames of 2^20 pixels and more: 1024 threads.
 cudaError_t launch_finalize(const LocParams& p, const MovieBufs& b, float sep, int link_grid, int frame0, int nf,
                             size_t smem, cudaStream_t st) {
     const bool big = (long long)p.H * p.W >= (1LL << 20);
-    const void* fn = big ? (const void*)finalize_kernel<1024> : (const void*)finalize_kernel<512>;
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = big ? allow_shared<finalize_kernel<1024>>() : allow_shared<finalize_kernel<512>>();
     if (e != cudaSuccess) return e;
     if (big) finalize_kernel<1024><<<nf, 1024, smem, st>>>(p, b, sep, link_grid, frame0);
     else finalize_kernel<512><<<nf, 512, smem, st>>>(p, b, sep, link_grid, frame0);

@@ -39,7 +39,6 @@ cudaError_t launch_link(const LinkBufs& L, int max_passes, int* passes, unsigned
 cudaError_t launch_link_multi(const LinkBufs* d_L, int nm, int max_passes, int* passes, unsigned long long* stat,
                               int grid, cudaStream_t st);
 __global__ void scan_frames_kernel(const int* in, int* out, int n);
-__global__ void scan_frames_from_kernel(const int* in, int* out, int f0, int n);
 __global__ void newid_kernel(const int* newrank, const int* newbase, const int* off, const int* npart,
                              int* newid, int T);
 cudaError_t launch_assemble(const AsmArgs& a, int num_sms, cudaStream_t st);
@@ -104,6 +103,7 @@ struct gt_ctx {
     char* arena = nullptr;
     size_t arena_size = 0;
     gt_stats stats{};
+    int stage_times = 0;  // 1: the stage times of stats are still in ev[0..4]
     int num_sms = 148;
     cudaEvent_t ev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
     int normalized_taps = 0;          // Gaussian taps divided by their sum on the host
@@ -141,6 +141,7 @@ constexpr int LOC_CMAX = 512;
 constexpr int FB_WIN_MAX = 100;
 constexpr long long SUBNET_BUDGET = 1LL << 26;  // option trials per subnet
 constexpr int LINK_WINDOWS = 16;  // upload chunks of the host-frames path, at most
+constexpr int STATUS_LSTAT = 8 + LINK_WINDOWS, STATUS_INTS = STATUS_LSTAT + 2 * (12 + 8);
 constexpr int LINK_RUNS = 4;      // linker launches over them, at most
 
 struct Resolved {
@@ -246,6 +247,7 @@ struct Plan {
     int fast_th = 32;
     std::vector<float> char_tab, gchar_tab;
     std::vector<int> char_off, sig_off, bg_off;
+    std::vector<int> tables;  // the five one after the other, as they are uploaded
     std::vector<std::string> names, types;
 };
 
@@ -346,6 +348,10 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     P.sig_off.clear(); P.bg_off.clear();
     if (r.has_sig) circle_inds_f(r.sig_radius, P.sig_off);
     if (r.has_bg) annulus_inds_f(r.bg_radius, r.sig_radius + r.gap_radius, P.bg_off);
+    P.tables.clear();
+    for (const auto* v : {&P.char_tab, &P.gchar_tab})
+        P.tables.insert(P.tables.end(), (const int*)v->data(), (const int*)v->data() + v->size());
+    for (const auto* v : {&P.char_off, &P.sig_off, &P.bg_off}) P.tables.insert(P.tables.end(), v->begin(), v->end());
     P.sep = (float)r.separation;
     P.link = r.has_search_range;
 
@@ -388,14 +394,17 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
 struct Work {
     void* frames;
     Cand* cand;
-    int *fcount, *rowcnt, *pend, *npend;
+    int *rowcnt, *pend;
     float *py, *px, *pm;
     int *prec, *npart, *gstart, *gidx;
     int *cperm, *crec, *ccell, *cstart, *cidx;
     float *cy, *cx, *cm;
+    int* tables;
     float *char_tab, *gchar_tab;
     int *char_off, *sig_off, *bg_off;
-    int* err;
+    // zeroed at the start of a call and read back as one at its end
+    int* status;
+    int *err, *nrows, *npend, *done, *fcount;
     int *off, *pred, *newrank, *newcount, *newbase, *root, *lroot, *newid;
     int* pbeg;  // fallback list position at the start of each chunk's locate
     // linker (LinkBufs)
@@ -426,10 +435,8 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->frames = c.take<char>(frame_bytes);
     const size_t cc = need_locate ? T * P.cap_c : 1;
     w->cand = c.take<Cand>(cc);
-    w->fcount = c.take<int>(T);
     w->rowcnt = c.take<int>(need_locate ? T * P.H * P.lp.ntx : 1);
     w->pend = c.take<int>(cc);
-    w->npend = c.take<int>(1);
     w->py = c.take<float>(T * P.cap_p);
     w->px = c.take<float>(T * P.cap_p);
     w->pm = c.take<float>(T * P.cap_p);
@@ -445,12 +452,23 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->cy = c.take<float>(cc);
     w->cx = c.take<float>(cc);
     w->cm = c.take<float>(cc);
-    w->char_tab = c.take<float>(P.char_tab.size());
-    w->gchar_tab = c.take<float>(P.gchar_tab.size());
-    w->char_off = c.take<int>(P.char_off.size());
-    w->sig_off = c.take<int>(P.sig_off.size());
-    w->bg_off = c.take<int>(P.bg_off.size());
-    w->err = c.take<int>(4);
+    int* tab = c.take<int>(P.tables.size());
+    w->tables = tab;
+    w->char_tab = (float*)tab;
+    w->gchar_tab = (float*)(tab += P.char_tab.size());
+    w->char_off = tab += P.gchar_tab.size();
+    w->sig_off = tab += P.char_off.size();
+    w->bg_off = tab += P.sig_off.size();
+    // {errors and linker passes, rows, pending walks, blocks done, the chunks'
+    // first pending walks, linker statistics, records per frame}
+    w->status = c.take<int>(STATUS_INTS + T);
+    w->err = w->status;
+    w->nrows = w->status + 4;
+    w->npend = w->status + 5;
+    w->done = w->status + 6;
+    w->pbeg = w->status + 8;
+    w->lstat = (unsigned long long*)(w->status + STATUS_LSTAT);
+    w->fcount = w->status + STATUS_INTS;
     w->off = c.take<int>(T + 1);
     const size_t np = P.link ? T * P.cap_p : 1;
     const size_t nm = P.link && P.r.memory > 0 ? np : 1;   // memory entries
@@ -464,7 +482,6 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->root = c.take<int>(np);
     w->lroot = c.take<int>(np);
     w->newid = c.take<int>(np);
-    w->pbeg = c.take<int>(LINK_WINDOWS);
     w->lnk = c.take<unsigned>(nm);
     w->mm = c.take<unsigned>(nm * nw);
     w->stamp = c.take<int>(nm);
@@ -480,7 +497,6 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->ent = c.take<int4>(nl);
     w->pres = c.take<unsigned>(nl * nw);
     w->fstamp = c.take<int>(T);
-    w->lstat = c.take<unsigned long long>(12 + 8);
     w->big = c.take<int>((size_t)P.nslot * big_ints(P));
     w->out = c.take<float>(need_locate && own_out ? T * P.cap_p * P.names.size() : 1);
     return c.off + 256;
@@ -537,11 +553,6 @@ LinkBufs link_bufs(const Plan& P, const Work& w, long long budget) {
 // order give the sequential result (the host-frames path links each
 // uploaded chunk while the next one is copied).  link_prepare runs once
 // before the first window, link_finish once after the last.
-int link_prepare(gt_ctx* ctx, const Work& w, cudaStream_t st) {
-    CK(cudaMemsetAsync(w.lstat, 0, sizeof(unsigned long long) * (12 + 8), st));
-    return GT_OK;
-}
-
 // Resident blocks of the one-movie (0) or the batched (1) linker.
 int link_grid(gt_ctx* ctx, int multi, int* grid) {
     if (!ctx->link_grid[multi]) {
@@ -577,23 +588,14 @@ int link_finish(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st) {
 }
 
 int run_link(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st) {
-    int rc = link_prepare(ctx, w, st);
-    if (!rc) rc = link_window(ctx, P, w, st, 0, P.T);
+    int rc = link_window(ctx, P, w, st, 0, P.T);
     if (!rc) rc = link_finish(ctx, P, w, st);
     return rc;
 }
 
 int upload_tables(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st) {
-    auto up = [&](void* dst, const void* src, size_t bytes) -> int {
-        if (bytes) CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
-        return GT_OK;
-    };
-    int rc;
-    if ((rc = up(w.char_tab, P.char_tab.data(), sizeof(float) * P.char_tab.size()))) return rc;
-    if ((rc = up(w.gchar_tab, P.gchar_tab.data(), sizeof(float) * P.gchar_tab.size()))) return rc;
-    if ((rc = up(w.char_off, P.char_off.data(), sizeof(int) * P.char_off.size()))) return rc;
-    if ((rc = up(w.sig_off, P.sig_off.data(), sizeof(int) * P.sig_off.size()))) return rc;
-    if ((rc = up(w.bg_off, P.bg_off.data(), sizeof(int) * P.bg_off.size()))) return rc;
+    if (!P.tables.empty())
+        CK(cudaMemcpyAsync(w.tables, P.tables.data(), sizeof(int) * P.tables.size(), cudaMemcpyHostToDevice, st));
     return GT_OK;
 }
 
@@ -609,6 +611,7 @@ MovieBufs movie_bufs(const Plan& P, const Work& w, const void* frames) {
     b.cstart = w.cstart; b.cidx = w.cidx;
     b.char_tab = w.char_tab; b.char_off = w.char_off; b.gchar_tab = w.gchar_tab;
     b.err = w.err;
+    b.off = w.off; b.done = w.done; b.nrows = w.nrows;
     return b;
 }
 
@@ -626,10 +629,9 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     MovieBufs b = movie_bufs(P, w, d_frames);
     int rc = upload_tables(ctx, P, w, st);
     if (rc) return rc;
-    CK(cudaMemsetAsync(w.fcount, 0, sizeof(int) * T, st));
-    CK(cudaMemsetAsync(w.npend, 0, sizeof(int), st));
-    CK(cudaMemsetAsync(w.err, 0, sizeof(int) * 4, st));
-    CK(cudaFuncSetAttribute(locate_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem_loc));
+    CK(cudaMemsetAsync(w.status, 0, sizeof(int) * (STATUS_INTS + (size_t)T), st));
+    CK(allow_shared<locate_tiles_kernel>());
+    CK(allow_shared<fallback_walk_kernel>());
     for (int i = 0; i < 5; ++i)
         if (!ctx->ev[i]) CK(cudaEventCreate(&ctx->ev[i]));
     const int ntiles = P.lp.ntx * P.lp.nty;
@@ -668,19 +670,12 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     // upload.
     const int nchunks = (T + chunk - 1) / chunk;
     const bool chunked = h_frames && P.link && nchunks > 1 && nchunks <= LINK_WINDOWS;
-    if (P.link) {
-        rc = link_prepare(ctx, w, st);
-        if (rc) return rc;
-    }
-    CK(cudaMemsetAsync(w.pbeg, 0, sizeof(int) * LINK_WINDOWS, st));
-    CK(cudaFuncSetAttribute(fallback_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem_fb));
     int wi = 0, linked = 0;
     auto post = [&](int f0, int nf) -> int {
         fallback_walk_kernel<<<ctx->num_sms * 4, 128, P.smem_fb, st>>>(P.lp, b, P.fb_win, w.pbeg + wi);
         CK(launch_finalize(P.lp, b, P.sep, P.link, f0, nf, P.smem_fin, st));
-        scan_frames_from_kernel<<<1, 1024, 0, st>>>(w.npart, w.off, f0, nf);
         CK(cudaGetLastError());
-        ctx->stats.launches += 3;
+        ctx->stats.launches += 2;
         ++wi;
         // linked in LINK_RUNS runs of chunks: a run costs its passes (about 15
         // us each) whatever its frames, 13 runs 2.0 ms of a 200-frame movie
@@ -734,9 +729,8 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
         // the whole movie as one window: finalize, then link
         fallback_walk_kernel<<<ctx->num_sms * 4, 128, P.smem_fb, st>>>(P.lp, b, P.fb_win, w.pbeg);
         CK(launch_finalize(P.lp, b, P.sep, P.link, 0, T, P.smem_fin, st));
-        scan_frames_from_kernel<<<1, 1024, 0, st>>>(w.npart, w.off, 0, T);
         CK(cudaGetLastError());
-        ctx->stats.launches += 3;
+        ctx->stats.launches += 2;
     }
     CK(cudaEventRecord(ctx->ev[2], st));
     if (P.link) {
@@ -765,8 +759,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     CK(cudaEventRecord(ctx->ev[4], st));
     // every statistic of the call in one readback: error words, row count,
     // pending walks, per-frame record counts, linker phases and frame counts
-    const size_t ph_off = (6 + (size_t)T + 1) & ~(size_t)1;  // 8-byte aligned for the linker's statistics
-    const size_t need_ints = ph_off + 2 * 12;
+    const size_t need_ints = STATUS_INTS + (size_t)T;
     if (ctx->h_stage_n < need_ints) {
         if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
         ctx->h_stage = nullptr;
@@ -775,17 +768,13 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
         ctx->h_stage_n = need_ints;
     }
     int* hs = ctx->h_stage;
-    CK(cudaMemcpyAsync(hs, w.err, sizeof(int) * 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hs + 4, w.off + T, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hs + 5, w.npend, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(hs + 6, w.fcount, sizeof(int) * T, cudaMemcpyDeviceToHost, st));
-    unsigned long long* hph = (unsigned long long*)(hs + ph_off);
-    if (P.link) CK(cudaMemcpyAsync(hph, w.lstat, sizeof(unsigned long long) * 12, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hs, w.status, sizeof(int) * need_ints, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    int hb[5] = {hs[0], hs[1], hs[2], hs[3], hs[4]};
+    const unsigned long long* hph = (const unsigned long long*)(hs + STATUS_LSTAT);
+    const int hb[5] = {hs[0], hs[1], hs[2], hs[3], hs[4]};
     const int np = hs[5];
     long long nc_total = 0;
-    for (int t = 0; t < T; ++t) nc_total += hs[6 + t];
+    for (int t = 0; t < T; ++t) nc_total += hs[STATUS_INTS + t];
     *err_bits = hb[0];
     *nrows = hb[4];
     ctx->stats.link_iterations = P.link ? hb[1] : 0;
@@ -796,11 +785,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     ctx->stats.fallback_walks = np;
     ctx->stats.particles = hb[4];
     ctx->stats.candidates = nc_total;
-    cudaEventElapsedTime(&ctx->stats.ms_locate, ctx->ev[0], ctx->ev[1]);
-    cudaEventElapsedTime(&ctx->stats.ms_finalize, ctx->ev[1], ctx->ev[2]);
-    cudaEventElapsedTime(&ctx->stats.ms_link, ctx->ev[2], ctx->ev[3]);
-    cudaEventElapsedTime(&ctx->stats.ms_assemble, ctx->ev[3], ctx->ev[4]);
-    cudaEventElapsedTime(&ctx->stats.ms_total, ctx->ev[0], ctx->ev[4]);
+    ctx->stage_times = 1;  // read from the events when asked for (gt_last_stats)
     return GT_OK;
 }
 
@@ -896,6 +881,7 @@ int batch_common(gt_ctx* ctx, const void* frames, bool host, int dtype, int T, i
     if (!ctx) return GT_ERR_ARG;
     ctx->err.clear();
     ctx->stats = gt_stats{};
+    ctx->stage_times = 0;
     if (!frames || !params || T < 1 || H < 1 || W < 1 || (dtype != GT_U16 && dtype != GT_F32)) {
         ctx->err = "invalid frames/shape/dtype";
         return GT_ERR_ARG;
@@ -1012,9 +998,7 @@ int tune_tile_rows(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t
             MovieBufs b = movie_bufs(Q, bm.w, frames);
             const int ntiles = Q.lp.ntx * Q.lp.nty;
             for (int rep = 0; rep < 2; ++rep) {
-                CK(cudaMemsetAsync(bm.w.fcount, 0, sizeof(int) * P.T, st));
-                CK(cudaMemsetAsync(bm.w.npend, 0, sizeof(int), st));
-                CK(cudaMemsetAsync(bm.w.err, 0, sizeof(int) * 4, st));
+                CK(cudaMemsetAsync(bm.w.status, 0, sizeof(int) * (STATUS_INTS + (size_t)P.T), st));
                 CK(cudaEventRecord(ctx->ev[0], st));
                 int used_tma = 0;
                 CK(launch_locate_fast(Q.lp.krad, Q.lp.D, Q.lp.rint_c, ths[v], dim3(ntiles, nf), st, Q.lp, b, P.T, 0,
@@ -1047,9 +1031,7 @@ int enqueue_front(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t 
     const Work& w = bm.w;
     const int T = P.T;
     MovieBufs b = movie_bufs(P, w, frames);
-    CK(cudaMemsetAsync(w.fcount, 0, sizeof(int) * T, s));
-    CK(cudaMemsetAsync(w.npend, 0, sizeof(int), s));
-    CK(cudaMemsetAsync(w.err, 0, sizeof(int) * 4, s));
+    CK(cudaMemsetAsync(w.status, 0, sizeof(int) * (STATUS_INTS + (size_t)T), s));
     const int ntiles = P.lp.ntx * P.lp.nty;
     if (bm.fast) {
         for (int f0 = 0; f0 < T; f0 += 65535) {
@@ -1073,10 +1055,7 @@ int enqueue_front(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t 
     CK(cudaGetLastError());
     fallback_walk_kernel<<<ctx->num_sms, 128, P.smem_fb, s>>>(P.lp, b, P.fb_win, nullptr);
     CK(launch_finalize(P.lp, b, P.sep, P.link, 0, T, P.smem_fin, s));
-    scan_frames_kernel<<<1, 1024, 0, s>>>(w.npart, w.off, T);
-    CK(cudaGetLastError());
-    *launches += 3;
-    if (P.link) return link_prepare(ctx, w, s);
+    *launches += 2;
     return GT_OK;
 }
 
@@ -1103,8 +1082,7 @@ int enqueue_back(gt_ctx* ctx, BatchMovie& bm, const gt_movie& mv, int* d_status,
     a.out_rows = mv.out ? mv.out_rows : 0;
     CK(launch_assemble(a, ctx->num_sms, s));
     *launches += 1;
-    CK(cudaMemcpyAsync(d_status, w.err, sizeof(int) * 4, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(d_status + 4, w.off + T, sizeof(int), cudaMemcpyDeviceToDevice, s));
+    CK(cudaMemcpyAsync(d_status, w.status, sizeof(int) * 5, cudaMemcpyDeviceToDevice, s));
     return GT_OK;
 }
 
@@ -1146,6 +1124,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
     if (!ctx) return GT_ERR_ARG;
     ctx->err.clear();
     ctx->stats = gt_stats{};
+    ctx->stage_times = 0;
     if (n < 0 || (n > 0 && !mv)) { ctx->err = "invalid movie list"; return GT_ERR_ARG; }
     if (n == 0) return GT_OK;
     CK(cudaSetDevice(ctx->device));
@@ -1291,13 +1270,8 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
                 rc = tune_tile_rows(ctx, B[i], mv[i].frames, st);
                 if (rc) return rc;
             }
-        size_t sl = 0, sf = 0;
-        for (int i = 0; i < n; ++i) {
-            sl = std::max(sl, B[i].P.smem_loc);
-            sf = std::max(sf, B[i].P.smem_fb);
-        }
-        CK(cudaFuncSetAttribute(locate_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl));
-        CK(cudaFuncSetAttribute(fallback_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf));
+        CK(allow_shared<locate_tiles_kernel>());
+        CK(allow_shared<fallback_walk_kernel>());
         CK(cudaStreamSynchronize(st));
         // capture; where capture is refused, run the same sequence directly
         cudaGraph_t graph = nullptr;
@@ -1338,7 +1312,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         int cnt = 0;
         for (int i = 0; i < n; ++i) {
             const Plan& P = B[i].P;
-            cnt += (P.T + 65534) / 65535 + 3 + (P.link ? 2 : 0) + 1;
+            cnt += (P.T + 65534) / 65535 + 2 + (P.link ? 2 : 0) + 1;
         }
         S.launches = cnt + (S.nlink > 0 ? 1 : 0);
     }
@@ -1375,6 +1349,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
     }
     ctx->err.clear();
     ctx->stats = keep;
+    ctx->stage_times = 0;
     ctx->stats.batch_fallbacks = fallbacks;
     ctx->stats.particles = rows_total;
     return GT_OK;
@@ -1389,6 +1364,7 @@ int adjoint_setup(gt_ctx* ctx, const float* d_frames, int T, int H, int W, const
     if (!ctx) return GT_ERR_ARG;
     ctx->err.clear();
     ctx->stats = gt_stats{};
+    ctx->stage_times = 0;
     if (!d_frames || !params || T < 1 || H < 1 || W < 1 || n < 0 || (n > 0 && !d_walk)) {
         ctx->err = "invalid frames/shape/walk";
         return GT_ERR_ARG;
@@ -1847,6 +1823,7 @@ int traj_begin(gt_ctx* ctx, int64_t n, bool ok_ptrs) {
     if (!ctx) return GT_ERR_ARG;
     ctx->err.clear();
     ctx->stats = gt_stats{};
+    ctx->stage_times = 0;
     if (n < 0 || (n > 0 && !ok_ptrs)) {
         ctx->err = "invalid arrays";
         return GT_ERR_ARG;
@@ -1923,6 +1900,13 @@ int gt_imsd(gt_ctx* ctx, const int64_t* ids, const int64_t* frames, const float*
 int gt_last_stats(const gt_ctx* ctx, gt_stats* out) {
     if (!ctx || !out) return GT_ERR_ARG;
     *out = ctx->stats;
+    if (ctx->stage_times) {
+        cudaEventElapsedTime(&out->ms_locate, ctx->ev[0], ctx->ev[1]);
+        cudaEventElapsedTime(&out->ms_finalize, ctx->ev[1], ctx->ev[2]);
+        cudaEventElapsedTime(&out->ms_link, ctx->ev[2], ctx->ev[3]);
+        cudaEventElapsedTime(&out->ms_assemble, ctx->ev[3], ctx->ev[4]);
+        cudaEventElapsedTime(&out->ms_total, ctx->ev[0], ctx->ev[4]);
+    }
     return GT_OK;
 }
 
@@ -1931,6 +1915,7 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
     if (!ctx) return GT_ERR_ARG;
     ctx->err.clear();
     ctx->stats = gt_stats{};
+    ctx->stage_times = 0;
     if ((!rows && n > 0) || ncols < 4 || n < 0 || (n > 0 && !ids)) { ctx->err = "invalid table"; return GT_ERR_ARG; }
     if (!(search_range > 0.0f && search_range < 4096.0f)) { ctx->err = "search_range must be in (0, 4096)"; return GT_ERR_ARG; }
     if (n == 0) return GT_OK;
@@ -1966,9 +1951,8 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         if (rc) return rc;
         carve(P, ctx->arena, &w, 0, false);
         CK(table_slabs(tab, P.cap_p, w.py, w.px, w.npart, ctx->num_sms, st));
-        CK(cudaMemsetAsync(w.err, 0, sizeof(int) * 4, st));
-        CK(cudaFuncSetAttribute(grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(int) * (size_t)P.lncx * P.lncy)));
+        CK(cudaMemsetAsync(w.status, 0, sizeof(int) * STATUS_INTS, st));
+        CK(allow_shared<grid_kernel>());
         grid_kernel<<<T, 512, sizeof(int) * (size_t)P.lncx * P.lncy, st>>>(w.py, w.px, w.npart, P.cap_p, P.LG,
                                                                         P.lncy, P.lncx, w.gstart, w.gidx, w.gpos);
         CK(cudaGetLastError());

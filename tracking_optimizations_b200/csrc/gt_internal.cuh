@@ -13,6 +13,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #define GT_MAX_TAPS 64
@@ -108,6 +109,9 @@ struct MovieBufs {
     const int* char_off;     // n_char x {di, dj}
     const float* gchar_tab;  // n_gchar x {sin2, cos2}, (d-1)/2 circle
     int* err;
+    int* off;             // exclusive prefix of npart, by the last block of finalize_kernel
+    int* nrows;           // rows of the frames so far
+    int* done;            // blocks of finalize_kernel that are done (0: not counted, null: no offsets)
 };
 
 struct LinkBufs {
@@ -213,5 +217,24 @@ struct AsmArgs {
     int* walk;            // optional n x 5 {frame, last-read row, col, final row, col}
     long long walk_rows;  // rows of `walk` (rows beyond are not written)
 };
+
+// Lets a kernel have as much dynamic shared memory as there is, once per
+// device: the limit is the process's, so every caller sets the same one.
+template <auto* FN>
+inline cudaError_t allow_shared() {
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    cudaFuncAttributes a;
+    e = cudaFuncGetAttributes(&a, (const void*)FN);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute((const void*)FN, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 227 * 1024 - (int)a.sharedSizeBytes);
+    if (e == cudaSuccess && dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
 
 }  // namespace gt

@@ -299,13 +299,13 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
                       sizeof(int) * 32 * 64 + 6 * sizeof(float) * 512 + 32 * 64;
         smem = (smem + 15) / 16 * 16;
         if (smem > 227 * 1024) return fail(GT_ERR_ARG, "diameter/separation too large for the tile plan");
-        SCK(cudaFuncSetAttribute(locate_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SCK(allow_shared<locate_tiles_kernel>());
         locate_tiles_kernel<<<dim3(lp.ntx * lp.nty, 1), 256, smem, st>>>(lp, b, 0);
         SCK(cudaGetLastError());
     }
     const int fb_win = std::min(100, std::max(lp.rint_c + 1, lp.max_iter - 1 + lp.rint_c + 1));
     const size_t smem_fb = sizeof(float) * (size_t)(2 * fb_win + 1) * (2 * fb_win + 1);
-    SCK(cudaFuncSetAttribute(fallback_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_fb));
+    SCK(allow_shared<fallback_walk_kernel>());
     fallback_walk_kernel<<<ds.num_sms * 4, 128, smem_fb, st>>>(lp, b, fb_win, nullptr);
     SCK(cudaGetLastError());
     SCK(launch_finalize(lp, b, (float)sep, 0, 0, 1, 4 * (size_t)ncell, st));
