@@ -332,7 +332,7 @@ typedef struct gt_stats {
     int32_t link_dirty[8];     /* frames relinked by fixed-point passes 1..8 */
     float ms_adjoint_particles; /* gt_adjoint_*: per-particle kernel */
     float ms_adjoint_dense;     /* gt_adjoint_backward: zeroing + transposed bandpass */
-    int32_t batch_graph;        /* gt_batch_many_device: 2 graph replayed, 1 graph built, 0 no graph */
+    int32_t batch_graph;        /* gt_batch_many_device: 2 graph replayed, 1 launched, graph built meanwhile, 0 no graph */
     int32_t batch_fallbacks;    /* gt_batch_many_device: movies rerun through gt_batch_device */
     float ms_msd;               /* gt_imsd: device time of the per-particle MSD kernel */
 } gt_stats;

@@ -45,7 +45,8 @@ def batch_many(movies, device=None, return_stats=False, outs=None):
     ``table`` an (n, ncols) float32 CUDA tensor; with ``return_stats`` also
     the call's gt_last_stats dict.
 
-    The CUDA graph of a batch is cached and replayed while the frames,
+    The first call on a set of buffers launches the batch and builds its CUDA
+    graph while the device works; the graph is replayed while the frames,
     parameters and output buffers stay the same: pass the same ``outs``
     (from ``output_buffers``) to successive calls to replay it; the returned
     tables are then views of those buffers."""

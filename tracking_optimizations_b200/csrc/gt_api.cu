@@ -1262,7 +1262,6 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         CK(cudaMemcpyAsync(S.d_L, hL.data(), sizeof(LinkBufs) * S.nlink, cudaMemcpyHostToDevice, st));
     }
     if (!replay) {
-        if (ctx->batch_exec) { cudaGraphExecDestroy(ctx->batch_exec); ctx->batch_exec = nullptr; }
         ctx->batch_key.clear();
         // autotuned tile rows (timed on this movie's frames and workspace)
         for (int i = 0; i < n; ++i)
@@ -1272,41 +1271,47 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
             }
         CK(allow_shared<locate_tiles_kernel>());
         CK(allow_shared<fallback_walk_kernel>());
-        CK(cudaStreamSynchronize(st));
-        // capture; where capture is refused, run the same sequence directly
+        CK(cudaEventRecord(ctx->ev[0], st));
+        rc = enqueue_batch(ctx, B, mv, n, S, st);
+        if (rc) return rc;
+        CK(cudaEventRecord(ctx->ev[1], st));
+        // The batch runs as plain launches (they hide behind the first
+        // movies' kernels); the graph that later calls replay is captured and
+        // instantiated while the device works.  Building it first kept the
+        // device idle for that time: 12 movies of 120 frames up to 1024 x 1024
+        // in new buffers 4.6 -> 3.3 ms a call.
+        // Where capture is refused, later calls launch the same way.
         cudaGraph_t graph = nullptr;
         bool captured = false;
         if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
-            const int erc = enqueue_batch(ctx, B, mv, n, S, st);
+            BatchShared Sc = S;
+            const int erc = enqueue_batch(ctx, B, mv, n, Sc, st);
             const cudaError_t ee = cudaStreamEndCapture(st, &graph);
             if (erc == GT_OK && ee == cudaSuccess && graph) {
-                cudaGraphExec_t ex = nullptr;
-                if (cudaGraphInstantiate(&ex, graph, 0) == cudaSuccess) {
-                    ctx->batch_exec = ex;
-                    ctx->batch_key = key;
-                    captured = true;
+                // the last batch's graph takes the new arguments if it has the
+                // same nodes and edges, else it is built anew
+                cudaGraphExecUpdateResultInfo info;
+                if (ctx->batch_exec && cudaGraphExecUpdate(ctx->batch_exec, graph, &info) != cudaSuccess) {
+                    cudaGetLastError();
+                    cudaGraphExecDestroy(ctx->batch_exec);
+                    ctx->batch_exec = nullptr;
                 }
+                captured = ctx->batch_exec || cudaGraphInstantiate(&ctx->batch_exec, graph, 0) == cudaSuccess;
+                if (captured) ctx->batch_key = key;
+                else ctx->batch_exec = nullptr;
             }
             if (graph) cudaGraphDestroy(graph);
-            if (!captured) {
-                cudaGetLastError();
-                ctx->err.clear();
-            }
-        } else {
-            cudaGetLastError();
         }
-        CK(cudaEventRecord(ctx->ev[0], st));
         if (captured) {
-            CK(cudaGraphLaunch(ctx->batch_exec, st));
             ctx->stats.batch_graph = 1;
         } else {
-            rc = enqueue_batch(ctx, B, mv, n, S, st);
-            if (rc) return rc;
+            cudaGetLastError();
+            ctx->err.clear();
         }
     } else {
-        CK(cudaStreamSynchronize(st));
         CK(cudaEventRecord(ctx->ev[0], st));
         CK(cudaGraphLaunch(ctx->batch_exec, st));
+        CK(cudaEventRecord(ctx->ev[1], st));
         ctx->stats.batch_graph = 2;
         // launches of the captured sequence
         int cnt = 0;
@@ -1316,7 +1321,6 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         }
         S.launches = cnt + (S.nlink > 0 ? 1 : 0);
     }
-    CK(cudaEventRecord(ctx->ev[1], st));
     CK(cudaStreamSynchronize(st));
     cudaEventElapsedTime(&ctx->stats.ms_total, ctx->ev[0], ctx->ev[1]);
     ctx->stats.launches = S.launches;
