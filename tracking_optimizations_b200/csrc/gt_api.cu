@@ -30,7 +30,7 @@
 
 namespace gt {
 __global__ void locate_tiles_kernel(const LocParams p, const MovieBufs b, int frame0);
-__global__ void fallback_walk_kernel(const LocParams p, const MovieBufs b, int win, const int* pbeg);
+cudaError_t launch_fallback(const LocParams& p, const MovieBufs& b, int win, const int* pbeg, int grid, cudaStream_t st);
 cudaError_t launch_finalize(const LocParams& p, const MovieBufs& b, float sep, int link_grid, int frame0, int nf,
                             size_t smem, cudaStream_t st);
 cudaError_t link_blocks_per_sm(bool multi, int* per_sm);
@@ -241,7 +241,7 @@ struct Plan {
     int LG = 8, lncx = 1, lncy = 1;  // linker's grid
     // linker scratch for components beyond a thread's own arrays
     int nslot = 0, big_d = 1, big_s = 1, big_e = 1;
-    size_t smem_loc = 0, smem_fb = 0, smem_fin = 0;
+    size_t smem_loc = 0, smem_fin = 0;
     int fb_win = 0;
     int fast = 0;
     int fast_th = 32;
@@ -362,7 +362,6 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     P.smem_loc = (P.smem_loc + 15) / 16 * 16;
     if (P.smem_loc > 227 * 1024) { *msg = "diameter/separation too large for the tile plan"; return GT_ERR_ARG; }
     P.fb_win = std::min(FB_WIN_MAX, std::max(lp.rint_c + 1, lp.max_iter - 1 + lp.rint_c + 1));
-    P.smem_fb = sizeof(float) * (size_t)(2 * P.fb_win + 1) * (2 * P.fb_win + 1);
 
     // capacities (bounds; overflow is detected on the device and retried)
     const long long HW = (long long)H * W;
@@ -631,7 +630,6 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     if (rc) return rc;
     CK(cudaMemsetAsync(w.status, 0, sizeof(int) * (STATUS_INTS + (size_t)T), st));
     CK(allow_shared<locate_tiles_kernel>());
-    CK(allow_shared<fallback_walk_kernel>());
     for (int i = 0; i < 5; ++i)
         if (!ctx->ev[i]) CK(cudaEventCreate(&ctx->ev[i]));
     const int ntiles = P.lp.ntx * P.lp.nty;
@@ -672,7 +670,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     const bool chunked = h_frames && P.link && nchunks > 1 && nchunks <= LINK_WINDOWS;
     int wi = 0, linked = 0;
     auto post = [&](int f0, int nf) -> int {
-        fallback_walk_kernel<<<ctx->num_sms * 4, 128, P.smem_fb, st>>>(P.lp, b, P.fb_win, w.pbeg + wi);
+        CK(launch_fallback(P.lp, b, P.fb_win, w.pbeg + wi, ctx->num_sms * 4, st));
         CK(launch_finalize(P.lp, b, P.sep, P.link, f0, nf, P.smem_fin, st));
         CK(cudaGetLastError());
         ctx->stats.launches += 2;
@@ -727,7 +725,7 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     CK(cudaEventRecord(ctx->ev[1], st));
     if (!chunked) {
         // the whole movie as one window: finalize, then link
-        fallback_walk_kernel<<<ctx->num_sms * 4, 128, P.smem_fb, st>>>(P.lp, b, P.fb_win, w.pbeg);
+        CK(launch_fallback(P.lp, b, P.fb_win, w.pbeg, ctx->num_sms * 4, st));
         CK(launch_finalize(P.lp, b, P.sep, P.link, 0, T, P.smem_fin, st));
         CK(cudaGetLastError());
         ctx->stats.launches += 2;
@@ -1053,7 +1051,7 @@ int enqueue_front(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t 
         }
     }
     CK(cudaGetLastError());
-    fallback_walk_kernel<<<ctx->num_sms, 128, P.smem_fb, s>>>(P.lp, b, P.fb_win, nullptr);
+    CK(launch_fallback(P.lp, b, P.fb_win, nullptr, ctx->num_sms, s));
     CK(launch_finalize(P.lp, b, P.sep, P.link, 0, T, P.smem_fin, s));
     *launches += 2;
     return GT_OK;
@@ -1270,8 +1268,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
                 if (rc) return rc;
             }
         CK(allow_shared<locate_tiles_kernel>());
-        CK(allow_shared<fallback_walk_kernel>());
-        CK(cudaEventRecord(ctx->ev[0], st));
+            CK(cudaEventRecord(ctx->ev[0], st));
         rc = enqueue_batch(ctx, B, mv, n, S, st);
         if (rc) return rc;
         CK(cudaEventRecord(ctx->ev[1], st));

@@ -270,20 +270,13 @@ __global__ void __launch_bounds__(NT) locate_tiles_kernel(const LocParams p, con
         b.rowcnt[((size_t)t * H + ty0 + r) * p.ntx + tj] = rowcount[r];
 }
 
-// Fallback walk for features whose walk left the tile halo (and for
-// max_iterations == 0): recompute the processed values it needs straight
-// from the frame, with the same arithmetic, into a shared-memory window.
-namespace {
-struct WinAcc {
-    const float* P;
-    int y0, x0, n;
-    __device__ bool covers(int u, int v) const { return u >= y0 && u < y0 + n && v >= x0 && v < x0 + n; }
-    __device__ float operator()(int u, int v) const { return P[(u - y0) * n + (v - x0)]; }
-};
-}  // namespace
+// Walks of the records that locate left pending (the walk left the tile halo,
+// a crowded tile, max_iterations == 0): the processed values that a walk can
+// read are recomputed from the frame, with the same arithmetic, into a
+// shared-memory window of n = 2 win + 1 pixels a side.
 
 // processed value at one pixel, straight from the frame (row pass then column
-// pass in shader order); used to fill the fallback window.
+// pass in shader order)
 __device__ float processed_at(const LocParams& p, const void* frames, size_t fbase, int u, int v) {
     const int kr = p.krad, H = p.H, W = p.W;
     float gs = 0.f, cs = 0.f;
@@ -311,29 +304,185 @@ __device__ float processed_at(const LocParams& p, const void* frames, size_t fba
     return res < 0.f ? 0.f : res;
 }
 
-__global__ void __launch_bounds__(128) fallback_walk_kernel(const LocParams p, const MovieBufs b, int win,
-                                                            const int* pbeg) {
+namespace {
+constexpr int FB_NT = 256;
+
+// Shared memory of a block, in floats: the window, raw pixels and row sums of
+// a chunk of its rows, and the centroid circle in the order of its sums (pixel
+// offsets, coordinates, and the pixels at the walk's position).
+struct FbPlan {
+    int n;     // window side
+    int rows;  // window rows filled at a time; 0: each pixel by itself
+    int kp;    // circle pixels, rounded up to 4
+};
+
+__host__ __device__ constexpr int up4(int x) { return (x + 3) / 4 * 4; }
+__host__ __device__ inline int fb_raw(const FbPlan& f) { return up4(f.n * f.n) + 4 * f.kp; }  // ints before the chunk
+
+// The n x n window at (y0, x0) in two passes like the tiles': a chunk of
+// output rows at a time, the raw rows that it reads (I, reflected at the
+// frame's edges), their row sums (G, B), then the columns.  Window pixels
+// outside the frame are 0 (no walk reads them).
+__device__ __forceinline__ void fill_window(const LocParams& p, const void* frames, size_t fbase, int y0, int x0, int n,
+                                            int rows, float* P, float* chunk) {
+    const int kr = p.krad, H = p.H, W = p.W, m = n + 2 * kr;
+    float* I = chunk;
+    float* G = I + (rows + 2 * kr) * m;
+    float* B = G + (rows + 2 * kr) * n;
+    for (int r0 = 0; r0 < n; r0 += rows) {
+        const int nr = min(rows, n - r0), nin = nr + 2 * kr;
+#pragma unroll 4
+        for (int q = threadIdx.x; q < nin * m; q += FB_NT) {
+            const int r = q / m;
+            int pu = y0 + r0 - kr + r, pv = x0 - kr + q - r * m;
+            if (pu < 0) pu = -pu - 1;
+            else if (pu >= H) pu = 2 * H - pu - 1;
+            if (pv < 0) pv = -pv - 1;
+            else if (pv >= W) pv = 2 * W - pv - 1;
+            const bool in = pu >= 0 && pu < H && pv >= 0 && pv < W;
+            I[q] = in ? load_px(frames, p.dtype, fbase + (size_t)pu * W + pv) : 0.f;
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < nin * n; q += FB_NT) {
+            const int r = q / n, v = x0 + q - r * n;
+            const float* in = I + r * m + (q - r * n);
+            float rg = 0.f, rb = 0.f;
+#pragma unroll 5
+            for (int j = 0; j <= 2 * kr; ++j) {
+                const int c = v + j - kr;
+                if (c >= 0 && c < W) rg = fmaf(p.w[j], in[j], rg);  // the Gaussian pads with 0
+                rb = rb + in[j];
+            }
+            G[q] = rg * p.rn;
+            B[q] = rb;
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < nr * n; q += FB_NT) {
+            const int r = q / n, u = y0 + r0 + r, v = x0 + q - r * n;
+            float gs = 0.f, cs = 0.f;
+#pragma unroll 5
+            for (int i = 0; i <= 2 * kr; ++i) {
+                const int c = u + i - kr;
+                if (c >= 0 && c < H) gs = fmaf(p.w[i], G[q + i * n], gs);
+                cs = cs + B[q + i * n];
+            }
+            const float res = fmaf(-cs, p.rkk, gs * p.rn);
+            P[r0 * n + q] = u < 0 || u >= H || v < 0 || v >= W || res < 0.f ? 0.f : res;
+        }
+        __syncthreads();
+    }
+}
+
+// walk_from by a warp: its lanes fetch the circle's pixels, then lanes 0, 1
+// and 2 run the three sums of the centroid (row offset, column offset, mass),
+// each in the shader's order (data * 1 is added exactly; a sum that starts at
+// +0 is never -0, so adding the padding's zeros changes nothing).
+__device__ __forceinline__ WalkOut walk_window(const LocParams& p, const float* P, int y0, int x0, int n, int kp,
+                                               const int* off, const float* cx, const float* cy, float* data, int u,
+                                               int v) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, b = p.border, rint = p.rint_c;
+    const float4* coef = (const float4*)(lane == 0 ? cx : cy);
+    const float4* d4 = (const float4*)data;
+    WalkOut o;
+    o.ul = 0; o.vl = 0;  // WGSL zero-initialised idx
+    float c0 = 0.f, c1 = 0.f, m = 0.f;
+    for (int it = 0; it < p.max_iter; ++it) {
+        if (u - b < 0 || u + b >= p.H || v - b < 0 || v + b >= p.W) {
+            c0 = c1 = m = 0.f;
+        } else {
+            const int r0 = u - y0, q0 = v - x0;
+            if (r0 < rint || r0 + rint >= n || q0 < rint || q0 + rint >= n) {
+                o.ok = 0; o.y = o.x = o.mass = 0.f;
+                return o;
+            }
+            const float* at = P + r0 * n + q0;
+            __syncwarp();
+#pragma unroll 4
+            for (int q = lane; q < kp; q += 32) data[q] = off[q] == INT_MIN ? 0.f : at[off[q]];
+            __syncwarp();
+            float acc = 0.f;
+#pragma unroll 4
+            for (int q = 0; q < kp / 4; ++q) {
+                const float4 d = d4[q];
+                float4 c = coef[q];
+                if (lane >= 2) c = make_float4(1.f, 1.f, 1.f, 1.f);
+                acc = fmaf(d.x, c.x, acc);
+                acc = fmaf(d.y, c.y, acc);
+                acc = fmaf(d.z, c.z, acc);
+                acc = fmaf(d.w, c.w, acc);
+            }
+            const float a0 = __shfl_sync(full, acc, 0), a1 = __shfl_sync(full, acc, 1);
+            m = __shfl_sync(full, acc, 2);
+            c0 = gpu_div(a0, m);  // centers.wgsl:82-83
+            c1 = gpu_div(a1, m);
+        }
+        o.ul = u; o.vl = v;
+        bool changed = false;
+        if (c0 > p.thr && u < p.H - 1) { u += 1; changed = true; }
+        else if (c0 < -p.thr && u > 0) { u -= 1; changed = true; }
+        if (c1 > p.thr && v < p.W - 1) { v += 1; changed = true; }
+        else if (c1 < -p.thr && v > 0) { v -= 1; changed = true; }
+        if (!changed) break;
+    }
+    o.y = (float)u + c0;
+    o.x = (float)v + c1;
+    o.mass = m;
+    o.ok = 1;
+    o.up = u; o.vp = v;
+    return o;
+}
+}  // namespace
+
+// A block walks one record after the other.  What bounds it: the latency of a
+// single walk (a few dozen records a movie).  Each window pixel straight from
+// the frame (krad^2 taps) and the walk by one thread took 177 us for 24
+// records of diameter 15; the passes and the three lanes take 25 us.
+__global__ void __launch_bounds__(FB_NT) fallback_walk_kernel(const LocParams p, const MovieBufs b, const FbPlan f,
+                                                              const int* pbeg) {
     extern __shared__ __align__(16) float wsm[];
     const int npend = *b.npend;
-    const int n = 2 * win + 1;
-    // entries from *pbeg on: those of the frames located since (chunked calls)
-    for (int k = (pbeg ? *pbeg : 0) + blockIdx.x; k < npend; k += gridDim.x) {
+    const int k0 = (pbeg ? *pbeg : 0) + blockIdx.x;  // entries from *pbeg on: those of the frames located since
+    if (k0 >= npend) return;
+    const int n = f.n, rint = p.rint_c;
+    int* off = (int*)(wsm + up4(n * n));
+    float* cx = (float*)off + f.kp;
+    float* cy = cx + f.kp;
+    float* data = cy + f.kp;
+    // the circle x^2 + y^2 <= r^2, rows then columns (a thread per row)
+    for (int i = (int)threadIdx.x - rint; i <= rint; i += FB_NT) {
+        auto half = [&](int x) { return (int)sqrtf((float)(rint * rint - x * x)); };
+        int at = 0;
+        for (int x = -rint; x < i; ++x) at += 2 * half(x) + 1;
+        for (int j = -half(i); j <= half(i); ++j, ++at) {
+            off[at] = i * n + j;
+            cx[at] = (float)i;
+            cy[at] = (float)j;
+        }
+        if (i == rint)
+            for (; at < f.kp; ++at) {
+                off[at] = INT_MIN;
+                cx[at] = cy[at] = 0.f;
+            }
+    }
+    for (int k = k0; k < npend; k += gridDim.x) {
         const int code = b.pend[k];
         const int t = code / b.cap_c;
         Cand* rec = b.cand + code;
         const int u0 = rec->u, v0 = rec->v;
         const size_t fbase = (size_t)t * p.H * p.W;
-        const int y0 = u0 - win, x0 = v0 - win;
-        __syncthreads();
-        for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
-            const int u = y0 + q / n, v = x0 + q % n;
-            float val = 0.f;
-            if (u >= 0 && u < p.H && v >= 0 && v < p.W) val = processed_at(p, b.frames, fbase, u, v);
-            wsm[q] = val;
+        const int y0 = u0 - n / 2, x0 = v0 - n / 2;
+        __syncthreads();  // the last record's walk is done with the window
+        if (p.max_iter > 0 && f.rows > 0) {
+            fill_window(p, b.frames, fbase, y0, x0, n, f.rows, wsm, wsm + fb_raw(f));
+        } else if (p.max_iter > 0) {
+            for (int q = threadIdx.x; q < n * n; q += FB_NT) {
+                const int u = y0 + q / n, v = x0 + q % n;
+                wsm[q] = u >= 0 && u < p.H && v >= 0 && v < p.W ? processed_at(p, b.frames, fbase, u, v) : 0.f;
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            WinAcc acc{wsm, y0, x0, n};
+        if (threadIdx.x < 32) {
             float y, x, m;
             bool ok = true;
             int ul = 0, vl = 0, up = u0, vp = v0;
@@ -344,21 +493,41 @@ __global__ void __launch_bounds__(128) fallback_walk_kernel(const LocParams p, c
                 y = (float)u0; x = (float)v0;
                 m = (p.border == 0) ? processed_at(p, b.frames, fbase, 0, 0) : 0.f;
             } else {
-                WalkOut wo = walk_from(p, acc, u0, v0);
+                const WalkOut wo = walk_window(p, wsm, y0, x0, n, f.kp, off, cx, cy, data, u0, v0);
                 ok = wo.ok != 0;
                 y = wo.y; x = wo.x; m = wo.mass;
                 ul = wo.ul; vl = wo.vl; up = wo.up; vp = wo.vp;
             }
-            if (!ok) {  // window too small for this walk: report, never guess
-                atomicOr(b.err, ERR_SCRATCH_OVERFLOW);
-                rec->state = CAND_REJECT;
-            } else {
-                rec->y = y; rec->x = x; rec->mass = m;
-                rec->ul = ul; rec->vl = vl; rec->up = up; rec->vp = vp;
-                rec->state = (m > p.minmass && m != 0.f) ? CAND_EMIT : CAND_REJECT;
+            if (threadIdx.x == 0) {
+                if (!ok) {  // window too small for this walk: report, never guess
+                    atomicOr(b.err, ERR_SCRATCH_OVERFLOW);
+                    rec->state = CAND_REJECT;
+                } else {
+                    rec->y = y; rec->x = x; rec->mass = m;
+                    rec->ul = ul; rec->vl = vl; rec->up = up; rec->vp = vp;
+                    rec->state = (m > p.minmass && m != 0.f) ? CAND_EMIT : CAND_REJECT;
+                }
             }
         }
     }
+}
+
+// Window rows filled at a time: all of them where the rows that they read fit
+// beside the window (diameter 31 up to 36 iterations), else as many as do.
+// None fit beside the largest windows with wide smoothing (diameter 31 from 81
+// iterations on): every pixel is then computed by itself.
+cudaError_t launch_fallback(const LocParams& p, const MovieBufs& b, int win, const int* pbeg, int grid, cudaStream_t st) {
+    cudaError_t e = allow_shared<fallback_walk_kernel>();
+    if (e != cudaSuccess) return e;
+    FbPlan f{2 * win + 1, 0, 0};
+    for (int i = -p.rint_c; i <= p.rint_c; ++i)
+        for (int j = -p.rint_c; j <= p.rint_c; ++j) f.kp += i * i + j * j <= p.rint_c * p.rint_c;
+    f.kp = up4(f.kp);
+    const int row = 3 * f.n + 2 * p.krad;  // floats of a raw row and its sums
+    f.rows = std::max(0, std::min(f.n, (227 * 1024 / 4 - fb_raw(f)) / row - 2 * p.krad));
+    const size_t smem = sizeof(float) * ((size_t)fb_raw(f) + (f.rows ? (size_t)(f.rows + 2 * p.krad) * row : 0));
+    fallback_walk_kernel<<<grid, FB_NT, smem, st>>>(p, b, f, pbeg);
+    return cudaGetLastError();
 }
 
 }  // namespace gt

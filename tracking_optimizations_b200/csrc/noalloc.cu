@@ -28,7 +28,7 @@
 
 namespace gt {
 __global__ void locate_tiles_kernel(const LocParams p, const MovieBufs b, int frame0);
-__global__ void fallback_walk_kernel(const LocParams p, const MovieBufs b, int win, const int* pbeg);
+cudaError_t launch_fallback(const LocParams& p, const MovieBufs& b, int win, const int* pbeg, int grid, cudaStream_t st);
 cudaError_t launch_finalize(const LocParams& p, const MovieBufs& b, float sep, int link_grid, int frame0, int nf,
                             size_t smem, cudaStream_t st);
 __global__ void scan_frames_kernel(const int* in, int* out, int n);
@@ -304,10 +304,7 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
         SCK(cudaGetLastError());
     }
     const int fb_win = std::min(100, std::max(lp.rint_c + 1, lp.max_iter - 1 + lp.rint_c + 1));
-    const size_t smem_fb = sizeof(float) * (size_t)(2 * fb_win + 1) * (2 * fb_win + 1);
-    SCK(allow_shared<fallback_walk_kernel>());
-    fallback_walk_kernel<<<ds.num_sms * 4, 128, smem_fb, st>>>(lp, b, fb_win, nullptr);
-    SCK(cudaGetLastError());
+    SCK(launch_fallback(lp, b, fb_win, nullptr, ds.num_sms * 4, st));
     SCK(launch_finalize(lp, b, (float)sep, 0, 0, 1, 4 * (size_t)ncell, st));
     scan_frames_kernel<<<1, 1024, 0, st>>>(b.npart, off, 1);
     AsmArgs a;
