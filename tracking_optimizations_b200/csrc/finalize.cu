@@ -3,14 +3,17 @@
 // Replaces the host-side raster scan (execute_gpu.rs:157-183) and the
 // kd-tree separation filter (execute_gpu.rs:258-284).  One CTA per frame:
 //   1. exclusive scan of the per-(row, tile column) record counts gives every
-//      record its raster position (the reference's pre-filter `idx`);
-//   2. records waiting on nothing (state EMIT) are compacted in raster order;
-//   3. a uniform grid (cell >= separation + 1) bins them, and a point is
-//      dropped if a neighbour closer than `separation` has a larger mass, or
-//      an equal mass and a smaller raster index (single pass, as the
-//      reference);
-//   4. survivors form the frame's particle table in raster order, and a
+//      record its raster position (the order of the reference's pre-filter
+//      `idx`); the records are listed in that order;
+//   2. a uniform grid (cell >= separation + 1) bins those waiting on nothing
+//      (state EMIT), and a point is dropped if a neighbour closer than
+//      `separation` has a larger mass, or an equal mass and a smaller raster
+//      position (single pass, as the reference);
+//   3. survivors form the frame's particle table in raster order, and a
 //      second grid over them serves the linker's candidate search.
+// What bounds it: the latency of its steps, each a pass over the frame's
+// records after a barrier.  The counts and the lists are in shared memory where
+// they are short (FIN_COUNTS, FIN_LIST).
 #include "gt_device.cuh"
 
 namespace gt {
@@ -76,24 +79,31 @@ __device__ __forceinline__ int cell_of(float y, float x, float G, int ncy, int n
     return cy * ncx + cx;
 }
 
-// Counting sort of n points into cells: start[ncell+1], idx[n] and, when
-// asked for, their positions in that order.
-template <int NT>
-__device__ void build_grid(const float* ys, const float* xs, int n, float G, int ncy, int ncx, int* cnt_s, int* start,
-                           int* idx, float2* pos, int* warp_tot, int* s_total) {
+// Counting sort of points into cells: item(i, &id, &y, &x) gives the i-th of n
+// (false: none).  The ids in cell order go to idx and, where asked for, the
+// cells' starts (ncell + 1) and the positions in that order to start and pos.
+// cnt_s is left with every cell's end.
+template <int NT, class F>
+__device__ void build_grid(int n, float G, int ncy, int ncx, int* cnt_s, int* start, int* idx, float2* pos,
+                           int* warp_tot, int* s_total, F&& item) {
     const int ncell = ncy * ncx;
+    int id;
+    float y, x;
     for (int c = threadIdx.x; c < ncell; c += NT) cnt_s[c] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n; i += NT) atomicAdd(&cnt_s[cell_of(ys[i], xs[i], G, ncy, ncx)], 1);
+    for (int i = threadIdx.x; i < n; i += NT)
+        if (item(i, &id, &y, &x)) atomicAdd(&cnt_s[cell_of(y, x, G, ncy, ncx)], 1);
     __syncthreads();
-    block_scan_inplace<NT>(cnt_s, ncell, warp_tot, s_total);
-    for (int c = threadIdx.x; c < ncell; c += NT) start[c] = cnt_s[c];
-    if (threadIdx.x == 0) start[ncell] = n;
-    __syncthreads();
+    const int total = block_scan_inplace<NT>(cnt_s, ncell, warp_tot, s_total);
+    if (start) {
+        for (int c = threadIdx.x; c < ncell; c += NT) start[c] = cnt_s[c];
+        if (threadIdx.x == 0) start[ncell] = total;
+        __syncthreads();
+    }
     for (int i = threadIdx.x; i < n; i += NT) {
-        const float y = ys[i], x = xs[i];
+        if (!item(i, &id, &y, &x)) continue;
         const int k = atomicAdd(&cnt_s[cell_of(y, x, G, ncy, ncx)], 1);
-        idx[k] = i;
+        idx[k] = id;
         if (pos) pos[k] = make_float2(y, x);
     }
     __syncthreads();
@@ -113,20 +123,21 @@ __device__ __forceinline__ bool within_r(float qy, float qx, float iy, float ix,
 }
 }  // namespace
 
+// Counts of a frame, and records of a frame, that the block keeps in shared
+// memory, which also holds the cells of the larger grid (FinShared: ints).
+constexpr int FIN_COUNTS = 4096, FIN_LIST = 1024;
+struct FinShared {
+    int cells, counts, list;  // list: records, six ints each
+};
+
 template <int NTF>
 __device__ __forceinline__ void finalize_frame(const LocParams& p, const MovieBufs& b, float sep, int link_grid,
-                                               int frame0, int* cnt_s, int* warp_tot, int& s_total) {
+                                               int frame0, int* cnt_s, FinShared sh, int* warp_tot, int& s_total) {
     const int t = frame0 + blockIdx.x;
     const int cap_c = b.cap_c;
     const int nrc = p.H * p.ntx;
     int* rc = b.rowcnt + (size_t)t * nrc;
     const Cand* cand = b.cand + (size_t)t * cap_c;
-    int* perm = b.cperm + (size_t)t * cap_c;
-    float* cy = b.cy + (size_t)t * cap_c;
-    float* cx = b.cx + (size_t)t * cap_c;
-    float* cm = b.cm + (size_t)t * cap_c;
-    int* crec = b.crec + (size_t)t * cap_c;
-    int* keep = b.ccell + (size_t)t * cap_c;
 
     const int nrec = b.fcount[t];
     if (nrec > cap_c) {
@@ -140,100 +151,111 @@ __device__ __forceinline__ void finalize_frame(const LocParams& p, const MovieBu
         }
         return;
     }
+    // the lists: positions, masses, records and the survivors' flags in raster
+    // order, and the grid's entries
+    const bool small = nrec <= sh.list;
+    int* list = cnt_s + sh.cells + sh.counts;
+    const size_t at = (size_t)t * cap_c;
+    float* cy = small ? (float*)list : b.cy + at;
+    float* cx = small ? (float*)list + sh.list : b.cx + at;
+    float* cm = small ? (float*)list + 2 * sh.list : b.cm + at;
+    int* crec = small ? list + 3 * sh.list : b.crec + at;
+    int* keep = small ? list + 4 * sh.list : b.ccell + at;
+    int* cidx = small ? list + 5 * sh.list : b.cidx + at;
 
-    // 1. raster positions
-    block_scan_inplace<NTF>(rc, nrc, warp_tot, &s_total);
-    for (int k = threadIdx.x; k < nrec; k += NTF) perm[k] = k;
+    // 1. raster order
+    if (nrc <= sh.counts) {
+        int* rs = cnt_s + sh.cells;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < nrc; i += NTF) rs[i] = rc[i];
+        rc = rs;
+    }
+    for (int i = threadIdx.x; i < nrec; i += NTF) keep[i] = 0;
     __syncthreads();
+    block_scan_inplace<NTF>(rc, nrc, warp_tot, &s_total);
     for (int k = threadIdx.x; k < nrec; k += NTF) {
         const Cand& c = cand[k];
-        if (c.u < 0 || c.u >= p.H || c.v < 0 || c.v >= p.W) continue;
-        const int dest = rc[c.u * p.ntx + c.v / p.TW] + c.rowrank;
-        if (dest >= 0 && dest < nrec) perm[dest] = k;
+        const int u = c.u, v = c.v, rank = c.rowrank, state = c.state;
+        const float y = c.y, x = c.x, mass = c.mass;
+        if (u < 0 || u >= p.H || v < 0 || v >= p.W) continue;
+        const int i = rc[u * p.ntx + v / p.TW] + rank;
+        if (i < 0 || i >= nrec || state != CAND_EMIT) continue;
+        keep[i] = 1;
+        cy[i] = y; cx[i] = x; cm[i] = mass; crec[i] = k;
     }
     __syncthreads();
 
-    // 2. compact emitted records in raster order
-    for (int i = threadIdx.x; i < nrec; i += NTF) keep[i] = cand[perm[i]].state == CAND_EMIT ? 1 : 0;
-    __syncthreads();
-    const int ne = block_scan_inplace<NTF>(keep, nrec, warp_tot, &s_total);
-    for (int i = threadIdx.x; i < nrec; i += NTF) {
-        const int k = perm[i];
-        const Cand& c = cand[k];
-        if (c.state != CAND_EMIT) continue;
-        const int e = keep[i];
-        cy[e] = c.y; cx[e] = c.x; cm[e] = c.mass; crec[e] = k;
-    }
-    __syncthreads();
-
-    // 3. separation filter on a uniform grid
+    // 2. separation filter on a uniform grid
     const float G = (float)b.G;
-    const int ncell = b.ncx * b.ncy;
-    int* cstart = b.cstart + (size_t)t * (ncell + 1);
-    int* cidx = b.cidx + (size_t)t * cap_c;
-    build_grid<NTF>(cy, cx, ne, G, b.ncy, b.ncx, cnt_s, cstart, cidx, nullptr, warp_tot, &s_total);
-    for (int i = threadIdx.x; i < ne; i += NTF) {
+    build_grid<NTF>(nrec, G, b.ncy, b.ncx, cnt_s, nullptr, cidx, nullptr, warp_tot, &s_total,
+                    [&](int i, int* id, float* y, float* x) {
+                        *id = i;
+                        *y = cy[i]; *x = cx[i];
+                        return keep[i] != 0;
+                    });
+    for (int i = threadIdx.x; i < nrec; i += NTF) {
+        if (!keep[i]) continue;
         const float qy = cy[i], qx = cx[i], qm = cm[i];
         const int c = cell_of(qy, qx, G, b.ncy, b.ncx);
         const int gy = c / b.ncx, gx = c - gy * b.ncx;
+        const int x0 = max(gx - 1, 0), x1 = min(gx + 1, b.ncx - 1);
         bool k = true;
-        for (int dy = -1; dy <= 1 && k; ++dy) {
-            const int yy = gy + dy;
-            if (yy < 0 || yy >= b.ncy) continue;
-            for (int dx = -1; dx <= 1 && k; ++dx) {
-                const int xx = gx + dx;
-                if (xx < 0 || xx >= b.ncx) continue;
-                const int cc = yy * b.ncx + xx;
-                for (int s = cstart[cc]; s < cstart[cc + 1]; ++s) {
-                    const int j = cidx[s];
-                    if (j == i) continue;
-                    float dd;
-                    if (!within_r(qy, qx, cy[j], cx[j], sep, &dd)) continue;
-                    const float nm = cm[j];
-                    if (qm < nm || (qm == nm && i > j)) { k = false; break; }
-                }
+        for (int yy = max(gy - 1, 0); yy <= min(gy + 1, b.ncy - 1) && k; ++yy) {
+            const int c0 = yy * b.ncx + x0;
+            const int s1 = cnt_s[yy * b.ncx + x1];
+            for (int s = c0 > 0 ? cnt_s[c0 - 1] : 0; s < s1; ++s) {
+                const int j = cidx[s];
+                if (j == i) continue;
+                float dd;
+                if (!within_r(qy, qx, cy[j], cx[j], sep, &dd)) continue;
+                const float nm = cm[j];
+                if (qm < nm || (qm == nm && i > j)) { k = false; break; }
             }
         }
-        keep[i] = k ? 1 : 0;
+        if (!k) keep[i] = 0;
     }
     __syncthreads();
 
-    // 4. survivors in raster order
-    const int np = block_scan_inplace<NTF>(keep, ne, warp_tot, &s_total);
+    // 3. survivors in raster order
+    const int np = block_scan_inplace<NTF>(keep, nrec, warp_tot, &s_total);
     const bool over = np > b.cap_p;
     if (over && threadIdx.x == 0) atomicOr(b.err, ERR_PART_OVERFLOW);
     float* py = b.py + (size_t)t * b.cap_p;
     float* px = b.px + (size_t)t * b.cap_p;
     float* pm = b.pm + (size_t)t * b.cap_p;
     int* prec = b.prec + (size_t)t * b.cap_p;
-    // keep[i] now holds the survivor index; recompute survivorship from the
-    // scan (a survivor is where the next prefix value increases)
-    for (int i = threadIdx.x; i < ne; i += NTF) {
+    // keep[i] now holds the survivor index; a survivor is where the next prefix
+    // value increases
+    auto survivor = [&](int i, int* id, float* y, float* x) {
         const int a = keep[i];
-        const int nxt = (i + 1 < ne) ? keep[i + 1] : np;
-        if (nxt > a && a < b.cap_p) {
-            py[a] = cy[i]; px[a] = cx[i]; pm[a] = cm[i]; prec[a] = crec[i];
+        *id = a;
+        if (((i + 1 < nrec) ? keep[i + 1] : np) <= a || a >= b.cap_p) return false;
+        *y = cy[i]; *x = cx[i];
+        return true;
+    };
+    for (int i = threadIdx.x; i < nrec; i += NTF) {
+        int a;
+        float y, x;
+        if (survivor(i, &a, &y, &x)) {
+            py[a] = y; px[a] = x; pm[a] = cm[i]; prec[a] = crec[i];
         }
     }
     if (threadIdx.x == 0) b.npart[t] = over ? b.cap_p : np;
-    __syncthreads();
 
-    // 5. grid over the particles for the linker
-    if (link_grid) {
-        const int n = over ? b.cap_p : np;
-        build_grid<NTF>(py, px, n, (float)b.LG, b.lncy, b.lncx, cnt_s,
+    // the grid over the particles for the linker
+    if (link_grid)
+        build_grid<NTF>(nrec, (float)b.LG, b.lncy, b.lncx, cnt_s,
                         b.gstart + (size_t)t * ((size_t)b.lncx * b.lncy + 1), b.gidx + (size_t)t * b.cap_p,
-                        b.gpos + (size_t)t * b.cap_p, warp_tot, &s_total);
-    }
+                        b.gpos + (size_t)t * b.cap_p, warp_tot, &s_total, survivor);
 }
 
 template <int NTF>
 __global__ void __launch_bounds__(NTF) finalize_kernel(const LocParams p, MovieBufs b, float sep,
-                                                       int link_grid, int frame0) {
+                                                       int link_grid, int frame0, FinShared sh) {
     __shared__ int warp_tot[NTF / 32];
     __shared__ int s_total, s_last;
-    extern __shared__ int cnt_s[];  // cells of the larger grid
-    finalize_frame<NTF>(p, b, sep, link_grid, frame0, cnt_s, warp_tot, s_total);
+    extern __shared__ int cnt_s[];  // cells of the larger grid, counts, lists
+    finalize_frame<NTF>(p, b, sep, link_grid, frame0, cnt_s, sh, warp_tot, s_total);
     if (!b.done) return;
     // the last block done: offsets of the launch's frames (a launch of its own
     // costs a short movie more than the sums)
@@ -268,8 +290,14 @@ cudaError_t launch_finalize(const LocParams& p, const MovieBufs& b, float sep, i
     const bool big = (long long)p.H * p.W >= (1LL << 20);
     const cudaError_t e = big ? allow_shared<finalize_kernel<1024>>() : allow_shared<finalize_kernel<512>>();
     if (e != cudaSuccess) return e;
-    if (big) finalize_kernel<1024><<<nf, 1024, smem, st>>>(p, b, sep, link_grid, frame0);
-    else finalize_kernel<512><<<nf, 512, smem, st>>>(p, b, sep, link_grid, frame0);
+    FinShared sh{(int)(smem / sizeof(int)), 0, 0};
+    const int nrc = p.H * p.ntx;
+    if (nrc <= FIN_COUNTS) sh.counts = nrc;
+    if (smem + sizeof(int) * (size_t)(sh.counts + 6 * FIN_LIST) <= 226 * 1024) sh.list = FIN_LIST;
+    else sh.counts = 0;  // cells of the finest grids fill the block's share
+    smem += sizeof(int) * (size_t)(sh.counts + 6 * sh.list);
+    if (big) finalize_kernel<1024><<<nf, 1024, smem, st>>>(p, b, sep, link_grid, frame0, sh);
+    else finalize_kernel<512><<<nf, 512, smem, st>>>(p, b, sep, link_grid, frame0, sh);
     return cudaGetLastError();
 }
 
@@ -283,8 +311,14 @@ __global__ void __launch_bounds__(NTG) grid_kernel(const float* py, const float*
     extern __shared__ int cnt_s[];
     const int t = blockIdx.x;
     const int ncell = ncx * ncy;
-    build_grid<NTG>(py + (size_t)t * cap_p, px + (size_t)t * cap_p, npart[t], (float)G, ncy, ncx, cnt_s,
-               gstart + (size_t)t * (ncell + 1), gidx + (size_t)t * cap_p, gpos + (size_t)t * cap_p, warp_tot, &s_total);
+    py += (size_t)t * cap_p;
+    px += (size_t)t * cap_p;
+    build_grid<NTG>(npart[t], (float)G, ncy, ncx, cnt_s, gstart + (size_t)t * (ncell + 1), gidx + (size_t)t * cap_p,
+                    gpos + (size_t)t * cap_p, warp_tot, &s_total, [&](int i, int* id, float* y, float* x) {
+                        *id = i;
+                        *y = py[i]; *x = px[i];
+                        return true;
+                    });
 }
 
 }  // namespace gt
