@@ -333,8 +333,10 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     P.fast = 0;
     const int want_fast = force_generic_flag ? 0 : fast_supported(lp.krad, lp.D, lp.rint_c, lp.d, dtype);
     P.char_tab.clear(); P.char_off.clear(); P.gchar_tab.clear();
-    circle_tables(lp.char_r, P.char_tab, &P.char_off, 1);
-    circle_tables(lp.rint_c, P.gchar_tab, nullptr, 0);
+    // only what the columns asked for read: most calls upload no table (8 us of
+    // a single frame's call)
+    if (r.cpu_processed) circle_tables(lp.char_r, P.char_tab, &P.char_off, 1);
+    if (r.characterize) circle_tables(lp.rint_c, P.gchar_tab, nullptr, 0);
     lp.n_char = (int)P.char_off.size() / 2;
     lp.n_gchar = (int)P.gchar_tab.size() / 2;
     if (want_fast) {
@@ -396,7 +398,7 @@ struct Work {
     int *rowcnt, *pend;
     float *py, *px, *pm;
     int *prec, *npart, *gstart, *gidx;
-    int *cperm, *crec, *ccell, *cstart, *cidx;
+    int *crec, *ccell, *cidx;
     float *cy, *cx, *cm;
     int* tables;
     float *char_tab, *gchar_tab;
@@ -430,7 +432,7 @@ struct Carver {
 size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_locate, bool own_out = true) {
     Carver c{base};
     const size_t T = P.T;
-    const size_t ncell = (size_t)P.ncx * P.ncy, lcell = (size_t)P.lncx * P.lncy;
+    const size_t lcell = (size_t)P.lncx * P.lncy;
     w->frames = c.take<char>(frame_bytes);
     const size_t cc = need_locate ? T * P.cap_c : 1;
     w->cand = c.take<Cand>(cc);
@@ -443,10 +445,8 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->npart = c.take<int>(T);
     w->gstart = c.take<int>(T * (lcell + 1));
     w->gidx = c.take<int>(T * P.cap_p);
-    w->cperm = c.take<int>(cc);
     w->crec = c.take<int>(cc);
     w->ccell = c.take<int>(cc);
-    w->cstart = c.take<int>(need_locate ? T * (ncell + 1) : 1);
     w->cidx = c.take<int>(cc);
     w->cy = c.take<float>(cc);
     w->cx = c.take<float>(cc);
@@ -606,8 +606,8 @@ MovieBufs movie_bufs(const Plan& P, const Work& w, const void* frames) {
     b.cand = w.cand; b.fcount = w.fcount; b.rowcnt = w.rowcnt; b.pend = w.pend; b.npend = w.npend;
     b.py = w.py; b.px = w.px; b.pm = w.pm; b.prec = w.prec; b.npart = w.npart;
     b.G = P.G; b.ncx = P.ncx; b.ncy = P.ncy; b.LG = P.LG; b.lncx = P.lncx; b.lncy = P.lncy; b.gstart = w.gstart; b.gidx = w.gidx; b.gpos = w.gpos;
-    b.cperm = w.cperm; b.cy = w.cy; b.cx = w.cx; b.cm = w.cm; b.crec = w.crec; b.ccell = w.ccell;
-    b.cstart = w.cstart; b.cidx = w.cidx;
+    b.cy = w.cy; b.cx = w.cx; b.cm = w.cm; b.crec = w.crec; b.ccell = w.ccell;
+    b.cidx = w.cidx;
     b.char_tab = w.char_tab; b.char_off = w.char_off; b.gchar_tab = w.gchar_tab;
     b.err = w.err;
     b.off = w.off; b.done = w.done; b.nrows = w.nrows;

@@ -97,13 +97,11 @@ struct MovieBufs {
     int* gstart;          // T*(lncx*lncy+1)
     int* gidx;            // T*cap_p
     float2* gpos;         // T*cap_p (y, x) of gidx's particles
-    int* cperm;           // T*cap_c finalize scratch (raster permutation)
     float* cy;            // T*cap_c emitted candidates in raster order
     float* cx;
     float* cm;
     int* crec;
     int* ccell;           // T*cap_c
-    int* cstart;          // T*(ncx*ncy+1) separation grid starts
     int* cidx;            // T*cap_c
     const float* char_tab;   // n_char x {r2, sin2, cos2}, d/2 circle
     const int* char_off;     // n_char x {di, dj}

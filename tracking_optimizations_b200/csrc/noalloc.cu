@@ -257,13 +257,11 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
     b.G = G; b.ncx = ncx; b.ncy = ncy;
     b.gstart = c.take<int>(ncell + 1);
     b.gidx = c.take<int>(cap_c);
-    b.cperm = c.take<int>(cap_c);
     b.cy = c.take<float>(cap_c);
     b.cx = c.take<float>(cap_c);
     b.cm = c.take<float>(cap_c);
     b.crec = c.take<int>(cap_c);
     b.ccell = c.take<int>(cap_c);
-    b.cstart = c.take<int>(ncell + 1);
     b.cidx = c.take<int>(cap_c);
     float* d_char_tab = c.take<float>(3 * lp.n_char);
     int* d_char_off = c.take<int>(2 * lp.n_char);
