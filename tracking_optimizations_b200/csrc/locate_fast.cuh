@@ -13,6 +13,7 @@
 // immediate and every loop has a constant trip count.  With RT the dilation
 // size is a run-time value of at most DD (and at least FM): the tile is laid
 // out for DD, and the two maxima over the window have one loop over its core.
+// COLS names the columns that the records carry.
 // Float frames add their boxcars in tap order (their sums round).  A CTA (256 or 512 threads) takes a
 // run of consecutive TH0 x 64 output tiles; per tile:
 //   0. the uint16 tile plus halo is staged by one TMA load (zero fill
@@ -43,6 +44,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "gt_device.cuh"
 #include "gt_simd.cuh"
@@ -57,6 +59,10 @@ constexpr int FNT = 256;  // threads of a 32-row tile
 // output row) keep 16 warps per SM slot at 2 CTAs per SM
 __host__ __device__ constexpr int fast_threads(int th) { return th == 32 ? FNT : 2 * FNT; }
 constexpr int FM = 8;     // outputs per thread item
+// Columns of the records: position and mass; the cpu_processed columns; the
+// characterize columns, with or without those.  An instance each: the code of
+// unused columns cost a call 1 to 2 %.
+enum { COLS_PLAIN = 0, COLS_CPU = 1, COLS_GPU = 2 };
 // Walker warps of a run of tiles (64-row tiles: 2 of 16 warps, 32-row
 // tiles: 2 of 8): they walk a tile of at most 32 NWO candidates while the
 // other warps start the next one.
@@ -261,13 +267,6 @@ struct P2Acc {
     }
 };
 
-template <class PX>
-struct GRawAcc {  // raw pixels straight from the frame (characterize only)
-    const PX* F;
-    int W;
-    __device__ float operator()(int u, int v) const { return (float)__ldg(F + (size_t)u * W + v); }
-};
-
 // Centroid sums at a centre whose processed row has parity E, fully unrolled
 // (centers.wgsl:39-85 order: i outer, j inner, mask x^2 + y^2 <= r^2).
 template <int RC, int E, int S>
@@ -346,6 +345,54 @@ __device__ __forceinline__ void circle_features_group(const float* P, int base, 
     sig = mx;
 }
 
+// characterize=True columns at the originating pixel (u, v) (centers.wgsl:64-80)
+// as {Rg_gpu, raw_mass_gpu, signal_gpu, ecc_gpu}, by the 8 lanes of a lane group
+// (l = lane & 7): lane 0 sums the mass, 1 data * r^2, 2 the raw pixels, 4 and 5
+// data * sin2 and cos2, each over the whole circle in the shader's order (data
+// * 1 is added exactly).  The group fetches the raw pixels together and hands
+// them on in order.  What bounds it: latency; a lane per record, with its raw
+// pixels loaded one by one, took 1.1 of 1.63 ms (12 frames of 2048 x 2560,
+// diameter 11, 5.7k records each), the lane groups 0.3.  Out of line and in
+// instances of its own (COLS_GPU): beside the other columns' code its registers
+// cost every call 1 to 3 %.  base is the P2 offset of (u, v), E the
+// parity of its processed row; every lane of the warp must call it.
+template <int RC, int S, class PX>
+__device__ __noinline__ float4 gpu_features_group(const float* P, int base, int E, const PX* frame, int H, int W, int u,
+                                                  int v, const float* tab, int l) {
+    constexpr int NV = (2 * RC + 1 + 7) / 8;  // raw pixels of a circle row per lane
+    const unsigned full = 0xffffffffu;
+    float raw[2 * RC + 1][NV];
+#pragma unroll
+    for (int i = -RC; i <= RC; ++i) {
+        const PX* row = frame + (size_t)clampi(u + i, 0, H - 1) * W;
+#pragma unroll
+        for (int h = 0; h < NV; ++h) raw[i + RC][h] = (float)__ldg(row + clampi(v - RC + 8 * h + l, 0, W - 1));
+    }
+    float acc = 0.f, mx = 0.f;
+    int t = 0;
+#pragma unroll
+    for (int i = -RC; i <= RC; ++i) {
+        const float* pr = P + base + ((((E + i) >> 1) * S) << 1) + ((E + i) & 1);
+#pragma unroll
+        for (int j = -RC; j <= RC; ++j) {
+            if (i * i + j * j > RC * RC) continue;
+            const float data = pr[2 * j];
+            const float rw = __shfl_sync(full, raw[i + RC][(j + RC) >> 3], (j + RC) & 7, 8);
+            float c = 1.f;
+            if (l >= 4) c = __ldg(tab + 2 * t + (l & 1));
+            if (l == 1) c = (float)(i * i + j * j);
+            acc = fmaf(l == 2 ? rw : data, c, acc);
+            mx = fmaxf(mx, data);
+            ++t;
+        }
+    }
+    const float m = __shfl_sync(full, acc, 0, 8), rg = __shfl_sync(full, acc, 1, 8), rm = __shfl_sync(full, acc, 2, 8);
+    float es = __shfl_sync(full, acc, 4, 8), ec = __shfl_sync(full, acc, 5, 8);
+    es = es * es;
+    ec = ec * ec;
+    return make_float4(sqrtf(gpu_div(rg, m)), rm, mx, gpu_div(sqrtf(es + ec), m - P[base + E]));
+}
+
 template <class G, int RC>
 __device__ __forceinline__ bool centroid_fixed(const LocParams& p, const P2Acc<G>& P, int u, int v, float& c0,
                                                float& c1, float& m) {
@@ -420,11 +467,12 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 // mask of the columns that emit, which is what finalize_kernel needs; slots
 // come from one atomic per warp.  Named barrier 1 syncs the nwt walker
 // threads.
-template <class G, int RC, class PX>
+template <class G, int RC, class PX, int COLS>
 __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b, const FTile& f, const float* P2f,
                                           const unsigned short* clist, unsigned long long* rowmask, int* stage,
                                           float4* sfeat, const int2* offs, const float* r2s, const float2* sc,
                                           int ncand, int c, bool have, int q, int wstride, int nwt) {
+    const bool cpu = COLS == COLS_CPU || (COLS == COLS_GPU && p.cpu_processed);
     const int H = p.H, W = p.W;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
@@ -490,7 +538,6 @@ __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b
     // records are computed by lane groups of 8, four records at a time
     // (circle_features_group); the slot atomic issued above completes
     // meanwhile.
-    GRawAcc<PX> racc{(const PX*)b.frames + (size_t)t * H * W, W};
     int roff = 0;
     for (int c0 = 0; c0 < ncand; c0 += wstride) {
         int rq = q, rtr = tr, rtc = tc, rst = st;
@@ -510,10 +557,12 @@ __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b
         const int ne = __popc(eb), e = __popc(eb & lt);
         const int ru = ty0 + rtr, rv = tx0 + rtc;
         float4 feat = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (p.cpu_processed && ne) {
-            // execute_gpu.rs:165-172, 286-299 at the originating pixel
+        if ((cpu || COLS == COLS_GPU) && ne) {
             if (em) stage[e] = ((ru - py0) << 16) | (rv - px0);
             __syncwarp();
+        }
+        if (cpu && ne) {
+            // execute_gpu.rs:165-172, 286-299 at the originating pixel
             for (int g = 0; g < ne; g += 4) {
                 const int er = min(g + (lane >> 3), ne - 1);
                 const int code = stage[er];
@@ -525,7 +574,7 @@ __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b
             }
             __syncwarp();
             if (em) feat = sfeat[e];
-            __syncwarp();  // stage and sfeat are reused by the next stride
+            __syncwarp();  // sfeat is reused by the next stride
         }
         // the slot base of lane 0's atomic, read only now: its latency
         // overlapped the sums above
@@ -545,13 +594,12 @@ __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b
             rec.ul = (int)(rlp >> 16); rec.vl = (int)(rlp & 0xffffu);
             rec.up = (int)(rfp >> 16); rec.vp = (int)(rfp & 0xffffu);
             rec.pad = 0;
-            if (p.cpu_processed) {
+            if (cpu) {
                 rec.rg_sum = feat.x;
                 rec.eccn = sqrtf(feat.y * feat.y + feat.z * feat.z);
                 rec.mid = acc(ru, rv);
                 rec.signal = feat.w;
             }
-            if (p.characterize) gpu_features(p, b, acc, racc, ru, rv, rec);
             if (gb >= 0) {
                 const int slot = gb + roff + e;
                 b.cand[(size_t)t * b.cap_c + slot] = rec;
@@ -561,6 +609,26 @@ __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b
                 }
             }
         }
+        if (COLS == COLS_GPU && ne && gb >= 0) {
+            // into the records just written, when no lane holds one any more
+            Cand* out = b.cand + (size_t)t * b.cap_c + gb + roff;
+            __syncwarp();
+            for (int g = 0; g < ne; g += 4) {
+                const int er = min(g + (lane >> 3), ne - 1);
+                const int code = stage[er];
+                const int rr = code >> 16, cc = code & 0xffff;
+                const float4 z = gpu_features_group<RC, G::P2S, PX>(
+                    P2f, ((rr >> 1) * G::P2S + cc) * 2, rr & 1, (const PX*)b.frames + (size_t)t * H * W, H, W,
+                    py0 + rr, px0 + cc, b.gchar_tab, lane & 7);
+                if ((lane & 7) == 0 && g + (lane >> 3) < ne) {
+                    out[er].g_rg = z.x;
+                    out[er].g_raw = z.y;
+                    out[er].g_sig = z.z;
+                    out[er].g_ecc = z.w;
+                }
+            }
+        }
+        __syncwarp();  // stage is reused by the next stride
         roff += ne;
     }
 }
@@ -583,7 +651,7 @@ __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b
 // copy that does not land within the bounded wait sets ERR_DEVICE_TIMEOUT;
 // the CTA then issues no further copies, lists no candidates and finishes its
 // run (every barrier is still reached; the host discards the results).
-template <int KR, int DD, int TH0, int RC, class PX, bool RT>
+template <int KR, int DD, int TH0, int RC, class PX, bool RT, int COLS>
 __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, RT>::CTAS))
     locate_fast_kernel(const LocParams p, const MovieBufs b, const __grid_constant__ CUtensorMap tmap, int use_tma,
                        int frame0, int ntiles, int total, int per_cta) {
@@ -637,7 +705,7 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
         // barrier then never completes and the bounded wait runs out
         if (!p.tma_withhold) tma_load_3d(U, &tmap, &bar, f.tx0 - G::L, f.ty0 - HP - KR, f.t);
     }
-    if (p.cpu_processed)
+    if (COLS == COLS_CPU || (COLS == COLS_GPU && p.cpu_processed))
         for (int k = tid; k < G::K; k += NTK) {
             sc[k] = make_float2(__ldg(b.char_tab + 3 * k + 1), __ldg(b.char_tab + 3 * k + 2));
             r2s[k] = __ldg(b.char_tab + 3 * k);
@@ -673,7 +741,7 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
                 const bool have = ov ? lane < h && c < ncand : c < ncand;
                 const int q = have ? clist[c] : 0;
                 if (ov && more) bar_arrive(2, NTK);  // the list (and s_nc) may be overwritten
-                walk_emit<G, RC, PX>(p, b, prev, P2w, clist, rowmask, (ov ? stage_ov : stage_bp) + warp * 32,
+                walk_emit<G, RC, PX, COLS>(p, b, prev, P2w, clist, rowmask, (ov ? stage_ov : stage_bp) + warp * 32,
                                  (ov ? sfeat_ov : sfeat_bp) + warp * 32, offs, r2s, sc, ncand, c, have, q, nwt, nwt);
                 if (!more) break;
                 if (nwt > 32) bar_sync(1, nwt);  // every walker reads rowmask until its last record
@@ -1118,11 +1186,16 @@ cudaError_t launch_instance(dim3 grid, cudaStream_t st, const LocParams& p, cons
     std::memset(&map, 0, sizeof(map));
     const int tma = make_tensor_map(&map, b.frames, (int)sizeof(PX), T, p.H, p.W, G::US, G::RH) ? 1 : 0;
     *used_tma = tma;
-    const auto fn = locate_fast_kernel<KR, DD, TH, RC, PX, RT>;
-    const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-    if (e != cudaSuccess) return e;
-    fn<<<nblk, fast_threads(TH), G::SMEM, st>>>(p, b, map, tma, frame0, (int)grid.x, (int)total, per);
-    return cudaGetLastError();
+    auto launch = [&](auto cols) {
+        constexpr auto* fn = locate_fast_kernel<KR, DD, TH, RC, PX, RT, decltype(cols)::value>;
+        const cudaError_t e = allow_shared<fn>();
+        if (e != cudaSuccess) return e;
+        fn<<<nblk, fast_threads(TH), G::SMEM, st>>>(p, b, map, tma, frame0, (int)grid.x, (int)total, per);
+        return cudaGetLastError();
+    };
+    return p.characterize    ? launch(std::integral_constant<int, COLS_GPU>())
+           : p.cpu_processed ? launch(std::integral_constant<int, COLS_CPU>())
+                             : launch(std::integral_constant<int, COLS_PLAIN>());
 }
 }  // namespace
 
