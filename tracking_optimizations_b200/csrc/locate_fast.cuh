@@ -25,13 +25,18 @@
 //      2^23) and filters 8 columns per thread (FFMA2 chains in tap order),
 //      Gaussian and boxcar -> Gp, Bp (row pairs); tiles at a frame edge
 //      then repair the boxcar's reflect padding (the Gaussian pads with 0);
-//   2. column pass: a thread filters one column over 8 rows (4 row pairs),
-//      scales by the reciprocal of the Gaussian norm, subtracts the boxcar
+//   2. column pass: a thread filters one column over 16 rows (8 row pairs; 8
+//      rows in 32-row tiles), scales by the reciprocal of the Gaussian norm, subtracts the boxcar
 //      as fma(-box, 1/k^2, gauss) and clips at 0 -> P2 (row pairs); tiles at
 //      a frame edge then write -inf outside the frame;
+//      (16 rows: one item a thread instead of 1.65, and the rows shared by two
+//      runs are loaded and summed once; 1000 frames of 512 x 512, diameter 7:
+//      1.272 -> 1.244 ms)
 //   3. row max over the dilation window (register sliding max) -> RM2;
-//   4. column max of RM2 compared with the centre: the local maxima of a
-//      warp's rows are listed at once by per-row ballots into the CTA list;
+//   4. column max of RM2 compared with the centre: a thread marks the local
+//      maxima of its 8 rows in a mask, and a warp appends its threads' first,
+//      second, ... marks to the CTA list (a ballot per row instead: 1.303 ms,
+//      so 1.272);
 //   5. the list is walked one candidate per lane by the walker warps, which
 //      compute the features and emit the records (ranks from per-row bit
 //      masks, one slot atomic per warp) while the other warps run the next
@@ -106,7 +111,9 @@ struct Geo {
     static constexpr int PW = RW - 2 * KR;
     static constexpr int NPW = (PW + FM - 1) / FM;
     static constexpr int PWC = FM * NPW;
-    static constexpr int NRQ = (PH + FM - 1) / FM;  // column-pass items per column
+    // column pass: an item covers HC runs of FM / 2 row pairs of a column
+    static constexpr int HC = TH0 == 64 ? 2 : 1;
+    static constexpr int NRQ = (PP + HC * (FM / 2) - 1) / (HC * (FM / 2));  // items per column
     static constexpr int GPS = PWC | 1;
     static constexpr int P2S = PW | 1;
     static constexpr int RMS = FT | 1;
@@ -145,9 +152,9 @@ struct Geo {
     static_assert(((TH0 - FM + HP - O) >> 1) + (FM + DD) / 2 - 1 <= PP, "column max rows allocated");
     static_assert(TH0 - 1 + HP + (DD - 1 - O) <= PH - 1, "column max window inside the processed rows");
     static_assert(FT + HX <= PW, "centre columns computed");
-    // a column-pass item covers row pairs p0 .. p0 + FM/2 - 1, p0 <= PP - FM/2,
-    // and reads row pairs up to p0 + FM/2 + KR - 1
-    static_assert(PP >= FM / 2 && PP + KR <= RP, "column pass reads computed row pairs");
+    // a column-pass item covers row pairs p0 .. p0 + HC FM/2 - 1, p0 <= PP - HC FM/2,
+    // and reads row pairs up to p0 + HC FM/2 + KR - 1
+    static_assert(PP >= HC * (FM / 2) && PP + KR <= RP, "column pass reads computed row pairs");
     static_assert(PWC <= GPS && PW <= P2S && FT <= RMS, "row strides");
     static_assert(US <= 256 && RH <= 256 && (US * sizeof(PX)) % 16 == 0, "TMA box");
     static_assert((NPW - 1) * FM < US && (FM * sizeof(PX)) % 16 == 0, "16-byte raw loads start inside a U row");
@@ -919,77 +926,85 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
         if (tid >= CB) {
             const int ctid = tid - CB;
             // ---- 2. column pass (preprocess_cols.wgsl) -> P2 ----
-            // item rq of a column covers row pairs p0 .. p0 + FM/2 - 1; the
+            // item rq of a column covers row pairs p0 .. p0 + HC FM/2 - 1; the
             // last one is moved up to end at the last processed row pair
             // (the rows it shares with the item before come out the same)
             for (int it = ctid; it < G::PW * G::NRQ; it += CN) {
                 const int rq = it / G::PW, c = it - rq * G::PW;
-                const int p0 = min(rq * (FM / 2), G::PP - FM / 2);
-                float2 L[FM / 2 + KR], ML[FM / 2 + KR - 1];
+                const int p0 = min(rq * (G::HC * (FM / 2)), G::PP - G::HC * (FM / 2));
+                // Gaussian and boxcar rows of a run; the last KR pairs carry over
+                const float2* gp = Gp + p0 * G::GPS + c;
+                const float2* bp = Bp + p0 * G::GPS + c;
+                float2* out = P2 + p0 * G::P2S + c;
+                float2 Lg[FM / 2 + KR], Lb[FM / 2 + KR];
+                float s0 = 0.f;
 #pragma unroll
-                for (int k2 = 0; k2 < FM / 2 + KR; ++k2) L[k2] = Gp[(p0 + k2) * G::GPS + c];
+                for (int k2 = 0; k2 < KR; ++k2) { Lg[k2] = gp[k2 * G::GPS]; Lb[k2] = bp[k2 * G::GPS]; }
 #pragma unroll
-                for (int k2 = 0; k2 < FM / 2 + KR - 1; ++k2) ML[k2] = make_float2(L[k2].y, L[k2 + 1].x);
-                float2 gq[FM / 2];
+                for (int h = 0; h < G::HC; ++h) {
+                    const int q0 = h * (FM / 2);
 #pragma unroll
-                for (int m = 0; m < FM / 2; ++m) {
-                    float2 acc = make_float2(0.f, 0.f);
+                    for (int k2 = KR; k2 < FM / 2 + KR; ++k2) Lg[k2] = gp[(q0 + k2) * G::GPS];
+                    float2 ML[FM / 2 + KR - 1];
 #pragma unroll
-                    for (int j = 0; j < TAPS; ++j)
-                        acc = fma2(W2[j], (j & 1) ? ML[m + (j >> 1)] : L[m + (j >> 1)], acc);
-                    gq[m] = mul2(acc, RN2);
-                }
-                // the rows' box sums, float frames: in tap order.  uint16 frames in
-                // scalar: the first window summed in tap
-                // order, each next row's window slid by one row; every partial
-                // sum is an integer below 2^24 (u16 frames), so all orders give
-                // the same bits
-                float2 cs[FM / 2];
-                {
+                    for (int k2 = 0; k2 < FM / 2 + KR - 1; ++k2) ML[k2] = make_float2(Lg[k2].y, Lg[k2 + 1].x);
+                    float2 gq[FM / 2], cs[FM / 2];
 #pragma unroll
-                    for (int k2 = 0; k2 < FM / 2 + KR; ++k2) L[k2] = Bp[(p0 + k2) * G::GPS + c];
+                    for (int m = 0; m < FM / 2; ++m) {
+                        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+                        for (int j = 0; j < TAPS; ++j)
+                            acc = fma2(W2[j], (j & 1) ? ML[m + (j >> 1)] : Lg[m + (j >> 1)], acc);
+                        gq[m] = mul2(acc, RN2);
+                    }
+#pragma unroll
+                    for (int k2 = KR; k2 < FM / 2 + KR; ++k2) Lb[k2] = bp[(q0 + k2) * G::GPS];
+                    // the rows' box sums, float frames: in tap order; uint16
+                    // frames: the first window summed in tap order, each next
+                    // row's window slid by one row (every partial sum is an
+                    // integer below 2^24, so all orders give the same bits)
                     if constexpr (F32) {
 #pragma unroll
-                        for (int k2 = 0; k2 < FM / 2 + KR - 1; ++k2) ML[k2] = make_float2(L[k2].y, L[k2 + 1].x);
+                        for (int k2 = 0; k2 < FM / 2 + KR - 1; ++k2) ML[k2] = make_float2(Lb[k2].y, Lb[k2 + 1].x);
 #pragma unroll
                         for (int m = 0; m < FM / 2; ++m) {
-                            float2 acc = L[m];
+                            float2 acc = Lb[m];
 #pragma unroll
-                            for (int j = 1; j < TAPS; ++j) acc = add2(acc, (j & 1) ? ML[m + (j >> 1)] : L[m + (j >> 1)]);
+                            for (int j = 1; j < TAPS; ++j) acc = add2(acc, (j & 1) ? ML[m + (j >> 1)] : Lb[m + (j >> 1)]);
                             cs[m] = acc;
                         }
                     } else {
-                    float bsum[FM + 2 * KR];
+                        auto row = [&](int r) { return (r & 1) ? Lb[r >> 1].y : Lb[r >> 1].x; };
+                        if (h == 0) {
 #pragma unroll
-                    for (int k2 = 0; k2 < FM / 2 + KR; ++k2) { bsum[2 * k2] = L[k2].x; bsum[2 * k2 + 1] = L[k2].y; }
-                    float sb[FM];
-                    float s0 = bsum[0];
+                            for (int j = 0; j < 2 * KR; ++j) s0 = s0 + row(j);
+                        }
+                        float sb[FM];
 #pragma unroll
-                    for (int j = 1; j < TAPS; ++j) s0 = s0 + bsum[j];
-                    sb[0] = s0;
+                        for (int m = 0; m < FM; ++m) {
+                            s0 = s0 + row(m + 2 * KR);
+                            sb[m] = s0;
+                            s0 = s0 - row(m);
+                        }
 #pragma unroll
-                    for (int m = 1; m < FM; ++m) {
-                        s0 = s0 + bsum[m + 2 * KR];
-                        s0 = s0 - bsum[m - 1];
-                        sb[m] = s0;
+                        for (int m = 0; m < FM / 2; ++m) cs[m] = make_float2(sb[2 * m], sb[2 * m + 1]);
                     }
 #pragma unroll
-                    for (int m = 0; m < FM / 2; ++m) cs[m] = make_float2(sb[2 * m], sb[2 * m + 1]);
+                    for (int m = 0; m < FM / 2; ++m) {
+                        // preprocess_cols.wgsl:54 contracted: fma(-cs, 1/k^2, gauss);
+                        // cs * -rkk is exactly -(cs * rkk)
+                        const float2 res = fma2(cs[m], NRKK2, gq[m]);
+                        // preprocess_cols.wgsl:55-60 clip at 0; res is never NaN or -0
+                        // here (u16 frames, non-negative sums), where max equals the
+                        // shader's select; positions outside the frame take -inf below
+                        // (float frames: the select, which keeps a NaN)
+                        float2 o;
+                        o.x = F32 ? (res.x < 0.f ? 0.f : res.x) : fmaxf(res.x, 0.f);
+                        o.y = F32 ? (res.y < 0.f ? 0.f : res.y) : fmaxf(res.y, 0.f);
+                        out[(q0 + m) * G::P2S] = o;
                     }
-                }
 #pragma unroll
-                for (int m = 0; m < FM / 2; ++m) {
-                    // preprocess_cols.wgsl:54 contracted: fma(-cs, 1/k^2, gauss);
-                    // cs * -rkk is exactly -(cs * rkk)
-                    const float2 res = fma2(cs[m], NRKK2, gq[m]);
-                    // preprocess_cols.wgsl:55-60 clip at 0; res is never NaN or -0
-                    // here (u16 frames, non-negative sums), where max equals the
-                    // shader's select; positions outside the frame take -inf below
-                    // (float frames: the select, which keeps a NaN)
-                    float2 o;
-                    o.x = F32 ? (res.x < 0.f ? 0.f : res.x) : fmaxf(res.x, 0.f);
-                    o.y = F32 ? (res.y < 0.f ? 0.f : res.y) : fmaxf(res.y, 0.f);
-                    P2[(p0 + m) * G::P2S + c] = o;
+                    for (int k2 = 0; k2 < KR; ++k2) { Lg[k2] = Lg[k2 + FM / 2]; Lb[k2] = Lb[k2 + FM / 2]; }
                 }
             }
             if (G::WS) bar_sync(5, NS);
@@ -1052,9 +1067,9 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
 
         // ---- 4. column max vs centre: non-strict local max (walk_cols.wgsl:19-36),
         //         listed at once: warp w owns tile rows 8 (w / 2) .. + 7 of
-        //         column half w % 2, ballots each row and appends its flagged
-        //         pixels to the CTA list (one shared atomic per warp; the order
-        //         of the list does not matter: records carry their rank) ----
+        //         column half w % 2 and appends their local maxima to the CTA
+        //         list (the order of the list does not matter: records carry
+        //         their rank) ----
         static_assert(FT * (TH0 / FM) == NTK && FT == 64, "one column of 8 rows per thread");
         {
             const int tc = tid % FT, rq = tid / FT;
@@ -1080,9 +1095,7 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
             }
             // a tile whose copy ran out of its wait lists nothing
             const bool col_in = f.tx0 + tc < W && !*(volatile int*)&s_fail;
-            unsigned bal[FM];
-            int nc = 0;
-            const int nin = col_in ? f.TH - tr0 : 0;  // rows m < nin are in the frame
+            const int nin = col_in ? min(max(f.TH - tr0, 0), FM) : 0;  // rows m < nin are in the frame
             // the centres: processed rows tr0 + HP .. tr0 + HP + FM - 1, read
             // as row pairs
             constexpr int CPO = HP & 1, NCP = (CPO + FM + 1) / 2;
@@ -1098,25 +1111,26 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
             }
             // in-frame centres are >= 0: with zero_skip a centre must be > 0
             const float zthr = p.zero_skip ? 0.f : -1.f;
+            unsigned mine = 0;
 #pragma unroll
             for (int m = 0; m < FM; ++m) {
                 const float center = cen[CPO + m];
                 // float frames: a NaN centre is no smaller than any maximum
-                const bool fl = m < nin && (F32 ? !(cm[m] > center) && !(p.zero_skip && center == 0.f)
-                                                : cm[m] <= center && center > zthr);
-                bal[m] = __ballot_sync(0xffffffffu, fl);
-                nc += __popc(bal[m]);
+                if (F32 ? !(cm[m] > center) && !(p.zero_skip && center == 0.f) : cm[m] <= center && center > zthr)
+                    mine |= 1u << m;
             }
+            mine &= (1u << nin) - 1u;
+            // a thread's first, then its second, ... (a ballot per row cost more
+            // than the few pixels that a warp lists)
             const unsigned lt = (1u << lane) - 1u;
-            int wbase = 0;
-            if (lane == 0 && nc) wbase = atomicAdd(&s_nc, nc);
-            wbase = __shfl_sync(0xffffffffu, wbase, 0);
-#pragma unroll
-            for (int m = 0; m < FM; ++m) {
-                if (bal[m] != 0u) {  // warp-uniform: most rows list nothing
-                    if ((bal[m] >> lane) & 1u)
-                        clist[wbase + __popc(bal[m] & lt)] = (unsigned short)((tr0 + m) * FT + tc);
-                    wbase += __popc(bal[m]);
+            for (unsigned bal = __ballot_sync(0xffffffffu, mine != 0); bal;
+                 bal = __ballot_sync(0xffffffffu, mine != 0)) {
+                int base = 0;
+                if (lane == 0) base = atomicAdd(&s_nc, __popc(bal));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (mine) {
+                    clist[base + __popc(bal & lt)] = (unsigned short)((tr0 + __ffs(mine) - 1) * FT + tc);
+                    mine &= mine - 1;
                 }
             }
         }
