@@ -131,6 +131,7 @@ struct gt_ctx {
     HostCopy hc;                         // pageable host arrays
     TrajMem traj;                        // scratch of the trajectory calls
     cudaEvent_t cev[9] = {};
+    cudaEvent_t lev = nullptr;        // work pending on the legacy default stream (call_stream)
 };
 
 namespace {
@@ -1480,6 +1481,20 @@ int adjoint_finish(gt_ctx* ctx, const AdjWork& aw, cudaStream_t st) {
 }  // namespace
 
 namespace {
+// The stream of a call on device pointers.  NULL is the context's stream, which
+// does not wait for the legacy default stream by itself: what that holds (torch
+// passes NULL for it) may still be writing the call's inputs or reading the
+// memory of its outputs.
+cudaStream_t call_stream(gt_ctx* ctx, void* stream) {
+    if (stream || !ctx) return (cudaStream_t)stream;
+    if (cudaSetDevice(ctx->device) != cudaSuccess ||
+        (!ctx->lev && cudaEventCreateWithFlags(&ctx->lev, cudaEventDisableTiming) != cudaSuccess) ||
+        cudaEventRecord(ctx->lev, cudaStreamLegacy) != cudaSuccess ||
+        cudaStreamWaitEvent(ctx->stream, ctx->lev, 0) != cudaSuccess)
+        cudaGetLastError();  // another stream is being captured: as without the wait
+    return ctx->stream;
+}
+
 thread_local std::string g_noctx_err;  // errors of calls made without a context
 }
 
@@ -1522,6 +1537,7 @@ void gt_ctx_destroy(gt_ctx* ctx) {
         if (e) cudaEventDestroy(e);
     for (auto& e : ctx->ev)
         if (e) cudaEventDestroy(e);
+    if (ctx->lev) cudaEventDestroy(ctx->lev);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -1667,7 +1683,7 @@ int gt_batch_file(gt_ctx* ctx, const char* path, int has_channel, uint32_t chann
 
 int gt_batch_device(gt_ctx* ctx, const void* d_frames, int dtype, int T, int H, int W,
                     const gt_params* params, float* d_out, int64_t out_rows, int64_t* nrows, void* stream) {
-    cudaStream_t st = stream ? (cudaStream_t)stream : (ctx ? ctx->stream : nullptr);
+    cudaStream_t st = call_stream(ctx, stream);
     return batch_common(ctx, d_frames, false, dtype, T, H, W, params, nullptr, d_out, out_rows, nrows, st);
 }
 
@@ -1678,7 +1694,7 @@ int gt_batch_device_walk(gt_ctx* ctx, const void* d_frames, int dtype, int T, in
         ctx->err = "null walk buffer";
         return GT_ERR_ARG;
     }
-    cudaStream_t st = stream ? (cudaStream_t)stream : (ctx ? ctx->stream : nullptr);
+    cudaStream_t st = call_stream(ctx, stream);
     return batch_common(ctx, d_frames, false, dtype, T, H, W, params, nullptr, d_out, out_rows, nrows, st,
                         (int*)d_walk);
 }
@@ -1690,7 +1706,7 @@ int gt_adjoint_forward(gt_ctx* ctx, const float* d_frames, int T, int H, int W, 
     int rc = adjoint_setup(ctx, d_frames, T, H, W, params, d_walk, n, &ap, &circ);
     if (rc) return rc;
     if (n > 0 && !d_yxm) { ctx->err = "null output"; return GT_ERR_ARG; }
-    cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
+    cudaStream_t st = call_stream(ctx, stream);
     AdjWork aw;
     rc = adjoint_work(ctx, ap, circ, -1, &aw, st);
     if (rc) return rc;
@@ -1713,7 +1729,7 @@ int gt_adjoint_backward(gt_ctx* ctx, const float* d_frames, int T, int H, int W,
     int rc = adjoint_setup(ctx, d_frames, T, H, W, params, d_walk, n, &ap, &circ);
     if (rc) return rc;
     if (!d_grad_frames || !d_grad_params || (n > 0 && !d_grad_yxm)) { ctx->err = "null output"; return GT_ERR_ARG; }
-    cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
+    cudaStream_t st = call_stream(ctx, stream);
     AdjWork aw;
     rc = adjoint_work(ctx, ap, circ, n, &aw, st);
     if (rc) return rc;
@@ -1763,7 +1779,7 @@ int gt_adjoint_uncertainty(gt_ctx* ctx, const float* d_frames, int T, int H, int
     }
     ap.gain = gain;
     ap.read_var = read_noise * read_noise;
-    cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
+    cudaStream_t st = call_stream(ctx, stream);
     AdjWork aw;
     rc = adjoint_work(ctx, ap, circ, -1, &aw, st);
     if (rc) return rc;
@@ -1779,7 +1795,7 @@ int gt_adjoint_uncertainty(gt_ctx* ctx, const float* d_frames, int T, int H, int
 }
 
 int gt_batch_many_device(gt_ctx* ctx, gt_movie* movies, int n, void* stream) {
-    cudaStream_t st = stream ? (cudaStream_t)stream : (ctx ? ctx->stream : nullptr);
+    cudaStream_t st = call_stream(ctx, stream);
     return batch_many(ctx, movies, n, st);
 }
 
