@@ -45,6 +45,32 @@ def test_pending_walks(gpu, d, iters, dtype):
     np.testing.assert_array_equal(got, want)
 
 
+# rows of no whole 16 bytes: one and several chunks of 64 MB, frames larger than
+# a chunk, and frames that start between words
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("dtype,T,H,W", [("u16", 3, 90, 131), ("f32", 3, 90, 131), ("u16", 35, 1001, 1003),
+                                         ("f32", 18, 1001, 1003), ("u16", 1, 5801, 5803)])
+def test_ragged_rows(gpu, dtype, T, H, W, shift):
+    import torch
+
+    from tracking_optimizations_b200 import _native, gpu_tracking
+
+    g = torch.Generator(device="cuda").manual_seed(W + T)
+    raw = torch.poisson(torch.full((T * H * W + 1,), 60.0, device="cuda"), generator=g)
+    raw[torch.randint(0, T * H * W, (T * H * W // 700,), device="cuda", generator=g)] += 500.0
+    raw = raw if dtype == "f32" else raw.to(torch.int16)
+    m = raw[shift: shift + T * H * W].view(T, H, W)
+    params = dict(separation=8, minmass=150.0, search_range=2.0, memory=1)
+    got = gpu_tracking.batch_device(m, 7, **params)
+    _native.set_option("force_generic", 1)
+    try:
+        want = gpu_tracking.batch_device(m, 7, **params)
+    finally:
+        _native.set_option("force_generic", 0)
+    assert len(got) > 20
+    assert torch.equal(got, want)
+
+
 def _chain_table(n, T, miss, seed, spacing):
     """Chains of n particles `spacing` apart that jitter and blink."""
     rng = np.random.default_rng(seed)

@@ -46,7 +46,9 @@ __global__ void grid_kernel(const float* py, const float* px, const int* npart, 
                             int ncy, int ncx, int* gstart, int* gidx, float2* gpos);
 int fast_supported(int kr, int dd, int rc, int diameter, int dtype);
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
-                               const MovieBufs& b, int T, int frame0, int* used_tma);
+                               const MovieBufs& b, const TileSource& src, int frame0, int* used_tma);
+cudaError_t launch_repack(const void* frames, int dtype, int frame0, int nf, int H, int W, int pitch, void* out,
+                          int num_sms, cudaStream_t st);
 void gauss_taps(int smoothing_size, float noise_size, int normalized, float* w, float* norm, float* rn);
 cudaError_t launch_adjoint_particles(int mode, const AdjParams& p, const float* frames, const int* walk, long long n,
                                      const int* circ, const float* grad, float* yxm, const AdjTiles& tl, double* gpar,
@@ -140,6 +142,10 @@ constexpr int LOC_TH = 32;
 constexpr int LOC_TW = 64;
 constexpr int LOC_CMAX = 512;
 constexpr int FB_WIN_MAX = 100;
+// Frames repacked at a time: few enough to be read back from L2 (126 MB), many
+// enough to fill the locate launch (300 frames of 507 x 517: 32 MB 0.577 ms, 64
+// 0.537, 128 0.540).
+constexpr long long REPACK_BYTES = 64LL << 20;
 constexpr long long SUBNET_BUDGET = 1LL << 26;  // option trials per subnet
 constexpr int LINK_WINDOWS = 16;  // upload chunks of the host-frames path, at most
 constexpr int STATUS_LSTAT = 8 + LINK_WINDOWS, STATUS_INTS = STATUS_LSTAT + 2 * (12 + 8);
@@ -245,6 +251,7 @@ struct Plan {
     size_t smem_loc = 0, smem_fin = 0;
     int fb_win = 0;
     int fast = 0;
+    int repack = 0, pitch = 0;  // frames of a chunk repacked for the tile copies (0: as given), their row pitch
     int fast_th = 32;
     std::vector<float> char_tab, gchar_tab;
     std::vector<int> char_off, sig_off, bg_off;
@@ -331,7 +338,7 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     lp.zero_skip = lp.max_iter >= 1 && lp.rint_c <= lp.o && lp.rint_c <= lp.D - 1 - lp.o;
     lp.tma_spin = 1 << 22;
     lp.tma_withhold = 0;
-    P.fast = 0;
+    P.fast = P.repack = 0;
     const int want_fast = force_generic_flag ? 0 : fast_supported(lp.krad, lp.D, lp.rint_c, lp.d, dtype);
     P.char_tab.clear(); P.char_off.clear(); P.gchar_tab.clear();
     // only what the columns asked for read: most calls upload no table (8 us of
@@ -347,6 +354,12 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
         lp.TW = 64;
         lp.ntx = (W + lp.TW - 1) / lp.TW;
         lp.nty = (H + lp.TH - 1) / lp.TH;
+        // widths that the tile copies can't take: chunks of frames with padded
+        // rows, small enough to be read back from L2
+        const int px = dtype == GT_U16 ? 2 : 4, vp = 16 / px;
+        P.pitch = (W + vp - 1) / vp * vp;
+        const long long frame = (long long)H * P.pitch * px;
+        if (P.pitch != W && frame <= REPACK_BYTES) P.repack = (int)std::min<long long>(T, REPACK_BYTES / frame);
     }
     P.sig_off.clear(); P.bg_off.clear();
     if (r.has_sig) circle_inds_f(r.sig_radius, P.sig_off);
@@ -399,6 +412,7 @@ struct Work {
     int *rowcnt, *pend;
     float *py, *px, *pm;
     int *prec, *npart, *gstart, *gidx;
+    char* repack;
     int *crec, *ccell, *cidx;
     float *cy, *cx, *cm;
     int* tables;
@@ -469,6 +483,7 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->pbeg = w->status + 8;
     w->lstat = (unsigned long long*)(w->status + STATUS_LSTAT);
     w->fcount = w->status + STATUS_INTS;
+    w->repack = c.take<char>(need_locate ? (size_t)P.repack * P.H * P.pitch * (P.dtype == GT_U16 ? 2 : 4) : 1);
     w->off = c.take<int>(T + 1);
     const size_t np = P.link ? T * P.cap_p : 1;
     const size_t nm = P.link && P.r.memory > 0 ? np : 1;   // memory entries
@@ -615,6 +630,30 @@ MovieBufs movie_bufs(const Plan& P, const Work& w, const void* frames) {
     return b;
 }
 
+// The specialised locate kernel over frames [f0, f0 + nf).  *used_tma: the tiles
+// were copied from the frames as they are.
+int locate_frames(gt_ctx* ctx, const Plan& P, const Work& w, const MovieBufs& b, int f0, int nf, cudaStream_t st,
+                  int* used_tma, int32_t* launches) {
+    const int ntiles = P.lp.ntx * P.lp.nty;
+    *used_tma = 0;
+    if (!P.repack) {
+        CK(launch_locate_fast(P.lp.krad, P.lp.D, P.lp.rint_c, P.fast_th, dim3(ntiles, nf), st, P.lp, b,
+                              TileSource{(const char*)b.frames + (size_t)f0 * P.H * P.W * (P.dtype == GT_U16 ? 2 : 4), P.W},
+                              f0, used_tma));
+        ++*launches;
+        return GT_OK;
+    }
+    for (int s = f0; s < f0 + nf; s += P.repack) {
+        const int m = std::min(P.repack, f0 + nf - s);
+        int tma = 0;
+        CK(launch_repack(b.frames, P.dtype, s, m, P.H, P.W, P.pitch, w.repack, ctx->num_sms, st));
+        CK(launch_locate_fast(P.lp.krad, P.lp.D, P.lp.rint_c, P.fast_th, dim3(ntiles, m), st, P.lp, b,
+                              TileSource{w.repack, P.pitch}, s, &tma));
+        *launches += 2;
+    }
+    return GT_OK;
+}
+
 // The whole locate(+link) pipeline on device frames; table left in w.out.
 // With h_frames set, d_frames is the workspace copy of host frames: the
 // copy runs in chunks of frames on the context's copy stream and each
@@ -633,7 +672,6 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
     CK(allow_shared<locate_tiles_kernel>());
     for (int i = 0; i < 5; ++i)
         if (!ctx->ev[i]) CK(cudaEventCreate(&ctx->ev[i]));
-    const int ntiles = P.lp.ntx * P.lp.nty;
     const bool fast = P.fast != 0;
     ctx->stats.locate_kernel = P.fast == 1 ? 1 : 0;
     // frame chunks: up to 16 for host frames (copy/locate overlap; the
@@ -697,10 +735,9 @@ int run_pipeline(gt_ctx* ctx, const Plan& P, const Work& w, const void* d_frames
             rc = stage(f0, nf);
             if (!rc) rc = mark();
             if (rc) return rc;
-            dim3 grid(ntiles, nf);
             int used_tma = 0;
-            CK(launch_locate_fast(P.lp.krad, P.lp.D, P.lp.rint_c, P.fast_th, grid, st, P.lp, b, T, f0, &used_tma));
-            ctx->stats.launches += 1;
+            rc = locate_frames(ctx, P, w, b, f0, nf, st, &used_tma, &ctx->stats.launches);
+            if (rc) return rc;
             if (P.fast == 1) ctx->stats.locate_kernel = used_tma ? 2 : 1;
             if (chunked && (rc = post(f0, nf))) return rc;
         }
@@ -995,13 +1032,12 @@ int tune_tile_rows(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t
             std::string msg;
             if (make_plan(P.r, P.T, P.H, P.W, P.dtype, 1, ctx->num_sms, &Q, &msg, 0, ths[v])) return GT_ERR_ARG;
             MovieBufs b = movie_bufs(Q, bm.w, frames);
-            const int ntiles = Q.lp.ntx * Q.lp.nty;
             for (int rep = 0; rep < 2; ++rep) {
                 CK(cudaMemsetAsync(bm.w.status, 0, sizeof(int) * (STATUS_INTS + (size_t)P.T), st));
                 CK(cudaEventRecord(ctx->ev[0], st));
-                int used_tma = 0;
-                CK(launch_locate_fast(Q.lp.krad, Q.lp.D, Q.lp.rint_c, ths[v], dim3(ntiles, nf), st, Q.lp, b, P.T, 0,
-                                      &used_tma));
+                int used_tma = 0, launches = 0;
+                const int rc = locate_frames(ctx, Q, bm.w, b, 0, nf, st, &used_tma, &launches);
+                if (rc) return rc;
                 CK(cudaEventRecord(ctx->ev[1], st));
                 CK(cudaEventSynchronize(ctx->ev[1]));
                 CK(cudaEventElapsedTime(&ms[v], ctx->ev[0], ctx->ev[1]));
@@ -1031,13 +1067,11 @@ int enqueue_front(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t 
     const int T = P.T;
     MovieBufs b = movie_bufs(P, w, frames);
     CK(cudaMemsetAsync(w.status, 0, sizeof(int) * (STATUS_INTS + (size_t)T), s));
-    const int ntiles = P.lp.ntx * P.lp.nty;
     if (bm.fast) {
         for (int f0 = 0; f0 < T; f0 += 65535) {
             int used_tma = 0;
-            CK(launch_locate_fast(P.lp.krad, P.lp.D, P.lp.rint_c, P.fast_th, dim3(ntiles, std::min(65535, T - f0)), s,
-                                  P.lp, b, T, f0, &used_tma));
-            ++*launches;
+            const int rc = locate_frames(ctx, P, w, b, f0, std::min(65535, T - f0), s, &used_tma, launches);
+            if (rc) return rc;
         }
     } else {
         LocParams lg = P.lp;
@@ -1150,6 +1184,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
                        ctx->batch_cap_div);
         if (rc) { ctx->err = who + msg; return rc; }
         B[i].P.lp.tiles_per_cta = ctx->tiles_per_cta;
+        if (ctx->batch_cap_div != 64) B[i].P.repack = 0;  // memory is short
         char buf[128];
         std::snprintf(buf, sizeof(buf), "%p|%d|%d|%d|%d|%p|%lld|", m.frames, m.dtype, m.T, m.H, m.W, (void*)m.out,
                       (long long)m.out_rows);
@@ -1315,7 +1350,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         int cnt = 0;
         for (int i = 0; i < n; ++i) {
             const Plan& P = B[i].P;
-            cnt += (P.T + 65534) / 65535 + 2 + (P.link ? 2 : 0) + 1;
+            cnt += (P.repack ? 2 * ((P.T + P.repack - 1) / P.repack) : (P.T + 65534) / 65535) + 2 + (P.link ? 2 : 0) + 1;
         }
         S.launches = cnt + (S.nlink > 0 ? 1 : 0);
     }

@@ -46,6 +46,14 @@ struct LocParams {
     int tma_spin;               // iteration limit of the bounded wait for a staged tile
     int tma_withhold;           // test switch: issue no tile copy, so the wait runs out
     int tiles_per_cta;          // specialised kernel: tiles per CTA (0 = chosen per launch)
+    int frame0;                 // specialised kernel: first frame of the launch (its buffers start there)
+};
+
+// Where the specialised kernel's tile copies read a launch's frames: rows
+// `pitch` pixels apart.
+struct TileSource {
+    const void* base;
+    int pitch;
 };
 
 // One located feature, keyed by its originating pixel (walk_cols.wgsl:87-91).

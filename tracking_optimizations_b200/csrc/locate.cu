@@ -270,6 +270,54 @@ __global__ void __launch_bounds__(NT) locate_tiles_kernel(const LocParams p, con
         b.rowcnt[((size_t)t * H + ty0 + r) * p.ntx + tj] = rowcount[r];
 }
 
+// Rows copied to a pitch of whole 16-byte groups, so that the tile copies (TMA)
+// take frames of any width: 16 bytes per item, as 32-bit words where the row
+// starts on one, else the words between the first and the last pixel, shifted.
+// Bound by memory.  Locate of 300 uint16 frames of 507 x 517, diameter 7: 0.652
+// ms with tiles read pixel by pixel, 0.536 with the copy (0.462 for 512 x 520
+// without one).
+template <class PX>
+__global__ void __launch_bounds__(256) repack_kernel(const PX* __restrict__ frames, long long rows, int W, int groups,
+                                                     uint4* __restrict__ out) {
+    constexpr int VP = 16 / sizeof(PX);
+    const long long n = rows * groups;
+    for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+        const long long r = i / groups;
+        const int c = (int)(i - r * groups) * VP;
+        const PX* src = frames + r * W + c;
+        uint4 o;
+        if (c + VP <= W) {
+            if (sizeof(PX) == 4 || ((uintptr_t)src & 2) == 0) {
+                const unsigned* w = (const unsigned*)src;
+                o = make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+            } else {
+                const unsigned* w = (const unsigned*)(src + 1);
+                const unsigned a = (unsigned)__ldg(src), z = (unsigned)__ldg(src + VP - 1);
+                const unsigned w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2);
+                o = make_uint4(a | w0 << 16, __funnelshift_l(w0, w1, 16), __funnelshift_l(w1, w2, 16), w2 >> 16 | z << 16);
+            }
+        } else {
+            __align__(16) PX v[VP];
+#pragma unroll
+            for (int q = 0; q < VP; ++q) v[q] = c + q < W ? __ldg(src + q) : (PX)0;
+            o = *(const uint4*)v;
+        }
+        out[i] = o;
+    }
+}
+
+cudaError_t launch_repack(const void* frames, int dtype, int frame0, int nf, int H, int W, int pitch, void* out,
+                          int num_sms, cudaStream_t st) {
+    const long long rows = (long long)nf * H, first = (long long)frame0 * H * W;
+    const int groups = pitch / (dtype == 0 ? 8 : 4);
+    const int grid = (int)std::min<long long>((rows * groups + 255) / 256, (long long)num_sms * 32);
+    if (dtype == 0)
+        repack_kernel<<<grid, 256, 0, st>>>((const unsigned short*)frames + first, rows, W, groups, (uint4*)out);
+    else
+        repack_kernel<<<grid, 256, 0, st>>>((const float*)frames + first, rows, W, groups, (uint4*)out);
+    return cudaGetLastError();
+}
+
 // Walks of the records that locate left pending (the walk left the tile halo,
 // a crowded tile, max_iterations == 0): the processed values that a walk can
 // read are recomputed from the frame, with the same arithmetic, into a

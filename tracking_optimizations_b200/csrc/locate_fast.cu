@@ -5,7 +5,7 @@
 namespace gt {
 
 cudaError_t launch_locate_flex(int kr, int rc, int dtype, dim3 grid, cudaStream_t st, const LocParams& p,
-                               const MovieBufs& b, int T, int frame0, int* used_tma);
+                               const MovieBufs& b, const TileSource& src, int frame0, int* used_tma);
 int flex_dilation(int rc, int dtype);
 
 // (smoothing radius, dilation size, centroid radius) triples with a kernel of
@@ -28,19 +28,19 @@ int fast_supported(int kr, int dd, int rc, int diameter, int dtype) {
 }
 
 // Launches the specialised kernel over frames [frame0, frame0 + grid.y),
-// grid.x tiles per frame.  *used_tma reports whether the raw tiles were
-// staged by TMA.
+// grid.x tiles per frame, whose raw tiles are copied from src.  *used_tma
+// reports whether they were staged by TMA; else they are read from b.frames.
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
-                               const MovieBufs& b, int T, int frame0, int* used_tma) {
+                               const MovieBufs& b, const TileSource& src, int frame0, int* used_tma) {
     if (p.dtype == 0) {
 #define GT_FAST_CASE(KR, DD, RC)                                                                              \
     if (kr == KR && dd == DD && rc == RC)                                                                     \
-        return th == 32 ? launch_instance<KR, DD, 32, RC, unsigned short, false>(grid, st, p, b, T, frame0, used_tma) \
-                        : launch_instance<KR, DD, 64, RC, unsigned short, false>(grid, st, p, b, T, frame0, used_tma);
+        return th == 32 ? launch_instance<KR, DD, 32, RC, unsigned short, false>(grid, st, p, b, src, frame0, used_tma) \
+                        : launch_instance<KR, DD, 64, RC, unsigned short, false>(grid, st, p, b, src, frame0, used_tma);
         GT_FAST_LIST(GT_FAST_CASE)
 #undef GT_FAST_CASE
     }
-    return launch_locate_flex(kr, rc, p.dtype, grid, st, p, b, T, frame0, used_tma);
+    return launch_locate_flex(kr, rc, p.dtype, grid, st, p, b, src, frame0, used_tma);
 }
 
 }  // namespace gt

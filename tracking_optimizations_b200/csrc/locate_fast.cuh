@@ -423,17 +423,17 @@ __device__ __forceinline__ bool centroid_fixed(const LocParams& p, const P2Acc<G
 }  // namespace
 
 namespace {
-// Output tile g of a launch: tiles are numbered frame by frame, frame0 first.
+// Output tile g of a launch: tiles are numbered frame by frame.
 struct FTile {
     int t, tj, ty0, tx0, TH;
 };
 
 template <int TH0>
-__device__ __forceinline__ FTile tile_of(const LocParams& p, int frame0, int ntiles, int g) {
+__device__ __forceinline__ FTile tile_of(const LocParams& p, int ntiles, int g) {
     FTile f;
     const int fr = g / ntiles, tile = g - fr * ntiles;
     const int ti = tile / p.ntx;
-    f.t = frame0 + fr;
+    f.t = fr;
     f.tj = tile - ti * p.ntx;
     f.ty0 = ti * TH0;
     f.tx0 = f.tj * FT;
@@ -612,7 +612,7 @@ __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b
                 b.cand[(size_t)t * b.cap_c + slot] = rec;
                 if (rec.state == CAND_PENDING) {
                     const int k = atomicAdd(b.npend, 1);
-                    b.pend[k] = t * b.cap_c + slot;
+                    b.pend[k] = (p.frame0 + t) * b.cap_c + slot;
                 }
             }
         }
@@ -661,7 +661,7 @@ __device__ __forceinline__ void walk_emit(const LocParams& p, const MovieBufs& b
 template <int KR, int DD, int TH0, int RC, class PX, bool RT, int COLS>
 __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, RT>::CTAS))
     locate_fast_kernel(const LocParams p, const MovieBufs b, const __grid_constant__ CUtensorMap tmap, int use_tma,
-                       int frame0, int ntiles, int total, int per_cta) {
+                       int ntiles, int total, int per_cta) {
     using G = Geo<KR, DD, TH0, RC, PX, RT>;
     constexpr bool F32 = G::F32;
     constexpr int NTK = fast_threads(TH0);
@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
     if (tid < TH0) rowmask[tid] = 0ull;
     if (use_tma && tid == PROD) {
         mbar_init(&bar, 1);
-        const FTile f = tile_of<TH0>(p, frame0, ntiles, g0);
+        const FTile f = tile_of<TH0>(p, ntiles, g0);
         mbar_expect_tx(&bar, (uint32_t)(G::RH * G::US * sizeof(PX)));
         // tma_withhold (a test of the timeout path) issues no copy: the
         // barrier then never completes and the bounded wait runs out
@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
     const float NEG = -CUDART_INF_F;
 
     FTile prev{};  // tile k - 1, walked at the top of iteration k
-    FTile f = tile_of<TH0>(p, frame0, ntiles, g0);  // tile k
+    FTile f = tile_of<TH0>(p, ntiles, g0);  // tile k
     int last = 0;  // the last tile whose copy was issued (copy-issuing thread)
     for (int k = 0; k <= ntl; ++k) {
         if (k > 0) {
@@ -1148,10 +1148,10 @@ __global__ void __launch_bounds__(fast_threads(TH0), (Geo<KR, DD, TH0, RC, PX, R
 }
 
 namespace {
-// TMA descriptor over the movie (dims W x H x T, pixels of `px` bytes: u16 or
-// f32) with a box of the raw tile.  Needs a 16-byte aligned base and a row
+// TMA descriptor over a launch's frames (dims W x H x T, pixels of `px` bytes: u16
+// or f32) with a box of the raw tile.  Needs a 16-byte aligned base and a row
 // pitch multiple of 16 bytes.
-inline bool make_tensor_map(CUtensorMap* map, const void* frames, int px, int T, int H, int W, int box_w, int box_h) {
+inline bool make_tensor_map(CUtensorMap* map, const TileSource& src, int px, int T, int H, int W, int box_w, int box_h) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
         void* fn = nullptr;
@@ -1161,12 +1161,12 @@ inline bool make_tensor_map(CUtensorMap* map, const void* frames, int px, int T,
             return false;
         encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
     }
-    if (((uintptr_t)frames & 15) || ((long long)W * px) % 16) return false;
+    if (((uintptr_t)src.base & 15) || ((long long)src.pitch * px) % 16) return false;
     cuuint64_t dims[3] = {(cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)T};
-    cuuint64_t strides[2] = {(cuuint64_t)W * px, (cuuint64_t)W * H * px};
+    cuuint64_t strides[2] = {(cuuint64_t)src.pitch * px, (cuuint64_t)src.pitch * H * px};
     cuuint32_t box[3] = {(cuuint32_t)box_w, (cuuint32_t)box_h, 1};
     cuuint32_t es[3] = {1, 1, 1};
-    CUresult r = encode(map, px == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(frames), dims, strides, box, es,
+    CUresult r = encode(map, px == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(src.base), dims, strides, box, es,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
@@ -1189,22 +1189,29 @@ inline int fast_tiles_per_cta(const LocParams& p, int total, int ctas) {
 // Launches one instance over frames [frame0, frame0 + grid.y), grid.x tiles
 // per frame.  *used_tma reports whether the raw tiles were staged by TMA.
 template <int KR, int DD, int TH, int RC, class PX, bool RT>
-cudaError_t launch_instance(dim3 grid, cudaStream_t st, const LocParams& p, const MovieBufs& b, int T, int frame0,
-                            int* used_tma) {
+cudaError_t launch_instance(dim3 grid, cudaStream_t st, const LocParams& lp, const MovieBufs& mb, const TileSource& src,
+                            int frame0, int* used_tma) {
     using G = Geo<KR, DD, TH, RC, PX, RT>;
     const long long total = (long long)grid.x * grid.y;
     if (total <= 0 || total > (1LL << 30)) return cudaErrorInvalidValue;
+    LocParams p = lp;
+    p.frame0 = frame0;
+    MovieBufs b = mb;  // the kernel counts its frames from 0
+    b.frames = (const PX*)mb.frames + (size_t)frame0 * p.H * p.W;
+    b.fcount += frame0;
+    b.rowcnt += (size_t)frame0 * p.H * p.ntx;
+    b.cand += (size_t)frame0 * b.cap_c;
     const int per = fast_tiles_per_cta(p, (int)total, RT ? G::CTAS : (TH == 32 ? 4 : 2));
     const unsigned nblk = (unsigned)((total + per - 1) / per);
     CUtensorMap map;
     std::memset(&map, 0, sizeof(map));
-    const int tma = make_tensor_map(&map, b.frames, (int)sizeof(PX), T, p.H, p.W, G::US, G::RH) ? 1 : 0;
+    const int tma = make_tensor_map(&map, src, (int)sizeof(PX), (int)grid.y, p.H, p.W, G::US, G::RH) ? 1 : 0;
     *used_tma = tma;
     auto launch = [&](auto cols) {
         constexpr auto* fn = locate_fast_kernel<KR, DD, TH, RC, PX, RT, decltype(cols)::value>;
         const cudaError_t e = allow_shared<fn>();
         if (e != cudaSuccess) return e;
-        fn<<<nblk, fast_threads(TH), G::SMEM, st>>>(p, b, map, tma, frame0, (int)grid.x, (int)total, per);
+        fn<<<nblk, fast_threads(TH), G::SMEM, st>>>(p, b, map, tma, (int)grid.x, (int)total, per);
         return cudaGetLastError();
     };
     return p.characterize    ? launch(std::integral_constant<int, COLS_GPU>())

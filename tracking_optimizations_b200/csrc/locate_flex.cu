@@ -20,12 +20,12 @@ int flex_dilation(int rc, int dtype) {
 }
 
 cudaError_t launch_locate_flex(int kr, int rc, int dtype, dim3 grid, cudaStream_t st, const LocParams& p,
-                               const MovieBufs& b, int T, int frame0, int* used_tma) {
+                               const MovieBufs& b, const TileSource& src, int frame0, int* used_tma) {
     if (kr != rc || p.D < FM || p.D > flex_dilation(rc, dtype)) return cudaErrorInvalidValue;
 #define GT_FLEX_CASE(R, DD)                                                                                   \
     if (rc == R)                                                                                              \
-        return dtype == 0 ? launch_instance<R, DD, 64, R, unsigned short, true>(grid, st, p, b, T, frame0, used_tma) \
-                          : launch_instance<R, DD, 64, R, float, true>(grid, st, p, b, T, frame0, used_tma);
+        return dtype == 0 ? launch_instance<R, DD, 64, R, unsigned short, true>(grid, st, p, b, src, frame0, used_tma) \
+                          : launch_instance<R, DD, 64, R, float, true>(grid, st, p, b, src, frame0, used_tma);
     GT_FLEX_LIST(GT_FLEX_CASE)
 #undef GT_FLEX_CASE
     return cudaErrorInvalidValue;

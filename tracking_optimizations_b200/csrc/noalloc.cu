@@ -35,7 +35,7 @@ __global__ void scan_frames_kernel(const int* in, int* out, int n);
 cudaError_t launch_assemble(const AsmArgs& a, int num_sms, cudaStream_t st);
 int fast_supported(int kr, int dd, int rc, int diameter, int dtype);
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
-                               const MovieBufs& b, int T, int frame0, int* used_tma);
+                               const MovieBufs& b, const TileSource& src, int frame0, int* used_tma);
 void gauss_taps(int smoothing_size, float noise_size, int normalized, float* w, float* norm, float* rn);
 void set_noctx_error(const char* msg);
 }  // namespace gt
@@ -289,7 +289,7 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
 
     if (fast) {
         int used_tma = 0;
-        SCK(launch_locate_fast(lp.krad, lp.D, lp.rint_c, 64, dim3(lp.ntx * lp.nty, 1), st, lp, b, 1, 0, &used_tma));
+        SCK(launch_locate_fast(lp.krad, lp.D, lp.rint_c, 64, dim3(lp.ntx * lp.nty, 1), st, lp, b, TileSource{b.frames, lp.W}, 0, &used_tma));
     } else {
         const int PH = 32 + 2 * lp.hp, PW = 64 + 2 * lp.hp;
         const int RH = PH + 2 * lp.krad, RW = PW + 2 * lp.krad;
