@@ -2013,14 +2013,17 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         if (rc) return rc;
         // ids in row order: compact index g == row index
         CK(table_ids(tab, w.root, w.newid, ctx->num_sms, st));
-        int bits = 0;
-        CK(cudaMemcpyAsync(&bits, w.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        // the error bits arrive before the ids: one wait for both
+        if (!ctx->h_stage) {
+            CK(cudaHostAlloc((void**)&ctx->h_stage, sizeof(int) * STATUS_INTS, cudaHostAllocDefault));
+            ctx->h_stage_n = STATUS_INTS;
+        }
+        CK(cudaMemcpyAsync(ctx->h_stage, w.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CK(ctx->hc.download(ids, tab.ids, sizeof(uint64_t) * (size_t)n, st));
         bool retry;
-        rc = err_status(ctx, bits, &retry);
+        rc = err_status(ctx, ctx->h_stage[0], &retry);
         if (rc && retry && scale < 64) continue;
         if (rc) return rc;
-        CK(ctx->hc.download(ids, tab.ids, sizeof(uint64_t) * (size_t)n, st));
         ctx->stats.particles = n;
         return GT_OK;
     }

@@ -58,6 +58,48 @@ __global__ void table_largest_kernel(const int* off, int T, int* stat) {
     if ((threadIdx.x & 31) == 0) atomicMax(stat + 3, m);
 }
 
+// The same of a small table by one block: its launches and waits cost more than
+// the rows (20 frames of 50: 187 us a call in five launches and two waits, 161 in one).
+constexpr int TINY = 8192, TINY_NT = 1024;
+
+__global__ void __launch_bounds__(TINY_NT) table_tiny_kernel(const float* rows, int n, int ncols, int* frame, int* off,
+                                                             int* stat) {
+    __shared__ int warp_tot[TINY_NT / 32], s_total, s_stat[4];
+    if (threadIdx.x < 4) s_stat[threadIdx.x] = 0;
+    if (threadIdx.x == 0) off[0] = 0;
+    __syncthreads();
+    int ym = 0, xm = 0, bad = 0, before = 0;
+    for (int i0 = 0; i0 < n; i0 += TINY_NT) {
+        const int i = i0 + threadIdx.x;
+        int start = 0;
+        if (i < n) {
+            const float* r = rows + (size_t)i * ncols;
+            const float f = r[0], y = r[2], x = r[3];
+            start = i == 0 ? f != 0.f : f != r[-ncols];
+            bad |= !isfinite(y) || !isfinite(x);
+            ym = max(ym, __float_as_int(fmaxf(y, 0.f)));
+            xm = max(xm, __float_as_int(fmaxf(x, 0.f)));
+        }
+        const int t = before + block_excl_scan<TINY_NT>(start, warp_tot, &s_total) + start;
+        if (i < n) frame[i] = t;
+        if (start) off[t] = i;
+        before += s_total;
+        __syncthreads();
+    }
+    const int T = before + 1;
+    if (threadIdx.x == 0) off[T] = n;
+    __syncthreads();
+    int m = 0;
+    for (int t = threadIdx.x; t < T; t += TINY_NT) m = max(m, off[t + 1] - off[t]);
+    atomicMax(s_stat, ym);
+    atomicMax(s_stat + 1, xm);
+    if (bad) atomicOr(s_stat + 2, 1);
+    atomicMax(s_stat + 3, m);
+    __syncthreads();
+    if (threadIdx.x < 4) stat[threadIdx.x] = s_stat[threadIdx.x];
+    if (threadIdx.x == 0) stat[4] = T;
+}
+
 __global__ void table_slabs_kernel(const float* rows, const int* frame, const int* off, int n, int ncols, int T, int cap,
                                    float* py, float* px, int* npart) {
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
@@ -94,7 +136,7 @@ int table_load(const float* h_rows, int n, int ncols, TrajMem& M, cudaStream_t s
     int* starts = M.get<int>(n);
     t->frame = M.get<int>(n);
     t->off = M.get<int>((size_t)n + 2);
-    int* stat = M.get<int>(4);
+    int* stat = M.get<int>(5);
     size_t tmp = 0;
     LK(cub::DeviceScan::InclusiveSum(nullptr, tmp, starts, t->frame, n, st));
     void* w = M.get<char>(tmp);
@@ -108,20 +150,29 @@ int table_load(const float* h_rows, int n, int ncols, TrajMem& M, cudaStream_t s
     t->ncols = ncols;
     const int nb = blocks_for(n, num_sms);
     LK(M.hc->upload(rows, h_rows, sizeof(float) * (size_t)n * ncols, st));
-    LK(cudaMemsetAsync(stat, 0, 4 * sizeof(int), st));
-    table_starts_kernel<<<nb, 256, 0, st>>>(rows, n, ncols, starts, stat);
-    LK(cudaGetLastError());
-    LK(cub::DeviceScan::InclusiveSum(w, tmp, starts, t->frame, n, st));
-    table_offsets_kernel<<<nb, 256, 0, st>>>(starts, t->frame, n, t->off);
-    LK(cudaGetLastError());
-    int last = 0, h[4];
-    LK(cudaMemcpyAsync(&last, t->frame + n - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
-    LK(cudaStreamSynchronize(st));
-    t->T = last + 1;
-    table_largest_kernel<<<blocks_for(t->T, num_sms), 256, 0, st>>>(t->off, t->T, stat);
-    LK(cudaGetLastError());
-    LK(cudaMemcpyAsync(h, stat, sizeof(h), cudaMemcpyDeviceToHost, st));
-    LK(cudaStreamSynchronize(st));
+    int h[5];
+    if (n <= TINY) {
+        table_tiny_kernel<<<1, TINY_NT, 0, st>>>(rows, n, ncols, t->frame, t->off, stat);
+        LK(cudaGetLastError());
+        LK(cudaMemcpyAsync(h, stat, sizeof(h), cudaMemcpyDeviceToHost, st));
+        LK(cudaStreamSynchronize(st));
+        t->T = h[4];
+    } else {
+        LK(cudaMemsetAsync(stat, 0, 4 * sizeof(int), st));
+        table_starts_kernel<<<nb, 256, 0, st>>>(rows, n, ncols, starts, stat);
+        LK(cudaGetLastError());
+        LK(cub::DeviceScan::InclusiveSum(w, tmp, starts, t->frame, n, st));
+        table_offsets_kernel<<<nb, 256, 0, st>>>(starts, t->frame, n, t->off);
+        LK(cudaGetLastError());
+        int last = 0;
+        LK(cudaMemcpyAsync(&last, t->frame + n - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        LK(cudaStreamSynchronize(st));
+        t->T = last + 1;
+        table_largest_kernel<<<blocks_for(t->T, num_sms), 256, 0, st>>>(t->off, t->T, stat);
+        LK(cudaGetLastError());
+        LK(cudaMemcpyAsync(h, stat, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        LK(cudaStreamSynchronize(st));
+    }
     if (h[2]) {
         *msg = "non-finite position";
         return GT_ERR_ARG;
