@@ -1899,6 +1899,7 @@ int gt_filter_stubs(gt_ctx* ctx, const int64_t* ids, int64_t n, int64_t threshol
     *nkept = 0;
     if (n == 0) return GT_OK;
     ctx->traj.hc = &ctx->hc;
+    const TrajEnd end{ctx->traj};
     return traj_filter_stubs(ids, n, threshold, keep, count, nkept, ctx->traj, ctx->stream, ctx->num_sms, &ctx->err);
 }
 
@@ -1908,6 +1909,7 @@ int gt_steps(gt_ctx* ctx, const int64_t* ids, const float* x, const float* y, in
     if (rc) return rc;
     if (n == 0) return GT_OK;
     ctx->traj.hc = &ctx->hc;
+    const TrajEnd end{ctx->traj};
     return traj_steps(ids, x, y, n, (float)mpp, xs, ys, x_step, y_step, steplength, order, ctx->traj, ctx->stream,
                       ctx->num_sms, &ctx->err);
 }
@@ -1925,6 +1927,7 @@ int gt_imsd(gt_ctx* ctx, const int64_t* ids, const int64_t* frames, const float*
     float ms = 0.f;
     if (n > 0) {
         ctx->traj.hc = &ctx->hc;
+        const TrajEnd end{ctx->traj};
         rc = traj_imsd(ids, frames, x, y, n, (float)mpp, max_lagtime, table_alloc, &data, &m, &ms, ctx->traj, ctx->stream,
                        ctx->num_sms, &ctx->err);
         if (rc) {
@@ -1977,6 +1980,7 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
     cudaStream_t st = ctx->stream;
     LinkTable tab;
     ctx->traj.hc = &ctx->hc;
+    const TrajEnd end{ctx->traj};
     int rc = table_load(rows, (int)n, ncols, ctx->traj, st, ctx->num_sms, &tab, &ctx->err);
     if (rc) return rc;
     const int T = tab.T;

@@ -12,8 +12,11 @@ namespace gt {
 
 // Scratch handed out piece by piece and taken back as a whole by the next
 // call's begin() (every call ends with its stream synchronised).  What a call
-// needed is one block for the next call.
+// needed is one block for the next call, up to KEEP bytes; end() gives more
+// than that back to the device.
 struct TrajMem {
+    static constexpr size_t KEEP = (size_t)1 << 30;  // tables of 10 million rows; beyond, a call takes far longer than
+                                                     // the allocations
     HostCopy* hc = nullptr;
     cudaEvent_t ev[2] = {nullptr, nullptr};
 
@@ -45,6 +48,13 @@ struct TrajMem {
         return (X*)p;
     }
 
+    // After a call, whose stream is synchronised.
+    void end() {
+        size_t sum = 0;
+        for (auto& b : blocks_) sum += b.size;
+        if (sum > KEEP) release();
+    }
+
     void release() {
         for (auto& b : blocks_) cudaFree(b.p);
         blocks_.clear();
@@ -73,6 +83,12 @@ struct TrajMem {
     }
     std::vector<Block> blocks_;
     size_t used_ = 0;
+};
+
+// Ends a call on the scratch when it leaves its scope, after an error too.
+struct TrajEnd {
+    TrajMem& m;
+    ~TrajEnd() { m.end(); }
 };
 
 // A position table on the device and its frames (linktable.cu).
