@@ -115,6 +115,7 @@ HostCopy::~HostCopy() {
         if (e) cudaEventDestroy(e);
     for (auto& s : slot_)
         if (s) cudaFreeHost(s);
+    if (small_) cudaFreeHost(small_);
 }
 
 cudaError_t HostCopy::ready() {
@@ -157,7 +158,14 @@ cudaError_t HostCopy::upload(void* dst, const void* src, size_t bytes, cudaStrea
 }
 
 cudaError_t HostCopy::download(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (bytes < SMALL || page_locked(dst) || ready() != cudaSuccess) {
+    if (bytes < SMALL) {
+        char* w = staged((char*)dst);
+        cudaError_t e = cudaMemcpyAsync(w, src, bytes, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess && w != dst) std::memcpy(dst, w, bytes);
+        return e;
+    }
+    if (page_locked(dst) || ready() != cudaSuccess) {
         cudaGetLastError();
         const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
         return e != cudaSuccess ? e : cudaStreamSynchronize(st);

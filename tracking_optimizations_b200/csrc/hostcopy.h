@@ -47,14 +47,25 @@ class HostCopy {
     cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st);
     // The device to dst (host); dst holds the data when the call returns.
     cudaError_t download(void* dst, const void* src, size_t bytes, cudaStream_t st);
+    // Page-locked words for results that the call waits for at once: copies into
+    // pageable memory wait one by one.  `words` where there are none.
+    template <class X>
+    X* staged(X* words) {
+        if (!small_ && cudaHostAlloc((void**)&small_, SMALL, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            small_ = nullptr;
+        }
+        return small_ ? (X*)small_ : words;
+    }
 
   private:
     static constexpr int SLOTS = 4;
     static constexpr size_t SLOT = (size_t)8 << 20;
-    static constexpr size_t SMALL = (size_t)64 << 10;  // below: the driver's own staging
+    static constexpr size_t SMALL = (size_t)64 << 10;  // below: uploads by the driver's own staging, downloads by small_
     cudaError_t ready();
     CopyPool pool_;
     char* slot_[SLOTS] = {};
+    char* small_ = nullptr;
     cudaEvent_t ev_[SLOTS] = {};
     int next_ = 0;
 };

@@ -150,11 +150,12 @@ int table_load(const float* h_rows, int n, int ncols, TrajMem& M, cudaStream_t s
     t->ncols = ncols;
     const int nb = blocks_for(n, num_sms);
     LK(M.hc->upload(rows, h_rows, sizeof(float) * (size_t)n * ncols, st));
-    int h[5];
+    int words[5];
+    int* h = M.hc->staged(words);
     if (n <= TINY) {
         table_tiny_kernel<<<1, TINY_NT, 0, st>>>(rows, n, ncols, t->frame, t->off, stat);
         LK(cudaGetLastError());
-        LK(cudaMemcpyAsync(h, stat, sizeof(h), cudaMemcpyDeviceToHost, st));
+        LK(cudaMemcpyAsync(h, stat, sizeof(words), cudaMemcpyDeviceToHost, st));
         LK(cudaStreamSynchronize(st));
         t->T = h[4];
     } else {
@@ -164,10 +165,9 @@ int table_load(const float* h_rows, int n, int ncols, TrajMem& M, cudaStream_t s
         LK(cub::DeviceScan::InclusiveSum(w, tmp, starts, t->frame, n, st));
         table_offsets_kernel<<<nb, 256, 0, st>>>(starts, t->frame, n, t->off);
         LK(cudaGetLastError());
-        int last = 0;
-        LK(cudaMemcpyAsync(&last, t->frame + n - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+        LK(cudaMemcpyAsync(h, t->frame + n - 1, sizeof(int), cudaMemcpyDeviceToHost, st));
         LK(cudaStreamSynchronize(st));
-        t->T = last + 1;
+        t->T = h[0] + 1;
         table_largest_kernel<<<blocks_for(t->T, num_sms), 256, 0, st>>>(t->off, t->T, stat);
         LK(cudaGetLastError());
         LK(cudaMemcpyAsync(h, stat, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));

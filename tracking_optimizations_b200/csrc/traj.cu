@@ -283,8 +283,7 @@ int sort_rows(const int64_t* h_ids, int64_t n, TrajMem& M, cudaStream_t st, int 
     id_range_kernel<<<grid, 256, 0, st>>>(ids, n, lohi);
     TK(cudaGetLastError());
     unsigned long long h[2];
-    TK(cudaMemcpyAsync(h, lohi, sizeof(h), cudaMemcpyDeviceToHost, st));
-    TK(cudaStreamSynchronize(st));
+    TK(M.hc->download(h, lohi, sizeof(h), st));
     out->idmin = (long long)h[0];
     const long long idmax = (long long)h[1];
     if (idmax - out->idmin >= (1LL << 31) || idmax < out->idmin) {
@@ -324,9 +323,12 @@ int find_groups(const Sorted& S, int64_t n, TrajMem& M, cudaStream_t st, int gri
     gstart_kernel<<<grid, 256, 0, st>>>(S.keys, n, *gid, *gstart);
     TK(cudaGetLastError());
     if (total) {
-        TK(cudaMemcpyAsync(&total[0], *gid + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-        TK(cudaMemcpyAsync(&total[1], heads + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        int64_t* h = M.hc->staged(total);
+        TK(cudaMemcpyAsync(&h[0], *gid + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        TK(cudaMemcpyAsync(&h[1], heads + n - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         TK(cudaStreamSynchronize(st));
+        total[0] = h[0];
+        total[1] = h[1];
     }
     return GT_OK;
 }
@@ -350,10 +352,9 @@ int traj_filter_stubs(const int64_t* h_ids, int64_t n, int64_t threshold, uint8_
     stubs_kernel<<<grid, 256, 0, st>>>(S.keys, n, gid, gstart, threshold, keep, count, cnt);
     TK(cudaGetLastError());
     unsigned long long hk = 0;
-    TK(cudaMemcpyAsync(&hk, cnt, sizeof(hk), cudaMemcpyDeviceToHost, st));
+    TK(M.hc->download(&hk, cnt, sizeof(hk), st));
     TK(M.hc->download(h_keep, keep, n, st));
     if (h_count) TK(M.hc->download(h_count, count, sizeof(int64_t) * n, st));
-    TK(cudaStreamSynchronize(st));
     *nkept = (int64_t)hk;
     return GT_OK;
 }
@@ -428,13 +429,15 @@ int traj_imsd(const int64_t* h_ids, const int64_t* h_frames, const float* h_x, c
     TK(cub::DeviceScan::ExclusiveSum(t, tmp, gspan, gbase, (int)G1, st));
     TK(cub::DeviceScan::ExclusiveSum(t, tmp, glags, gout, (int)G1, st));
     TK(cub::DeviceScan::ExclusiveSum(t, tmp, gchunks, cstart, (int)G1, st));
-    int64_t tot_span = 0, tot_out = 0, nchunks = 0;
-    unsigned long long hs[3] = {0, 0, 0};
-    TK(cudaMemcpyAsync(&tot_span, gbase + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    TK(cudaMemcpyAsync(&tot_out, gout + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    TK(cudaMemcpyAsync(&nchunks, cstart + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    TK(cudaMemcpyAsync(hs, stat, sizeof(hs), cudaMemcpyDeviceToHost, st));
+    int64_t words[6];
+    int64_t* h = M.hc->staged(words);
+    TK(cudaMemcpyAsync(&h[0], gbase + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    TK(cudaMemcpyAsync(&h[1], gout + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    TK(cudaMemcpyAsync(&h[2], cstart + G, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    TK(cudaMemcpyAsync(&h[3], stat, 3 * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     TK(cudaStreamSynchronize(st));
+    const int64_t tot_span = h[0], tot_out = h[1], nchunks = h[2];
+    unsigned long long hs[3] = {(unsigned long long)h[3], (unsigned long long)h[4], (unsigned long long)h[5]};
     if (hs[0]) {
         *msg = "a particle spans more than 2^31 frames";
         return GT_ERR_ARG;
@@ -480,8 +483,7 @@ int traj_imsd(const int64_t* h_ids, const int64_t* h_frames, const float* h_x, c
                                                tab, stat + 2);
         TK(cudaGetLastError());
     }
-    TK(cudaMemcpyAsync(hs, stat, sizeof(hs), cudaMemcpyDeviceToHost, st));
-    TK(cudaStreamSynchronize(st));
+    TK(M.hc->download(hs, stat, sizeof(hs), st));
     if (hs[0]) {
         *msg = "more than one position for a particle in one frame (one trajectory per particle expected)";
         return GT_ERR_ARG;
