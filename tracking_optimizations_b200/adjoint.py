@@ -150,8 +150,8 @@ class RefineAtPeaks(torch.autograd.Function):
         st = lib.gt_adjoint_backward(gctx, _ptr(frames), T, H, W, ctypes.byref(ctx.p), _ptr(walk), n, _ptr(g),
                                      _ptr(grad_frames), _ptr(grad_par), _stream())
         _native.check(st, gctx)
-        gs = grad_par[0].to(ctx.params_dtype[0])
-        gk = grad_par[1].to(ctx.params_dtype[1])
+        gs = grad_par[0].to(ctx.params_dtype[0]) if ctx.needs_input_grad[1] else None
+        gk = grad_par[1].to(ctx.params_dtype[1]) if ctx.needs_input_grad[2] else None
         return grad_frames, gs, gk, None, None
 
 
@@ -169,8 +169,10 @@ def refine(frames, walk, diameter, noise_size=None, smoothing_size=None, **param
         float(diameter if smoothing_size is None else smoothing_size), dtype=torch.float64)
     opts = dict(params)
     opts["diameter"] = diameter
-    return RefineAtPeaks.apply(frames, ns.to(dev) if ns.device != dev else ns,
-                               ks.to(dev) if ks.device != dev else ks, walk, opts)
+    # values without a gradient stay where they are: on the host they cost the
+    # call no copy and no wait to be read
+    ns, ks = (v.to(dev) if v.requires_grad and v.device != dev else v for v in (ns, ks))
+    return RefineAtPeaks.apply(frames, ns, ks, walk, opts)
 
 
 def uncertainty(frames, walk, diameter, gain=1.0, read_noise=0.0, **params):

@@ -1505,8 +1505,7 @@ int adjoint_work(gt_ctx* ctx, const AdjParams& ap, const std::vector<int>& circ,
 
 int adjoint_finish(gt_ctx* ctx, const AdjWork& aw, cudaStream_t st) {
     int herr = 0;
-    CK(cudaMemcpyAsync(&herr, aw.err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CK(ctx->hc.download(&herr, aw.err, sizeof(int), st));
     if (herr) {
         ctx->err = "a walk record lies outside the frames";
         return GT_ERR_ARG;
