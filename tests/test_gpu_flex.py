@@ -58,6 +58,24 @@ def test_shapes(gpu, H, W, dtype):
         np.testing.assert_array_equal(got, want)
 
 
+# instances whose tiles are shorter than 64 rows: a frame of one row less and more than a tile or two, runs of tiles
+@pytest.mark.parametrize("dtype,d,rows", [("u16", 11, 56), ("u16", 13, 56), ("u16", 15, 40), ("f32", 9, 48),
+                                          ("f32", 11, 48), ("f32", 13, 48)])
+def test_tile_rows(gpu, dtype, d, rows):
+    from tracking_optimizations_b200 import _native
+
+    for H in (rows - 1, rows, rows + 1, 2 * rows - 1, 2 * rows + 1, 3 * rows + 7):
+        m = _movie(3, H, 136, d + H, dtype)
+        got, want = _both(m, diameter=d, cpu_processed=True, characterize=True)
+        np.testing.assert_array_equal(got, want)
+        _native.set_option("locate_tiles_per_cta", 4)
+        try:
+            got, _ = _both(m, diameter=d, cpu_processed=True)
+        finally:
+            _native.set_option("locate_tiles_per_cta", 0)
+        np.testing.assert_array_equal(got[:, :7], want[:, :7])
+
+
 @pytest.mark.parametrize("d", [5, 9, 15])
 def test_non_finite_pixels(gpu, d):
     m = _movie(4, 140, 160, d, "f32")

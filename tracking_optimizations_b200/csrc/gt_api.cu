@@ -45,6 +45,7 @@ cudaError_t launch_assemble(const AsmArgs& a, int num_sms, cudaStream_t st);
 __global__ void grid_kernel(const float* py, const float* px, const int* npart, int cap_p, int G,
                             int ncy, int ncx, int* gstart, int* gidx, float2* gpos);
 int fast_supported(int kr, int dd, int rc, int diameter, int dtype);
+int fast_rows(int kr, int dd, int rc, int dtype, int th);
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, const TileSource& src, int frame0, int* used_tma);
 cudaError_t launch_repack(const void* frames, int dtype, int frame0, int nf, int H, int W, int pitch, void* out,
@@ -349,7 +350,7 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     lp.n_gchar = (int)P.gchar_tab.size() / 2;
     if (want_fast) {
         P.fast = want_fast;
-        P.fast_th = want_fast == 2 ? 64 : fast_tile_rows;
+        P.fast_th = fast_rows(lp.krad, lp.D, lp.rint_c, dtype, fast_tile_rows);
         lp.TH = P.fast_th;
         lp.TW = 64;
         lp.ntx = (W + lp.TW - 1) / lp.TW;

@@ -14,7 +14,7 @@
 // size is a run-time value of at most DD (and at least FM): the tile is laid
 // out for DD, and the two maxima over the window have one loop over its core.
 // COLS names the columns that the records carry.
-// Float frames add their boxcars in tap order (their sums round).  A CTA (256 or 512 threads) takes a
+// Float frames add their boxcars in tap order (their sums round).  A CTA (8 threads a tile row) takes a
 // run of consecutive TH0 x 64 output tiles; per tile:
 //   0. the uint16 tile plus halo is staged by one TMA load (zero fill
 //      outside the frame) into U[RH][US] (US >= RW: rows padded so that
@@ -58,11 +58,10 @@ namespace gt {
 
 namespace {
 constexpr int FT = 64;    // output tile width
-constexpr int FNT = 256;  // threads of a 32-row tile
 
-// 8 warps per 32 output rows: 64-row tiles (less halo recomputed per
-// output row) keep 16 warps per SM slot at 2 CTAs per SM
-__host__ __device__ constexpr int fast_threads(int th) { return th == 32 ? FNT : 2 * FNT; }
+// A thread per 8 output pixels (256 for 32 rows, 512 for 64): 64-row tiles (less
+// halo recomputed per output row) keep 16 warps per SM slot at 2 CTAs per SM
+__host__ __device__ constexpr int fast_threads(int th) { return th * (FT / 8); }
 constexpr int FM = 8;     // outputs per thread item
 // Columns of the records: position and mass; the cpu_processed columns; the
 // characterize columns, with or without those.  An instance each: the code of
@@ -112,7 +111,7 @@ struct Geo {
     static constexpr int NPW = (PW + FM - 1) / FM;
     static constexpr int PWC = FM * NPW;
     // column pass: an item covers HC runs of FM / 2 row pairs of a column
-    static constexpr int HC = TH0 == 64 ? 2 : 1;
+    static constexpr int HC = TH0 == 32 ? 1 : 2;
     static constexpr int NRQ = (PP + HC * (FM / 2) - 1) / (HC * (FM / 2));  // items per column
     static constexpr int GPS = PWC | 1;
     static constexpr int P2S = PW | 1;
@@ -164,6 +163,22 @@ struct Geo {
     static_assert(RC + 2 <= HP && RC <= HX, "walk and feature circles inside the processed region");
     static_assert(NTK / 32 > 2 * NWO, "stencil warps besides the walkers");
 };
+
+// Tile rows of an instance, where the caller asks for 64: as many as let two CTAs
+// share an SM.  Alone on its SM a CTA leaves every barrier between its phases
+// unhidden, which costs more than the halo of the shorter tile: 64 rows alone
+// and two of fewer, 200 float frames of 524 x 800, diameter 9, 0.929 and 0.762 ms
+// (48 rows); 12 frames of 2048 x 2560, diameter 11, characterize, 0.825 and 0.707
+// (56); 100 frames of 512 x 512, diameter 13, 0.342 and 0.295 (56); of 389 x 517,
+// diameter 15, 0.466 and 0.403 (40).  Float frames of diameter 13: 0.408 either way.
+template <int KR, int DD, int RC, class PX, bool RT>
+__host__ __device__ constexpr int tile_rows() {
+    return Geo<KR, DD, 64, RC, PX, RT>::CTAS > 1   ? 64
+           : Geo<KR, DD, 56, RC, PX, RT>::CTAS > 1 ? 56
+           : Geo<KR, DD, 48, RC, PX, RT>::CTAS > 1 ? 48
+           : Geo<KR, DD, 40, RC, PX, RT>::CTAS > 1 ? 40
+                                                   : 64;
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);

@@ -6,7 +6,7 @@
 namespace gt {
 
 namespace {
-// (radius, dilation size of separation = diameter + 1); tiles of 64 rows
+// (radius, dilation size of separation = diameter + 1)
 #define GT_FLEX_LIST(X) X(2, 8) X(3, 11) X(4, 14) X(5, 16) X(6, 19) X(7, 22)
 }  // namespace
 
@@ -19,13 +19,23 @@ int flex_dilation(int rc, int dtype) {
     return 0;
 }
 
+int flex_rows(int rc, int dtype) {
+#define GT_FLEX_CASE(R, DD) \
+    if (rc == R) return dtype == 0 ? tile_rows<R, DD, R, unsigned short, true>() : tile_rows<R, DD, R, float, true>();
+    GT_FLEX_LIST(GT_FLEX_CASE)
+#undef GT_FLEX_CASE
+    return 64;
+}
+
 cudaError_t launch_locate_flex(int kr, int rc, int dtype, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, const TileSource& src, int frame0, int* used_tma) {
     if (kr != rc || p.D < FM || p.D > flex_dilation(rc, dtype)) return cudaErrorInvalidValue;
 #define GT_FLEX_CASE(R, DD)                                                                                   \
     if (rc == R)                                                                                              \
-        return dtype == 0 ? launch_instance<R, DD, 64, R, unsigned short, true>(grid, st, p, b, src, frame0, used_tma) \
-                          : launch_instance<R, DD, 64, R, float, true>(grid, st, p, b, src, frame0, used_tma);
+        return dtype == 0 ? launch_instance<R, DD, tile_rows<R, DD, R, unsigned short, true>(), R, unsigned short, \
+                                            true>(grid, st, p, b, src, frame0, used_tma)                       \
+                          : launch_instance<R, DD, tile_rows<R, DD, R, float, true>(), R, float, true>(        \
+                                grid, st, p, b, src, frame0, used_tma);
     GT_FLEX_LIST(GT_FLEX_CASE)
 #undef GT_FLEX_CASE
     return cudaErrorInvalidValue;

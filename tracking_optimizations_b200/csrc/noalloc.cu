@@ -34,6 +34,7 @@ cudaError_t launch_finalize(const LocParams& p, const MovieBufs& b, float sep, i
 __global__ void scan_frames_kernel(const int* in, int* out, int n);
 cudaError_t launch_assemble(const AsmArgs& a, int num_sms, cudaStream_t st);
 int fast_supported(int kr, int dd, int rc, int diameter, int dtype);
+int fast_rows(int kr, int dd, int rc, int dtype, int th);
 cudaError_t launch_locate_fast(int kr, int dd, int rc, int th, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, const TileSource& src, int frame0, int* used_tma);
 void gauss_taps(int smoothing_size, float noise_size, int normalized, float* w, float* norm, float* rn);
@@ -226,7 +227,7 @@ extern "C" int gt_locate_frame_static(const void* d_frame, int dtype, int H, int
     const int n_bg = bg ? annulus_f(pr->bg_radius, pr->sig_radius + gap, bg_off) : 0;
 
     const bool fast = fast_supported(lp.krad, lp.D, lp.rint_c, lp.d, dtype) != 0;
-    const int th = fast ? 64 : 32;
+    const int th = fast ? fast_rows(lp.krad, lp.D, lp.rint_c, dtype, 64) : 32;
     lp.TH = th;
     lp.TW = 64;
     lp.ntx = (W + 63) / 64;
