@@ -808,14 +808,13 @@ __device__ __forceinline__ void flush_seeds(const LinkBufs& L, SeedBuf& sb, int 
     __shared__ int s_base;
     __syncthreads();
     const int n = min(sb.n, SEED_BUF);
-    if (n > 0) {
-        if (threadIdx.x == 0) s_base = atomicAdd(L.ctr + (k & 3) * 4, n);
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += NTL) L.seedq[s_base + i] = sb.h[i];
-        __syncthreads();
-        if (threadIdx.x == 0) sb.n = 0;
-        __syncthreads();
-    }
+    if (threadIdx.x == 0 && n > 0) s_base = atomicAdd(L.ctr + (k & 3) * 4, n);
+    // every thread has read the count: the next movie's seeds may come in
+    __syncthreads();
+    if (n == 0) return;
+    for (int i = threadIdx.x; i < n; i += NTL) L.seedq[s_base + i] = sb.h[i];
+    if (threadIdx.x == 0) sb.n = 0;
+    __syncthreads();
 }
 
 // Sets the bits `wm` of word w of the lanes' particles' membership (particle
