@@ -510,8 +510,9 @@ __global__ void __launch_bounds__(TR_NT) adjoint_transpose_kernel(AdjParams p, A
                 if (g != 0.f && r >= 0 && r < SH && x >= 0 && x < SW) atomicAdd(&at(S, SS, r, x), g);
             }
         }
+        const int rest = s_entry;  // read by all before thread 0 writes the next one
         __syncthreads();
-        if (s_entry == 0) break;
+        if (rest == 0) break;
         if (threadIdx.x == 0) {
             int entry = s_entry, q = 0;
             for (; entry > 0 && q < LIST; entry = __ldg(tl.next + entry - 1)) s_list[q++] = (entry - 1) / tl.slots;
