@@ -42,3 +42,32 @@ def test_seeds_of_many_linked_movies(gpu, n):
         assert stats["link_iterations"] > 2
         for (table, _), w in zip(got, want):
             np.testing.assert_array_equal(table.cpu().numpy(), w)
+
+
+@pytest.mark.parametrize("short", [0, 1])
+def test_tile_rows_timed_in_the_movies_workspace(gpu, short):
+    """Frame sizes that no call has timed yet, rows of no whole 16 bytes among
+    them, with the usual and with short capacities: the timing runs stay inside
+    the movies' workspaces (the linker's tables lie behind them), and a movie
+    with more features than the short capacities hold is rerun."""
+    import torch
+
+    from tracking_optimizations_b200 import _native, batched
+
+    g = torch.Generator(device="cuda").manual_seed(3)
+    crowded = (torch.rand((2, 700, 700 + 3 * short), device="cuda", generator=g) * 200).to(torch.int16)
+    movies = [(_movie(20, 600, 601 + 2 * short, 700, 1), dict(diameter=7, search_range=4.0, memory=1, cpu_processed=True)),
+              (_movie(40, 203 + short, 205, 60, 2), dict(diameter=5, search_range=4.0, memory=3)),
+              (crowded, dict(diameter=5)),
+              (_movie(9, 160 + 16 * short, 320, 60, 3), dict(diameter=9, search_range=4.0))]
+    want = _each(movies)
+    outs = [torch.empty((len(w) + 5, w.shape[1]), device="cuda") for w in want]
+    _native.set_option("test_short_memory", short)
+    try:
+        for turn in range(3):
+            got, stats = batched.batch_many(movies, outs=outs, return_stats=True)
+            for (table, _), w in zip(got, want):
+                np.testing.assert_array_equal(table.cpu().numpy(), w)
+    finally:
+        _native.set_option("test_short_memory", 0)
+    assert stats["batch_fallbacks"] >= short

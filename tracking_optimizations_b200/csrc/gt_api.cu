@@ -130,6 +130,7 @@ struct gt_ctx {
     size_t h_status_n = 0;
     int tune_disabled = 0;
     int batch_cap_div = 64;           // first candidate capacity of batched movies: H*W / this
+    int short_memory = 0;             // test switch: batches start with the capacities of short memory
     cudaStream_t copy_stream = nullptr;  // host->device frame chunks
     HostCopy hc;                         // pageable host arrays
     TrajMem traj;                        // scratch of the trajectory calls
@@ -307,6 +308,15 @@ void link_scratch(Plan* pl, int scale) {
     P.big_e = (int)std::min<long long>(32768LL * scale, (long long)P.big_d * P.big_s);
 }
 
+// The specialised locate kernel's tile height, 32 or fast_rows: nothing in the
+// workspace depends on it.
+void set_tile_rows(Plan* pl, int rows) {
+    LocParams& lp = pl->lp;
+    pl->fast_th = fast_rows(lp.krad, lp.D, lp.rint_c, pl->dtype, rows);
+    lp.TH = pl->fast_th;
+    lp.nty = (lp.H + lp.TH - 1) / lp.TH;
+}
+
 int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int num_sms, Plan* pl,
               std::string* msg, int force_generic_flag = 0, int fast_tile_rows = 32, int cap_div = 64) {
     Plan& P = *pl;
@@ -350,11 +360,9 @@ int make_plan(const Resolved& r, int T, int H, int W, int dtype, int scale, int 
     lp.n_gchar = (int)P.gchar_tab.size() / 2;
     if (want_fast) {
         P.fast = want_fast;
-        P.fast_th = fast_rows(lp.krad, lp.D, lp.rint_c, dtype, fast_tile_rows);
-        lp.TH = P.fast_th;
         lp.TW = 64;
         lp.ntx = (W + lp.TW - 1) / lp.TW;
-        lp.nty = (H + lp.TH - 1) / lp.TH;
+        set_tile_rows(&P, fast_tile_rows);
         // widths that the tile copies can't take: chunks of frames with padded
         // rows, small enough to be read back from L2
         const int px = dtype == GT_U16 ? 2 : 4, vp = 16 / px;
@@ -1029,9 +1037,8 @@ int tune_tile_rows(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t
         float ms[2] = {0.f, 0.f};
         const int ths[2] = {32, 64};
         for (int v = 0; v < 2; ++v) {
-            Plan Q;
-            std::string msg;
-            if (make_plan(P.r, P.T, P.H, P.W, P.dtype, 1, ctx->num_sms, &Q, &msg, 0, ths[v])) return GT_ERR_ARG;
+            Plan Q = P;  // the workspace is carved for P's capacities
+            set_tile_rows(&Q, ths[v]);
             MovieBufs b = movie_bufs(Q, bm.w, frames);
             for (int rep = 0; rep < 2; ++rep) {
                 CK(cudaMemsetAsync(bm.w.status, 0, sizeof(int) * (STATUS_INTS + (size_t)P.T), st));
@@ -1047,16 +1054,7 @@ int tune_tile_rows(gt_ctx* ctx, BatchMovie& bm, const void* frames, cudaStream_t
         best = ms[1] < ms[0] ? 64 : 32;
         ctx->tile_rows[key] = best;
     }
-    if (best != P.fast_th) {
-        Plan Q;
-        std::string msg;
-        if (make_plan(P.r, P.T, P.H, P.W, P.dtype, 1, ctx->num_sms, &Q, &msg, 0, best)) return GT_ERR_ARG;
-        Work w2{};
-        Plan Qc = Q, Pc = P;
-        Qc.nslot = 0;
-        Pc.nslot = 0;
-        if (carve(Qc, nullptr, &w2, 0, true, false) == carve(Pc, nullptr, &w2, 0, true, false)) P = Q;
-    }
+    set_tile_rows(&P, best);
     return GT_OK;
 }
 
@@ -1255,9 +1253,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         if (need > avail - avail / 8) {
             if (ctx->batch_cap_div < 1024) {
                 ctx->batch_cap_div *= 4;
-                const int rc2 = batch_many(ctx, mv, n, st);
-                ctx->batch_cap_div = 64;
-                return rc2;
+                return batch_many(ctx, mv, n, st);
             }
             ctx->err = "the batch does not fit in device memory; split it";
             return GT_ERR_OOM;
@@ -1831,6 +1827,7 @@ int gt_adjoint_uncertainty(gt_ctx* ctx, const float* d_frames, int T, int H, int
 
 int gt_batch_many_device(gt_ctx* ctx, gt_movie* movies, int n, void* stream) {
     cudaStream_t st = call_stream(ctx, stream);
+    if (ctx) ctx->batch_cap_div = ctx->short_memory ? 256 : 64;
     return batch_many(ctx, movies, n, st);
 }
 
@@ -1843,6 +1840,7 @@ int gt_ctx_set_option(gt_ctx* ctx, const char* key, int value) {
     if (k == "subnet_budget" && value > 0) { ctx->subnet_budget = value; return GT_OK; }
     if (k == "subnet_budget" && value == 0) { ctx->subnet_budget = SUBNET_BUDGET; return GT_OK; }
     if (k == "test_withhold_tile_copy" && (value == 0 || value == 1)) { ctx->withhold_tma = value; return GT_OK; }
+    if (k == "test_short_memory" && (value == 0 || value == 1)) { ctx->short_memory = value; return GT_OK; }
     if (k == "locate_tiles_per_cta" && value >= 0 && value <= 64) {
         ctx->tiles_per_cta = value;
         if (ctx->batch_exec) {  // the cached batch graph holds the old launch shape
