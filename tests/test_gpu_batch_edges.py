@@ -71,3 +71,36 @@ def test_tile_rows_timed_in_the_movies_workspace(gpu, short):
     finally:
         _native.set_option("test_short_memory", 0)
     assert stats["batch_fallbacks"] >= short
+
+
+def test_larger_batch_refused_between_replays(gpu):
+    """A batch of more movies that does not fit in device memory takes larger
+    status words before it is refused; the batch before it then runs again
+    into those."""
+    import ctypes
+
+    from tracking_optimizations_b200 import _native, batched
+
+    movies = [(_movie(8, 96, 96, 30, s), dict(diameter=7, search_range=4.0, memory=1)) for s in range(2)]
+    want = _each(movies)
+    outs = batched.output_buffers(movies)
+
+    def turn():
+        for o in outs:
+            o.fill_(-1.0)
+        got, stats = batched.batch_many(movies, outs=outs, return_stats=True)
+        for (table, _), w in zip(got, want):
+            np.testing.assert_array_equal(table.cpu().numpy(), w)
+        return stats["batch_graph"]
+
+    modes = [turn(), turn()]
+    many = (_native.GtMovie * 400)()
+    for m in many:  # frames that nothing reads: the plan alone is too large
+        m.frames, m.dtype = movies[0][0].data_ptr(), _native.GT_U16
+        m.T, m.H, m.W = 100000, 1024, 1024
+        m.params = _native.make_params(7)
+        m.out, m.out_rows = outs[0].data_ptr(), 0
+    ctx = _native.context(0)
+    st = _native.load().gt_batch_many_device(ctx, many, len(many), None)
+    assert st == _native.GT_ERR_OOM, _native.load().gt_last_error(ctx)
+    assert modes + [turn(), turn()] == [1, 2, 1, 2]

@@ -1152,6 +1152,12 @@ int enqueue_batch(gt_ctx* ctx, std::vector<BatchMovie>& B, gt_movie* mv, int n, 
     return GT_OK;
 }
 
+void drop_batch_graph(gt_ctx* ctx) {
+    if (ctx->batch_exec) cudaGraphExecDestroy(ctx->batch_exec);
+    ctx->batch_exec = nullptr;
+    ctx->batch_key.clear();
+}
+
 int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
     if (!ctx) return GT_ERR_ARG;
     ctx->err.clear();
@@ -1192,6 +1198,7 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
     }
     // pinned status words, side streams, events
     if (ctx->h_status_n < (size_t)8 * n) {
+        drop_batch_graph(ctx);  // it reads back into the old words
         if (ctx->h_status) cudaFreeHost(ctx->h_status);
         ctx->h_status = nullptr;
         ctx->h_status_n = 0;
@@ -1843,20 +1850,12 @@ int gt_ctx_set_option(gt_ctx* ctx, const char* key, int value) {
     if (k == "test_short_memory" && (value == 0 || value == 1)) { ctx->short_memory = value; return GT_OK; }
     if (k == "locate_tiles_per_cta" && value >= 0 && value <= 64) {
         ctx->tiles_per_cta = value;
-        if (ctx->batch_exec) {  // the cached batch graph holds the old launch shape
-            cudaGraphExecDestroy(ctx->batch_exec);
-            ctx->batch_exec = nullptr;
-            ctx->batch_key.clear();
-        }
+        drop_batch_graph(ctx);  // it holds the old launch shape
         return GT_OK;
     }
     if (k == "normalized_taps" && (value == 0 || value == 1)) {
         ctx->normalized_taps = value;
-        if (ctx->batch_exec) {  // the cached batch graph holds the old taps
-            cudaGraphExecDestroy(ctx->batch_exec);
-            ctx->batch_exec = nullptr;
-            ctx->batch_key.clear();
-        }
+        drop_batch_graph(ctx);  // it holds the old taps
         return GT_OK;
     }
     ctx->err = "unknown option or value: " + k;
