@@ -126,8 +126,9 @@ GT_API int gt_batch(gt_ctx* ctx, const void* frames, int dtype, int T, int H, in
  * buffer `d_out` (capacity out_rows x ncols floats); *nrows receives the row
  * count (rows beyond out_rows are not written, *nrows still reports them).
  * `stream` is a cudaStream_t (NULL = the context's stream, after the work
- * that the legacy default stream holds); the call returns after the work on
- * it has finished. */
+ * that the legacy default stream holds, unless a stream that synchronises
+ * with that one is being captured); the call returns after the work on it
+ * has finished. */
 GT_API int gt_batch_device(gt_ctx* ctx, const void* d_frames, int dtype, int T, int H, int W,
                     const gt_params* params, float* d_out, int64_t out_rows,
                     int64_t* nrows, void* stream);

@@ -1525,11 +1525,15 @@ namespace {
 // memory of its outputs.
 cudaStream_t call_stream(gt_ctx* ctx, void* stream) {
     if (stream || !ctx) return (cudaStream_t)stream;
-    if (cudaSetDevice(ctx->device) != cudaSuccess ||
+    // While a stream that synchronises with the default stream is captured, a
+    // record there would end the capture: the query does not, and the call runs
+    // without the wait.
+    cudaStreamCaptureStatus cap;
+    if (cudaSetDevice(ctx->device) != cudaSuccess || cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess ||
         (!ctx->lev && cudaEventCreateWithFlags(&ctx->lev, cudaEventDisableTiming) != cudaSuccess) ||
         cudaEventRecord(ctx->lev, cudaStreamLegacy) != cudaSuccess ||
         cudaStreamWaitEvent(ctx->stream, ctx->lev, 0) != cudaSuccess)
-        cudaGetLastError();  // another stream is being captured: as without the wait
+        cudaGetLastError();
     return ctx->stream;
 }
 
