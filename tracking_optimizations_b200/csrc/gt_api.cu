@@ -150,7 +150,7 @@ constexpr int FB_WIN_MAX = 100;
 constexpr long long REPACK_BYTES = 64LL << 20;
 constexpr long long SUBNET_BUDGET = 1LL << 26;  // option trials per subnet
 constexpr int LINK_WINDOWS = 16;  // upload chunks of the host-frames path, at most
-constexpr int STATUS_LSTAT = 8 + LINK_WINDOWS, STATUS_INTS = STATUS_LSTAT + 2 * (12 + 8);
+constexpr int STATUS_LSTAT = 8 + LINK_WINDOWS, STATUS_INTS = STATUS_LSTAT + 2 * 12 + 4 * NCTR;
 constexpr int LINK_RUNS = 4;      // linker launches over them, at most
 
 struct Resolved {
@@ -248,7 +248,7 @@ struct Plan {
     int cap_c = 0, cap_p = 0;
     int G = 8, ncx = 1, ncy = 1;      // separation grid
     int LG = 8, lncx = 1, lncy = 1;  // linker's grid
-    // linker scratch for components beyond a thread's own arrays
+    // linker scratch for components beyond a block's own arrays
     int nslot = 0, big_d = 1, big_s = 1, big_e = 1;
     size_t smem_loc = 0, smem_fin = 0;
     int fb_win = 0;
@@ -294,18 +294,23 @@ void annulus_inds_f(float outer, float inner, std::vector<int>& off) {
         }
 }
 
-size_t big_ints(const Plan& P) { return 8 * (size_t)P.big_d + 1 + 3 * (size_t)P.big_s + 5 * (size_t)P.big_e; }
+size_t big_ints(const Plan& P) { return comp_bytes(P.big_d, P.big_s, P.big_e, sizeof(int)) / sizeof(int); }
 
-// Scratch slots of the linker's large components: room for 4096
-// destinations, 8192 sources and 32768 edges each (a component that the
-// search budget lets finish is far smaller), four times more per capacity
-// retry.
+// Scratch slots of the linker's largest components, a block's each: as many as
+// fit 256 MB, 64 at least and a block's on every SM four times over at most.
+int big_slots(const Plan& P) {
+    return (int)std::max<size_t>(64, std::min<size_t>(4 * 148, ((size_t)64 << 20) / big_ints(P)));
+}
+
+// Their sizes: room for 4096 destinations, 8192 sources and 32768 edges (a
+// component that the search budget lets finish is far smaller), four times
+// more per capacity retry.
 void link_scratch(Plan* pl, int scale) {
     Plan& P = *pl;
-    P.nslot = P.link ? 64 : 0;
     P.big_d = (int)std::min<long long>(4096LL * scale, P.cap_p);
     P.big_s = (int)std::min<long long>(8192LL * scale, (long long)P.cap_p * (P.r.memory + 1));
     P.big_e = (int)std::min<long long>(32768LL * scale, (long long)P.big_d * P.big_s);
+    P.nslot = P.link ? big_slots(P) : 0;
 }
 
 // The specialised locate kernel's tile height, 32 or fast_rows: nothing in the
@@ -437,7 +442,7 @@ struct Work {
     unsigned *lnk, *mm, *pres;
     int *stamp, *rstamp, *seedq, *recq, *deferq, *gframe, *cstamp, *head, *fstamp, *big;
     int4* ent;
-    unsigned long long* lstat;  // 4 phase times, 8 frame counts, then the linker's counters (16 ints)
+    unsigned long long* lstat;  // 4 phase times, 8 frame counts, then the linker's counters
     float* out;
 };
 
@@ -510,7 +515,7 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->mm = c.take<unsigned>(nm * nw);
     w->stamp = c.take<int>(nm);
     w->rstamp = c.take<int>(nm);
-    w->seedq = c.take<int>(nm);
+    w->seedq = c.take<int>(np);
     w->recq = c.take<int>(nm);
     w->deferq = c.take<int>(np);
     w->gframe = c.take<int>(nl);
@@ -596,7 +601,7 @@ int link_window(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st, int 
     const int rc = link_grid(ctx, 0, &grid);
     if (rc) return rc;
     // the pass counters start at zero (the statistics add up over windows)
-    if (tb > 0) CK(cudaMemsetAsync(w.lstat + 12, 0, sizeof(unsigned long long) * 8, st));
+    if (tb > 0) CK(cudaMemsetAsync(w.lstat + 12, 0, sizeof(int) * 4 * NCTR, st));
     CK(launch_link(L, te - tb + 1, w.err + 1, w.lstat, grid, st));
     ctx->stats.launches += 1;
     return GT_OK;
@@ -1224,10 +1229,10 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         if (!P.link) continue;
         B[i].link_slot = S.nlink++;
         S.max_passes = std::max(S.max_passes, P.T + 1);
-        big.nslot = std::max(big.nslot, P.nslot);
         big.big_d = std::max(big.big_d, P.big_d);
         big.big_s = std::max(big.big_s, P.big_s);
         big.big_e = std::max(big.big_e, P.big_e);
+        big.nslot = big_slots(big);
     }
     // arena layout: movies, link pool, shared arrays
     size_t total = 0;

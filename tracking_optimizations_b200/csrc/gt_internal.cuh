@@ -120,6 +120,29 @@ struct MovieBufs {
     int* done;            // blocks of finalize_kernel that are done (0: not counted, null: no offsets)
 };
 
+// A component's arrays in memory for cd destinations, cs sources and ce edges,
+// with indices of `isz` bytes (link.cu, MemComp): the lists, then the hash
+// tables of the exploration, whose place the search's arrays take.
+__host__ __device__ constexpr int hash_size(int cap) {
+    int n = 64;
+    while (n < 2 * cap || n < cap + 33) n <<= 1;  // a warp's 32 keys may come on top of cap
+    return n;
+}
+__host__ __device__ constexpr size_t comp_lists(size_t cd, size_t cs, size_t ce, size_t isz) {
+    return (4 * (ce + cd + cs) + isz * (2 * ce + cd + 1) + 3) / 4 * 4;
+}
+__host__ __device__ constexpr size_t comp_bytes(int cd, int cs, int ce, size_t isz) {
+    const size_t search = 4 * (size_t)cs + isz * (6 * (size_t)cd + 2 * (size_t)cs);
+    const size_t hash = (4 + isz) * ((size_t)hash_size(cd) + hash_size(cs));
+    return comp_lists(cd, cs, ce, isz) + ((search > hash ? search : hash) + 3) / 4 * 4;
+}
+
+// The linker's counters, a set of NCTR per pass (4 sets in turn): seeds (of the
+// first linking: components beyond a thread's arrays), membership checks,
+// components beyond a warp's registers, frames, components beyond a block's
+// arrays, and those of them that are done.
+enum { C_SEEDS = 0, C_CHECKS = 1, C_MEM = 2, C_FRAMES = 3, C_SLOT = 4, C_DONE = 5, NCTR = 8 };
+
 struct LinkBufs {
     int T, cap_p, memory;
     int tb, te;           // frames linked by this launch; earlier frames are final
@@ -140,10 +163,10 @@ struct LinkBufs {
     unsigned* mm;         // word w, bit b: memory entry of the frame 2 + 32 w + b later
     int* stamp;           // last pass in which the particle was a seed
     int* rstamp;          // last pass that listed it for a membership check
-    int* seedq;           // slab handles of the pass's seeds
+    int* seedq;           // slab handles of the pass's seeds, np
     int* recq;            // particles whose linked bits the pass changed (memory 1, 2),
                           // or those of the trajectories that it changed
-    int* deferq;          // seeds whose component is resolved in scratch
+    int* deferq;          // seeds whose component is resolved in memory, np
     int* newrank;         // rank among new particles of its frame
     int* root;
     int* lroot;           // where the pred chain enters the particle's chunk
@@ -156,10 +179,10 @@ struct LinkBufs {
     unsigned* pres;       // as mm: the id is present in the frame 1 + 32 w + b later
     int* newcount;        // T
     int* fstamp;          // T: last pass with a seed in the frame
-    int* ctr;             // 4 passes x {seeds, membership checks, deferred, frames}
+    int* ctr;             // 4 passes x NCTR
     int* err;
     long long budget;     // branch-and-bound option trials per subnet
-    // scratch of the components beyond a thread's own arrays: nslot slots of
+    // scratch of the components beyond a block's own arrays: nslot slots of
     // big_ints for big_d destinations, big_s sources and big_e edges
     int nslot, big_d, big_s, big_e;
     size_t big_ints;

@@ -24,14 +24,18 @@
 //     or removing entries alters exactly the components that hold a
 //     destination in reach of one (every piece that a removed entry leaves
 //     behind was next to it), so those destinations are the pass's seeds;
-//   - a thread explores one seed's component through the frames' cell grids
-//     and resolves it; of the seeds of a component the smallest does it.
+//   - a warp (in the first linking a thread) explores one seed's component
+//     through the frames' cell grids and resolves it; of the seeds of a
+//     component the smallest does it.
 //     There is no per-frame state, so the work spreads over the whole grid
 //     whatever the frames' sizes.
 // Relinking whole frames instead, a block per changed frame with the graph in
 // shared memory, took 0.99 ms for that movie, 64 ms for 200 frames of 15k
 // particles with memory 3 and 9.2 ms for a table of 500 frames of 760.
 #include <cooperative_groups.h>
+
+#include <climits>
+#include <type_traits>
 
 #include "gt_device.cuh"
 
@@ -117,11 +121,18 @@ __device__ __forceinline__ int push_slot(int* ctr) {
 
 // One component: destinations (index in frame t), sources (keys that order
 // them as linking.rs:244-259 does: frame t-1 by index, then the memory
-// entries by (frame, index): cap_p + slab handle) and their edges.  At most 32
-// destinations and 32 sources fit a thread's local arrays (SmallComp, the first
-// linking) or a warp (WarpComp, the passes); larger components are resolved by
-// one thread per block with arrays in global memory (LinkBufs::big).
-constexpr int CAP_N = 32, CAP_E = 112;
+// entries by (frame, index): cap_p + slab handle) and their edges.  By size:
+//   8 destinations, 8 sources, 24 edges   a thread's local arrays (SmallComp),
+//                                         in the first linking;
+//   32, 32, 112                           a warp's registers (WarpComp), in the
+//                                         first linking and the passes;
+//   256, 256, 1024                        a warp with the block's arrays (MemComp);
+//   beyond                                a warp with a slot of LinkBufs::big.
+// A thread that goes on to 32 takes far longer than a warp: tables of 300 chains
+// of 31 particles 1.22 ms a call, 0.28 with the warps; and one thread of 64
+// blocks at a time for all that is larger 0.78 ms and more (4000 chains of 40:
+// 217 ms, 1.4 with the block's arrays; 300 of 400: 2.7).
+constexpr int CAP_T = 8, CAP_TE = 24, CAP_N = 32, CAP_E = 112;
 
 // Set of at most 32 sources or destinations.
 struct BitSet {
@@ -132,8 +143,9 @@ struct BitSet {
     __device__ void clear(int) { m = 0; }
 };
 
+template <class I>
 struct ArraySet {
-    int* p;
+    I* p;
     __device__ bool has(int i) const { return p[i] != 0; }
     __device__ void add(int i) { p[i] = 1; }
     __device__ void del(int i) { p[i] = 0; }
@@ -143,55 +155,92 @@ struct ArraySet {
 };
 
 struct SmallComp {
-    int D[CAP_N];
-    unsigned S[CAP_N];
-    float ew[CAP_E], dw[CAP_E];
-    unsigned char ed[CAP_E], es[CAP_E], dsrc[CAP_E];
-    unsigned char doff[CAP_N + 1], path[CAP_N], oi[CAP_N], stk[2 * CAP_N];
-    signed char cur[CAP_N], best[CAP_N];
-    __device__ int md() const { return CAP_N; }
-    __device__ int ms() const { return CAP_N; }
-    __device__ int me() const { return CAP_E; }
-    __device__ BitSet dset() { return BitSet(); }
+    int D[CAP_T];
+    unsigned S[CAP_T];
+    float ew[CAP_TE], dw[CAP_TE];
+    unsigned char ed[CAP_TE], es[CAP_TE], dsrc[CAP_TE];
+    unsigned char doff[CAP_T + 1], path[CAP_T], oi[CAP_T], stk[2 * CAP_T];
+    signed char cur[CAP_T], best[CAP_T];
     __device__ BitSet sset() { return BitSet(); }
 };
 
-struct BigComp {
+// Arrays for cd destinations, cs sources and ce edges (comp_bytes), in shared
+// memory (I: 16 bits) or in a slot of LinkBufs::big (I: int).
+template <class I>
+struct MemComp {
+    int cd, cs, ce;
+    float* dw;               // edges, grouped by destination in the order found
     int* D;
     unsigned* S;
-    float *ew, *dw;
-    int *ed, *es, *dsrc, *doff, *path, *oi, *used, *vis, *stk, *cur, *best;
-    int cd, cs, ce;
-    __device__ int md() const { return cd; }
-    __device__ int ms() const { return cs; }
-    __device__ int me() const { return ce; }
-    __device__ ArraySet dset() { return ArraySet{vis}; }
-    __device__ ArraySet sset() { return ArraySet{used}; }
+    I *dsrc, *list, *doff;   // source per edge; the sources' lists
+    int* soff;               // ends of the sources' lists
+    I *path, *oi, *stk, *used, *vis;
+    typename std::make_signed<I>::type *cur, *best;
+    char* hash;              // during the exploration, in the place of soff and the others
+    __device__ ArraySet<I> sset() const { return ArraySet<I>{used}; }
+
+    __device__ MemComp(void* mem, int cd_, int cs_, int ce_) : cd(cd_), cs(cs_), ce(ce_) {
+        dw = (float*)mem;
+        D = (int*)(dw + ce);
+        S = (unsigned*)(D + cd);
+        dsrc = (I*)(S + cs);
+        list = dsrc + ce;
+        doff = list + ce;
+        hash = (char*)mem + comp_lists(cd, cs, ce, sizeof(I));
+        soff = (int*)hash;
+        I* q = (I*)(soff + cs);
+        auto take = [&](int n) { I* r = q; q += n; return r; };
+        path = take(cd); oi = take(cd); stk = take(cd + cs); used = take(cs); vis = take(cd);
+        cur = (decltype(cur))take(cd); best = (decltype(best))take(cd);
+    }
 };
 
-__device__ __forceinline__ BigComp big_comp(const LinkBufs& L, int slot) {
-    BigComp b;
-    int* p = L.big + (size_t)slot * L.big_ints;
-    auto take = [&](int n) { int* q = p; p += n; return q; };
-    const int nd = L.big_d, ns = L.big_s, ne = L.big_e;
-    b.cd = nd; b.cs = ns; b.ce = ne;
-    b.D = take(nd); b.S = (unsigned*)take(ns);
-    b.ew = (float*)take(ne); b.dw = (float*)take(ne);
-    b.ed = take(ne); b.es = take(ne); b.dsrc = take(ne);
-    b.doff = take(nd + 1); b.path = take(nd); b.oi = take(nd); b.used = take(ns); b.vis = take(nd);
-    b.stk = take(nd + ns); b.cur = take(nd); b.best = take(nd);
-    return b;
-}
+// Keys and their numbers in the order of arrival: a warp's lanes put theirs in
+// side by side (a search among the arrived ones: 300 chains of 255 2.03 ms a
+// call instead of 1.27).
+constexpr unsigned NO_KEY = 0xffffffffu;
+template <class I>
+struct KeyTable {
+    unsigned* key;
+    I* val;
+    int size;  // a power of two
+    __device__ void clear() {
+        for (int i = threadIdx.x & 31; i < size; i += 32) key[i] = NO_KEY;
+    }
+    // The number of each key that is wanted: new ones from *n on, if cap holds
+    // them (else false).  Every lane calls it.
+    __device__ bool put(unsigned k, bool want, int cap, int* n, int* idx, bool* fresh) {
+        const unsigned full = 0xffffffffu;
+        unsigned h = (k * 2654435761u) >> (__clz(size) + 1);
+        bool is_new = false;
+        if (want)
+            while (true) {
+                const unsigned old = atomicCAS(key + h, NO_KEY, k);
+                is_new = old == NO_KEY;
+                if (is_new || old == k) break;
+                h = (h + 1) & (size - 1);
+            }
+        const unsigned news = __ballot_sync(full, is_new);
+        *fresh = is_new;
+        *idx = *n + __popc(news & ((1u << (threadIdx.x & 31)) - 1u));
+        if (*n + __popc(news) > cap) return false;
+        if (is_new) val[h] = (I)*idx;
+        __syncwarp();
+        if (want && !is_new) *idx = val[h];
+        *n += __popc(news);
+        return true;
+    }
+};
+
+// A component of the block's own arrays.
+constexpr int MID_N = 256, MID_E = 1024;
+constexpr int MID_BYTES = (int)comp_bytes(MID_N, MID_N, MID_E, 2);
 
 // DFS preorder of the destinations from `first` (linking.rs:316-342) over
 // the per-destination lists: neighbours in ascending order, so the next node
-// is the smallest one not yet visited.  Returns the number of destinations.
-template <class C>
-__device__ int dfs_order(C& c, int first, int nd, int ns, int ne) {
-    auto vis = c.dset();
-    auto used = c.sset();
-    vis.clear(nd);
-    used.clear(ns);
+// is the smallest one not yet visited.
+__device__ void dfs_order(SmallComp& c, int first, int nd, int ne) {
+    BitSet vis, used;
     int top = 1, np = 0;
     c.stk[0] = first;
     vis.add(first);
@@ -218,7 +267,43 @@ __device__ int dfs_order(C& c, int first, int nd, int ns, int ne) {
         if (next < 0) --top;
         else c.stk[top++] = next;
     }
-    return np;
+}
+
+// The same over the lists of both sides.
+template <class I>
+__device__ void dfs_order(const MemComp<I>& c, int first, int nd) {
+    int top = 1, np = 0;
+    c.stk[0] = (I)first;
+    c.vis[first] = 1;
+    c.path[np++] = (I)first;
+    while (top > 0) {
+        const int node = c.stk[top - 1];
+        int next = -1;
+        if (node < nd) {
+            const int z1 = c.doff[node + 1];
+            for (int z = c.doff[node]; z < z1 && next < 0; ++z)
+                if (!c.used[c.dsrc[z]]) next = c.dsrc[z];
+            if (next >= 0) {
+                c.used[next] = 1;
+                next += nd;
+            }
+        } else {
+            const int s = node - nd, z1 = c.soff[s];
+            int dn = 0;
+            for (int z = s > 0 ? c.soff[s - 1] : 0; z < z1; ++z) {
+                const int q = c.list[z];
+                if (c.vis[q]) continue;
+                const int dq = c.D[q];
+                if (next < 0 || dq < dn) { next = q; dn = dq; }
+            }
+            if (next >= 0) {
+                c.vis[next] = 1;
+                c.path[np++] = (I)next;
+            }
+        }
+        if (next < 0) --top;
+        else c.stk[top++] = (I)next;
+    }
 }
 
 // Exhaustive search of one subnet (linking.rs:390-452): destinations in DFS
@@ -298,7 +383,7 @@ __device__ __forceinline__ void mark_linked(const LinkBufs& L, int src, int fs, 
         if (set) atomicOr(L.lnk + src, 1u << j);
         else atomicAnd(L.lnk + src, ~(1u << j));
         if (k > 0 && L.memory <= 2 && atomicExch(L.rstamp + src, k) != k)
-            L.recq[push_slot(L.ctr + (k & 3) * 4 + 1)] = src;
+            L.recq[push_slot(L.ctr + (k & 3) * NCTR + C_CHECKS)] = src;
     }
 }
 
@@ -339,12 +424,11 @@ __device__ __forceinline__ void take_up(const LinkBufs& L, long long key, int g,
     if (src >= 0 && L.memory > 0) mark_linked(L, src, fs, t, k, true);
 }
 
-// Explores the component of destination d of frame t and resolves it.
-// k = 0: every destination is a seed and there are no memory entries.
+// Explores the component of destination d of frame t and resolves it, in the
+// first linking: every destination is a seed and there are no memory entries.
 // COMP_SKIP: a smaller seed of the same component does it; COMP_BIG: it does
 // not fit c (nothing is written).
-template <class C>
-__device__ int link_component(const LinkBufs& L, C& c, int t, int d, int k) {
+__device__ int link_component(const LinkBufs& L, SmallComp& c, int t, int d) {
     const float r = L.r;
     const int offt = __ldg(L.off + t);
     const size_t bt = (size_t)t * L.cap_p;
@@ -354,56 +438,38 @@ __device__ int link_component(const LinkBufs& L, C& c, int t, int d, int k) {
         if (qd < nd) {
             const int di = qd++;
             const float y = __ldg(L.py + bt + c.D[di]), x = __ldg(L.px + bt + c.D[di]);
-            auto edge = [&](unsigned key, float w) {
-                int s = 0;
-                while (s < ns && c.S[s] != key) ++s;
-                if (s == ns) {
-                    if (ns == c.ms()) { res = COMP_BIG; return false; }
-                    c.S[ns++] = key;
-                }
-                if (ne == c.me()) { res = COMP_BIG; return false; }
-                c.ed[ne] = di;
-                c.es[ne] = s;
-                c.ew[ne++] = w;
-                return true;
-            };
-            bool go = true;
             if (t > 0)
-                go = near(L, t - 1, y, x, [&](int i, float sy, float sx) {
+                near(L, t - 1, y, x, [&](int i, float sy, float sx) {
                     float w;
-                    return !within_r(sy, sx, y, x, r, &w) || edge((unsigned)i, w);
+                    if (!within_r(sy, sx, y, x, r, &w)) return true;
+                    int s = 0;
+                    while (s < ns && c.S[s] != (unsigned)i) ++s;
+                    if (ne == CAP_TE || s == CAP_T) { res = COMP_BIG; return false; }
+                    if (s == ns) c.S[ns++] = (unsigned)i;
+                    c.ed[ne] = di;
+                    c.es[ne] = s;
+                    c.ew[ne++] = w;
+                    return true;
                 });
-            if (k > 0)
-                for (int j = 1; go && j <= L.memory && t - 1 - j >= 0; ++j) {
-                    const int f = t - 1 - j, of = __ldg(L.off + f);
-                    go = near(L, f, y, x, [&](int i, float sy, float sx) {
-                        float w;
-                        if (!within_r(sy, sx, y, x, r, &w) || !in_memory(L, of + i, j)) return true;
-                        return edge((unsigned)L.cap_p + (unsigned)(f * L.cap_p + i), w);
-                    });
-                }
-            if (!go) return res;
         } else if (qs < ns) {
-            const unsigned key = c.S[qs++];
-            const size_t h = key < (unsigned)L.cap_p ? (size_t)(t - 1) * L.cap_p + key : (size_t)(key - (unsigned)L.cap_p);
+            const size_t h = (size_t)(t - 1) * L.cap_p + c.S[qs++];
             const float sy = __ldg(L.py + h), sx = __ldg(L.px + h);
-            const bool go = near(L, t, sy, sx, [&](int i, float y, float x) {
+            near(L, t, sy, sx, [&](int i, float y, float x) {
                 float w;
                 if (!within_r(sy, sx, y, x, r, &w)) return true;
                 int q = 0;
                 while (q < nd && c.D[q] != i) ++q;
                 if (q < nd) return true;
-                if (i < d && (k == 0 || __ldcg(L.stamp + offt + i) == k)) { res = COMP_SKIP; return false; }
-                if (nd == c.md()) { res = COMP_BIG; return false; }
+                if (i < d) { res = COMP_SKIP; return false; }
+                if (nd == CAP_T) { res = COMP_BIG; return false; }
                 c.D[nd++] = i;
                 return true;
             });
-            if (!go) return res;
         } else {
             break;
         }
+        if (res != COMP_DONE) return res;
     }
-    int np = nd;
     if (nd == 1 && ns <= 1) {
         c.path[0] = 0;
         c.best[0] = ns - 1;  // the only source, or none
@@ -430,19 +496,15 @@ __device__ int link_component(const LinkBufs& L, C& c, int t, int d, int k) {
         int first = 0;
         for (int q = 1; q < nd; ++q)
             if (c.D[q] < c.D[first]) first = q;
-        np = dfs_order(c, first, nd, ns, ne);
-        for (int q = 0; q < np; ++q) c.best[q] = -1;
-        if (!solve_subnet(c, np, ns, L.budget, r * r)) atomicOr(L.err, ERR_SUBNET_BUDGET);
+        dfs_order(c, first, nd, ne);
+        for (int q = 0; q < nd; ++q) c.best[q] = -1;
+        if (!solve_subnet(c, nd, ns, L.budget, r * r)) atomicOr(L.err, ERR_SUBNET_BUDGET);
     }
-    // the links: first every source given up, then every source taken (a
-    // source that changes destination ends up linked)
-    if (k > 0)
-        for (int q = 0; q < np; ++q) give_up(L, c.best[q] < 0 ? -1 : (long long)c.S[c.best[q]], offt + c.D[c.path[q]], t, k);
-    for (int q = 0; q < np; ++q) take_up(L, c.best[q] < 0 ? -1 : (long long)c.S[c.best[q]], offt + c.D[c.path[q]], t, k);
+    for (int q = 0; q < nd; ++q) take_up(L, c.best[q] < 0 ? -1 : (long long)c.S[c.best[q]], offt + c.D[c.path[q]], t, 0);
     return COMP_DONE;
 }
 
-// A pass's seeds are resolved by a warp each: what a thread does one
+// A seed's component by a warp: what a thread does one
 // dependent load after the other (up to 100k cycles for a component of 3
 // destinations and 5 sources with memory 3) the lanes do side by side.  The
 // nodes of a search level are expanded together: their cell ranges in all
@@ -497,8 +559,8 @@ __device__ __forceinline__ bool each_in_rows(unsigned a, int n, int nrows, F&& f
     return true;
 }
 
-// The component of seed d of frame t (t >= 1) in pass k >= 1; as
-// link_component.
+// The component of seed d of frame t (t >= 1) in pass k, as link_component (k =
+// 0: the first linking).
 __device__ int link_component_warp(const LinkBufs& L, WarpComp& c, int t, int d, int k) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -509,7 +571,7 @@ __device__ int link_component_warp(const LinkBufs& L, WarpComp& c, int t, int d,
     unsigned myS = 0;
     float sy = 0.f, sx = 0.f;
     int nd = 1, ns = 0, ne = 0, qd = 0, qs = 0, res = COMP_DONE;
-    const int ngr = min(L.memory, t - 1) + 1;  // source frames t-1, t-2, ...
+    const int ngr = k == 0 ? 1 : min(L.memory, t - 1) + 1;  // source frames t-1, t-2, ...
     while (true) {
         if (qd < nd) {
             // 3 rows of cells in each source frame; several destinations at
@@ -580,7 +642,7 @@ __device__ int link_component_warp(const LinkBufs& L, WarpComp& c, int t, int d,
                     i = __ldg(L.gidx + at);
                     float w;
                     hit = within_r(y, x, p.x, p.y, r, &w);
-                    smaller = hit && i < d && __ldcg(L.stamp + offt + i) == k;
+                    smaller = hit && i < d && (k == 0 || __ldcg(L.stamp + offt + i) == k);
                 }
                 if (__any_sync(full, smaller)) { res = COMP_SKIP; return false; }
                 for (unsigned m = __ballot_sync(full, hit); m; m &= m - 1) {
@@ -744,9 +806,185 @@ __device__ int link_component_warp(const LinkBufs& L, WarpComp& c, int t, int d,
         mine = __shfl_sync(full, mine, dest);
     }
     // every source given up before any is taken
-    if (lane < nd) give_up(L, key, offt + mine, t, k);
+    if (k > 0 && lane < nd) give_up(L, key, offt + mine, t, k);
     __syncwarp();
     if (lane < nd) take_up(L, key, offt + mine, t, k);
+    __syncwarp();
+    return COMP_DONE;
+}
+
+// The component of seed d of frame t (t >= 1) in pass k by a warp, with arrays
+// in memory: explored as in link_component_warp, then lanes sort the
+// destinations' lists and make the sources', and lane 0 orders and searches.
+// What bounds it: latency, of the exploration's steps and of the search's loads.
+template <class I>
+__device__ int link_component_mem(const LinkBufs& L, MemComp<I> c, int t, int d, int k) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const float r = L.r;
+    const int offt = __ldg(L.off + t);
+    const size_t bt = (size_t)t * L.cap_p;
+    int nd = 0, ns = 0, ne = 0, qd = 0, qs = 0, res = COMP_DONE;
+    const int ngr = k == 0 ? 1 : min(L.memory, t - 1) + 1;  // source frames t-1, t-2, ...
+    const int hd = hash_size(c.cd), hs = hash_size(c.cs);
+    unsigned* keys = (unsigned*)c.hash;
+    KeyTable<I> dt{keys, (I*)(keys + hd + hs), hd}, stab{keys + hd, (I*)(keys + hd + hs) + hd, hs};
+    dt.clear();
+    stab.clear();
+    if (lane == 0) c.D[0] = d;
+    __syncwarp();
+    int idx;
+    bool fresh;
+    dt.put((unsigned)d, lane == 0, c.cd, &nd, &idx, &fresh);
+    while (true) {
+        if (qd < nd) {
+            const int nb = 3 * ngr <= 16 ? min(nd - qd, 32 / (3 * ngr)) : 1;
+            for (int j0 = 0; j0 < ngr; j0 += 10) {
+                const int per = 3 * min(10, ngr - j0);
+                const int mine = qd + min(lane / per, nb - 1);
+                const float y = __ldg(L.py + bt + c.D[mine]), x = __ldg(L.px + bt + c.D[mine]);
+                const int q = lane - (mine - qd) * per;
+                unsigned a = 0;
+                int n = 0;
+                if (lane < nb * per) cell_row(L, t - 1 - j0 - q / 3, q % 3, y, x, &a, &n);
+                const bool go = each_in_rows(a, n, nb * per, [&](int row, unsigned at) {
+                    const int node = max(row, 0) / per;
+                    const float y1 = __shfl_sync(full, y, node * per), x1 = __shfl_sync(full, x, node * per);
+                    unsigned key = 0;
+                    float w = 0.f;
+                    bool hit = false;
+                    if (row >= 0) {
+                        const int j = j0 + (row - node * per) / 3, f = t - 1 - j;
+                        const float2 p = __ldg(L.gpos + at);
+                        const int i = __ldg(L.gidx + at);
+                        hit = within_r(p.x, p.y, y1, x1, r, &w);
+                        if (hit && j > 0) hit = in_memory(L, __ldg(L.off + f) + i, j);
+                        key = j == 0 ? (unsigned)i : (unsigned)L.cap_p + (unsigned)(f * L.cap_p + i);
+                    }
+                    const unsigned hits = __ballot_sync(full, hit);
+                    int s;
+                    bool first;
+                    if (ne + __popc(hits) > c.ce || !stab.put(key, hit, c.cs, &ns, &s, &first)) {
+                        res = COMP_BIG;
+                        return false;
+                    }
+                    // a destination's edges follow one another: rows are in its order
+                    const int e = ne + __popc(hits & ((1u << lane) - 1u));
+                    if (first) c.S[s] = key;
+                    if (hit) {
+                        c.dsrc[e] = (I)s;
+                        c.dw[e] = w;
+                        c.list[e] = (I)(qd + node);  // the edge's destination, for now
+                    }
+                    ne += __popc(hits);
+                    __syncwarp();
+                    return true;
+                });
+                if (!go) return res;
+            }
+            qd += nb;
+        } else if (qs < ns) {
+            const int nb = min(ns - qs, 10);
+            const unsigned key = c.S[qs + min(lane / 3, nb - 1)];
+            const size_t h = key < (unsigned)L.cap_p ? (size_t)(t - 1) * L.cap_p + key : (size_t)(key - (unsigned)L.cap_p);
+            const float y = __ldg(L.py + h), x = __ldg(L.px + h);
+            unsigned a = 0;
+            int n = 0;
+            if (lane < 3 * nb) cell_row(L, t, lane % 3, y, x, &a, &n);
+            const bool go = each_in_rows(a, n, 3 * nb, [&](int row, unsigned at) {
+                const int from = max(row, 0) / 3 * 3;
+                const float y1 = __shfl_sync(full, y, from), x1 = __shfl_sync(full, x, from);
+                int i = 0;
+                bool hit = false, smaller = false;
+                if (row >= 0) {
+                    const float2 p = __ldg(L.gpos + at);
+                    float w;
+                    i = __ldg(L.gidx + at);
+                    hit = within_r(y1, x1, p.x, p.y, r, &w);
+                    smaller = hit && i < d && (k == 0 || __ldcg(L.stamp + offt + i) == k);
+                }
+                if (__any_sync(full, smaller)) { res = COMP_SKIP; return false; }
+                int q;
+                bool first;
+                if (!dt.put((unsigned)i, hit, c.cd, &nd, &q, &first)) { res = COMP_BIG; return false; }
+                if (first) c.D[q] = i;
+                __syncwarp();
+                return true;
+            });
+            if (!go) return res;
+            qs += nb;
+        } else {
+            break;
+        }
+    }
+    __syncwarp();  // the tables' place is free
+    // the destinations' lists (every destination has an edge, or it is alone)
+    for (int e = lane; e < ne; e += 32)
+        if (e == 0 || c.list[e - 1] != c.list[e]) c.doff[c.list[e]] = (I)e;
+    if (lane == 0) {
+        c.doff[0] = 0;
+        c.doff[nd] = (I)ne;
+    }
+    for (int q = lane; q < nd; q += 32) c.vis[q] = 0;
+    for (int s = lane; s < ns; s += 32) {
+        c.used[s] = 0;
+        c.soff[s] = 0;
+    }
+    __syncwarp();
+    for (int e = lane; e < ne; e += 32) atomicAdd(c.soff + c.dsrc[e], 1);
+    __syncwarp();
+    // in ascending source order (linking.rs:310-315)
+    for (int q = lane; q < nd; q += 32) {
+        const int z0 = c.doff[q], z1 = c.doff[q + 1];
+        for (int e = z0 + 1; e < z1; ++e) {
+            const int s = c.dsrc[e];
+            const float w = c.dw[e];
+            const unsigned key = c.S[s];
+            int z = e;
+            for (; z > z0 && c.S[c.dsrc[z - 1]] > key; --z) {
+                c.dsrc[z] = c.dsrc[z - 1];
+                c.dw[z] = c.dw[z - 1];
+            }
+            c.dsrc[z] = (I)s;
+            c.dw[z] = w;
+        }
+    }
+    __syncwarp();
+    // the sources' lists: starts, which the entries move on to the ends
+    for (int s0 = 0, before = 0; s0 < ns; s0 += 32) {
+        const int n = s0 + lane < ns ? c.soff[s0 + lane] : 0;
+        int incl = n;
+#pragma unroll
+        for (int b = 1; b < 32; b <<= 1) {
+            const int v = __shfl_up_sync(full, incl, b);
+            if (lane >= b) incl += v;
+        }
+        if (s0 + lane < ns) c.soff[s0 + lane] = before + incl - n;
+        before += __shfl_sync(full, incl, 31);
+    }
+    __syncwarp();
+    for (int q = lane; q < nd; q += 32)
+        for (int z = c.doff[q]; z < c.doff[q + 1]; ++z) c.list[atomicAdd(c.soff + c.dsrc[z], 1)] = (I)q;
+    int low = INT_MAX;
+    for (int q = lane; q < nd; q += 32) low = min(low, c.D[q]);
+    low = __reduce_min_sync(full, low);
+    int first = INT_MAX;
+    for (int q = lane; q < nd; q += 32)
+        if (c.D[q] == low) first = q;
+    first = __reduce_min_sync(full, first);
+    for (int q = lane; q < nd; q += 32) c.best[q] = -1;
+    __syncwarp();
+    if (lane == 0) {
+        dfs_order(c, first, nd);
+        if (!solve_subnet(c, nd, ns, L.budget, r * r)) atomicOr(L.err, ERR_SUBNET_BUDGET);
+    }
+    __syncwarp();
+    // every source given up before any is taken
+    auto source = [&](int q) { return c.best[q] < 0 ? -1 : (long long)c.S[c.best[q]]; };
+    if (k > 0)
+        for (int q = lane; q < nd; q += 32) give_up(L, source(q), offt + c.D[c.path[q]], t, k);
+    __syncwarp();
+    for (int q = lane; q < nd; q += 32) take_up(L, source(q), offt + c.D[c.path[q]], t, k);
     __syncwarp();
     return COMP_DONE;
 }
@@ -758,41 +996,77 @@ __device__ void link_all(const LinkBufs& L, int tid, int nthr) {
         const int t = frame_of(L, g, L.tb, L.te);
         const int d = g - __ldg(L.off + t);
         SmallComp c;
-        if (link_component(L, c, t, d, 0) == COMP_BIG) L.deferq[push_slot(L.ctr + 2)] = t * L.cap_p + d;
+        if (link_component(L, c, t, d) == COMP_BIG) L.seedq[push_slot(L.ctr + C_SEEDS)] = t * L.cap_p + d;
     }
 }
 
-// Resolves the components of pass k's seeds, starting with a warp per block.
-__device__ void link_seeds(const LinkBufs& L, int k, int vw, int nwarp) {
-    __shared__ WarpComp wc[NTL / 32];
-    int* ctr = L.ctr + (k & 3) * 4;
-    const int n = __ldcg(ctr);
+// Resolves the components of pass k's seeds (k = 0: of those that link_all left),
+// starting with a warp per block.
+__device__ void link_seeds(const LinkBufs& L, WarpComp* wc, int k, int vw, int nwarp) {
+    int* ctr = L.ctr + (k & 3) * NCTR;
+    const int n = __ldcg(ctr + C_SEEDS);
     for (int q = vw; q < n; q += nwarp) {
         const int h = __ldcg(L.seedq + q);
         const int t = h / L.cap_p;
         if (link_component_warp(L, wc[threadIdx.x >> 5], t, h - t * L.cap_p, k) == COMP_BIG && (threadIdx.x & 31) == 0)
-            L.deferq[push_slot(ctr + 2)] = h;
+            L.deferq[push_slot(ctr + C_MEM)] = h;
         __syncwarp();
     }
 }
 
-// The components that do not fit a thread's arrays, one thread per block and
-// scratch slot.
-__device__ void link_deferred(const LinkBufs& L, int k) {
-    const int n = __ldcg(L.ctr + (k & 3) * 4 + 2);
-    if (threadIdx.x != 0 || (int)blockIdx.x >= L.nslot) return;
-    for (int q = blockIdx.x; q < n; q += min((int)gridDim.x, L.nslot)) {
+// The components that do not fit a warp's registers: a warp per block with the
+// block's arrays (`mem`).  Those that do not fit these are marked in the queue,
+// for link_slots.  Movies begin at block *r.
+__device__ void link_deferred(const LinkBufs& L, void* mem, int k, int* r) {
+    int* ctr = L.ctr + (k & 3) * NCTR;
+    const int n = __ldcg(ctr + C_MEM);
+    const int b = (int)blockIdx.x - *r;
+    *r = (*r + n) % (int)gridDim.x;
+    if (threadIdx.x >= 32) return;
+    const MemComp<unsigned short> c(mem, MID_N, MID_N, MID_E);
+    for (int q = b < 0 ? b + (int)gridDim.x : b; q < n; q += gridDim.x) {
         const int h = __ldcg(L.deferq + q);
         const int t = h / L.cap_p;
-        BigComp c = big_comp(L, blockIdx.x);
-        if (link_component(L, c, t, h - t * L.cap_p, k) == COMP_BIG) {
+        if (link_component_mem(L, c, t, h - t * L.cap_p, k) == COMP_BIG && threadIdx.x == 0) {
+            L.deferq[q] = ~h;
+            atomicAdd(ctr + C_SLOT, 1);
+        }
+        __syncwarp();
+    }
+}
+
+// A warp per block and scratch slot.
+__device__ void link_slots(const LinkBufs& L, int k) {
+    int* ctr = L.ctr + (k & 3) * NCTR;
+    const int n = __ldcg(ctr + C_MEM);
+    if (threadIdx.x >= 32 || (int)blockIdx.x >= L.nslot) return;
+    const MemComp<int> c(L.big + (size_t)blockIdx.x * L.big_ints, L.big_d, L.big_s, L.big_e);
+    for (int q = blockIdx.x; q < n; q += min((int)gridDim.x, L.nslot)) {
+        const int h = ~__ldcg(L.deferq + q);
+        if (h < 0) continue;
+        const int t = h / L.cap_p;
+        if (link_component_mem(L, c, t, h - t * L.cap_p, k) == COMP_BIG) {
             // the host retries with larger slots; until the launch ends every
             // link of the frame must be a valid index
-            atomicOr(L.err, ERR_EDGE_OVERFLOW);
+            if (threadIdx.x == 0) atomicOr(L.err, ERR_EDGE_OVERFLOW);
             if (k == 0)
-                for (int g = __ldg(L.off + t); g < __ldg(L.off + t + 1); ++g) L.pred[g] = -1;
+                for (int g = __ldg(L.off + t) + threadIdx.x; g < __ldg(L.off + t + 1); g += 32) L.pred[g] = -1;
         }
+        __syncwarp();
+        if (threadIdx.x == 0) atomicAdd(ctr + C_DONE, 1);
     }
+}
+
+// Until the slots are done, asleep: the grid barrier's polling keeps emptying
+// the L1 that a busy block on the same SM works from (lattices of 10 x 10 in
+// slots 174 ms a call beside it, 52 beside sleepers).  The limit only ends the
+// sleep: the barrier follows.
+__device__ void wait_slots(const LinkBufs& L, int k) {
+    const int* ctr = L.ctr + (k & 3) * NCTR;
+    const int n = __ldcg(ctr + C_SLOT);
+    const volatile int* done = ctr + C_DONE;
+    if (threadIdx.x == 0)
+        for (int i = 0; i < (1 << 24) && *done < n; ++i) __nanosleep(1000);
 }
 
 // A block's seeds on their way to the queue: one global atomic per block
@@ -808,7 +1082,7 @@ __device__ __forceinline__ void flush_seeds(const LinkBufs& L, SeedBuf& sb, int 
     __shared__ int s_base;
     __syncthreads();
     const int n = min(sb.n, SEED_BUF);
-    if (threadIdx.x == 0 && n > 0) s_base = atomicAdd(L.ctr + (k & 3) * 4, n);
+    if (threadIdx.x == 0 && n > 0) s_base = atomicAdd(L.ctr + (k & 3) * NCTR + C_SEEDS, n);
     // every thread has read the count: the next movie's seeds may come in
     __syncthreads();
     if (n == 0) return;
@@ -864,9 +1138,9 @@ __device__ __forceinline__ void set_members(const LinkBufs& L, SeedBuf& sb, int 
                         if (atomicExch(L.stamp + __ldg(L.off + tt) + i, k) != k) {
                             const int slot = atomicAdd(&sb.n, 1);
                             if (slot < SEED_BUF) sb.h[slot] = h;
-                            else L.seedq[push_slot(L.ctr + (k & 3) * 4)] = h;
+                            else L.seedq[push_slot(L.ctr + (k & 3) * NCTR + C_SEEDS)] = h;
                             if (__ldcg(L.fstamp + tt) != k && atomicExch(L.fstamp + tt, k) != k)
-                                atomicAdd(L.ctr + (k & 3) * 4 + 3, 1);
+                                atomicAdd(L.ctr + (k & 3) * NCTR + C_FRAMES, 1);
                         }
                     }
                 }
@@ -905,7 +1179,7 @@ __device__ void members_short(const LinkBufs& L, SeedBuf& sb, int k, int tid, in
     const int fb = first_member(L);
     const int g0 = __ldg(L.off + fb);
     // pass 1: all, in order; later: spread over the grid's warps
-    const int n = k == 1 ? __ldg(L.off + L.te) - g0 : __ldcg(L.ctr + ((k - 1) & 3) * 4 + 1);
+    const int n = k == 1 ? __ldg(L.off + L.te) - g0 : __ldcg(L.ctr + ((k - 1) & 3) * NCTR + C_CHECKS);
     for (int i = tid; __any_sync(0xffffffffu, i < n); i += nthr) {
         int g = 0, f = 0;
         unsigned wm = 0, bits = 0;
@@ -970,7 +1244,7 @@ __device__ __forceinline__ void each_unused(const LinkBufs& L, int mask, int roo
 
 // The particles that pass k evaluates: number, and the i-th.
 __device__ __forceinline__ int find_count(const LinkBufs& L, int k) {
-    return k == 1 ? __ldg(L.off + L.te) - __ldg(L.off + first_member(L)) : __ldcg(L.ctr + (k & 3) * 4 + 1);
+    return k == 1 ? __ldg(L.off + L.te) - __ldg(L.off + first_member(L)) : __ldcg(L.ctr + (k & 3) * NCTR + C_CHECKS);
 }
 
 __device__ __forceinline__ int find_item(const LinkBufs& L, int k, int i) {
@@ -980,7 +1254,7 @@ __device__ __forceinline__ int find_item(const LinkBufs& L, int k, int i) {
 __device__ void members_find(const LinkBufs& L, int k, int tid, int nthr) {
     const int g1 = __ldg(L.off + L.te);
     for (int g = __ldg(L.off + first_member(L)) + tid; g < g1; g += nthr)
-        if (__ldcg(L.cstamp + __ldcg(L.root + g)) == k) L.recq[push_slot(L.ctr + (k & 3) * 4 + 1)] = g;
+        if (__ldcg(L.cstamp + __ldcg(L.root + g)) == k) L.recq[push_slot(L.ctr + (k & 3) * NCTR + C_CHECKS)] = g;
 }
 
 __device__ void members_chain(const LinkBufs& L, int k, int tid, int nthr) {
@@ -1161,6 +1435,9 @@ template <class M>
 __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_passes, int* passes,
                                               unsigned long long* stat) {
     __shared__ SeedBuf sb;
+    // the warps' edges, then (a grid barrier between) a deferred component
+    constexpr int WARP_BYTES = (int)sizeof(WarpComp) * (NTL / 32);
+    __shared__ __align__(16) unsigned char buf[WARP_BYTES > MID_BYTES ? WARP_BYTES : MID_BYTES];
     if (threadIdx.x == 0) sb.n = 0;
     cg::grid_group grid = cg::this_grid();
     const int nthr = gridDim.x * NTL;
@@ -1202,19 +1479,36 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
         }
     }
     grid.sync();
+    auto any = [&](int k, int what) {
+        bool b = false;
+        for (int m = 0; m < nm; ++m) b |= __ldcg(movie(m).ctr + (k & 3) * NCTR + what) > 0;
+        return b;
+    };
     auto deferred = [&](int k) {
-        bool any = false;
-        for (int m = 0; m < nm; ++m) any |= __ldcg(movie(m).ctr + (k & 3) * 4 + 2) > 0;
-        if (!any) return;
-        for (int m = 0; m < nm; ++m) link_deferred(movie(m), k);
+        if (!any(k, C_MEM)) return;
+        int r = 0;
+        for (int m = 0; m < nm; ++m) link_deferred(movie(m), buf, k, &r);
+        grid.sync();
+        if (!any(k, C_SLOT)) return;
+        for (int m = 0; m < nm; ++m) link_slots(movie(m), k);
+        for (int m = 0; m < nm; ++m) wait_slots(movie(m), k);
         grid.sync();
     };
+    if (any(0, C_SEEDS)) {
+        int r = 0;
+        for (int m = 0; m < nm; ++m) {
+            const LinkBufs L = movie(m);
+            const int id = rot(vw0 * 32, r, L) >> 5;
+            link_seeds(L, (WarpComp*)buf, 0, id, nthr >> 5);
+        }
+        grid.sync();
+    }
     deferred(0);
     tick(0);
     int k = 0;
     if (any_mem) {
         auto active = [&](const LinkBufs& L, int kk) {
-            return L.memory > 0 && L.te > 2 && (kk == 1 || __ldcg(L.ctr + ((kk - 1) & 3) * 4) > 0);
+            return L.memory > 0 && L.te > 2 && (kk == 1 || __ldcg(L.ctr + ((kk - 1) & 3) * NCTR + C_SEEDS) > 0);
         };
         for (k = 1; k <= max_passes; ++k) {
             bool longs = false;
@@ -1250,7 +1544,7 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
                 const int id = rot(vt0, r, L);
                 // the counters of pass k + 1 were last read in pass k - 2
                 if (stamp)
-                    for (int q = 0; q < 4; ++q) L.ctr[((k + 1) & 3) * 4 + q] = 0;
+                    for (int q = 0; q < NCTR; ++q) L.ctr[((k + 1) & 3) * NCTR + q] = 0;
                 if (!active(L, k)) continue;
                 if (L.memory <= 2) members_short(L, sb, k, k == 1 ? tid0 : id, nthr);
                 else members_long(L, sb, k, find_count(L, k) > nthr / 8 ? tid0 : id, nthr);
@@ -1258,11 +1552,11 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
             }
             grid.sync();
             int total = 0;
-            for (int m = 0; m < nm; ++m) total += __ldcg(movie(m).ctr + (k & 3) * 4);
+            for (int m = 0; m < nm; ++m) total += __ldcg(movie(m).ctr + (k & 3) * NCTR + C_SEEDS);
             tick(2);
             if (stamp && k <= 8) {
                 unsigned long long nf = 0;
-                for (int m = 0; m < nm; ++m) nf += (unsigned)__ldcg(movie(m).ctr + (k & 3) * 4 + 3);
+                for (int m = 0; m < nm; ++m) nf += (unsigned)__ldcg(movie(m).ctr + (k & 3) * NCTR + C_FRAMES);
                 stat[4 + k - 1] += nf;
             }
             if (total == 0) break;
@@ -1272,7 +1566,7 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
                 const int id = rot(vw0 * 32, r, L) >> 5;
                 if (!active(L, k)) continue;
                 if (L.memory > 2) members_clear(L, k, tid0, nthr);
-                link_seeds(L, k, id, nthr >> 5);
+                link_seeds(L, (WarpComp*)buf, k, id, nthr >> 5);
             }
             grid.sync();
             deferred(k);
