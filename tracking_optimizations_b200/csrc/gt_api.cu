@@ -2002,7 +2002,11 @@ int gt_link(gt_ctx* ctx, const float* rows, int64_t n, int ncols, float search_r
         // cells of absolute positions; negative coordinates clamp into the
         // first cell (clamping is monotone, so neighbours stay adjacent)
         const double ext = (double)std::max(tab.ymax, tab.xmax) + 1.0;
-        P.LG = std::max({(int)std::ceil(search_range) + 1, 8, (int)std::ceil(ext / 200.0)});
+        // at most 200 x 200 of them and about 16 a particle of the largest
+        // frame (32 x 32 at least): every frame has its own, and 1.2 million
+        // frames of one particle would want 194 GB of 200 x 200
+        const double side = std::min(200.0, std::max(32.0, std::ceil(std::sqrt(16.0 * tab.largest))));
+        P.LG = std::max({(int)std::ceil(search_range) + 1, 8, (int)std::ceil(ext / side)});
         P.lncy = (int)(tab.ymax / P.LG) + 1;
         P.lncx = (int)(tab.xmax / P.LG) + 1;
         link_scratch(&P, scale);
