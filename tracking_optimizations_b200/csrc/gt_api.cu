@@ -296,10 +296,12 @@ void annulus_inds_f(float outer, float inner, std::vector<int>& off) {
 
 size_t big_ints(const Plan& P) { return comp_bytes(P.big_d, P.big_s, P.big_e, sizeof(int)) / sizeof(int); }
 
-// Scratch slots of the linker's largest components, a block's each: as many as
-// fit 256 MB, 64 at least and a block's on every SM four times over at most.
-int big_slots(const Plan& P) {
-    return (int)std::max<size_t>(64, std::min<size_t>(4 * 148, ((size_t)64 << 20) / big_ints(P)));
+// Scratch slots of the linker's largest components in T frames, a block's each:
+// 16 a pair of frames, as many as fit 256 MB (64 in any case), and a block's
+// on every SM four times over at most.
+int big_slots(const Plan& P, long long T) {
+    const size_t fit = std::max<size_t>(64, std::min<size_t>(4 * 148, ((size_t)64 << 20) / big_ints(P)));
+    return (int)std::min<long long>(fit, 16 * (T - 1));
 }
 
 // Their sizes: room for 4096 destinations, 8192 sources and 32768 edges (a
@@ -310,7 +312,7 @@ void link_scratch(Plan* pl, int scale) {
     P.big_d = (int)std::min<long long>(4096LL * scale, P.cap_p);
     P.big_s = (int)std::min<long long>(8192LL * scale, (long long)P.cap_p * (P.r.memory + 1));
     P.big_e = (int)std::min<long long>(32768LL * scale, (long long)P.big_d * P.big_s);
-    P.nslot = P.link ? big_slots(P) : 0;
+    P.nslot = P.link ? big_slots(P, P.T) : 0;
 }
 
 // The specialised locate kernel's tile height, 32 or fast_rows: nothing in the
@@ -469,8 +471,8 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->pend = c.take<int>(cc);
     w->py = c.take<float>(T * P.cap_p);
     w->px = c.take<float>(T * P.cap_p);
-    w->pm = c.take<float>(T * P.cap_p);
-    w->prec = c.take<int>(T * P.cap_p);
+    w->pm = c.take<float>(need_locate ? T * P.cap_p : 1);
+    w->prec = c.take<int>(need_locate ? T * P.cap_p : 1);
     w->npart = c.take<int>(T);
     w->gstart = c.take<int>(T * (lcell + 1));
     w->gidx = c.take<int>(T * P.cap_p);
@@ -544,7 +546,11 @@ int ensure_arena(gt_ctx* ctx, size_t bytes) {
     if (ctx->arena_size >= bytes) return GT_OK;
     if (ctx->arena) { cudaFree(ctx->arena); ctx->arena = nullptr; ctx->arena_size = 0; }
     size_t want = bytes + bytes / 8;
-    CK(cudaMalloc((void**)&ctx->arena, want));
+    if (cudaMalloc((void**)&ctx->arena, want) != cudaSuccess) {
+        ctx->err = "workspace of " + std::to_string(want >> 20) + " MB: " + cudaGetErrorString(cudaGetLastError());
+        ctx->arena = nullptr;
+        return GT_ERR_OOM;
+    }
     ctx->arena_size = want;
     return GT_OK;
 }
@@ -942,22 +948,30 @@ int batch_common(gt_ctx* ctx, const void* frames, bool host, int dtype, int T, i
     if (rc) return rc;
     r.normalized_taps = ctx->normalized_taps;
     CK(cudaSetDevice(ctx->device));
+    int cap_div = 64;
     for (int scale = 1; scale <= 64; scale *= 4) {
         Plan P;
-        rc = make_plan(r, T, H, W, dtype, scale, ctx->num_sms, &P, &ctx->err, ctx->force_generic,
-                       ctx->fast_tile_rows);
-        if (rc) return rc;
+        Work w{};
+        const size_t fbytes = host ? (size_t)T * H * W * elem_size(dtype) : 0;
+        while (true) {
+            rc = make_plan(r, T, H, W, dtype, scale, ctx->num_sms, &P, &ctx->err, ctx->force_generic,
+                           ctx->fast_tile_rows, cap_div);
+            if (rc) return rc;
+            if (cap_div != 64) P.repack = 0;  // memory is short
+            // a caller's device buffer receives the rows directly: no table slab
+            rc = ensure_arena(ctx, carve(P, nullptr, &w, fbytes, true, d_out == nullptr));
+            if (!rc) break;
+            // the largest capacities that fit; more features than they hold ask
+            // for larger ones again
+            if (rc != GT_ERR_OOM || scale > 1 || cap_div >= 1024) return rc;
+            cap_div *= 2;
+        }
+        ctx->err.clear();
         if (ctx->withhold_tma) {
             P.lp.tma_withhold = 1;
             P.lp.tma_spin = 1 << 10;
         }
         P.lp.tiles_per_cta = ctx->tiles_per_cta;
-        const size_t fbytes = host ? (size_t)T * H * W * elem_size(dtype) : 0;
-        Work w{};
-        // a caller's device buffer receives the rows directly: no table slab
-        const size_t need = carve(P, nullptr, &w, fbytes, true, d_out == nullptr);
-        rc = ensure_arena(ctx, need);
-        if (rc) return rc;
         carve(P, ctx->arena, &w, fbytes, true, d_out == nullptr);
         const void* dfr = host ? w.frames : frames;
         int bits = 0;
@@ -1232,8 +1246,9 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
         big.big_d = std::max(big.big_d, P.big_d);
         big.big_s = std::max(big.big_s, P.big_s);
         big.big_e = std::max(big.big_e, P.big_e);
-        big.nslot = big_slots(big);
+        big.T += P.T;
     }
+    if (S.nlink > 0) big.nslot = big_slots(big, big.T);
     // arena layout: movies, link pool, shared arrays
     size_t total = 0;
     for (int i = 0; i < n; ++i) {
