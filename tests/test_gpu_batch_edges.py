@@ -104,3 +104,38 @@ def test_larger_batch_refused_between_replays(gpu):
     st = _native.load().gt_batch_many_device(ctx, many, len(many), None)
     assert st == _native.GT_ERR_OOM, _native.load().gt_last_error(ctx)
     assert modes + [turn(), turn()] == [1, 2, 1, 2]
+
+
+def test_repacked_rows_share_buffers(gpu):
+    """Movies of odd width need room for repacked rows, by side stream and not
+    by movie: 24 of them take little more than 24 of even width."""
+    import ctypes
+
+    import torch
+
+    from tracking_optimizations_b200 import batched, gpu_tracking
+
+    lib, used = gpu.load(), []
+    for W in (1008, 1003):
+        g = torch.Generator(device="cuda").manual_seed(W)
+        frames = torch.poisson(torch.full((8, 601, W), 60.0, device="cuda"), generator=g).to(torch.int16)
+        frames.view(-1)[torch.randint(0, frames.numel(), (frames.numel() // 900,), device="cuda", generator=g)] += 900
+        movies = [(frames.roll(i, 1).contiguous(), dict(diameter=7, minmass=400.0)) for i in range(24)]
+        want = _each(movies[:1] + movies[-1:])
+        outs = batched.output_buffers(movies)
+        ctx = ctypes.c_void_p()
+        arr = (gpu.GtMovie * len(movies))()
+        for m, (fr, kw), out in zip(arr, movies, outs):
+            m.frames, m.dtype, (m.T, m.H, m.W) = fr.data_ptr(), gpu.GT_U16, fr.shape
+            m.params, m.out, m.out_rows = gpu.make_params(**kw), out.data_ptr(), len(out)
+        torch.cuda.synchronize()
+        assert lib.gt_ctx_create(0, ctypes.byref(ctx)) == 0
+        before = torch.cuda.mem_get_info()[0]
+        for _ in range(3):
+            assert lib.gt_batch_many_device(ctx, arr, len(movies), None) == 0, lib.gt_last_error(ctx)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        for i, w in ((0, want[0]), (-1, want[1])):
+            assert len(w) > 100
+            np.testing.assert_array_equal(outs[i][: arr[i if i >= 0 else 23].nrows].cpu().numpy(), w)
+        lib.gt_ctx_destroy(ctx)
+    assert used[1] < 1.3 * used[0], used

@@ -99,6 +99,8 @@ void gauss_taps(int smoothing_size, float noise_size, int normalized, float* w, 
 
 using namespace gt;
 
+constexpr int BATCH_STREAMS = 8;
+
 struct gt_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -119,8 +121,8 @@ struct gt_ctx {
     std::map<std::array<int, 6>, int> tile_rows;  // autotuned tile rows per (H, W, krad, D, rc, dtype)
     std::string batch_key;            // inputs of the cached graph
     cudaGraphExec_t batch_exec = nullptr;
-    cudaStream_t side[8] = {};
-    cudaEvent_t bev[20] = {};         // fork/join events
+    cudaStream_t side[BATCH_STREAMS] = {};
+    cudaEvent_t bev[2 + 2 * BATCH_STREAMS] = {};  // fork/join events
     int* h_status = nullptr;          // pinned: 8 ints per movie
     int* h_stage = nullptr;           // pinned: one call's statistics, read back in one go
     int link_grid[2] = {0, 0};        // resident blocks of the one-movie and the batched linker (queried once)
@@ -460,6 +462,8 @@ struct Carver {
     }
 };
 
+size_t repack_bytes(const Plan& P) { return (size_t)P.repack * P.H * P.pitch * (P.dtype == GT_U16 ? 2 : 4); }
+
 size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_locate, bool own_out = true) {
     Carver c{base};
     const size_t T = P.T;
@@ -499,7 +503,7 @@ size_t carve(const Plan& P, char* base, Work* w, size_t frame_bytes, bool need_l
     w->pbeg = w->status + 8;
     w->lstat = (unsigned long long*)(w->status + STATUS_LSTAT);
     w->fcount = w->status + STATUS_INTS;
-    w->repack = c.take<char>(need_locate ? (size_t)P.repack * P.H * P.pitch * (P.dtype == GT_U16 ? 2 : 4) : 1);
+    w->repack = c.take<char>(need_locate ? repack_bytes(P) : 1);
     w->off = c.take<int>(T + 1);
     const size_t np = P.link ? T * P.cap_p : 1;
     const size_t nm = P.link && P.r.memory > 0 ? np : 1;   // memory entries
@@ -1137,9 +1141,10 @@ int enqueue_back(gt_ctx* ctx, BatchMovie& bm, const gt_movie& mv, int* d_status,
     return GT_OK;
 }
 
-// The whole batch on `st`, fanned out over the context's side streams.
+// The whole batch on `st`, fanned out over the context's side streams: movie i
+// on stream i % BATCH_STREAMS.
 int enqueue_batch(gt_ctx* ctx, std::vector<BatchMovie>& B, gt_movie* mv, int n, BatchShared& S, cudaStream_t st) {
-    const int K = 8;
+    const int K = BATCH_STREAMS;
     S.launches = 0;
     CK(cudaEventRecord(ctx->bev[0], st));
     for (int k = 0; k < K; ++k) CK(cudaStreamWaitEvent(ctx->side[k], ctx->bev[0], 0));
@@ -1157,15 +1162,15 @@ int enqueue_batch(gt_ctx* ctx, std::vector<BatchMovie>& B, gt_movie* mv, int n, 
         CK(launch_link_multi(S.d_L, S.nlink, S.max_passes, S.d_passes, S.d_stat, S.link_grid, st));
         S.launches += 1;
     }
-    CK(cudaEventRecord(ctx->bev[9], st));
-    for (int k = 0; k < K; ++k) CK(cudaStreamWaitEvent(ctx->side[k], ctx->bev[9], 0));
+    CK(cudaEventRecord(ctx->bev[1 + K], st));
+    for (int k = 0; k < K; ++k) CK(cudaStreamWaitEvent(ctx->side[k], ctx->bev[1 + K], 0));
     for (int i = 0; i < n; ++i) {
         int rc = enqueue_back(ctx, B[i], mv[i], S.d_status + 8 * i, ctx->side[i % K], &S.launches);
         if (rc) return rc;
     }
     for (int k = 0; k < K; ++k) {
-        CK(cudaEventRecord(ctx->bev[10 + k], ctx->side[k]));
-        CK(cudaStreamWaitEvent(st, ctx->bev[10 + k], 0));
+        CK(cudaEventRecord(ctx->bev[2 + K + k], ctx->side[k]));
+        CK(cudaStreamWaitEvent(st, ctx->bev[2 + K + k], 0));
     }
     CK(cudaMemcpyAsync(ctx->h_status, S.d_status, sizeof(int) * 8 * (size_t)n, cudaMemcpyDeviceToHost, st));
     return GT_OK;
@@ -1251,17 +1256,27 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
     if (S.nlink > 0) big.nslot = big_slots(big, big.T);
     // arena layout: movies, link pool, shared arrays
     size_t total = 0;
-    for (int i = 0; i < n; ++i) {
+    // one buffer of repacked rows per side stream, whose movies follow one another
+    size_t rows[BATCH_STREAMS] = {};
+    auto own = [&](int i) {  // what a movie does not share
         Plan Pc = B[i].P;
         Pc.nslot = 0;
+        Pc.repack = 0;
+        return Pc;
+    };
+    for (int i = 0; i < n; ++i) {
+        size_t& r = rows[i % BATCH_STREAMS];
+        r = std::max(r, repack_bytes(B[i].P));
         Work w{};
         B[i].off = total;
-        total += carve(Pc, nullptr, &w, 0, true, false);
+        total += carve(own(i), nullptr, &w, 0, true, false);
         total = (total + 255) / 256 * 256;
     }
     Carver pc{nullptr};
     int* big_pool = nullptr;
+    char* repack[BATCH_STREAMS];
     auto pool_layout = [&](Carver& c) {
+        for (int k = 0; k < BATCH_STREAMS; ++k) repack[k] = c.take<char>(rows[k]);
         big_pool = c.take<int>((size_t)big.nslot * big_ints(big));
         S.d_L = c.take<LinkBufs>(std::max(1, S.nlink));
         S.d_stat = c.take<unsigned long long>(12);
@@ -1294,13 +1309,12 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
                       ctx->tune_disabled, ctx->batch_cap_div);
         key += buf;
     }
-    for (int i = 0; i < n; ++i) {
-        Plan Pc = B[i].P;
-        Pc.nslot = 0;
-        carve(Pc, ctx->arena + B[i].off, &B[i].w, 0, true, false);
-    }
     Carver c2{ctx->arena + total};
     pool_layout(c2);
+    for (int i = 0; i < n; ++i) {
+        carve(own(i), ctx->arena + B[i].off, &B[i].w, 0, true, false);
+        B[i].w.repack = repack[i % BATCH_STREAMS];
+    }
     const bool replay = ctx->batch_exec && key == ctx->batch_key;
     // constant tables and linker descriptors (other calls may have reused
     // the arena since the graph was built)
