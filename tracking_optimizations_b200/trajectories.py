@@ -19,6 +19,12 @@ from . import _native
 from .gpu_tracking import _adopt_table as adopt_table
 
 
+# A view of the table's third column keeps the whole table, page-locked memory
+# in steps of 2 MB: short results are copied out of it (24 us for 65536 values;
+# 750k, 9 MB, would take 0.4 ms more than the view).
+MSD_COPY = 1 << 16
+
+
 def _i64(a):
     return np.ascontiguousarray(a, dtype=np.int64)
 
@@ -111,7 +117,10 @@ def imsd(ids, frames, x, y, mpp, fps, max_lagtime=100, device=0):
         raise
     lag = a[:, 0].astype(np.float64)
     lag /= float(fps)
-    return lag, a[:, 1].astype(np.int64), a[:, 2]
+    msd = a[:, 2]
+    if len(msd) <= MSD_COPY:
+        msd = msd.copy()
+    return lag, a[:, 1].astype(np.int64), msd
 
 
 def postprocess(df, params):
