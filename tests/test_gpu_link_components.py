@@ -71,3 +71,24 @@ def test_time_of_many(gpu):
             link_rust(table, 5.0, 1)
         took.append(time.perf_counter() - t0)
     assert took[1] < 20 * took[0], took
+
+
+@pytest.mark.parametrize("memory", [0, 2, 3])
+def test_movies(gpu, memory):
+    """Movies whose components reach a few dozen particles: from the host, linked
+    in runs of frames, and on the device, alone and in a batch."""
+    import torch
+
+    from tracking_optimizations_b200 import batch_rust, batched, synth
+
+    movies, want = [], []
+    for seed in range(3):
+        spec = synth.scaled(synth.PLAIN_1000, frames=80, height=128, width=128, spots=130, seed=seed)
+        m = synth.make_movie(spec)
+        params = dict(separation=4, minmass=150.0, search_range=6.0, memory=memory)
+        want.append(oracle.batch(m, 5, **params)[0])
+        got, _ = batch_rust(m, 5, **params)
+        np.testing.assert_array_equal(got, want[-1])
+        movies.append((torch.from_numpy(m.view(np.int16)).cuda(), dict(params, diameter=5)))
+    for (table, _), w in zip(batched.batch_many(movies), want):
+        np.testing.assert_array_equal(table.cpu().numpy(), w)
