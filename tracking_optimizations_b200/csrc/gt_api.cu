@@ -563,11 +563,11 @@ LinkBufs link_bufs(const Plan& P, const Work& w, long long budget) {
     LinkBufs L{};
     L.tb = 0;
     L.te = P.T;
-    L.T = P.T; L.cap_p = P.cap_p; L.memory = (int)std::min<uint32_t>(P.r.memory, (uint32_t)P.T);
+    L.cap_p = P.cap_p; L.memory = (int)std::min<uint32_t>(P.r.memory, (uint32_t)P.T);
     L.r = P.r.search_range;
     L.inv_g = 1.0f / (float)P.LG;
     L.ncx = P.lncx; L.ncy = P.lncy;
-    L.py = w.py; L.px = w.px; L.npart = w.npart; L.off = w.off; L.gstart = w.gstart; L.gidx = w.gidx; L.gpos = w.gpos;
+    L.py = w.py; L.px = w.px; L.off = w.off; L.gstart = w.gstart; L.gidx = w.gidx; L.gpos = w.gpos;
     L.np = (size_t)P.T * P.cap_p;
     L.pred = w.pred; L.lnk = w.lnk; L.mm = w.mm; L.stamp = w.stamp; L.rstamp = w.rstamp;
     L.seedq = w.seedq; L.recq = w.recq; L.deferq = w.deferq;
@@ -581,17 +581,6 @@ LinkBufs link_bufs(const Plan& P, const Work& w, long long budget) {
     return L;
 }
 
-// Linking over the particle tables already in the workspace (npart, py, px,
-// gstart/gidx, off): cooperative launches of link_fixpoint_kernel run the
-// fixed point, then new trajectory ids are numbered.  Leaves the trajectory
-// id of particle g in newid[root[g]].
-//
-// The linker in frame windows.  link_window links frames [tb, te) to their
-// fixed point, given final links for the frames before tb: the memory
-// entries of a frame depend only on earlier frames, so windows taken in
-// order give the sequential result (the host-frames path links each
-// uploaded chunk while the next one is copied).  link_prepare runs once
-// before the first window, link_finish once after the last.
 // Resident blocks of the one-movie (0) or the batched (1) linker.
 int link_grid(gt_ctx* ctx, int multi, int* grid) {
     if (!ctx->link_grid[multi]) {
@@ -603,6 +592,17 @@ int link_grid(gt_ctx* ctx, int multi, int* grid) {
     return GT_OK;
 }
 
+// Linking over the particle tables already in the workspace (npart, py, px,
+// gstart/gidx, off): cooperative launches of link_fixpoint_kernel run the
+// fixed point, then new trajectory ids are numbered.  Leaves the trajectory
+// id of particle g in newid[root[g]].
+//
+// The linker in frame windows.  link_window links frames [tb, te) to their
+// fixed point, given final links for the frames before tb: the memory
+// entries of a frame depend only on earlier frames, so windows taken in
+// order give the sequential result (the host-frames path links each
+// uploaded chunk while the next one is copied).  link_finish runs once after
+// the last.
 int link_window(gt_ctx* ctx, const Plan& P, const Work& w, cudaStream_t st, int tb, int te) {
     LinkBufs L = link_bufs(P, w, ctx->subnet_budget);
     L.tb = tb;
@@ -859,7 +859,7 @@ int err_status(gt_ctx* ctx, int bits, bool* retry) {
         ctx->err = "a linking subnetwork exceeded the search budget";
         return GT_ERR_SUBNET_BUDGET;
     }
-    if (bits & (ERR_CAND_OVERFLOW | ERR_PART_OVERFLOW | ERR_EDGE_OVERFLOW | ERR_MEM_OVERFLOW |
+    if (bits & (ERR_CAND_OVERFLOW | ERR_PART_OVERFLOW | ERR_EDGE_OVERFLOW |
                 ERR_SCRATCH_OVERFLOW)) {
         *retry = true;
         ctx->err = "per-frame capacity exceeded (bits " + std::to_string(bits) + ")";

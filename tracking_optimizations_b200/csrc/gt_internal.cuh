@@ -80,7 +80,6 @@ enum ErrBits {
     ERR_PART_OVERFLOW = 2,
     ERR_EDGE_OVERFLOW = 4,
     ERR_SUBNET_BUDGET = 8,
-    ERR_MEM_OVERFLOW = 16,
     ERR_SCRATCH_OVERFLOW = 32,
     ERR_DEVICE_TIMEOUT = 64,
 };
@@ -144,14 +143,13 @@ __host__ __device__ constexpr size_t comp_bytes(int cd, int cs, int ce, size_t i
 enum { C_SEEDS = 0, C_CHECKS = 1, C_MEM = 2, C_FRAMES = 3, C_SLOT = 4, C_DONE = 5, NCTR = 8 };
 
 struct LinkBufs {
-    int T, cap_p, memory;
+    int cap_p, memory;
     int tb, te;           // frames linked by this launch; earlier frames are final
     float r;              // search range
     float inv_g;          // 1 / cell size
     int ncx, ncy;
     const float* py;
     const float* px;
-    const int* npart;
     const int* off;       // exclusive prefix of npart (compact particle index)
     const int* gstart;
     const int* gidx;

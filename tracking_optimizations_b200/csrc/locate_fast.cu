@@ -6,7 +6,7 @@ namespace gt {
 
 cudaError_t launch_locate_flex(int kr, int rc, int dtype, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, const TileSource& src, int frame0, int* used_tma);
-int flex_dilation(int rc, int dtype);
+int flex_dilation(int rc);
 int flex_rows(int rc, int dtype);
 
 // (smoothing radius, dilation size, centroid radius) triples with a kernel of
@@ -25,7 +25,7 @@ int fast_supported(int kr, int dd, int rc, int diameter, int dtype) {
         GT_FAST_LIST(GT_FAST_CASE)
 #undef GT_FAST_CASE
     }
-    return dd >= FM && dd <= flex_dilation(rc, dtype) ? 2 : 0;
+    return dd >= FM && dd <= flex_dilation(rc) ? 2 : 0;
 }
 
 // Tile rows of those kernels: 32 where asked for and there is a choice, else the

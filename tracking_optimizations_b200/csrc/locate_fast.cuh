@@ -70,10 +70,7 @@ enum { COLS_PLAIN = 0, COLS_CPU = 1, COLS_GPU = 2 };
 // Walker warps of a run of tiles (64-row tiles: 2 of 16 warps, 32-row
 // tiles: 2 of 8): they walk a tile of at most 32 NWO candidates while the
 // other warps start the next one.
-#ifndef GT_WALKERS64
-#define GT_WALKERS64 2
-#endif
-__host__ __device__ constexpr int walker_warps(int th) { return th == 32 ? 2 : GT_WALKERS64; }
+constexpr int WALKERS = 2;
 
 __host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 __host__ __device__ constexpr int round8(int x) { return (x + 7) / 8 * 8; }
@@ -129,7 +126,7 @@ struct Geo {
     static constexpr int SZ_BP = align128(cmax(RP * GPS * 8, TH0 * FT * 2 + (NTK / 32) * 32 * 20));
     static constexpr int K = circle_size(RC);
     static constexpr int SZ_TAB = align128(K * 20);  // (sin2, cos2), P2 offsets by parity, r2
-    static constexpr int NWO = walker_warps(TH0);
+    static constexpr int NWO = WALKERS;
     static constexpr int SZ_STG = align128(NWO * 32 * 20);  // emission staging of the overlapping walkers
     static constexpr int SMEM1 = SZ_P2 + SZ_GP + SZ_BP + SZ_U + SZ_TAB + SZ_STG;
     // Two processed planes (the walkers read the previous tile's while the

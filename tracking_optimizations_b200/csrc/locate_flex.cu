@@ -11,11 +11,10 @@ namespace {
 }  // namespace
 
 // The largest dilation size of radius rc's instance, 0 without one.
-int flex_dilation(int rc, int dtype) {
+int flex_dilation(int rc) {
 #define GT_FLEX_CASE(R, DD) if (rc == R) return DD;
     GT_FLEX_LIST(GT_FLEX_CASE)
 #undef GT_FLEX_CASE
-    (void)dtype;
     return 0;
 }
 
@@ -29,7 +28,7 @@ int flex_rows(int rc, int dtype) {
 
 cudaError_t launch_locate_flex(int kr, int rc, int dtype, dim3 grid, cudaStream_t st, const LocParams& p,
                                const MovieBufs& b, const TileSource& src, int frame0, int* used_tma) {
-    if (kr != rc || p.D < FM || p.D > flex_dilation(rc, dtype)) return cudaErrorInvalidValue;
+    if (kr != rc || p.D < FM || p.D > flex_dilation(rc)) return cudaErrorInvalidValue;
 #define GT_FLEX_CASE(R, DD)                                                                                   \
     if (rc == R)                                                                                              \
         return dtype == 0 ? launch_instance<R, DD, tile_rows<R, DD, R, unsigned short, true>(), R, unsigned short, \
