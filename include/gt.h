@@ -311,8 +311,7 @@ GT_API void gt_table_free(gt_table* table);
  *                       limit and the call returns GT_ERR_DEVICE_TIMEOUT (a
  *                       test of the timeout path; no fault, nothing in flight)
  *   "test_short_memory" 1 = gt_batch_many_device plans as for a batch that does not
- *                       fit beside the caller's data: tighter first capacities,
- *                       rows not repacked
+ *                       fit beside the caller's data: tighter first capacities
  * Returns GT_ERR_ARG for an unknown key or value. */
 GT_API int gt_ctx_set_option(gt_ctx* ctx, const char* key, int value);
 

@@ -1213,7 +1213,6 @@ int batch_many(gt_ctx* ctx, gt_movie* mv, int n, cudaStream_t st) {
                        ctx->batch_cap_div);
         if (rc) { ctx->err = who + msg; return rc; }
         B[i].P.lp.tiles_per_cta = ctx->tiles_per_cta;
-        if (ctx->batch_cap_div != 64) B[i].P.repack = 0;  // memory is short
         char buf[128];
         std::snprintf(buf, sizeof(buf), "%p|%d|%d|%d|%d|%p|%lld|", m.frames, m.dtype, m.T, m.H, m.W, (void*)m.out,
                       (long long)m.out_rows);
