@@ -1502,8 +1502,8 @@ __device__ __forceinline__ void link_fixpoint(const M& movie, int nm, int max_pa
             link_seeds(L, (WarpComp*)buf, 0, id, nthr >> 5);
         }
         grid.sync();
+        deferred(0);
     }
-    deferred(0);
     tick(0);
     int k = 0;
     if (any_mem) {
